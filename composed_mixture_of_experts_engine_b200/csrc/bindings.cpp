@@ -197,6 +197,7 @@ void router_fwd(const Tensor& X, const Tensor& Wg, int64_t K, Tensor& logits, Te
   a.workspace = reinterpret_cast<uint32_t*>(workspace.data_ptr());
   a.status = opt_ptr<int>(status);
   a.timeout_ns = static_cast<unsigned long long>(timeout_ns);
+  a.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   check_cuda(cmoe::launch_router_fwd(a, cur_stream()), "launch_router_fwd");
 }
 
@@ -399,6 +400,7 @@ void combine_bwd_w(const Tensor& rows, const Tensor& slot_row, const Tensor& dy,
 
 void register_attention(pybind11::module_& m);
 void register_ep(pybind11::module_& m);
+void register_router(pybind11::module_& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "sm_100a kernels of the composed MoE engine";
@@ -421,4 +423,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("combine_bwd_w", &combine_bwd_w);
   register_attention(m);
   register_ep(m);
+  register_router(m);
 }

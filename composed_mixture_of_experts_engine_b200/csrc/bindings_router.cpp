@@ -1,0 +1,94 @@
+// Native host path of the router: one call allocates every output of a routing pass and launches the kernel, so that
+// a small routing call costs one binding call instead of eight tensor constructions and three casts in Python.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <map>
+#include <mutex>
+#include <optional>
+#include <tuple>
+#include <utility>
+
+#include "router.cuh"
+
+namespace {
+
+using torch::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// Statistics workspace, zero between launches (the kernel leaves it so).  One per (device, stream): launches on one
+// stream run in order, launches on two streams must not share the accumulators.  At most kMaxWorkspaces are kept
+// (3 KiB each); further streams get a fresh zeroed one per call.
+constexpr size_t kMaxWorkspaces = 256;
+Tensor router_workspace(const c10::Device& dev, cudaStream_t stream) {
+  static std::mutex mu;
+  static std::map<std::pair<int, cudaStream_t>, Tensor> kept;
+  const auto opt = at::TensorOptions().device(dev).dtype(at::kInt);
+  const int64_t words = static_cast<int64_t>(cmoe::router_workspace_words(cmoe::kRouterMaxExperts));
+  const std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(static_cast<int>(dev.index()), stream);
+  auto it = kept.find(key);
+  if (it != kept.end()) return it->second;
+  Tensor t = at::zeros({words}, opt);
+  if (kept.size() < kMaxWorkspaces) kept.emplace(key, t);
+  return t;
+}
+
+// (idx32, w32, idx64, w16, logits, lse, counts, counts64, mean_prob, stats).  `full` false: only the routing decision
+// in its public types (idx64, w16) is produced, for callers that want no gradient and no statistics.
+using RouteResult = std::tuple<OptTensor, OptTensor, Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor,
+                               OptTensor, OptTensor>;
+RouteResult router_route(const Tensor& X, const Tensor& Wg, int64_t K, bool full, const OptTensor& status) {
+  TORCH_CHECK(X.is_cuda() && X.scalar_type() == at::kBFloat16 && X.dim() == 2 && X.stride(1) == 1,
+              "X must be a CUDA bf16 matrix with unit inner stride");
+  TORCH_CHECK(Wg.is_cuda() && Wg.scalar_type() == at::kBFloat16 && Wg.dim() == 2 && Wg.is_contiguous() &&
+                  Wg.size(0) == X.size(1),
+              "Wg must be contiguous bf16 [H, E]");
+  const c10::cuda::CUDAGuard guard(X.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+  const int64_t N = X.size(0), E = Wg.size(1);
+  const auto f32 = X.options().dtype(at::kFloat), i32 = X.options().dtype(at::kInt), i64 = X.options().dtype(at::kLong);
+  cmoe::RouterFwdArgs a;
+  a.X = X.data_ptr();
+  a.n_tokens = N;
+  a.H = static_cast<int>(X.size(1));
+  a.ldx = X.stride(0);
+  a.Wg = Wg.data_ptr();
+  a.E = static_cast<int>(E);
+  a.K = static_cast<int>(K);
+  a.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  Tensor idx64 = at::empty({N, K}, i64), w16 = at::empty({N, K}, X.options());
+  a.topk_idx64 = reinterpret_cast<long long*>(idx64.data_ptr<int64_t>());
+  a.topk_w_bf16 = w16.data_ptr();
+  OptTensor idx32, w32, logits, lse, counts, counts64, mean_prob, stats;
+  Tensor ws;
+  if (full) {
+    idx32 = at::empty({N, K}, i32);
+    w32 = at::empty({N, K}, f32);
+    logits = at::empty({N, E}, f32);
+    lse = at::empty({N}, f32);
+    counts = at::empty({E}, i32);
+    counts64 = at::empty({E}, i64);
+    mean_prob = at::empty({E}, f32);
+    stats = at::empty({4}, f32);
+    ws = router_workspace(X.device(), stream);
+    a.topk_idx = idx32->data_ptr<int>();
+    a.topk_w = w32->data_ptr<float>();
+    a.logits = logits->data_ptr<float>();
+    a.lse = lse->data_ptr<float>();
+    a.counts = counts->data_ptr<int>();
+    a.counts64 = reinterpret_cast<long long*>(counts64->data_ptr<int64_t>());
+    a.mean_prob = mean_prob->data_ptr<float>();
+    a.stats = stats->data_ptr<float>();
+    a.workspace = reinterpret_cast<uint32_t*>(ws.data_ptr());
+  }
+  a.status = status.has_value() ? status->data_ptr<int>() : nullptr;
+  const cudaError_t e = cmoe::launch_router_fwd(a, stream);
+  TORCH_CHECK(e == cudaSuccess, "cmoe: launch_router_fwd failed: ", cudaGetErrorString(e));
+  return {idx32, w32, idx64, w16, logits, lse, counts, counts64, mean_prob, stats};
+}
+
+}  // namespace
+
+void register_router(pybind11::module_& m) { m.def("router_route", &router_route); }

@@ -1,10 +1,21 @@
 // Fused top-k router for sm_100a.
 //
 // Forward, one launch: gate GEMM (tokens [N,H] x gate_w [H,E]) on tcgen05 with the fp32 logits in
-// tensor memory, then per token row (one thread per row, straight out of TMEM): fp32 softmax
-// statistics, top-k with lowest-index tie break, renormalised gate weights, per-expert counts,
-// per-expert probability sums (load-balance loss), z-loss, and a last-CTA finalisation that turns
-// those sums into the loss values.  The tokens are read from HBM exactly once.
+// tensor memory, then per token row out of shared memory: top-k with lowest-index tie break, fp32 softmax
+// statistics, renormalised gate weights, per-expert counts, per-expert probability sums (load-balance loss),
+// z-loss, and a last-CTA finalisation that turns those sums into the loss values.  The tokens are read from HBM
+// exactly once.
+//
+// What bounds it: with many tokens the read of the tokens, with few tokens (or many experts) what one SM can pull
+// in, and in both cases the epilogue that no other work hides.  Hence
+//   * few row tiles are split along H over a cluster of up to 8 CTAs, each with its share of the k-blocks; the partial
+//     logits meet through distributed shared memory in rank order and every CTA finishes its share of the rows
+//     (64 tokens, H 2048, E 64: the k loop 9.6 -> ~2 us);
+//   * the epilogue runs on 16 warps with four lanes per row over logits in shared memory.  A thread per row straight
+//     out of tensor memory took longer than the GEMM: 54 us of 88 at 8190 tokens, E 256, top-8.
+// Launch to end with a cold L2, before (one CTA per tile, a thread per row) and now: 8190 tokens H 4096 E 256 top-8
+// 94 -> 49 us, 64 x 2048 E 64 top-8 33 -> 18, 1000 x 2048 E 64 top-8 35 -> 21, 16384 x 4096 E 64 top-2 51 -> 47
+// (134 MB of tokens: 21 us at the copy rate).
 //
 // Backward: the analytic gradient of the gate weights, load-balance loss and z-loss with respect
 // to the logits (one warp per token); the two contractions with it (grad_tokens, grad_gate_w) run
@@ -15,6 +26,7 @@
 // (pkg/kernels/moe_router.py:102-251, 545-546, 690-734).
 #include "router.cuh"
 
+#include <climits>
 #include <cstdio>
 #include <mutex>
 
@@ -28,8 +40,10 @@ constexpr int RT_BM = 128;
 constexpr int RT_BK = 64;
 constexpr int RT_A_BYTES = RT_BM * RT_BK * 2;  // 16 KiB
 constexpr int RT_CHUNK_BYTES = 64 * RT_BK * 2;  // 8 KiB: 64 experts x 64 k
-constexpr int RT_THREADS = 192;
+constexpr int RT_EPI = 512;                     // epilogue threads (warps 2..17)
+constexpr int RT_THREADS = 64 + RT_EPI;
 constexpr int RT_MAX_STAGES = 8;
+constexpr int RT_MAX_SPLIT = 8;  // portable cluster size
 constexpr int RT_SMEM_BUDGET = 200 * 1024;
 
 struct RouterParams {
@@ -37,35 +51,69 @@ struct RouterParams {
   int H, E, K;
   int n_chunks;  // ceil(E / 64)
   int stages;
+  int split;   // CTAs per row tile (the cluster size): each takes its share of the k-blocks
   int umma_n;  // E rounded up to 16
   int tmem_cols;
   float* logits;
   int* topk_idx;
   float* topk_w;
+  long long* topk_idx64;
+  __nv_bfloat16* topk_w16;
   float* lse;
   int* counts;
+  long long* counts64;
   float* mean_prob;
-  float* stats;
+  float* stats;  // nullptr: no statistics are gathered
   uint32_t* workspace;
   int* status;
   unsigned long long timeout_ns;
 };
 
-// sum v[i] over the 32 lanes of the warp for all 32 i at once (31 shuffles); afterwards lane L
-// holds the total of column L in v[0]
-__device__ __forceinline__ void warp_transpose_reduce(float (&v)[32], int lane) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < off; ++i) {
-      const float send = upper ? v[i] : v[i + off];
-      const float keep = upper ? v[i + off] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-}
+// row stride (floats) of the logits tile in shared memory: 4 more than a multiple of 32 banks, so that both the
+// 16-byte stores of 32 neighbouring rows and the reads of 8 rows x 4 lanes touch every bank once
+__host__ __device__ constexpr int rt_row_stride(int E) { return (E + 31) / 32 * 32 + 4; }
+// per-CTA tables behind the pipeline stages (bytes); the barriers come first
+constexpr int RT_TABLES = 512 /* barriers, slots */ + RT_BM * 4 /* 1/sum */ + RT_BM * 4 /* lse^2 */ + RT_EPI * 4 /* column partials */ +
+                          kRouterMaxExperts * 4 /* counts */ + 2 * kRouterMaxTopK * RT_BM * 4 /* picks */;
 
+// order-preserving map of a logit to an integer: +0 and -0 agree, NaN takes a place at the end of the order (so every
+// pick is a valid expert whatever the input), and nothing maps to INT_MIN, which stands for "taken"
+__device__ __forceinline__ int logit_key(float v) {
+  const int b = __float_as_int(v + 0.f);
+  return max(b ^ ((b >> 31) & 0x7fffffff), INT_MIN + 1);
+}
+__device__ __forceinline__ float key_logit(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t rt_cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void rt_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void rt_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t smem_addr, uint32_t rank) {
+  float4 v;
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+
+// NG: groups of eight experts per lane (a row's four lanes take the experts 4 j + lane): E <= 32 NG
+template <int NG>
 __global__ void __launch_bounds__(RT_THREADS, 1)
 router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                   const RouterParams p) {
@@ -73,25 +121,30 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int b_bytes = p.n_chunks * RT_CHUNK_BYTES;
   const int stage_bytes = RT_A_BYTES + b_bytes;
-  uint8_t* tail = smem + p.stages * stage_bytes;
+  const int SE = rt_row_stride(p.E);
+  const int front = max(p.stages * stage_bytes, RT_BM * SE * 4);
+  float* s_logit = reinterpret_cast<float*>(smem);  // [128][SE], over the drained pipeline stages
+  uint8_t* tail = smem + front;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(tail);   // [RT_MAX_STAGES]
   uint64_t* empty_bar = full_bar + RT_MAX_STAGES;           // [RT_MAX_STAGES]
   uint64_t* tfull_bar = empty_bar + RT_MAX_STAGES;          // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* s_last = const_cast<int*>(abort_flag) + 1;
-  // per-tile sums as 64-bit fixed point (integer adds commute: the result does not depend on the order of the warps)
-  unsigned long long* s_prob = reinterpret_cast<unsigned long long*>(
-      (reinterpret_cast<uintptr_t>(s_last + 1) + 7) & ~uintptr_t(7));  // [256]
-  unsigned long long* s_z = s_prob + kRouterMaxExperts;
-  int* s_cnt = reinterpret_cast<int*>(s_z + 1);  // [256]
-  int* s_topi = s_cnt + kRouterMaxExperts;                      // [kRouterMaxTopK][128] chosen experts, one column per row
-  float* s_topp = reinterpret_cast<float*>(s_topi + kRouterMaxTopK * 128);  // [kRouterMaxTopK][128] their probabilities
+  float* s_inv = reinterpret_cast<float*>(tail + 512);  // [128] 1 / sum of exponentials (0: no such token)
+  float* s_z = s_inv + RT_BM;                           // [128] lse^2
+  float* s_part = s_z + RT_BM;                          // [512] column sums of row ranges
+  int* s_cnt = reinterpret_cast<int*>(s_part + RT_EPI);        // [256]
+  int* s_topi = s_cnt + kRouterMaxExperts;                     // [kRouterMaxTopK][128] chosen experts
+  float* s_topv = reinterpret_cast<float*>(s_topi + kRouterMaxTopK * RT_BM);  // ... their logits, then gate weights
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const long long row0 = static_cast<long long>(blockIdx.x) * RT_BM;
-  const int k_blocks = (p.H + RT_BK - 1) / RT_BK;
+  const int split = p.split;
+  const int rank = split > 1 ? static_cast<int>(rt_cluster_rank()) : 0;
+  const long long row0 = static_cast<long long>(blockIdx.x / split) * RT_BM;
+  const int all_blocks = (p.H + RT_BK - 1) / RT_BK;
+  const int kb0 = all_blocks * rank / split, kb1 = all_blocks * (rank + 1) / split;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -119,11 +172,13 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   wc.status = p.status;
   wc.timeout_ns = p.timeout_ns;
 
+  const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread
+  const int E = p.E;
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
         mbar_arrive_expect_tx(&full_bar[stage], stage_bytes);
         uint8_t* a_dst = smem + stage * stage_bytes;
@@ -137,12 +192,13 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = make_idesc_bf16(RT_BM, p.umma_n, 0, 1);
       int stage = 0;
       uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&full_bar[stage], phase, wc, ST_TIMEOUT_SMEM_FULL)) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
@@ -151,7 +207,7 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         for (int k = 0; k < RT_BK / 16; ++k) {
           const uint64_t ad = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
           const uint64_t bd = make_smem_desc_sw128(b_addr + k * 2048, RT_CHUNK_BYTES, 1024);
-          umma_bf16_ss(tmem_base, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_bf16_ss(tmem_base, ad, bd, idesc, kb != kb0 || k != 0 ? 1u : 0u);
         }
         umma_commit(&empty_bar[stage]);
         if (++stage == p.stages) {
@@ -161,167 +217,248 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       }
       umma_commit(tfull_bar);
     }
+    __syncwarp();
   } else {
-    // ---------------------------------------------------------------- epilogue: one thread per token row
-    const int et = threadIdx.x - 64;  // 0..127
-    const int quad = warp & 3;
-    const long long row = row0 + quad * 32 + lane;
-    const bool row_ok = row < p.n_tokens;
-    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    const int E = p.E;
-    const int nch = (E + 31) / 32;
-    for (int e = et; e < kRouterMaxExperts; e += 128) {
-      s_prob[e] = 0ull;
-      s_cnt[e] = 0;
-    }
-    if (et == 0) *s_z = 0ull;
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-
+    for (int e = et; e < kRouterMaxExperts; e += RT_EPI) s_cnt[e] = 0;
     const bool ok = mbar_wait(tfull_bar, 0, wc, ST_TIMEOUT_TMEM_FULL);
     tc_fence_after();
     if (ok) {
-      // pass 1: row maximum, and the logits go out to global memory
-      float mx = -INFINITY;
+      // logits: tensor memory -> shared memory, every warp its own quadrant of lanes and every fourth 16 columns
+      const int quad = warp & 3;
+      float* dst = s_logit + (quad * 32 + lane) * SE;
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < nch; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
+      for (int c = (et >> 7) * 16; c < E; c += 64) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(t_row + c, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c * 32 + j < E) mx = fmaxf(mx, __uint_as_float(r[j]));
-        if (row_ok) {
-          float* dst = p.logits + row * E + c * 32;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            if (c * 32 + j < E)
-              *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+        for (int j = 0; j < 16; j += 4)  // the row stride has room for all 16 columns
+          *reinterpret_cast<float4*>(dst + c + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
                                                                 __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+      }
+    }
+    __syncwarp();
+  }
+  if (split > 1) {  // every CTA's partial logits are in its shared memory
+    rt_cluster_arrive();
+    rt_cluster_wait();
+  }
+  if (warp >= 2) {
+    const int R = RT_BM / split;  // this CTA finishes the rows [r_lo, r_lo + R) of the tile
+    const int r_lo = rank * R;
+    if (split == 1) epi_sync();
+    // add the partial logits of the cluster in rank order; the logits go out to global memory
+    if (split > 1 || p.logits != nullptr) {
+      const int e4 = E / 4;
+      for (int i = et; i < R * e4; i += RT_EPI) {
+        const int r = i / e4, c = (i - r * e4) * 4;
+        float* cell = s_logit + (r_lo + r) * SE + c;
+        float4 v;
+        if (split > 1) {
+          v = make_float4(0.f, 0.f, 0.f, 0.f);
+          const uint32_t a = smem_u32(cell);
+          for (int q = 0; q < split; ++q) {
+            const float4 o = ld_cluster_f4(a, q);
+            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+          }
+          *reinterpret_cast<float4*>(cell) = v;  // no other CTA reads these rows of this CTA
+        } else {
+          v = *reinterpret_cast<const float4*>(cell);
         }
+        const long long row = row0 + r_lo + r;
+        if (p.logits != nullptr && row < p.n_tokens) *reinterpret_cast<float4*>(p.logits + row * E + c) = v;
       }
-      // pass 2: log-sum-exp
-      float se = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < nch; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
-        tmem_ld_wait();
+      if (split > 1) epi_sync();
+    }
+  }
+  if (split > 1) rt_cluster_arrive();  // done with the other CTAs' shared memory; waited for before the exit
+  if (warp >= 2) {
+    const int R = RT_BM / split;
+    const int r_lo = rank * R;
+    const int t = et >> 2, l = et & 3;  // row of this CTA's share, lane of the row
+    const int n = E / 4;                // experts per lane (E is a multiple of 8)
+    const long long row = row0 + r_lo + t;
+    const bool row_ok = row < p.n_tokens;
+    if (t < R) {  // whole warps: R is a multiple of 16
+      float* mine = s_logit + (r_lo + t) * SE + l;
+      // best of every group of eight of this lane's experts
+      int gk[NG], gj[NG];
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c * 32 + j < E) se += expf(__uint_as_float(r[j]) - mx);
-      }
-      const float lse = mx + logf(se);
-      if (row_ok) p.lse[row] = lse;
-      // pass 3: per-expert probability sums over the 128 rows of this tile
-#pragma unroll 1
-      for (int c = 0; c < nch; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        float pv[32];
+      for (int g = 0; g < NG; ++g) {
+        gk[g] = INT_MIN;
+        gj[g] = g * 8;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          pv[j] = (row_ok && (c * 32 + j < E)) ? expf(__uint_as_float(r[j]) - lse) : 0.f;
-        warp_transpose_reduce(pv, lane);
-        if (c * 32 + lane < E) atomicAdd(&s_prob[c * 32 + lane], __float2ull_rn(pv[0] * kRouterProbScale));
-      }
-      // pass 4: top-k by repeated arg-max over TMEM (already chosen experts are masked by bit sets).  The loops
-      // over k and over the 32-expert chunks stay rolled: this code runs once per CTA, so every instruction is a
-      // cold fetch, and eight unrolled copies of the compare block cost more in instruction fetches than they
-      // save in loop overhead.  The K results wait in shared memory (one column per thread) for the renormalisation.
-      uint32_t sel[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) sel[c] = 0u;
-      float psum = 0.f;
-#pragma unroll 1
-      for (int kk = 0; kk < p.K; ++kk) {
-        float best = -INFINITY;
-        int bi = -1;
-#pragma unroll 1
-        for (int c = 0; c < nch; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_row + c * 32, r);
-          tmem_ld_wait();
-          uint32_t m = 0u;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) m = (q == c) ? sel[q] : m;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = __uint_as_float(r[j]);
-            const bool cand = (c * 32 + j < E) && (((m >> j) & 1u) == 0u);
-            if (cand && (bi < 0 || v > best)) {
-              best = v;
-              bi = c * 32 + j;
+        for (int q = 0; q < 8; ++q) {
+          const int j = g * 8 + q;
+          if (j < n) {
+            const int k = logit_key(mine[4 * j]);
+            if (k > gk[g]) {
+              gk[g] = k;
+              gj[g] = j;
             }
           }
         }
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c == (bi >> 5)) sel[c] |= 1u << (bi & 31);
-        const float pk = expf(best - lse);
-        psum += pk;
-        s_topi[kk * 128 + et] = bi;
-        s_topp[kk * 128 + et] = pk;
       }
-      if (row_ok) {
-        const float inv = 1.f / psum;
+      // top-k: best group, best of the four lanes, then the winning lane looks through its one group again.  The loop
+      // over k stays rolled: this code runs once per CTA, so every instruction is a cold fetch.
+      unsigned long long taken = 0ull;
+      float mx = 0.f, psum = 0.f;
 #pragma unroll 1
-        for (int kk = 0; kk < p.K; ++kk) {
-          const int e = s_topi[kk * 128 + et];
-          p.topk_idx[row * p.K + kk] = e;
-          p.topk_w[row * p.K + kk] = s_topp[kk * 128 + et] * inv;
-          atomicAdd(&s_cnt[e], 1);
+      for (int kk = 0; kk < p.K; ++kk) {
+        int bk = gk[0], bj = gj[0];
+#pragma unroll
+        for (int g = 1; g < NG; ++g)
+          if (gk[g] > bk) {
+            bk = gk[g];
+            bj = gj[g];
+          }
+        int e = 4 * bj + l;
+#pragma unroll
+        for (int off = 1; off <= 2; off <<= 1) {
+          const int ok = __shfl_xor_sync(0xffffffffu, bk, off), oe = __shfl_xor_sync(0xffffffffu, e, off);
+          if (ok > bk || (ok == bk && oe < e)) {
+            bk = ok;
+            e = oe;
+          }
+        }
+        const float v = key_logit(bk);
+        if (kk == 0) mx = v;
+        psum += expf(v - mx);
+        if (l == 0) {
+          s_topi[kk * RT_BM + t] = e;
+          s_topv[kk * RT_BM + t] = v;
+          if (row_ok) atomicAdd(&s_cnt[e], 1);
+        }
+        if (l == (e & 3)) {
+          const int wj = e >> 2, wg = wj >> 3;
+          taken |= 1ull << wj;
+          const uint32_t tk = static_cast<uint32_t>(taken >> (wg * 8)) & 0xffu;
+          int nk = INT_MIN, nj = wg * 8;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int j = wg * 8 + q;
+            if (j < n && ((tk >> q) & 1u) == 0u) {
+              const int k = logit_key(mine[4 * j]);
+              if (k > nk) {
+                nk = k;
+                nj = j;
+              }
+            }
+          }
+#pragma unroll
+          for (int g = 0; g < NG; ++g)
+            if (g == wg) {
+              gk[g] = nk;
+              gj[g] = nj;
+            }
+        }
+        __syncwarp();
+      }
+      const float inv_psum = 1.f / psum;
+      for (int kk = l; kk < p.K; kk += 4) s_topv[kk * RT_BM + t] = expf(s_topv[kk * RT_BM + t] - mx) * inv_psum;
+      // softmax statistics (the first pick is the row maximum); the exponentials replace the logits
+      if (p.stats != nullptr || p.lse != nullptr) {
+        float se = 0.f;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) {
+          const float ex = expf(mine[4 * j] - mx);
+          mine[4 * j] = ex;
+          se += ex;
+        }
+        se += __shfl_xor_sync(0xffffffffu, se, 1);
+        se += __shfl_xor_sync(0xffffffffu, se, 2);
+        if (l == 0) {
+          const float lse = mx + logf(se);
+          if (row_ok && p.lse != nullptr) p.lse[row] = lse;
+          s_inv[t] = row_ok ? 1.f / se : 0.f;
+          s_z[t] = row_ok ? lse * lse : 0.f;
         }
       }
-      const float z = warp_sum(row_ok ? lse * lse : 0.f);
-      if (lane == 0) atomicAdd(s_z, __float2ull_rn(z * kRouterZScale));
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    // flush this tile's sums; the last CTA to finish turns them into the loss values
-    unsigned long long* ws_prob = reinterpret_cast<unsigned long long*>(p.workspace);
-    unsigned long long* ws_z = ws_prob + E;
-    int* ws_cnt = reinterpret_cast<int*>(ws_z + 1);
-    unsigned int* ws_done = reinterpret_cast<unsigned int*>(ws_cnt + E);
-    for (int e = et; e < E; e += 128) {
-      if (s_prob[e] != 0ull) atomicAdd(&ws_prob[e], s_prob[e]);
-      if (s_cnt[e] != 0) atomicAdd(&ws_cnt[e], s_cnt[e]);
+    epi_sync();
+    // the picks, whole rows of K at a time
+    const int live = static_cast<int>(min(static_cast<long long>(R), p.n_tokens - (row0 + r_lo)));
+    for (int i = et; i < live * p.K; i += RT_EPI) {
+      const int r = i / p.K, kk = i - r * p.K;
+      const long long o = (row0 + r_lo) * p.K + i;
+      const int e = s_topi[kk * RT_BM + r];
+      const float w = s_topv[kk * RT_BM + r];
+      if (p.topk_idx != nullptr) p.topk_idx[o] = e;
+      if (p.topk_idx64 != nullptr) p.topk_idx64[o] = e;
+      if (p.topk_w != nullptr) p.topk_w[o] = w;
+      if (p.topk_w16 != nullptr) p.topk_w16[o] = __float2bfloat16(w);
     }
-    if (et == 0) atomicAdd(ws_z, *s_z);
-    __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (et == 0) {
-      const unsigned int ticket = atomicAdd(ws_done, 1u);
-      *s_last = (ticket == gridDim.x - 1) ? 1 : 0;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (*s_last && et < 32) {
+    if (p.stats != nullptr) {
+      // probability sums: thread = (expert, range of rows), then the ranges of an expert in order
+      const int cols = NG == 1 ? 32 : (NG == 2 ? 64 : (NG == 4 ? 128 : 256));
+      const int parts = RT_EPI / cols, per = (R + parts - 1) / parts;
+      const int e = et & (cols - 1), part = et / cols;
+      float sum = 0.f;
+      if (e < E) {
+        const int r1 = min(R, (part + 1) * per);
+#pragma unroll 8
+        for (int r = part * per; r < r1; ++r) sum += s_logit[(r_lo + r) * SE + e] * s_inv[r];
+      }
+      s_part[part * cols + e] = sum;
+      epi_sync();
+      // flush this share's sums as 64-bit fixed point (integer adds commute: the result does not depend on the order
+      // of the CTAs); the last CTA to finish turns them into the loss values
+      unsigned long long* ws_prob = reinterpret_cast<unsigned long long*>(p.workspace);
+      unsigned long long* ws_z = ws_prob + E;
+      int* ws_cnt = reinterpret_cast<int*>(ws_z + 1);
+      unsigned int* ws_done = reinterpret_cast<unsigned int*>(ws_cnt + E);
+      if (et < E) {
+        float pr = 0.f;
+        for (int q = 0; q < parts; ++q) pr += s_part[q * cols + et];
+        const unsigned long long fx = __float2ull_rn(pr * kRouterProbScale);
+        if (fx != 0ull) atomicAdd(&ws_prob[et], fx);
+        if (s_cnt[et] != 0) atomicAdd(&ws_cnt[et], s_cnt[et]);
+      } else if (et >= RT_EPI - 32) {  // E <= 256: this warp has no expert
+        float z = 0.f;
+        for (int r = lane; r < R; r += 32) z += s_z[r];
+        z = warp_sum(z);
+        if (lane == 0) atomicAdd(ws_z, __float2ull_rn(z * kRouterZScale));
+      }
       __threadfence();
-      const float n_tok = static_cast<float>(p.n_tokens);
-      float aux = 0.f, mxc = 0.f, sumc = 0.f;
-      for (int e = lane; e < E; e += 32) {
-        const float pr = static_cast<float>(static_cast<double>(__ldcg(&ws_prob[e])) / kRouterProbScale);
-        const int cn = __ldcg(&ws_cnt[e]);
-        p.counts[e] = cn;
-        p.mean_prob[e] = pr / n_tok;
-        aux += (static_cast<float>(cn) / (n_tok * p.K)) * (pr / n_tok);
-        mxc = fmaxf(mxc, static_cast<float>(cn));
-        sumc += static_cast<float>(cn);
-        ws_prob[e] = 0ull;
-        ws_cnt[e] = 0;
+      epi_sync();
+      if (et == 0) {
+        const unsigned int ticket = atomicAdd(ws_done, 1u);
+        *s_last = (ticket == gridDim.x - 1) ? 1 : 0;
       }
-      aux = warp_sum(aux);
-      mxc = warp_max(mxc);
-      sumc = warp_sum(sumc);
-      if (lane == 0) {
-        p.stats[0] = aux * E;
-        p.stats[1] = static_cast<float>(static_cast<double>(__ldcg(ws_z)) / kRouterZScale) / n_tok;
-        p.stats[2] = sumc > 0.f ? mxc / (sumc / E) : 1.f;
-        p.stats[3] = sumc;
-        *ws_z = 0ull;
-        *ws_done = 0u;
+      epi_sync();
+      if (*s_last && et < 32) {
+        __threadfence();
+        const float n_tok = static_cast<float>(p.n_tokens);
+        float aux = 0.f, mxc = 0.f, sumc = 0.f;
+        for (int x = lane; x < E; x += 32) {
+          const float pr = static_cast<float>(static_cast<double>(__ldcg(&ws_prob[x])) / kRouterProbScale);
+          const int cn = __ldcg(&ws_cnt[x]);
+          if (p.counts != nullptr) p.counts[x] = cn;
+          if (p.counts64 != nullptr) p.counts64[x] = cn;
+          if (p.mean_prob != nullptr) p.mean_prob[x] = pr / n_tok;
+          aux += (static_cast<float>(cn) / (n_tok * p.K)) * (pr / n_tok);
+          mxc = fmaxf(mxc, static_cast<float>(cn));
+          sumc += static_cast<float>(cn);
+          ws_prob[x] = 0ull;
+          ws_cnt[x] = 0;
+        }
+        aux = warp_sum(aux);
+        mxc = warp_max(mxc);
+        sumc = warp_sum(sumc);
+        if (lane == 0) {
+          p.stats[0] = aux * E;
+          p.stats[1] = static_cast<float>(static_cast<double>(__ldcg(ws_z)) / kRouterZScale) / n_tok;
+          p.stats[2] = sumc > 0.f ? mxc / (sumc / E) : 1.f;
+          p.stats[3] = sumc;
+          *ws_z = 0ull;
+          *ws_done = 0u;
+        }
       }
+      __syncwarp();
     }
   }
+  if (split > 1) rt_cluster_wait();  // nobody still reads this CTA's shared memory
 
   tc_fence_before();
   __syncthreads();
@@ -429,9 +566,29 @@ cudaError_t encode_bf16_2d(CUtensorMap* out, const void* ptr, long long rows, lo
 
 }  // namespace
 
+template <int NG>
+static cudaError_t launch_router_variant(const CUtensorMap& tmX, const CUtensorMap& tmW, const RouterParams& p,
+                                         unsigned tiles, int smem, cudaStream_t stream) {
+  static const cudaError_t configured = cudaFuncSetAttribute(
+      router_fwd_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM_BUDGET + 1024 + RT_TABLES);
+  if (configured != cudaSuccess) return configured;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.split);
+  cfg.blockDim = dim3(RT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, router_fwd_kernel<NG>, tmX, tmW, p);
+}
+
 cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   if (a.E <= 0 || a.E > kRouterMaxExperts || a.E % 8 != 0 || a.K <= 0 || a.K > kRouterMaxTopK || a.K > a.E ||
-      a.H % 8 != 0 || a.n_tokens <= 0)
+      a.H % 8 != 0 || a.n_tokens <= 0 || (a.stats != nullptr && a.workspace == nullptr))
     return cudaErrorInvalidValue;
   CUtensorMap tmX, tmW;
   cudaError_t e = encode_bf16_2d(&tmX, a.X, a.n_tokens, a.H, a.ldx, 128);
@@ -446,9 +603,18 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   p.K = a.K;
   p.n_chunks = (a.E + 63) / 64;
   const int stage_bytes = RT_A_BYTES + p.n_chunks * RT_CHUNK_BYTES;
+  // Split along H while the clusters still fit one wave of SMs and every CTA keeps at least four k-blocks: below
+  // that the exchange of the partial logits (about 1 us) costs what the shorter k loop saves.
+  const unsigned tiles = static_cast<unsigned>((a.n_tokens + RT_BM - 1) / RT_BM);
+  const int k_blocks = (a.H + RT_BK - 1) / RT_BK;
+  const int sms = a.num_sms > 0 ? a.num_sms : 148;
+  p.split = 1;
+  while (p.split < RT_MAX_SPLIT && tiles * p.split * 2 <= static_cast<unsigned>(sms) && k_blocks >= 8 * p.split)
+    p.split *= 2;
   int stages = RT_SMEM_BUDGET / stage_bytes;
   if (stages > RT_MAX_STAGES) stages = RT_MAX_STAGES;
-  p.stages = stages;
+  const int per_cta = (k_blocks + p.split - 1) / p.split;
+  p.stages = stages < per_cta ? stages : per_cta;
   p.umma_n = ((a.E + 15) / 16) * 16;
   int cols = 32;
   while (cols < p.umma_n) cols <<= 1;
@@ -456,24 +622,24 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   p.logits = a.logits;
   p.topk_idx = a.topk_idx;
   p.topk_w = a.topk_w;
+  p.topk_idx64 = a.topk_idx64;
+  p.topk_w16 = reinterpret_cast<__nv_bfloat16*>(a.topk_w_bf16);
   p.lse = a.lse;
   p.counts = a.counts;
+  p.counts64 = a.counts64;
   p.mean_prob = a.mean_prob;
   p.stats = a.stats;
   p.workspace = a.workspace;
   p.status = a.status;
   p.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
 
-  const int smem = stages * stage_bytes + 1024 + 512 + kRouterMaxExperts * (8 + 4) + kRouterMaxTopK * 128 * 8 + 64;
-  static int configured_smem = 0;
-  if (smem > configured_smem) {
-    e = cudaFuncSetAttribute(router_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured_smem = smem;
-  }
-  const unsigned grid = static_cast<unsigned>((a.n_tokens + RT_BM - 1) / RT_BM);
-  router_fwd_kernel<<<grid, RT_THREADS, smem, stream>>>(tmX, tmW, p);
-  return cudaGetLastError();
+  const int tile_bytes = RT_BM * rt_row_stride(a.E) * 4;
+  const int ring = p.stages * stage_bytes;
+  const int smem = (ring > tile_bytes ? ring : tile_bytes) + 1024 + RT_TABLES;
+  if (a.E <= 32) return launch_router_variant<1>(tmX, tmW, p, tiles, smem, stream);
+  if (a.E <= 64) return launch_router_variant<2>(tmX, tmW, p, tiles, smem, stream);
+  if (a.E <= 128) return launch_router_variant<4>(tmX, tmW, p, tiles, smem, stream);
+  return launch_router_variant<8>(tmX, tmW, p, tiles, smem, stream);
 }
 
 cudaError_t launch_router_bwd(const RouterBwdArgs& a, cudaStream_t stream) {

@@ -24,16 +24,21 @@ struct RouterFwdArgs {
   const void* Wg = nullptr;  // [H, E] bf16 row-major (E contiguous)
   int E = 0;
   int K = 0;
+  // every output may be nullptr; counts, mean_prob and stats are produced together, where stats is set
   float* logits = nullptr;   // [n_tokens, E] fp32
   int* topk_idx = nullptr;   // [n_tokens, K] int32, descending probability, ties -> lowest index
   float* topk_w = nullptr;   // [n_tokens, K] fp32, renormalised over the K picks
+  long long* topk_idx64 = nullptr;  // the same two as int64 and bf16 (what the public entry points return)
+  void* topk_w_bf16 = nullptr;
   float* lse = nullptr;      // [n_tokens] fp32 log-sum-exp of the logits (saved for the backward)
   int* counts = nullptr;     // [E] int32 number of (token, slot) pairs routed to each expert
+  long long* counts64 = nullptr;  // ... as int64
   float* mean_prob = nullptr;  // [E] fp32 mean softmax probability of each expert (P_i)
   float* stats = nullptr;    // [4]: E*sum_i f_i*P_i (aux loss), mean lse^2 (z loss), max/mean load, sum(counts)
   uint32_t* workspace = nullptr;  // router_workspace_words(E) zeroed words
   int* status = nullptr;
   unsigned long long timeout_ns = 0;
+  int num_sms = 0;  // 0: those of a B200
 };
 
 cudaError_t launch_router_fwd(const RouterFwdArgs& args, cudaStream_t stream);

@@ -29,6 +29,7 @@ _SOURCES = [
     "bindings.cpp",
     "bindings_attention.cpp",
     "bindings_ep.cpp",
+    "bindings_router.cpp",
     "gemm.cu",
     "gemm2.cu",
     "router.cu",

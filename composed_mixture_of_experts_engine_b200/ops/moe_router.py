@@ -109,82 +109,78 @@ def _should_use_triton(tokens: torch.Tensor, gate_w: torch.Tensor, force_referen
 # --------------------------------------------------------------------------------------------------
 # fused device path
 # --------------------------------------------------------------------------------------------------
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
-
-
-def _router_workspace(device: torch.device, E: int) -> torch.Tensor:
-    key = (device.index or 0, E)
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = torch.zeros(3 * E + 4, dtype=torch.int32, device=device)  # csrc/router.cuh: router_workspace_words
-        _workspaces[key] = ws
-    return ws
-
-
 class RouterOutput:
-    """Everything the fused forward produced, all on the device."""
+    """Everything the fused forward produced, all on the device.  ``idx32`` / ``w32`` are what the kernels downstream
+    read, ``idx64`` / ``w16`` / ``counts64`` the same values in the types that the public entry points return."""
 
-    __slots__ = ("idx32", "w32", "logits", "lse", "counts", "mean_prob", "stats", "events")
+    __slots__ = ("idx32", "w32", "idx64", "w16", "logits", "lse", "counts", "counts64", "mean_prob", "stats", "events")
 
-    def __init__(self, idx32, w32, logits, lse, counts, mean_prob, stats, events=None):
-        self.idx32, self.w32, self.logits, self.lse = idx32, w32, logits, lse
-        self.counts, self.mean_prob, self.stats, self.events = counts, mean_prob, stats, events
+    def __init__(self, idx32, w32, idx64, w16, logits, lse, counts, counts64, mean_prob, stats, events=None):
+        self.idx32, self.w32, self.idx64, self.w16 = idx32, w32, idx64, w16
+        self.logits, self.lse, self.counts, self.counts64 = logits, lse, counts, counts64
+        self.mean_prob, self.stats, self.events = mean_prob, stats, events
 
 
 def fused_router_forward(tokens: torch.Tensor, gate_w_bf16: torch.Tensor, k: int, timed: bool = False) -> RouterOutput:
     from .kernels import status_word
 
-    N, _ = tokens.shape
-    E = gate_w_bf16.shape[1]
-    dev = tokens.device
-    f32 = dict(device=dev, dtype=torch.float32)
-    out = RouterOutput(
-        torch.empty(N, k, device=dev, dtype=torch.int32), torch.empty(N, k, **f32), torch.empty(N, E, **f32),
-        torch.empty(N, **f32), torch.empty(E, device=dev, dtype=torch.int32), torch.empty(E, **f32),
-        torch.empty(4, **f32),
-    )
-    if timed:
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-    _ext.ext().router_fwd(tokens, gate_w_bf16, k, out.logits, out.idx32, out.w32, out.lse, out.counts, out.mean_prob,
-                          out.stats, _router_workspace(dev, E), status_word(dev), 0)
-    if timed:
-        e1.record()
-        out.events = (e0, e1)
+    ext, status = _ext.ext(), status_word(tokens.device)
+    if not timed:
+        return RouterOutput(*ext.router_route(tokens, gate_w_bf16, k, True, status))
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    out = RouterOutput(*ext.router_route(tokens, gate_w_bf16, k, True, status), events=(e0, e1))
+    e1.record()
     return out
 
 
+def _bf16_gate(gate_w: torch.Tensor) -> torch.Tensor:
+    return (gate_w if gate_w.dtype == torch.bfloat16 else gate_w.to(torch.bfloat16)).contiguous()
+
+
+def _needs_grad(*tensors: torch.Tensor) -> bool:
+    return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
+
+
+def _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w, grad_aux, grad_z, gate_dtype):
+    """(grad_tokens, grad_gate): the analytic d(logits) kernel and the two contractions with it."""
+    from .kernels import linear_nt, linear_tn
+
+    gl16 = torch.empty(logits.shape, device=logits.device, dtype=torch.bfloat16)
+    _ext.ext().router_bwd(logits, lse, idx32, grad_w, counts, grad_aux, grad_z, gl16, None)
+    grad_tokens = grad_gate = None
+    if ctx.needs_input_grad[0]:
+        grad_tokens = linear_nt(gl16, gw16)  # [N, E] x [H, E]^T
+    if ctx.needs_input_grad[1]:
+        grad_gate = linear_tn(tokens, gl16).to(gate_dtype)  # tokens^T [H, N] x gl [N, E]
+    return grad_tokens, grad_gate
+
+
 class FusedRouterFunction(torch.autograd.Function):
-    """(tokens, gate_w) -> (gate weights fp32 [N,K], aux loss, z loss); indices and statistics ride on ``holder``."""
+    """(tokens, gate_w) -> (gate weights fp32, gate weights in bf16 [N,K], aux loss, z loss, idx32, idx64); the two
+    weight tensors hold the same values and take gradients each.  Everything else rides on ``holder``."""
 
     @staticmethod
     def forward(ctx, tokens, gate_w, k: int, holder: Dict[str, Any], timed: bool):
-        gw16 = gate_w if gate_w.dtype == torch.bfloat16 else gate_w.to(torch.bfloat16)
-        gw16 = gw16.contiguous()
+        gw16 = _bf16_gate(gate_w)
         out = fused_router_forward(tokens, gw16, k, timed)
         holder["out"] = out
+        ctx.set_materialize_grads(False)
         ctx.save_for_backward(tokens, gw16, out.logits, out.lse, out.idx32, out.counts)
         ctx.gate_dtype = gate_w.dtype
-        ctx.mark_non_differentiable(out.idx32)
-        return out.w32, out.stats[0], out.stats[1], out.idx32
+        ctx.mark_non_differentiable(out.idx32, out.idx64)
+        return out.w32, out.w16, out.stats[0], out.stats[1], out.idx32, out.idx64
 
     @staticmethod
-    def backward(ctx, grad_w, grad_aux, grad_z, _grad_idx):
-        from .kernels import linear_nt, linear_tn
-
-        tokens, gw16, logits, lse, idx32, counts = ctx.saved_tensors
-        N, E = logits.shape
-        gl16 = torch.empty(N, E, device=logits.device, dtype=torch.bfloat16)
-        gw = None if grad_w is None else grad_w.float().contiguous()
+    def backward(ctx, grad_w32, grad_w16, grad_aux, grad_z, _grad_idx32, _grad_idx64):
+        gw = grad_w32
+        if grad_w16 is not None:
+            gw = grad_w16.float() if gw is None else gw + grad_w16
+        gw = None if gw is None else gw.float().contiguous()
         ga = None if grad_aux is None else grad_aux.float().reshape(1).contiguous()
         gz = None if grad_z is None else grad_z.float().reshape(1).contiguous()
-        _ext.ext().router_bwd(logits, lse, idx32, gw, counts, ga, gz, gl16, None)
-        grad_tokens = grad_gate = None
-        if ctx.needs_input_grad[0]:
-            grad_tokens = linear_nt(gl16, gw16)  # [N, E] x [H, E]^T
-        if ctx.needs_input_grad[1]:
-            grad_gate = linear_tn(tokens, gl16).to(ctx.gate_dtype)  # tokens^T [H, N] x gl [N, E]
-        return grad_tokens, grad_gate, None, None, None
+        gt, gg = _fused_router_backward(ctx, *ctx.saved_tensors, gw, ga, gz, ctx.gate_dtype)
+        return gt, gg, None, None, None
 
 
 # --------------------------------------------------------------------------------------------------
@@ -199,9 +195,9 @@ class MoERouterFunction(torch.autograd.Function):
         E = gate_w.shape[1]
         fused = _should_use_fused(tokens, gate_w, force_reference, k)
         if fused:
-            gw16 = gate_w.to(torch.bfloat16).contiguous()
+            gw16 = _bf16_gate(gate_w)
             out = fused_router_forward(tokens, gw16, k, timed=report is not None)
-            idx, w, logits = out.idx32.long(), out.w32.to(tokens.dtype), out.logits
+            idx, w, logits = out.idx64, out.w16, out.logits
             ctx.fused_saved = (gw16, out.lse, out.idx32, out.counts)
             if report is not None:
                 report["output"] = out
@@ -221,14 +217,10 @@ class MoERouterFunction(torch.autograd.Function):
     def backward(ctx, _grad_idx, grad_w):
         tokens, gate_w, logits, idx = ctx.saved_tensors
         if ctx.fused:
-            from .kernels import linear_nt, linear_tn
-
             gw16, lse, idx32, counts = ctx.fused_saved
-            gl16 = torch.empty(logits.shape, device=logits.device, dtype=torch.bfloat16)
-            _ext.ext().router_bwd(logits, lse, idx32, grad_w.float().contiguous(), counts, None, None, gl16, None)
-            grad_tokens = linear_nt(gl16, gw16).to(tokens.dtype) if ctx.needs_input_grad[0] else None
-            grad_gate = linear_tn(tokens, gl16).to(gate_w.dtype) if ctx.needs_input_grad[1] else None
-            return grad_tokens, grad_gate, None, None, None
+            gt, gg = _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w.float().contiguous(),
+                                            None, None, gate_w.dtype)
+            return gt, gg, None, None, None
         gl = _reference_backward_fp64(logits, idx, grad_w, ctx.k, ctx.E)
         grad_tokens = (gl @ gate_w.to(torch.float64).t()).to(tokens.dtype) if ctx.needs_input_grad[0] else None
         grad_gate = (tokens.to(torch.float64).t() @ gl).to(gate_w.dtype) if ctx.needs_input_grad[1] else None
@@ -247,6 +239,12 @@ def moe_topk_route(tokens: torch.Tensor, gate_w: torch.Tensor, k: int, force_ref
         raise ValueError(f"tokens must be [B,S,H] or [N,H], got shape {list(tokens.shape)}")
     if not (1 <= k <= gate_w.shape[1]):
         raise ValueError(f"k={k} must be in [1, {gate_w.shape[1]}]")
+    if not _needs_grad(tokens, gate_w) and _should_use_fused(tokens, gate_w, force_reference, k):
+        # no gradient wanted: one native call, one kernel, and only the decision itself is written
+        from .kernels import status_word
+
+        out = _ext.ext().router_route(tokens, _bf16_gate(gate_w), k, False, status_word(tokens.device))
+        return out[2], out[3]
     return MoERouterFunction.apply(tokens, gate_w, k, force_reference, None)
 
 
@@ -328,8 +326,10 @@ class MoERouter(nn.Module):
             e1.synchronize()
             kernel_ms = e0.elapsed_time(e1)
         bytes_moved = N * H * pend["elem"] + H * E * pend["elem"] + N * E * 4 + N * K * 8
-        z = float(pend["z_loss"]) if pend.get("z_loss") is not None else 0.0
-        aux = float(pend["aux_loss"]) if pend.get("aux_loss") is not None else 0.0
+        if pend.get("stats") is not None:  # the fused kernel's {aux loss, z loss, ...}
+            aux, z = pend["stats"].tolist()[:2]
+        else:
+            aux, z = float(pend["aux_loss"]), float(pend["z_loss"])
         mean = float(counts.mean())
         return RouterProfile(
             sram_bytes_per_block=_fused_stage_bytes(E),
@@ -356,15 +356,20 @@ class MoERouter(nn.Module):
         E, K = self.num_experts, self.top_k
         fused = self.bias is None and _should_use_fused(tokens, self.gate_w, force_reference, K)
         if fused:
-            holder: Dict[str, Any] = {}
-            w32, aux, z, idx32 = FusedRouterFunction.apply(tokens, self.gate_w, K, holder, self.profile_timing)
-            out: RouterOutput = holder["out"]
-            idx, w, counts = idx32.long(), w32.to(tokens.dtype), out.counts.long()
+            if _needs_grad(tokens, self.gate_w):
+                holder: Dict[str, Any] = {}
+                w32, w, aux, z, idx32, idx = FusedRouterFunction.apply(tokens, self.gate_w, K, holder,
+                                                                       self.profile_timing)
+                out: RouterOutput = holder["out"]
+            else:
+                out = fused_router_forward(tokens, _bf16_gate(self.gate_w), K, self.profile_timing)
+                w32, w, idx32, idx = out.w32, out.w16, out.idx32, out.idx64
+                aux, z = out.stats[0], out.stats[1]
             self._last_logits, self.last_aux_loss, self.last_z_loss = out.logits, aux, z
             self.last_idx32, self.last_w32 = idx32, w32
-            self._pending = dict(counts=out.counts, N=N, fused=True, events=out.events, z_loss=z.detach(),
-                                 aux_loss=aux.detach(), elem=2, sram=16384 + ((E + 63) // 64) * 8192)
-            return idx, w, counts
+            self._pending = dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2,
+                                 sram=16384 + ((E + 63) // 64) * 8192)
+            return idx, w, out.counts64
         # PyTorch path (bias, CPU, fp32 tokens, shapes the kernel does not cover): fp64 math under autograd
         logits64 = tokens.to(torch.float64) @ self.gate_w.to(torch.float64)
         if self.bias is not None:
