@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "gemm.cuh"
+#include "host_ops.h"
 #include "ops.cuh"
 #include "router.cuh"
 
@@ -100,16 +101,12 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& D, int64_t mode, int64_t epi
   cmoe::GemmArgs g = gemm_args(A, B, D, mode, epilogue, M, N, K, a_mn, b_mn, groups, b_group_rows, split_n, tile_group,
                                num_m_tiles, max_m_tiles, group_offsets, d_group_stride, accumulate, aux_in, aux_out,
                                ready_flags, ready_stride, ready_count, ready_target, status, timeout_ns);
-  // dense and grouped-K launches with plain results run on the two-SM kernel (CMOE_GEMM_2CTA=0: one-CTA kernel)
-  static const bool two_cta = [] {
-    const char* v = std::getenv("CMOE_GEMM_2CTA");
-    return v == nullptr || (v[0] != '\0' && v[0] != '0');
-  }();
-  if (two_cta && cmoe::gemm_2cta_supported(g)) {
-    check_cuda(cmoe::launch_gemm_2cta(g, cur_stream()), "launch_gemm_2cta");
-    return;
-  }
-  check_cuda(cmoe::launch_gemm(g, cur_stream()), "launch_gemm");
+  cmoe::launch_gemm_any(g, cur_stream());
+}
+
+// out (+)= a^T @ b over the rows, cut into pieces where the output alone would leave SMs idle
+void wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, const OptTensor& status) {
+  cmoe::dense_wgrad(a, b, out, accumulate, opt_ptr<int>(status));
 }
 
 // GEMM (dense or grouped-M) whose output rows are scattered by the epilogue: row r goes to rank
@@ -405,6 +402,7 @@ void register_router(pybind11::module_& m);
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "sm_100a kernels of the composed MoE engine";
   m.def("gemm", &gemm);
+  m.def("wgrad", &wgrad);
   m.def("gemm_pull", &gemm_pull);
   m.def("gemm_scatter", &gemm_scatter);
   m.def("router_fwd", &router_fwd);

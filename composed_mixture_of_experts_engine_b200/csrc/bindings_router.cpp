@@ -10,6 +10,7 @@
 #include <tuple>
 #include <utility>
 
+#include "host_ops.h"
 #include "router.cuh"
 
 namespace {
@@ -89,6 +90,49 @@ RouteResult router_route(const Tensor& X, const Tensor& Wg, int64_t K, bool full
   return {idx32, w32, idx64, w16, logits, lse, counts, counts64, mean_prob, stats};
 }
 
+// (grad_tokens, grad_gate) from the upstream gradients of the gate weights (fp32 and / or bf16 view of the same
+// values), the load-balance loss and the z-loss: the d(logits) kernel, then the two contractions with it.
+std::tuple<OptTensor, OptTensor> router_grad(const Tensor& X, const Tensor& Wg, const Tensor& logits, const Tensor& lse,
+                                             const Tensor& idx32, const Tensor& counts, const OptTensor& grad_w32,
+                                             const OptTensor& grad_w16, const OptTensor& grad_aux,
+                                             const OptTensor& grad_z, bool need_tokens, bool need_gate, bool gate_bf16,
+                                             const OptTensor& status) {
+  const c10::cuda::CUDAGuard guard(X.device());
+  const auto as_f32 = [](const OptTensor& t) {
+    return t.has_value() ? OptTensor(t->to(at::kFloat).contiguous()) : OptTensor();
+  };
+  OptTensor gw = as_f32(grad_w32);
+  if (grad_w16.has_value()) gw = gw.has_value() ? (*gw + *grad_w16).contiguous() : as_f32(grad_w16);
+  const OptTensor ga = as_f32(grad_aux), gz = as_f32(grad_z);
+  Tensor gl = at::empty(logits.sizes(), X.options());
+  cmoe::RouterBwdArgs a;
+  a.logits = logits.data_ptr<float>();
+  a.lse = lse.data_ptr<float>();
+  a.topk_idx = idx32.data_ptr<int>();
+  a.grad_w = gw.has_value() ? gw->data_ptr<float>() : nullptr;
+  a.counts = counts.data_ptr<int>();
+  a.grad_aux = ga.has_value() ? ga->data_ptr<float>() : nullptr;
+  a.grad_z = gz.has_value() ? gz->data_ptr<float>() : nullptr;
+  a.n_tokens = logits.size(0);
+  a.E = static_cast<int>(logits.size(1));
+  a.K = static_cast<int>(idx32.size(1));
+  a.grad_logits_bf16 = gl.data_ptr();
+  const cudaError_t e = cmoe::launch_router_bwd(a, at::cuda::getCurrentCUDAStream().stream());
+  TORCH_CHECK(e == cudaSuccess, "cmoe: launch_router_bwd failed: ", cudaGetErrorString(e));
+  int* st = status.has_value() ? status->data_ptr<int>() : nullptr;
+  std::tuple<OptTensor, OptTensor> out;
+  if (need_tokens) std::get<0>(out) = cmoe::dense_nt(gl, Wg, Tensor(), st);  // [N, E] x [H, E]^T
+  if (need_gate) {                                                          // tokens^T [H, N] x gl [N, E]
+    Tensor g = at::empty({X.size(1), gl.size(1)}, gate_bf16 ? X.options() : X.options().dtype(at::kFloat));
+    cmoe::dense_wgrad(X, gl, g, false, st);
+    std::get<1>(out) = g;
+  }
+  return out;
+}
+
 }  // namespace
 
-void register_router(pybind11::module_& m) { m.def("router_route", &router_route); }
+void register_router(pybind11::module_& m) {
+  m.def("router_route", &router_route);
+  m.def("router_grad", &router_grad);
+}

@@ -65,6 +65,7 @@ struct KParams {
   const int* tile_group;
   const int* num_m_tiles;
   const int* group_offsets;
+  int k_chunk, k_rows;
   void* D;
   long long ldd, d_group_stride;
   int d_fp32, accumulate;
@@ -162,8 +163,8 @@ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles
     }
     ti.k_blocks = (p.K + BK - 1) / BK;
   } else {  // grouped-K: both operands are MN-major, contraction over the rows of group g
-    const int r0 = p.group_offsets[g];
-    const int r1 = p.group_offsets[g + 1];
+    const int r0 = p.k_chunk > 0 ? min(g * p.k_chunk, p.k_rows) : p.group_offsets[g];
+    const int r1 = p.k_chunk > 0 ? min((g + 1) * p.k_chunk, p.k_rows) : p.group_offsets[g + 1];
     ti.a_mn0 = ti.m0;
     ti.a_k0 = r0;
     ti.b_n0 = ti.n0;
@@ -1160,7 +1161,8 @@ cudaError_t launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const
 
 cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   if (a.N % 8 != 0 || a.N <= 0) return cudaErrorInvalidValue;
-  if (a.mode == GEMM_GROUPED_K && !(a.a_mn && a.b_mn)) return cudaErrorInvalidValue;
+  if (a.mode == GEMM_GROUPED_K && (!(a.a_mn && a.b_mn) || (a.group_offsets == nullptr && (a.k_chunk <= 0 || a.k_chunk % 64 != 0))))
+    return cudaErrorInvalidValue;
   if (a.mode == GEMM_GROUPED_M && a.a_mn) return cudaErrorInvalidValue;
   if (a.epilogue == EPI_SWIGLU_FWD && (a.b_mn || a.split_n <= 0)) return cudaErrorInvalidValue;
 
@@ -1183,6 +1185,8 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.tile_group = a.tile_group;
   kp.num_m_tiles = a.num_m_tiles;
   kp.group_offsets = a.group_offsets;
+  kp.k_chunk = a.k_chunk;
+  kp.k_rows = static_cast<int>(a.a_rows);
   kp.D = a.D;
   kp.ldd = a.ldd;
   kp.d_group_stride = a.d_group_stride;

@@ -49,6 +49,8 @@ struct GemmArgs {
   const int* num_m_tiles = nullptr;    // grouped-M: number of live 128-row tiles, device scalar
   int max_m_tiles = 0;                 // grouped-M: upper bound on *num_m_tiles (sizes the grid)
   const int* group_offsets = nullptr;  // grouped-K: [groups+1] row offsets (multiples of 64), device memory
+  int k_chunk = 0;                     // grouped-K without group_offsets: group g contracts over the rows
+                                       // [g * k_chunk, (g + 1) * k_chunk) (a multiple of 64) of the a_rows rows
 
   void* D = nullptr;
   long long ldd = 0;

@@ -51,6 +51,7 @@ struct K2Params {
   int mode, M, N, K, groups;
   int a_mn, b_mn;
   const int* group_offsets;
+  int k_chunk, k_rows;  // regular groups of k_chunk rows instead of group_offsets
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
   int* status;
   unsigned long long timeout_ns;
@@ -74,7 +75,8 @@ __device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, 
   ti.n0 = (r / band_rows) * T_BN;
   ti.group = g;
   if (p.mode == GEMM_GROUPED_K) {
-    const int r0 = p.group_offsets[g], r1 = p.group_offsets[g + 1];
+    const int r0 = p.k_chunk > 0 ? min(g * p.k_chunk, p.k_rows) : p.group_offsets[g];
+    const int r1 = p.k_chunk > 0 ? min((g + 1) * p.k_chunk, p.k_rows) : p.group_offsets[g + 1];
     ti.a_k0 = ti.b_k0 = r0;
     ti.k_blocks = (r1 - r0 + T_BK - 1) / T_BK;
   } else {
@@ -466,7 +468,7 @@ bool gemm_2cta_supported(const GemmArgs& a) {
   if (a.mode == GEMM_DENSE) {
     if (a.a_mn) return false;
   } else if (a.mode == GEMM_GROUPED_K) {
-    if (!(a.a_mn && a.b_mn)) return false;
+    if (!(a.a_mn && a.b_mn) || (a.group_offsets == nullptr && (a.k_chunk <= 0 || a.k_chunk % 64 != 0))) return false;
   } else {
     return false;
   }
@@ -499,6 +501,8 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   kp.a_mn = a.a_mn;
   kp.b_mn = a.b_mn;
   kp.group_offsets = a.group_offsets;
+  kp.k_chunk = a.k_chunk;
+  kp.k_rows = static_cast<int>(a.a_rows);
   kp.d_fp32 = a.d_fp32;
   kp.reduce = a.accumulate;
   kp.status = a.status;

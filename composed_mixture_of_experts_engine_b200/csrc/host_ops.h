@@ -1,0 +1,19 @@
+// Native host building blocks shared by the binding files: GEMM launches on tensors, without Python in between.
+#pragma once
+#include <torch/extension.h>
+
+#include "gemm.cuh"
+
+namespace cmoe {
+
+// Launches `g` on the two-SM kernel where it qualifies (CMOE_GEMM_2CTA=0: never), on the one-CTA kernel otherwise.
+void launch_gemm_any(const GemmArgs& g, cudaStream_t stream);
+
+// y[M, N] = x[M, K] @ w[N, K]^T (out: bf16, allocated when undefined)
+torch::Tensor dense_nt(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
+// y[M, K] = x[M, N] @ w[N, K]
+torch::Tensor dense_nn(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
+// out[M, N] (+)= a[R, M]^T @ b[R, N]; out fp32 (stored, or added to) or bf16 (stored)
+void dense_wgrad(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool accumulate, int* status);
+
+}  // namespace cmoe

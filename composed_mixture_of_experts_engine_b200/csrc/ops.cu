@@ -435,6 +435,31 @@ __global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restric
   if (threadIdx.x == 0) *out += acc;
 }
 
+// Sum of the partial results of a contraction that was cut into `parts` pieces, always in the same order; the result
+// replaces or is added to fp32, or is rounded once to bf16.
+template <int OUT>  // 0: fp32 store, 1: fp32 add, 2: bf16 store
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float4* __restrict__ part, int parts, long long n4,
+                                                            void* __restrict__ out) {
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= n4) return;
+  float4 acc = __ldcs(part + i);
+#pragma unroll 8
+  for (int s = 1; s < parts; ++s) {
+    const float4 v = __ldcs(part + s * n4 + i);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  if (OUT == 2) {
+    reinterpret_cast<uint2*>(out)[i] = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+  } else {
+    float4* o = reinterpret_cast<float4*>(out) + i;
+    if (OUT == 1) {
+      const float4 v = *o;
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+    *o = acc;
+  }
+}
+
 // ------------------------------------------------------------------------------------ cross-entropy
 constexpr int CE_THREADS = 512;
 __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
@@ -891,6 +916,19 @@ cudaError_t launch_sumsq(const void* x, int is_bf16, long long n, float* out, fl
   const unsigned grid = static_cast<unsigned>(sumsq_partial_count(n));
   sumsq_kernel<<<grid, 256, 0, stream>>>(x, is_bf16, n, out, partials);
   if (partials != nullptr) sumsq_final_kernel<<<1, 256, 0, stream>>>(partials, static_cast<int>(grid), out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void* out, int out_bf16, int accumulate,
+                                 cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (n % 4 != 0 || parts < 1 || (out_bf16 && accumulate)) return cudaErrorInvalidValue;
+  const long long n4 = n / 4;
+  const unsigned grid = static_cast<unsigned>((n4 + 255) / 256);
+  const float4* p = reinterpret_cast<const float4*>(part);
+  if (out_bf16) splitk_reduce_kernel<2><<<grid, 256, 0, stream>>>(p, parts, n4, out);
+  else if (accumulate) splitk_reduce_kernel<1><<<grid, 256, 0, stream>>>(p, parts, n4, out);
+  else splitk_reduce_kernel<0><<<grid, 256, 0, stream>>>(p, parts, n4, out);
   return cudaGetLastError();
 }
 

@@ -59,6 +59,11 @@ cudaError_t launch_adamw(const AdamWArgs& a, cudaStream_t stream);
 int sumsq_partial_count(long long n);
 cudaError_t launch_sumsq(const void* x, int is_bf16, long long n, float* out, float* partials, cudaStream_t stream);
 
+// out[i] (fp32: stored or added to; bf16: stored) = sum over s < parts of part[s * n + i], in order of s.  n % 4 == 0,
+// 16-byte aligned pointers.
+cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void* out, int out_bf16, int accumulate,
+                                 cudaStream_t stream);
+
 // ---- cross-entropy, forward and gradient in one pass ------------------------------------------
 // logits [rows, V] bf16 are overwritten with d(loss)/d(logits) = (softmax - onehot) * grad_scale;
 // *loss_sum += sum over rows of the per-row loss (fp32), or, with `row_loss` [rows], the per-row losses are written

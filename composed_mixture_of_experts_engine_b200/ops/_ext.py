@@ -30,6 +30,7 @@ _SOURCES = [
     "bindings_attention.cpp",
     "bindings_ep.cpp",
     "bindings_router.cpp",
+    "host_ops.cpp",
     "gemm.cu",
     "gemm2.cu",
     "router.cu",
@@ -161,7 +162,7 @@ def build_io_lib(force: bool = False) -> Path:
 
 
 # kernels launched by one call of each entry point (cudaMemsetAsync calls are not counted)
-_KERNELS_PER_CALL = {"moe_plan": 3, "moe_plan_scratch_words": 0}
+_KERNELS_PER_CALL = {"moe_plan": 3, "moe_plan_scratch_words": 0, "router_grad": 3}
 _launch_counts: dict = {}
 
 

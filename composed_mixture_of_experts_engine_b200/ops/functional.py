@@ -98,7 +98,7 @@ class _LinearFn(torch.autograd.Function):
             if main is not None:
                 kernels.linear_tn_acc(dy2, x2, main)
             else:
-                dw = kernels.linear_tn(dy2, x2).to(weight.dtype)
+                dw = kernels.linear_tn(dy2, x2, out_dtype=weight.dtype)
         return dx, dw
 
 

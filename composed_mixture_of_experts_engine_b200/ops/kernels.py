@@ -114,57 +114,21 @@ def linear_nn(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
     return gemm(x, w, out, M=M, N=N, K=K, b_mn=True, accumulate=accumulate)
 
 
-_offsets_cache: Dict[Tuple[int, Tuple[int, ...]], torch.Tensor] = {}
-
-
-def _offsets_i32(device: torch.device, offs: Tuple[int, ...]) -> torch.Tensor:
-    """Device copy of a short host list of row offsets, made once per distinct list (a fresh ``torch.tensor``
-    per call would be a pageable host-to-device copy in the middle of the backward pass)."""
-    key = (device.index or 0, offs)
-    t = _offsets_cache.get(key)
-    if t is None:
-        if len(_offsets_cache) > 256:
-            _offsets_cache.clear()
-        t = torch.tensor(offs, device=device, dtype=torch.int32)
-        _offsets_cache[key] = t
-    return t
-
-
 def linear_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
-              splits: int = 0) -> torch.Tensor:
-    """out[M, N] (fp32) = a[R, M]^T @ b[R, N]: the weight-gradient contraction over R rows.
-
-    The R rows are cut into ``splits`` chunks (multiples of 64 rows) that run as separate tiles and
-    are summed afterwards, so that small outputs still fill the GPU.
-    """
-    R, M = a.shape
-    N = b.shape[1]
-    if splits <= 0:
-        tiles = ((M + 127) // 128) * ((N + 255) // 256)
-        splits = max(1, min(R // 512 if R >= 512 else 1, (148 + tiles - 1) // tiles))
-    chunk = ((R + splits - 1) // splits + 63) // 64 * 64
-    offs = tuple(min(i * chunk, R) for i in range(splits)) + (R,)
-    offs_t = _offsets_i32(a.device, offs)
-    part = torch.empty(splits, M, N, device=a.device, dtype=torch.float32)
-    gemm(a, b, part, mode=GEMM_GROUPED_K, M=M, N=N, a_mn=True, b_mn=True, groups=splits, group_offsets=offs_t,
-         d_group_stride=M * N)
-    red = part[0] if splits == 1 else part.sum(0)
+              out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    """out[M, N] = a[R, M]^T @ b[R, N]: the weight-gradient contraction over R rows (fp32 accumulation; a bf16 result
+    is rounded once).  Small outputs are cut into pieces of rows that run side by side and are added in order
+    (csrc/host_ops.cpp)."""
     if out is None:
-        return red
-    if accumulate:
-        out.add_(red.to(out.dtype))
-    else:
-        out.copy_(red)
+        out = torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=out_dtype)
+    _ext.ext().wgrad(a, b, out, accumulate, status_word(a.device))
     return out
 
 
 def linear_tn_acc(a: torch.Tensor, b: torch.Tensor, acc: torch.Tensor, accumulate: bool = True) -> torch.Tensor:
-    """acc[M, N] (fp32, in place) += a[R, M]^T @ b[R, N] with the addition done by the kernel's TMA reduce-add
-    epilogue (no read-modify-write pass over ``acc`` on the SMs, no temporary); ``accumulate=False`` stores."""
-    R, M = a.shape
-    N = b.shape[1]
-    gemm(a, b, acc, mode=GEMM_GROUPED_K, M=M, N=N, a_mn=True, b_mn=True, groups=1,
-         group_offsets=_offsets_i32(a.device, (0, R)), d_group_stride=M * N, accumulate=accumulate)
+    """acc[M, N] (fp32, in place) += a[R, M]^T @ b[R, N]; one piece adds with the kernel's TMA reduce-add epilogue (no
+    read-modify-write pass over ``acc`` on the SMs, no temporary); ``accumulate=False`` stores."""
+    _ext.ext().wgrad(a, b, acc, accumulate, status_word(a.device))
     return acc
 
 

@@ -142,18 +142,15 @@ def _needs_grad(*tensors: torch.Tensor) -> bool:
     return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
 
 
-def _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w, grad_aux, grad_z, gate_dtype):
+def _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w32, grad_w16, grad_aux, grad_z,
+                           gate_dtype):
     """(grad_tokens, grad_gate): the analytic d(logits) kernel and the two contractions with it."""
-    from .kernels import linear_nt, linear_tn
+    from .kernels import status_word
 
-    gl16 = torch.empty(logits.shape, device=logits.device, dtype=torch.bfloat16)
-    _ext.ext().router_bwd(logits, lse, idx32, grad_w, counts, grad_aux, grad_z, gl16, None)
-    grad_tokens = grad_gate = None
-    if ctx.needs_input_grad[0]:
-        grad_tokens = linear_nt(gl16, gw16)  # [N, E] x [H, E]^T
-    if ctx.needs_input_grad[1]:
-        grad_gate = linear_tn(tokens, gl16).to(gate_dtype)  # tokens^T [H, N] x gl [N, E]
-    return grad_tokens, grad_gate
+    gt, gg = _ext.ext().router_grad(tokens, gw16, logits, lse, idx32, counts, grad_w32, grad_w16, grad_aux, grad_z,
+                                    ctx.needs_input_grad[0], ctx.needs_input_grad[1], gate_dtype == torch.bfloat16,
+                                    status_word(tokens.device))
+    return gt, (gg if gg is None or gg.dtype == gate_dtype else gg.to(gate_dtype))
 
 
 class FusedRouterFunction(torch.autograd.Function):
@@ -173,13 +170,7 @@ class FusedRouterFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_w32, grad_w16, grad_aux, grad_z, _grad_idx32, _grad_idx64):
-        gw = grad_w32
-        if grad_w16 is not None:
-            gw = grad_w16.float() if gw is None else gw + grad_w16
-        gw = None if gw is None else gw.float().contiguous()
-        ga = None if grad_aux is None else grad_aux.float().reshape(1).contiguous()
-        gz = None if grad_z is None else grad_z.float().reshape(1).contiguous()
-        gt, gg = _fused_router_backward(ctx, *ctx.saved_tensors, gw, ga, gz, ctx.gate_dtype)
+        gt, gg = _fused_router_backward(ctx, *ctx.saved_tensors, grad_w32, grad_w16, grad_aux, grad_z, ctx.gate_dtype)
         return gt, gg, None, None, None
 
 
@@ -218,8 +209,8 @@ class MoERouterFunction(torch.autograd.Function):
         tokens, gate_w, logits, idx = ctx.saved_tensors
         if ctx.fused:
             gw16, lse, idx32, counts = ctx.fused_saved
-            gt, gg = _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w.float().contiguous(),
-                                            None, None, gate_w.dtype)
+            gt, gg = _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, None, grad_w, None, None,
+                                            gate_w.dtype)
             return gt, gg, None, None, None
         gl = _reference_backward_fp64(logits, idx, grad_w, ctx.k, ctx.E)
         grad_tokens = (gl @ gate_w.to(torch.float64).t()).to(tokens.dtype) if ctx.needs_input_grad[0] else None

@@ -186,7 +186,7 @@ class _AllGatherLinear(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             # dy [rows, out_l] @ W [out_l, in], summed over ranks, this rank's sequence shard
             dx = _gemm_reduce_scatter(c, dy2, weight, True, B, S_l, "ag_dx").view(B, S_l, -1)
-        dw = kernels.linear_tn(dy2, full).to(weight.dtype) if ctx.needs_input_grad[1] else None
+        dw = kernels.linear_tn(dy2, full, out_dtype=weight.dtype) if ctx.needs_input_grad[1] else None
         return dx, dw, None
 
 
@@ -206,7 +206,7 @@ class _LinearReduceScatter(torch.autograd.Function):
         x2, weight = ctx.saved_tensors
         c, (B, S_l) = ctx.c, ctx.dims
         dy_full, dx = _gathered_gemm(c, dy.reshape(B * S_l, -1).contiguous(), weight, B, S_l, True, "rs_dy")
-        dw = kernels.linear_tn(dy_full.contiguous(), x2).to(weight.dtype) if ctx.needs_input_grad[1] else None
+        dw = kernels.linear_tn(dy_full.contiguous(), x2, out_dtype=weight.dtype) if ctx.needs_input_grad[1] else None
         return dx.reshape(B, c.world * S_l, -1) if ctx.needs_input_grad[0] else None, dw, None
 
 

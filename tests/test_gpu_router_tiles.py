@@ -11,11 +11,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("N,H,E,K", [
     (1, 8, 8, 8),          # one token, one k-block, K = E
-    (64, 2048, 64, 8),     # one row tile split over a cluster of eight CTAs
-    (129, 520, 256, 8),    # two row tiles, a ragged last k-block, the widest expert variant
-    (300, 4096, 128, 6),   # cluster of eight, 128 experts
+    (64, 2048, 64, 8),     # short tiles of 16 rows
+    (129, 520, 256, 8),    # a cluster of four CTAs per tile, a ragged last k-block, the widest expert variant
+    (300, 4096, 128, 6),   # clusters of two CTAs, 128 experts
     (127, 1024, 24, 3),    # expert count that is no multiple of 16
-    (8190, 1024, 40, 1),   # 64 row tiles: cluster of two
+    (8190, 1024, 40, 1),   # tiles of 64 rows
     (20000, 256, 32, 4),   # more row tiles than SMs
 ])
 def test_route_matches_the_oracle_at_tile_edges(N, H, E, K):
