@@ -398,6 +398,7 @@ void combine_bwd_w(const Tensor& rows, const Tensor& slot_row, const Tensor& dy,
 void register_attention(pybind11::module_& m);
 void register_ep(pybind11::module_& m);
 void register_router(pybind11::module_& m);
+void register_moe(pybind11::module_& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "sm_100a kernels of the composed MoE engine";
@@ -422,4 +423,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   register_attention(m);
   register_ep(m);
   register_router(m);
+  register_moe(m);
 }

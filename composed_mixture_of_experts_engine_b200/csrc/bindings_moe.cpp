@@ -1,0 +1,242 @@
+// Native host path of the expert layer on one GPU: row plan -> gather -> grouped SwiGLU GEMMs -> weighted combine, and
+// its backward, each as one binding call that allocates and launches everything.  A layer call of a few hundred
+// tokens is bound by its host work: fourteen tensor constructions, six binding calls and their argument checks took
+// longer in Python than the kernels on the GPU.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <algorithm>
+#include <optional>
+#include <tuple>
+
+#include "host_ops.h"
+#include "ops.cuh"
+
+namespace {
+
+using torch::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+void check(cudaError_t e, const char* what) {
+  TORCH_CHECK(e == cudaSuccess, "cmoe: ", what, " failed: ", cudaGetErrorString(e));
+}
+int* status_ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr<int>() : nullptr; }
+
+// The tables of a row plan in one int32 buffer (see MoePlanArgs in ops.cuh for their meaning).
+struct PlanTables {
+  int64_t n_slots, cap_rows, E;
+  int64_t row_slot, group_offsets, tile_group, num_m_tiles, counts_kept, words;  // offsets; slot_row is at 0
+  PlanTables(int64_t n_slots_, int64_t E_) : n_slots(n_slots_), E(E_) {
+    // worst case of the padded layout: every slot kept, up to 127 padding rows for every expert that has a slot
+    cap_rows = (n_slots + std::min(E, n_slots) * 127 + 127) / 128 * 128;
+    row_slot = n_slots;
+    group_offsets = row_slot + cap_rows;
+    tile_group = group_offsets + E + 1;
+    num_m_tiles = tile_group + cap_rows / 128;
+    counts_kept = num_m_tiles + 1;
+    words = counts_kept + E;
+  }
+};
+
+struct Shapes {
+  int64_t N, K, H, E, F;
+};
+Shapes check_shapes(const Tensor& x, const Tensor& idx32, const Tensor& w13, const Tensor& w2) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1,
+              "x must be a CUDA bf16 matrix with unit inner stride");
+  TORCH_CHECK(idx32.scalar_type() == at::kInt && idx32.dim() == 2 && idx32.is_contiguous() && idx32.size(0) == x.size(0),
+              "idx must be contiguous int32 [N, K]");
+  TORCH_CHECK(w13.scalar_type() == at::kBFloat16 && w13.dim() == 3 && w13.is_contiguous() && w13.size(2) == x.size(1) &&
+                  w13.size(1) % 2 == 0,
+              "w13 must be contiguous bf16 [E, 2F, H]");
+  const Shapes s{x.size(0), idx32.size(1), x.size(1), w13.size(0), w13.size(1) / 2};
+  TORCH_CHECK(w2.scalar_type() == at::kBFloat16 && w2.is_contiguous() && w2.dim() == 3 && w2.size(0) == s.E &&
+                  w2.size(1) == s.H && w2.size(2) == s.F,
+              "w2 must be contiguous bf16 [E, H, F]");
+  return s;
+}
+
+// a grouped-by-rows launch over the tiles of `plan`: D[rows, N] = A[rows, K] * B (one [b_rows, b_cols] block per expert)
+cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_rows, bool b_mn, const Tensor& D, int64_t N,
+                            int64_t K, const PlanTables& pt, int* plan, int* status) {
+  cmoe::GemmArgs g;
+  g.A = A.data_ptr();
+  g.a_rows = A.size(0);
+  g.a_cols = A.size(1);
+  g.a_ld = A.stride(0);
+  g.B = B.data_ptr();
+  g.b_rows = pt.E * b_group_rows;
+  g.b_cols = B.size(2);
+  g.b_ld = B.size(2);
+  g.b_mn = b_mn;
+  g.mode = cmoe::GEMM_GROUPED_M;
+  g.N = static_cast<int>(N);
+  g.K = static_cast<int>(K);
+  g.groups = static_cast<int>(pt.E);
+  g.b_group_rows = b_group_rows;
+  g.tile_group = plan + pt.tile_group;
+  g.num_m_tiles = plan + pt.num_m_tiles;
+  g.max_m_tiles = static_cast<int>(pt.cap_rows / 128);
+  g.D = D.data_ptr();
+  g.ldd = D.stride(0);
+  g.status = status;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  return g;
+}
+
+// (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads)
+using Forward = std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor>;
+Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
+                          const Tensor& w2, int64_t capacity, bool keep, const OptTensor& status,
+                          const OptTensor& overflow) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+  const Shapes s = check_shapes(x, idx32, w13, w2);
+  TORCH_CHECK(gate_w32.scalar_type() == at::kFloat && gate_w32.is_contiguous() && gate_w32.numel() == s.N * s.K,
+              "gate weights must be contiguous fp32 [N, K]");
+  const PlanTables pt(s.N * s.K, s.E);
+  const auto i32 = x.options().dtype(at::kInt), bf = x.options();
+  Tensor plan_t = at::empty({pt.words}, i32);
+  int* plan = plan_t.data_ptr<int>();
+  {
+    const int per_k = capacity > 0;
+    Tensor scratch = at::empty(
+        {static_cast<int64_t>(cmoe::moe_plan_scratch_words(pt.n_slots, static_cast<int>(s.E), static_cast<int>(s.K), per_k))},
+        i32);
+    cmoe::MoePlanArgs a;
+    a.topk_idx = idx32.data_ptr<int>();
+    a.n_slots = pt.n_slots;
+    a.K = static_cast<int>(s.K);
+    a.num_experts = a.n_local = static_cast<int>(s.E);
+    a.per_k_bins = per_k;
+    a.capacity = static_cast<int>(capacity);
+    a.cap_rows = pt.cap_rows;
+    a.slot_row = plan;
+    a.row_slot = plan + pt.row_slot;
+    a.group_offsets = plan + pt.group_offsets;
+    a.tile_group = plan + pt.tile_group;
+    a.num_m_tiles = plan + pt.num_m_tiles;
+    a.counts_kept = plan + pt.counts_kept;
+    a.scratch = scratch.data_ptr<int>();
+    a.overflow = status_ptr(overflow);
+    check(cmoe::launch_moe_plan(a, stream), "moe_plan");
+  }
+  Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
+  check(cmoe::launch_gather_rows(x.data_ptr(), plan + pt.row_slot, static_cast<int>(s.K), nullptr, xp.data_ptr(),
+                                 pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(s.H), x.stride(0), s.H, stream),
+        "gather_rows");
+  Tensor hact = at::empty({pt.cap_rows, s.F}, bf);
+  OptTensor gu;
+  {
+    cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status));
+    g.epilogue = cmoe::EPI_SWIGLU_FWD;
+    g.split_n = static_cast<int>(s.F);
+    if (keep) {
+      gu = at::empty({pt.cap_rows, 2 * s.F}, bf);
+      g.aux_out = gu->data_ptr();
+      g.ld_aux_out = 2 * s.F;
+    }
+    cmoe::launch_gemm_any(g, stream);
+  }
+  Tensor yp = at::empty({pt.cap_rows, s.H}, bf);
+  cmoe::launch_gemm_any(grouped_rows(hact, w2, s.H, false, yp, s.H, s.F, pt, plan, status_ptr(status)), stream);
+  Tensor y = at::empty({s.N, s.H}, bf);
+  check(cmoe::launch_combine_rows(yp.data_ptr(), plan, gate_w32.data_ptr<float>(), y.data_ptr(), s.N,
+                                  static_cast<int>(s.K), static_cast<int>(s.H), s.H, s.H, stream),
+        "combine_rows");
+  if (!keep) return {y, plan_t, std::nullopt, std::nullopt, std::nullopt, std::nullopt};
+  return {y, plan_t, xp, hact, gu, yp};
+}
+
+// dW[e] = a[rows of e]^T b[rows of e]: added into the fp32 `main` buffer when there is one (returns nothing), else
+// rounded once into a new tensor of the weight's type
+OptTensor expert_wgrad(const Tensor& a, const Tensor& b, const Tensor& weight, const OptTensor& main, const PlanTables& pt,
+                       const int* plan, int* status, cudaStream_t stream) {
+  cmoe::GemmArgs g;
+  g.A = a.data_ptr();
+  g.a_rows = a.size(0);
+  g.a_cols = a.size(1);
+  g.a_ld = a.stride(0);
+  g.a_mn = 1;
+  g.B = b.data_ptr();
+  g.b_rows = b.size(0);
+  g.b_cols = b.size(1);
+  g.b_ld = b.stride(0);
+  g.b_mn = 1;
+  g.mode = cmoe::GEMM_GROUPED_K;
+  g.M = static_cast<int>(a.size(1));
+  g.N = static_cast<int>(b.size(1));
+  g.groups = static_cast<int>(pt.E);
+  g.group_offsets = plan + pt.group_offsets;
+  g.d_group_stride = a.size(1) * b.size(1);
+  g.ldd = b.size(1);
+  g.status = status;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  OptTensor out;
+  if (main.has_value()) {
+    TORCH_CHECK(main->scalar_type() == at::kFloat && main->is_contiguous() && main->numel() == weight.numel(),
+                "main_grad must be a contiguous fp32 tensor of the weight's shape");
+    g.D = main->data_ptr();
+    g.d_fp32 = g.accumulate = 1;
+  } else {
+    out = at::empty(weight.sizes(), weight.options());
+    g.D = out->data_ptr();
+  }
+  cmoe::launch_gemm_any(g, stream);
+  return out;
+}
+
+// (dx, d_gate, dw13, dw2)
+using Backward = std::tuple<OptTensor, OptTensor, OptTensor, OptTensor>;
+Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor& xp, const Tensor& hact, const Tensor& gu,
+                            const Tensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2, bool need_dx,
+                            bool need_gate, const OptTensor& main13, const OptTensor& main2, const OptTensor& status) {
+  const c10::cuda::CUDAGuard guard(dy.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+  const int64_t N = gate_w32.size(0), K = gate_w32.size(1), H = xp.size(1), E = w13.size(0), F = hact.size(1);
+  TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && dy.size(0) == N && dy.size(1) == H, "bad dy");
+  const PlanTables pt(N * K, E);
+  TORCH_CHECK(plan_t.numel() == pt.words && xp.size(0) == pt.cap_rows, "the row plan belongs to another layer call");
+  int* plan = plan_t.data_ptr<int>();
+  int* st = status_ptr(status);
+  Backward out;
+  if (need_gate) {
+    Tensor d_gate = at::empty({N, K}, gate_w32.options());
+    check(cmoe::launch_combine_bwd_w(yp.data_ptr(), plan, dy.data_ptr(), d_gate.data_ptr<float>(), N,
+                                     static_cast<int>(K), static_cast<int>(H), H, H, stream),
+          "combine_bwd_w");
+    std::get<1>(out) = d_gate;
+  }
+  Tensor dyp = at::empty({pt.cap_rows, H}, dy.options());
+  check(cmoe::launch_gather_rows(dy.data_ptr(), plan + pt.row_slot, static_cast<int>(K), gate_w32.data_ptr<float>(),
+                                 dyp.data_ptr(), pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(H), H, H, stream),
+        "gather_rows");
+  Tensor dgu = at::empty({pt.cap_rows, 2 * F}, dy.options());
+  {
+    cmoe::GemmArgs g = grouped_rows(dyp, w2, H, true, dgu, F, H, pt, plan, st);
+    g.epilogue = cmoe::EPI_SWIGLU_BWD;
+    g.aux_in = gu.data_ptr();
+    g.ld_aux_in = gu.stride(0);
+    cmoe::launch_gemm_any(g, stream);
+  }
+  if (need_dx) {
+    Tensor dxp = at::empty({pt.cap_rows, H}, dy.options());
+    cmoe::launch_gemm_any(grouped_rows(dgu, w13, 2 * F, true, dxp, H, 2 * F, pt, plan, st), stream);
+    Tensor dx = at::empty({N, H}, dy.options());
+    check(cmoe::launch_combine_rows(dxp.data_ptr(), plan, nullptr, dx.data_ptr(), N, static_cast<int>(K),
+                                    static_cast<int>(H), H, H, stream),
+          "combine_rows");
+    std::get<0>(out) = dx;
+  }
+  std::get<3>(out) = expert_wgrad(dyp, hact, w2, main2, pt, plan, st, stream);
+  std::get<2>(out) = expert_wgrad(dgu, xp, w13, main13, pt, plan, st, stream);
+  return out;
+}
+
+}  // namespace
+
+void register_moe(pybind11::module_& m) {
+  m.def("moe_local_forward", &moe_local_forward);
+  m.def("moe_local_backward", &moe_local_backward);
+}

@@ -1,11 +1,10 @@
 // Bandwidth-bound kernels of the training step: RMSNorm, RoPE, fused AdamW (+ global-norm clipping
-// without a host round trip), cross-entropy with in-place gradient, and the MoE bookkeeping kernels
-// (deterministic expert-sorted row plan, row gather, weighted combine).
+// without a host round trip), cross-entropy with in-place gradient, and the MoE row kernels (row gather, weighted
+// combine; the row plan is in plan.cu).
 //
 // Reference counterparts: RMSNorm eager ops (pkg/models/moe.py:83-86); torch.optim.AdamW +
-// clip_grad_norm_ + F.cross_entropy (train.py:207-212, 297-303, 322-323); argsort /
-// repeat_interleave / per-k scatter loop of the MoE layer (pkg/distributed/moe_layer.py:309-353);
-// capacity dropping (moe_layer.py:64-155).  RoPE has no counterpart there.
+// clip_grad_norm_ + F.cross_entropy (train.py:207-212, 297-303, 322-323); the per-k scatter loop of the
+// MoE layer (pkg/distributed/moe_layer.py:309-353).  RoPE has no counterpart there.
 #include "ops.cuh"
 
 #include <cstdlib>
@@ -539,150 +538,6 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   }
 }
 
-// ------------------------------------------------------------------------------------ MoE plan
-constexpr int PLAN_UNIT_SLOTS = 256;  // slots ranked by one warp
-constexpr int PLAN_WARPS = 8;
-
-__device__ __forceinline__ int plan_bin(const MoePlanArgs& a, long long slot) {
-  const int e = a.topk_idx[slot] - a.expert_lo;
-  if (e < 0 || e >= a.n_local) return -1;
-  return a.per_k_bins ? e * a.K + static_cast<int>(slot % a.K) : e;
-}
-
-// pass 1: per-unit histogram.  hist[unit][bin]
-__global__ void __launch_bounds__(PLAN_WARPS * 32) moe_plan_hist_kernel(const MoePlanArgs a, int nbins, int n_units) {
-  const int unit = blockIdx.x * PLAN_WARPS + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (unit >= n_units) return;
-  int* hist = a.scratch + static_cast<long long>(unit) * nbins;
-  for (int b = lane; b < nbins; b += 32) hist[b] = 0;
-  __syncwarp();
-  const long long s0 = static_cast<long long>(unit) * PLAN_UNIT_SLOTS;
-  for (int r = 0; r < PLAN_UNIT_SLOTS / 32; ++r) {
-    const long long slot = s0 + r * 32 + lane;
-    const int bin = slot < a.n_slots ? plan_bin(a, slot) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    if (bin >= 0 && (peers & ((1u << lane) - 1u)) == 0u) hist[bin] += __popc(peers);
-    __syncwarp();
-  }
-}
-
-// pass 2 (one CTA): exclusive prefix of hist over units within each bin, clipped bin totals,
-// 128-row-padded expert offsets, tile table
-__global__ void __launch_bounds__(1024) moe_plan_scan_kernel(const MoePlanArgs a, int nbins, int n_units) {
-  int* hist = a.scratch;
-  int* bin_base = a.scratch + static_cast<long long>(n_units) * nbins;
-  int* bin_total = bin_base + nbins;
-  __shared__ int s_part[1024];
-  if (nbins <= 1024) {
-    // all 1024 threads: thread = (chunk of units, bin).  Chunk sums, a short serial prefix over the chunks of the
-    // bin in shared memory, then the exclusive prefix inside the chunk.  Loads of neighbouring threads are
-    // neighbouring bins (coalesced) and independent of the running sum.
-    int chunks = 1024 / nbins;
-    if (chunks > n_units) chunks = n_units;
-    const int per = (n_units + chunks - 1) / chunks;
-    const int b = threadIdx.x % nbins, c = threadIdx.x / nbins;
-    const bool live = c < chunks;
-    const int u0 = c * per, u1 = min(n_units, u0 + per);
-    int sum = 0;
-    if (live) {
-#pragma unroll 8
-      for (int u = u0; u < u1; ++u) sum += hist[static_cast<long long>(u) * nbins + b];
-    }
-    s_part[threadIdx.x] = sum;
-    __syncthreads();
-    if (live) {
-      int run = 0;
-      for (int cc = 0; cc < c; ++cc) run += s_part[cc * nbins + b];
-#pragma unroll 8
-      for (int u = u0; u < u1; ++u) {
-        const int cnt = hist[static_cast<long long>(u) * nbins + b];
-        hist[static_cast<long long>(u) * nbins + b] = run;
-        run += cnt;
-      }
-      if (c == chunks - 1) {  // the last chunk's running sum is the bin total
-        for (int cc = c + 1; cc < chunks; ++cc) run += s_part[cc * nbins + b];
-        bin_total[b] = (a.capacity > 0 && run > a.capacity) ? a.capacity : run;
-      }
-    }
-  } else {
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
-      int run = 0;
-      for (int u = 0; u < n_units; ++u) {
-        const int c = hist[static_cast<long long>(u) * nbins + b];
-        hist[static_cast<long long>(u) * nbins + b] = run;
-        run += c;
-      }
-      bin_total[b] = (a.capacity > 0 && run > a.capacity) ? a.capacity : run;
-    }
-  }
-  __syncthreads();
-  __shared__ int s_total_rows;
-  if (threadIdx.x == 0) {
-    const int kb = a.per_k_bins ? a.K : 1;
-    int off = 0;
-    for (int e = 0; e < a.n_local; ++e) {
-      a.group_offsets[e] = off;
-      int cnt = 0;
-      for (int k = 0; k < kb; ++k) {
-        bin_base[e * kb + k] = off + cnt;
-        cnt += bin_total[e * kb + k];
-      }
-      // rows that do not fit the buffer are dropped by the assign pass (and counted in `overflow`)
-      const long long room = a.cap_rows - off;
-      if (cnt > room) cnt = room > 0 ? static_cast<int>(room) : 0;
-      a.counts_kept[e] = cnt;
-      off += (cnt + 127) / 128 * 128;
-      if (off > a.cap_rows) off = static_cast<int>(a.cap_rows / 128 * 128);
-    }
-    a.group_offsets[a.n_local] = off;
-    *a.num_m_tiles = off / 128;
-    s_total_rows = off;
-  }
-  __syncthreads();
-  const int tiles = s_total_rows / 128;
-  for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
-    const int row = t * 128;
-    int lo = 0, hi = a.n_local;  // largest e with group_offsets[e] <= row
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (a.group_offsets[mid] <= row) lo = mid; else hi = mid;
-    }
-    a.tile_group[t] = lo;
-  }
-}
-
-// pass 3: destination row of every slot
-__global__ void __launch_bounds__(PLAN_WARPS * 32) moe_plan_assign_kernel(const MoePlanArgs a, int nbins, int n_units) {
-  const int unit = blockIdx.x * PLAN_WARPS + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (unit >= n_units) return;
-  int* hist = a.scratch + static_cast<long long>(unit) * nbins;
-  const int* bin_base = a.scratch + static_cast<long long>(n_units) * nbins;
-  const long long s0 = static_cast<long long>(unit) * PLAN_UNIT_SLOTS;
-  for (int r = 0; r < PLAN_UNIT_SLOTS / 32; ++r) {
-    const long long slot = s0 + r * 32 + lane;
-    const int bin = slot < a.n_slots ? plan_bin(a, slot) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    int row = -1;
-    if (bin >= 0) {
-      const int rank = hist[bin] + __popc(peers & ((1u << lane) - 1u));
-      if (a.capacity <= 0 || rank < a.capacity) row = bin_base[bin] + rank;
-      if (row >= a.cap_rows) {  // the row buffer is full: drop the slot and report it
-        row = -1;
-        if (a.overflow) atomicAdd(a.overflow, 1);
-      }
-    }
-    __syncwarp();
-    if (bin >= 0 && (peers & ((1u << lane) - 1u)) == 0u) hist[bin] += __popc(peers);
-    __syncwarp();
-    if (slot < a.n_slots) {
-      a.slot_row[slot] = row;
-      if (row >= 0 && row < a.cap_rows) a.row_slot[row] = static_cast<int>(slot);
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------ gather / combine
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ row_slot,
                                    int slot_div, const float* __restrict__ slot_scale,
@@ -938,27 +793,6 @@ cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* 
   if (ld % 8 != 0) return cudaErrorInvalidValue;
   cross_entropy_kernel<<<static_cast<unsigned>(rows), CE_THREADS, 0, stream>>>(
       reinterpret_cast<__nv_bfloat16*>(logits), targets, loss_sum, row_loss, rows, V, ld, grad_scale);
-  return cudaGetLastError();
-}
-
-size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_bins) {
-  const long long nbins = static_cast<long long>(n_local) * (per_k_bins ? K : 1);
-  const long long n_units = (n_slots + PLAN_UNIT_SLOTS - 1) / PLAN_UNIT_SLOTS;
-  return static_cast<size_t>(n_units * nbins + 2 * nbins);
-}
-
-cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
-  if (a.n_slots <= 0 || a.n_local <= 0) return cudaErrorInvalidValue;
-  const int nbins = a.n_local * (a.per_k_bins ? a.K : 1);
-  const int n_units = static_cast<int>((a.n_slots + PLAN_UNIT_SLOTS - 1) / PLAN_UNIT_SLOTS);
-  cudaError_t e = cudaMemsetAsync(a.row_slot, 0xFF, sizeof(int) * a.cap_rows, stream);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(a.tile_group, 0xFF, sizeof(int) * ((a.cap_rows + 127) / 128), stream);
-  if (e != cudaSuccess) return e;
-  const unsigned blocks = static_cast<unsigned>((n_units + PLAN_WARPS - 1) / PLAN_WARPS);
-  moe_plan_hist_kernel<<<blocks, PLAN_WARPS * 32, 0, stream>>>(a, nbins, n_units);
-  moe_plan_scan_kernel<<<1, 1024, 0, stream>>>(a, nbins, n_units);
-  moe_plan_assign_kernel<<<blocks, PLAN_WARPS * 32, 0, stream>>>(a, nbins, n_units);
   return cudaGetLastError();
 }
 

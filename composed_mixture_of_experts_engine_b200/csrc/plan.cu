@@ -1,0 +1,328 @@
+// Expert-sorted row plan of the MoE layer (see ops.cuh for what it produces): ranks every (token, k) slot within its
+// expert, in slot order and without atomics on the order.
+// Reference counterpart: argsort / repeat_interleave of the MoE layer (pkg/distributed/moe_layer.py:309-353) and its
+// capacity dropping (moe_layer.py:64-155).
+//
+// What bounds it: latency.  The slots are a few hundred KiB at most, so the time is the number of dependent launches
+// and of dependent passes inside them.
+//   * up to 8192 slots: one launch of one CTA, 32 warps that each rank 256 slots;
+//   * more: a counting launch (histogram per unit of slots), then one launch whose CTAs each add up the histograms of
+//     the units before theirs (a few KiB out of L2, redundantly, which is cheaper than a launch or a last-CTA hand-over
+//     in between), derive the expert offsets and rank their slots;
+//   * only where units x bins exceed 16384 words a scan launch replaces the redundant sums.
+// The first form took two memsets and three launches, one of them a single CTA whose first thread walked the experts
+// through global memory: 22.8 us of kernels for 64 tokens x top-8 of 64 experts, 41 us for 16384 tokens.
+#include "ops.cuh"
+
+#include "common.cuh"
+
+namespace cmoe {
+
+namespace {
+
+constexpr int kCountThreads = 256;
+constexpr int kWarpsMulti = 8;
+constexpr int kWarpsSingle = 32;
+constexpr int kSingleSlots = 8192;
+constexpr int kRedundantWords = 16384;
+constexpr int kSmemLimit = 200 * 1024;
+
+__device__ __forceinline__ int plan_bin(const MoePlanArgs& a, long long slot) {
+  const int e = a.topk_idx[slot] - a.expert_lo;
+  if (e < 0 || e >= a.n_local) return -1;
+  return a.per_k_bins ? e * a.K + static_cast<int>(slot % a.K) : e;
+}
+
+// hist[unit][bin]; also clears the row -> slot table
+__global__ void __launch_bounds__(kCountThreads) plan_count_kernel(const MoePlanArgs a, int nbins, int unit_slots,
+                                                                   int in_smem) {
+  extern __shared__ int plan_smem[];
+  int* hist = a.scratch + static_cast<long long>(blockIdx.x) * nbins;
+  int* h = in_smem ? plan_smem : hist;
+  for (int b = threadIdx.x; b < nbins; b += kCountThreads) h[b] = 0;
+  for (long long r = blockIdx.x * static_cast<long long>(kCountThreads) + threadIdx.x; r < a.cap_rows;
+       r += static_cast<long long>(gridDim.x) * kCountThreads)
+    a.row_slot[r] = -1;
+  __syncthreads();
+  const long long s0 = static_cast<long long>(blockIdx.x) * unit_slots;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < unit_slots; i += kCountThreads) {  // whole warps: unit_slots is a multiple of 1024
+    const long long slot = s0 + i;
+    const int bin = slot < a.n_slots ? plan_bin(a, slot) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && (peers & ((1u << lane) - 1u)) == 0u) atomicAdd(h + bin, __popc(peers));
+  }
+  if (in_smem) {
+    __syncthreads();
+    for (int b = threadIdx.x; b < nbins; b += kCountThreads) hist[b] = h[b];
+  }
+}
+
+// In place: hist[unit][bin] -> sum over the units before it; total[bin] behind the histograms.  A CTA takes 32 bins,
+// its 32 warps a chunk of the units each.
+__global__ void __launch_bounds__(1024) plan_scan_kernel(const MoePlanArgs a, int nbins, int n_units) {
+  __shared__ int part[32][33];
+  int* hist = a.scratch;
+  int* total = a.scratch + static_cast<long long>(n_units) * nbins;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.x * 32 + lane;
+  const int per = (n_units + 31) / 32;
+  const int u0 = min(n_units, w * per), u1 = min(n_units, u0 + per);
+  int sum = 0;
+  if (b < nbins)
+#pragma unroll 8
+    for (int u = u0; u < u1; ++u) sum += hist[static_cast<long long>(u) * nbins + b];
+  part[w][lane] = sum;
+  __syncthreads();
+  int run = 0;
+  for (int q = 0; q < w; ++q) run += part[q][lane];
+  if (b < nbins) {
+#pragma unroll 8
+    for (int u = u0; u < u1; ++u) {
+      const int c = hist[static_cast<long long>(u) * nbins + b];
+      hist[static_cast<long long>(u) * nbins + b] = run;
+      run += c;
+    }
+    if (w == 31) total[b] = run;
+  }
+}
+
+// int words of working storage of one CTA of the ranking kernel: warp counts, slots before this unit, totals, first
+// row of every bin, first row of every expert
+__host__ __device__ inline long long rank_words(int warps, int nbins, int n_local) {
+  return (static_cast<long long>(warps) + 3) * nbins + n_local + 1;
+}
+
+// SINGLE: one CTA does everything.  Otherwise CTA u ranks the slots of unit u; `prescanned` says that
+// plan_scan_kernel has run.  `work` is this launch's working storage in global memory, one piece per CTA, where shared
+// memory would not hold it (thousands of bins); nullptr: shared memory.
+template <int WARPS, bool SINGLE>
+__global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs a, int nbins, int unit_slots,
+                                                               int n_units, int prescanned, int* work) {
+  extern __shared__ int plan_smem[];
+  constexpr int T = WARPS * 32;
+  int* s_warp = work != nullptr ? work + blockIdx.x * rank_words(WARPS, nbins, a.n_local) : plan_smem;  // [WARPS][nbins]
+  int* s_pre = s_warp + WARPS * nbins;  // slots of the bin in units before this one
+  int* s_tot = s_pre + nbins;           // all slots of the bin
+  int* s_base = s_tot + nbins;          // first row of the bin
+  int* s_goff = s_base + nbins;         // [n_local + 1] first row of the expert
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int unit = blockIdx.x;
+  const unsigned below = (1u << lane) - 1u;
+
+  for (int i = tid; i < (WARPS + 2) * nbins; i += T) s_warp[i] = 0;
+  if (SINGLE)
+    for (long long r = tid; r < a.cap_rows; r += T) a.row_slot[r] = -1;
+  __syncthreads();
+
+  // counts of this warp's range of slots
+  const int warp_slots = unit_slots / WARPS;
+  const long long s0 = static_cast<long long>(unit) * unit_slots + warp * warp_slots;
+  int* mine = s_warp + warp * nbins;
+  // (the expert numbers of up to eight rounds of 32 slots are fetched together)
+  int bins[8];
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = i0 + q * 32;
+      const long long slot = s0 + i + lane;
+      bins[q] = i < warp_slots && slot < a.n_slots ? plan_bin(a, slot) : -1;
+    }
+  };
+  for (int i0 = 0; i0 < warp_slots; i0 += 256) {
+    fetch(i0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int bin = bins[q];
+      const unsigned peers = __match_any_sync(0xffffffffu, bin);
+      if (bin >= 0 && (peers & below) == 0u) mine[bin] += __popc(peers);
+      __syncwarp();
+    }
+  }
+  // counts of the other units
+  if (!SINGLE) {
+    const int* hist = a.scratch;
+    if (prescanned) {
+      const int* total = hist + static_cast<long long>(n_units) * nbins;
+      for (int b = tid; b < nbins; b += T) {
+        s_pre[b] = hist[static_cast<long long>(unit) * nbins + b];
+        s_tot[b] = total[b];
+      }
+    } else {
+      // thread = (bin, range of units)
+      const int lanes_b = min(nbins, T);
+      const int ranges = T / lanes_b, range = tid / lanes_b;
+      if (range < ranges) {
+        const int per = (n_units + ranges - 1) / ranges;
+        const int u0 = min(n_units, range * per), u1 = min(n_units, u0 + per);
+        for (int b = tid - range * lanes_b; b < nbins; b += lanes_b) {
+          int before = 0, all = 0;
+#pragma unroll 8
+          for (int u = u0; u < u1; ++u) {
+            const int c = hist[static_cast<long long>(u) * nbins + b];
+            all += c;
+            before += u < unit ? c : 0;
+          }
+          atomicAdd(s_pre + b, before);
+          atomicAdd(s_tot + b, all);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // per bin: exclusive prefix over the warps
+  for (int b = tid; b < nbins; b += T) {
+    int run = 0;
+#pragma unroll 8
+    for (int w = 0; w < WARPS; ++w) {
+      const int c = s_warp[w * nbins + b];
+      s_warp[w * nbins + b] = run;
+      run += c;
+    }
+    if (SINGLE) s_tot[b] = run;
+    if (a.capacity > 0) {
+      const int t = SINGLE ? run : s_tot[b];
+      s_tot[b] = min(t, a.capacity);
+    }
+  }
+  __syncthreads();
+  // expert offsets: 128-row-padded exclusive prefix over the experts (one warp), clipped to the buffer
+  const int kb = a.per_k_bins ? a.K : 1;
+  const int cap128 = static_cast<int>(a.cap_rows / 128 * 128);
+  if (warp == 0) {
+    long long carry = 0;
+    for (int e0 = 0; e0 < a.n_local; e0 += 32) {
+      const int e = e0 + lane;
+      int cnt = 0;
+      if (e < a.n_local)
+        for (int k = 0; k < kb; ++k) cnt += s_tot[e * kb + k];
+      const int padded = (cnt + 127) / 128 * 128;
+      int incl = padded;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const long long raw = carry + incl - padded;
+      const int off = raw < cap128 ? static_cast<int>(raw) : cap128;
+      if (e < a.n_local) {
+        s_goff[e] = off;
+        int base = off;
+        for (int k = 0; k < kb; ++k) {
+          s_base[e * kb + k] = base;
+          base += s_tot[e * kb + k];
+        }
+        if (unit == 0) {
+          // rows that do not fit the buffer are dropped below (and counted in `overflow`)
+          const long long room = a.cap_rows - off;
+          a.counts_kept[e] = cnt > room ? static_cast<int>(room > 0 ? room : 0) : cnt;
+          a.group_offsets[e] = off;
+        }
+      }
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) {
+      const int off = carry < cap128 ? static_cast<int>(carry) : cap128;
+      s_goff[a.n_local] = off;
+      if (unit == 0) {
+        a.group_offsets[a.n_local] = off;
+        *a.num_m_tiles = off / 128;
+      }
+    }
+  }
+  __syncthreads();
+  // destination row of every slot
+  for (int i0 = 0; i0 < warp_slots; i0 += 256) {
+    if (warp_slots > 256) fetch(i0);  // otherwise still at hand
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = i0 + q * 32;
+      const long long slot = s0 + i + lane;
+      const int bin = bins[q];
+      const unsigned peers = __match_any_sync(0xffffffffu, bin);
+      int row = -1;
+      if (bin >= 0) {
+        const int rank = s_pre[bin] + mine[bin] + __popc(peers & below);
+        if (a.capacity <= 0 || rank < a.capacity) row = s_base[bin] + rank;
+        if (row >= a.cap_rows) {  // the row buffer is full: drop the slot and report it
+          row = -1;
+          if (a.overflow) atomicAdd(a.overflow, 1);
+        }
+      }
+      __syncwarp();
+      if (bin >= 0 && (peers & below) == 0u) mine[bin] += __popc(peers);
+      __syncwarp();
+      if (i < warp_slots && slot < a.n_slots) {
+        a.slot_row[slot] = row;
+        if (row >= 0) a.row_slot[row] = static_cast<int>(slot);
+      }
+    }
+  }
+  // expert of every tile, spread over the CTAs
+  const int tiles = s_goff[a.n_local] / 128, all_tiles = static_cast<int>((a.cap_rows + 127) / 128);
+  for (int t = unit * T + tid; t < all_tiles; t += gridDim.x * T) {
+    int e = -1;
+    if (t < tiles) {
+      int lo = 0, hi = a.n_local;  // largest e with goff[e] <= row
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (s_goff[mid] <= t * 128) lo = mid; else hi = mid;
+      }
+      e = lo;
+    }
+    a.tile_group[t] = e;
+  }
+}
+
+struct PlanShape {
+  int nbins, unit_slots, n_units;
+  bool single, scan, wide;  // wide: the ranking kernel's working storage lies in global memory
+  PlanShape(long long n_slots, int n_local, int K, int per_k_bins) {
+    nbins = n_local * (per_k_bins ? K : 1);
+    single = n_slots <= kSingleSlots && rank_words(kWarpsSingle, nbins, n_local) * 4 <= kSmemLimit;
+    wide = !single && rank_words(kWarpsMulti, nbins, n_local) * 4 > kSmemLimit;
+    // a unit has at least as many slots as bins twice over, so that its histogram is not larger than its slots
+    unit_slots = single ? static_cast<int>((n_slots + 1023) / 1024 * 1024) : 1024 * ((nbins + 511) / 512);
+    n_units = single ? 1 : static_cast<int>((n_slots + unit_slots - 1) / unit_slots);
+    scan = !single && static_cast<long long>(n_units) * nbins > kRedundantWords;
+  }
+  long long hist_words() const { return single ? 0 : (static_cast<long long>(n_units) + 1) * nbins; }
+};
+
+}  // namespace
+
+size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_bins) {
+  const PlanShape s(n_slots, n_local, K, per_k_bins);
+  const long long work = s.wide ? s.n_units * rank_words(kWarpsMulti, s.nbins, n_local) : 0;
+  return static_cast<size_t>(s.hist_words() + work + 1);
+}
+
+cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
+  if (a.n_slots <= 0 || a.n_local <= 0) return cudaErrorInvalidValue;
+  const PlanShape s(a.n_slots, a.n_local, a.K, a.per_k_bins);
+  static const cudaError_t configured = [] {
+    cudaError_t e = cudaFuncSetAttribute(plan_rank_kernel<kWarpsSingle, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(plan_rank_kernel<kWarpsMulti, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSmemLimit);
+  }();
+  if (configured != cudaSuccess) return configured;
+  if (s.single) {
+    const size_t smem = rank_words(kWarpsSingle, s.nbins, a.n_local) * 4;
+    plan_rank_kernel<kWarpsSingle, true>
+        <<<1, kWarpsSingle * 32, smem, stream>>>(a, s.nbins, s.unit_slots, 1, 0, nullptr);
+    return cudaGetLastError();
+  }
+  const bool hist_in_smem = s.nbins * 4 <= 48 * 1024;
+  plan_count_kernel<<<s.n_units, kCountThreads, hist_in_smem ? s.nbins * 4 : 0, stream>>>(a, s.nbins, s.unit_slots,
+                                                                                          hist_in_smem ? 1 : 0);
+  if (s.scan) plan_scan_kernel<<<(s.nbins + 31) / 32, 1024, 0, stream>>>(a, s.nbins, s.n_units);
+  const size_t smem = s.wide ? 0 : rank_words(kWarpsMulti, s.nbins, a.n_local) * 4;
+  plan_rank_kernel<kWarpsMulti, false><<<s.n_units, kWarpsMulti * 32, smem, stream>>>(
+      a, s.nbins, s.unit_slots, s.n_units, s.scan ? 1 : 0, s.wide ? a.scratch + s.hist_words() : nullptr);
+  return cudaGetLastError();
+}
+
+}  // namespace cmoe

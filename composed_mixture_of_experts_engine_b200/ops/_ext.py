@@ -30,11 +30,13 @@ _SOURCES = [
     "bindings_attention.cpp",
     "bindings_ep.cpp",
     "bindings_router.cpp",
+    "bindings_moe.cpp",
     "host_ops.cpp",
     "gemm.cu",
     "gemm2.cu",
     "router.cu",
     "ops.cu",
+    "plan.cu",
     "attention.cu",
     "attention_fwd2.cu",
     "ep.cu",
@@ -162,7 +164,7 @@ def build_io_lib(force: bool = False) -> Path:
 
 
 # kernels launched by one call of each entry point (cudaMemsetAsync calls are not counted)
-_KERNELS_PER_CALL = {"moe_plan": 3, "moe_plan_scratch_words": 0, "router_grad": 3}
+_KERNELS_PER_CALL = {"moe_plan": 2, "moe_plan_scratch_words": 0, "router_grad": 3, "moe_local_forward": 5, "moe_local_backward": 7}
 _launch_counts: dict = {}
 
 

@@ -401,7 +401,7 @@ class _LocalMoEFn(torch.autograd.Function):
             y = torch.empty(N, H, device=x.device, dtype=torch.bfloat16)
             _ext.ext().combine_rows(ys, ident, gate_w32, y, K)
             ctx.save_for_backward(xp, hact, gu, ys, gate_w32, w13, w2, ident)
-        else:
+        else:  # debug checks on: the plan is validated between the launches
             xp = kernels.gather_rows(x, plan)
             hact, gu, yp = grouped_swiglu_forward(xp, w13, w2, plan)
             y = kernels.combine_rows(yp, plan, gate_w32)
@@ -446,12 +446,59 @@ class _LocalMoEFn(torch.autograd.Function):
         return dx, d_gate, None, dw13, dw2, None, None
 
 
+class _LocalPlan:
+    """What telemetry reads of a native row plan: the kept rows per expert, the tail of its table buffer."""
+
+    __slots__ = ("buf", "n_local")
+
+    def __init__(self, buf: torch.Tensor, n_local: int):
+        self.buf, self.n_local = buf, n_local
+
+    @property
+    def counts_kept(self) -> torch.Tensor:
+        return self.buf[-self.n_local:]
+
+
+def _native_forward(x, gate_w32, idx32, w13, w2, capacity: int, keep: bool, holder: Optional[dict]):
+    dev = x.device
+    out = _ext.ext().moe_local_forward(x, gate_w32, idx32, w13, w2, capacity, keep, kernels.status_word(dev),
+                                       kernels.overflow_counter(dev))
+    if holder is not None:
+        holder["plan"] = _LocalPlan(out[1], w13.shape[0])
+    return out
+
+
+class _NativeLocalMoEFn(torch.autograd.Function):
+    """The same layer math, with each direction one native call (csrc/bindings_moe.cpp)."""
+
+    @staticmethod
+    def forward(ctx, x, gate_w32, idx32, w13, w2, capacity: int, holder: Optional[dict]):
+        y, plan, xp, hact, gu, yp = _native_forward(x, gate_w32, idx32, w13, w2, capacity, True, holder)
+        ctx.save_for_backward(plan, xp, hact, gu, yp, gate_w32, w13, w2)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        plan, xp, hact, gu, yp, gate_w32, w13, w2 = ctx.saved_tensors
+        dx, d_gate, dw13, dw2 = _ext.ext().moe_local_backward(
+            dy.contiguous(), plan, xp, hact, gu, yp, gate_w32, w13, w2, ctx.needs_input_grad[0],
+            ctx.needs_input_grad[1], getattr(w13, "main_grad", None), getattr(w2, "main_grad", None),
+            kernels.status_word(dy.device))
+        return dx, d_gate, None, dw13, dw2, None, None
+
+
 def local_moe(x: torch.Tensor, gate_w: torch.Tensor, idx: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
               capacity: int = 0, holder: Optional[dict] = None) -> torch.Tensor:
     """All experts on this rank.  ``x`` [N,H], ``gate_w`` [N,K] gate weights, ``idx`` [N,K] expert ids."""
     if on_device_path(x, w13, w2):
-        return _LocalMoEFn.apply(x, gate_w.float().contiguous(), idx.to(torch.int32).contiguous(), w13, w2, capacity,
-                                 holder)
+        from . import debug
+
+        gate_w32, idx32 = gate_w.float().contiguous(), idx.to(torch.int32).contiguous()
+        if _local_fused() or debug.enabled():
+            return _LocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
+        if torch.is_grad_enabled() and any(t.requires_grad for t in (x, gate_w32, w13, w2)):
+            return _NativeLocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
+        return _native_forward(x, gate_w32, idx32, w13, w2, capacity, False, holder)[0]
     keep = None
     if capacity > 0:
         keep = ~capacity_drop_mask_reference(idx, w13.shape[0], capacity)
