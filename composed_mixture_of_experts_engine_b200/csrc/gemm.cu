@@ -20,12 +20,11 @@
 // one piece ahead, overwrites them in place with dGate / dUp and stores those with TMA.
 #include "gemm.cuh"
 
-#include <cstdio>
 #include <cstdlib>
-#include <mutex>
-#include <unordered_map>
 
 #include "common.cuh"
+#include "swiglu_epilogue.cuh"
+#include "tensor_maps.h"
 
 namespace cmoe {
 
@@ -175,10 +174,6 @@ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles
   return ti;
 }
 
-// ex2.approx + rcp.approx: two special-function instructions instead of an IEEE division (the epilogue warps are
-// issue-bound: one warp per scheduler, so every instruction saved per element shortens the tile)
-__device__ __forceinline__ float sigmoidf_fast(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
-
 // 32 fp32 values of one output row -> bf16 (or fp32) in global memory, columns [col, col+32) masked by n_limit
 __device__ __forceinline__ void store_row_chunk(void* D, long long ldd, int d_fp32, int accumulate, long long row,
                                                 int col, int n_limit, const float (&v)[32]) {
@@ -231,32 +226,6 @@ __device__ __forceinline__ void prefetch_f32_chunk(const float* row_ptr, int col
   for (int j = 0; j < 8; ++j) {
     v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row_ok && col + j * 4 < n_limit) v[j] = *reinterpret_cast<const float4*>(row_ptr + col + j * 4);
-  }
-}
-
-// SwiGLU backward for 32 columns of one row: dH (fp32 bits in r) with the saved gate / up values (bf16, packed in
-// cg / cu) -> dGate / dUp (bf16, packed) written over cg / cu.  Eight columns at a time, straight from the packed
-// inputs to the packed outputs.
-__device__ __forceinline__ void swiglu_bwd_math(const uint32_t (&r)[32], uint4 (&cg)[4], uint4 (&cu)[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t gw[4] = {cg[j].x, cg[j].y, cg[j].z, cg[j].w};
-    const uint32_t uw[4] = {cu[j].x, cu[j].y, cu[j].z, cu[j].w};
-    uint32_t og[4], ou[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float2 g = unpack_bf16x2(gw[q]);
-      const float2 u = unpack_bf16x2(uw[q]);
-      const float dh0 = __uint_as_float(r[8 * j + 2 * q]), dh1 = __uint_as_float(r[8 * j + 2 * q + 1]);
-      const float s0 = sigmoidf_fast(g.x), s1 = sigmoidf_fast(g.y);
-      // d silu(g)/dg = s (1 + g (1 - s))
-      const float dg0 = dh0 * u.x * (s0 * fmaf(g.x, 1.f - s0, 1.f));
-      const float dg1 = dh1 * u.y * (s1 * fmaf(g.y, 1.f - s1, 1.f));
-      og[q] = pack_bf16x2(dg0, dg1);
-      ou[q] = pack_bf16x2(dh0 * (g.x * s0), dh1 * (g.y * s1));
-    }
-    cg[j] = make_uint4(og[0], og[1], og[2], og[3]);
-    cu[j] = make_uint4(ou[0], ou[1], ou[2], ou[3]);
   }
 }
 
@@ -952,188 +921,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-  });
-  return fn;
-}
-
-struct TmapKey {
-  const void* ptr;
-  long long rows, cols, ld;
-  int box_rows, box_cols;
-  bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows &&
-           box_cols == o.box_cols;
-  }
-};
-struct TmapKeyHash {
-  size_t operator()(const TmapKey& k) const {
-    size_t h = reinterpret_cast<size_t>(k.ptr);
-    h = h * 1000003u ^ static_cast<size_t>(k.rows);
-    h = h * 1000003u ^ static_cast<size_t>(k.cols);
-    h = h * 1000003u ^ static_cast<size_t>(k.ld);
-    h = h * 1000003u ^ static_cast<size_t>(k.box_rows);
-    h = h * 1000003u ^ static_cast<size_t>(k.box_cols);
-    return h;
-  }
-};
-
-// bf16 row-major [rows, cols] (leading dimension ld), box = box_cols columns x box_rows rows; 64 columns use the
-// 128-byte swizzle (operands), 32 columns the 64-byte swizzle (epilogue pieces)
-cudaError_t make_tmap(CUtensorMap* out, const void* ptr, long long rows, long long cols, long long ld, int box_rows,
-                      int box_cols = 64) {
-  static std::mutex mu;
-  static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-  if (box_cols != 64 && box_cols != 32) return cudaErrorInvalidValue;
-  TmapKey key{ptr, rows, cols, ld, box_rows, box_cols};
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
-      *out = it->second;
-      return cudaSuccess;
-    }
-  }
-  EncodeTiledFn enc = get_encode_fn();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0 || (ld * 2) % 16 != 0 || cols <= 0 || rows <= 0)
-    return cudaErrorInvalidValue;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estride[2] = {1u, 1u};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estride,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    std::fprintf(stderr, "cmoe: cuTensorMapEncodeTiled failed (%d) rows=%lld cols=%lld ld=%lld box_rows=%d\n",
-                 static_cast<int>(r), rows, cols, ld, box_rows);
-    return cudaErrorInvalidValue;
-  }
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (cache.size() > 8192) cache.clear();
-    cache.emplace(key, *out);
-  }
-  return cudaSuccess;
-}
-
-// Output map: [groups, rows, cols] of fp32 or bf16 with row stride ld and group stride gstride (elements); the box
-// is one staging buffer, 128 rows x 128 bytes, 128-byte swizzle.
-cudaError_t make_tmap_out(CUtensorMap* out, const void* ptr, int fp32, long long groups, long long rows,
-                          long long cols, long long ld, long long gstride, int box_bytes = 128) {
-  struct Key {
-    const void* ptr;
-    long long groups, rows, cols, ld, gstride;
-    int fp32, box_bytes;
-    bool operator==(const Key& o) const {
-      return ptr == o.ptr && groups == o.groups && rows == o.rows && cols == o.cols && ld == o.ld &&
-             gstride == o.gstride && fp32 == o.fp32 && box_bytes == o.box_bytes;
-    }
-  };
-  struct KeyHash {
-    size_t operator()(const Key& k) const {
-      size_t h = reinterpret_cast<size_t>(k.ptr);
-      for (long long v : {k.groups, k.rows, k.cols, k.ld, k.gstride, static_cast<long long>(k.fp32),
-                          static_cast<long long>(k.box_bytes)})
-        h = h * 1000003u ^ static_cast<size_t>(v);
-      return h;
-    }
-  };
-  static std::mutex mu;
-  static std::unordered_map<Key, CUtensorMap, KeyHash> cache;
-  if (box_bytes != 128 && box_bytes != 64) return cudaErrorInvalidValue;
-  Key key{ptr, groups, rows, cols, ld, gstride, fp32, box_bytes};
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
-      *out = it->second;
-      return cudaSuccess;
-    }
-  }
-  EncodeTiledFn enc = get_encode_fn();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  const long long es = fp32 ? 4 : 2;
-  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(groups)};
-  cuuint64_t gstr[2] = {static_cast<cuuint64_t>(ld * es), static_cast<cuuint64_t>(gstride * es)};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(box_bytes / es), static_cast<cuuint32_t>(BM), 1u};
-  cuuint32_t estride[3] = {1u, 1u, 1u};
-  CUresult r = enc(out, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-                   const_cast<void*>(ptr), gdim, gstr, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    std::fprintf(stderr, "cmoe: cuTensorMapEncodeTiled (output) failed (%d) groups=%lld rows=%lld cols=%lld ld=%lld\n",
-                 static_cast<int>(r), groups, rows, cols, ld);
-    return cudaErrorInvalidValue;
-  }
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (cache.size() > 8192) cache.clear();
-    cache.emplace(key, *out);
-  }
-  return cudaSuccess;
-}
-
-// bf16 [rows, 2N] viewed as [rows, 2 halves, N] (gate | up): dims (N, 2, rows), box 32 columns x 1 half x 128 rows,
-// 64-byte swizzle; a store of columns [c, c+32) of one half is clipped at N and never reaches into the other half
-cudaError_t make_tmap_halves(CUtensorMap* out, const void* ptr, long long rows, long long n, long long ld) {
-  struct Key {
-    const void* ptr;
-    long long rows, n, ld;
-    bool operator==(const Key& o) const { return ptr == o.ptr && rows == o.rows && n == o.n && ld == o.ld; }
-  };
-  struct KeyHash {
-    size_t operator()(const Key& k) const {
-      size_t h = reinterpret_cast<size_t>(k.ptr);
-      for (long long v : {k.rows, k.n, k.ld}) h = h * 1000003u ^ static_cast<size_t>(v);
-      return h;
-    }
-  };
-  static std::mutex mu;
-  static std::unordered_map<Key, CUtensorMap, KeyHash> cache;
-  Key key{ptr, rows, n, ld};
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
-      *out = it->second;
-      return cudaSuccess;
-    }
-  }
-  EncodeTiledFn enc = get_encode_fn();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(n), 2u, static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstr[2] = {static_cast<cuuint64_t>(n * 2), static_cast<cuuint64_t>(ld * 2)};
-  cuuint32_t box[3] = {32u, 1u, static_cast<cuuint32_t>(BM)};
-  cuuint32_t estride[3] = {1u, 1u, 1u};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstr, box, estride,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (cache.size() > 8192) cache.clear();
-    cache.emplace(key, *out);
-  }
-  return cudaSuccess;
-}
-
 // CMOE_GEMM_DIRECT_EPILOGUE=1 keeps every epilogue on per-thread stores from registers (for A/B measurements)
 bool direct_epilogue_forced() {
   static const bool forced = [] {

@@ -47,6 +47,12 @@ struct GemmArgs {
 
   const int* tile_group = nullptr;     // grouped-M: group of each 128-row tile (-1: skip), device memory
   const int* num_m_tiles = nullptr;    // grouped-M: number of live 128-row tiles, device scalar
+  // grouped-M, optional (the launch may then run on pairs of SMs): the same tiles in pairs of neighbours of one group,
+  // (first tile) * 2 + (1 if the pair has only that tile), and the number of pairs; device memory
+  const int* pair_tile = nullptr;
+  const int* num_pairs = nullptr;
+  long long rows_per_group = 0;        // grouped-M: expected rows of a group (chooses the order of the tiles only)
+  const int* group_order = nullptr;    // grouped-K, optional: the groups from most to fewest rows, device memory
   int max_m_tiles = 0;                 // grouped-M: upper bound on *num_m_tiles (sizes the grid)
   const int* group_offsets = nullptr;  // grouped-K: [groups+1] row offsets (multiples of 64), device memory
   int k_chunk = 0;                     // grouped-K without group_offsets: group g contracts over the rows
@@ -111,8 +117,9 @@ struct GemmArgs {
 // encoding tensor maps or launching.
 cudaError_t launch_gemm(const GemmArgs& args, cudaStream_t stream);
 
-// Two-SM variant (clusters of two CTAs, `tcgen05.mma.cta_group::2`, 256 x 256 tiles) for dense GEMMs and grouped-K
-// weight-gradient GEMMs with plain results; `gemm_2cta_supported` says whether a launch description qualifies.
+// Two-SM variant (clusters of two CTAs, `tcgen05.mma.cta_group::2`, 256 x 256 tiles) for dense GEMMs, grouped-K
+// weight-gradient GEMMs with plain results and grouped-M GEMMs that come with a table of tile pairs;
+// `gemm_2cta_supported` says whether a launch description qualifies.
 bool gemm_2cta_supported(const GemmArgs& args);
 constexpr int kPullFlagsPerTile = 4;  // words of GemmArgs::tile_ready per 128-row tile
 cudaError_t launch_gemm_2cta(const GemmArgs& args, cudaStream_t stream);

@@ -5,14 +5,20 @@
 // operands for 128 x 256 x 64 multiply-adds instead of the 48 KiB of the one-CTA kernel, so the L2 -> SM traffic per
 // FLOP drops by a third and six stages fit where four did.
 //
-// Scope: dense GEMMs and the grouped-K weight-gradient GEMMs with plain (staged, TMA-stored or TMA-reduced) results.
-// Everything that needs the fused epilogues, the row pull or the scatter stays on the one-CTA kernel in gemm.cu.
-// The host side sends every launch that qualifies here (`CMOE_GEMM_2CTA=0` keeps them on the one-CTA kernel).
+// Scope: dense GEMMs, the grouped-K weight-gradient GEMMs, and the grouped-by-rows expert GEMMs with plain and SwiGLU
+// results (there a pair takes two neighbouring 128-row tiles of one expert; where an expert has an odd number of tiles
+// its last pair computes and discards a half).  The row pull, the scatter and unaligned results stay on the one-CTA
+// kernel in gemm.cu.  The host side sends every launch that qualifies here (`CMOE_GEMM_2CTA=0` keeps them on the
+// one-CTA kernel).
+// What bounds it: the tensor pipe at the clock that the power limit leaves (1.55 GHz of 1.96 in a capture of the expert
+// GEMMs; pipe active 78 - 84 % of the cycles), so what counts is operand traffic per FLOP and evenly filled SMs.
 // Measured on a B200: dense 8192^3 1543 TFLOP/s against 1407 for the one-CTA kernel (cuBLAS in the same run: 1707),
-// grouped weight gradient with fp32 accumulation 1352 against 1144.
+// grouped weight gradient with fp32 accumulation 1352 against 1144; expert layer of 64 experts, 2048 rows each, H 2048,
+// F 1024, one-CTA / this kernel: first GEMM 869 / 823 us, second 475 / 436, gradient of the activation 513 / 482 (481
+// with two groups of epilogue warps, 497 with one), gradient of the tokens 884 / 838.
 //
-// CTA layout (192 threads): warp 0 TMA producer, warp 1 TMEM allocation (both CTAs) + MMA issue (leader only),
-// warps 2..5 epilogue of this CTA's 128 rows.  Barriers:
+// CTA layout (192 threads, 320 with two epilogue groups): warp 0 TMA producer, warp 1 TMEM allocation (both CTAs) + MMA issue (leader only),
+// warps 2.. epilogue of this CTA's 128 rows.  Barriers:
 //   full[s]   in the leader: one arrival with the byte count of both CTAs' loads; both CTAs' TMA loads complete on it
 //   empty[s]  in each CTA: the leader's MMA commits to its own and to the peer's barrier
 //   tfull[a]  in each CTA: committed by the leader to both when an accumulator is complete
@@ -20,12 +26,9 @@
 // Every wait is bounded as in gemm.cu; a wait that runs out ends the kernel normally with a status code.
 #include "gemm.cuh"
 
-#include <cstdio>
-#include <cstdlib>
-#include <mutex>
-#include <unordered_map>
-
 #include "common.cuh"
+#include "swiglu_epilogue.cuh"
+#include "tensor_maps.h"
 
 namespace cmoe {
 
@@ -34,17 +37,20 @@ namespace {
 constexpr int T_BM = 256;   // tile rows (128 per CTA)
 constexpr int T_BN = 256;   // tile columns (each CTA loads 128 of B's rows / columns)
 constexpr int T_BK = 64;
-constexpr int T_STAGES = 6;
 constexpr int T_A_BYTES = 128 * T_BK * 2;  // 16 KiB
 constexpr int T_B_BYTES = 128 * T_BK * 2;  // 16 KiB
 constexpr int T_STAGE_BYTES = T_A_BYTES + T_B_BYTES;
 constexpr int T_CHUNK_BYTES = 64 * T_BK * 2;  // one 64 x 64 bf16 box of an MN-major operand
 constexpr int T_STAGING_BUF = 128 * 128;
-constexpr int T_STAGING = 2 * T_STAGING_BUF;
-constexpr int T_THREADS = 192;
+constexpr int T_STAGING = 2 * T_STAGING_BUF;  // per group of four epilogue warps
+constexpr int T_MAX_GROUPS = 2;
 constexpr int T_TMEM_COLS = 512;
-constexpr int T_SMEM = T_STAGES * T_STAGE_BYTES + T_STAGING + 1024 + 256;
-constexpr int T_SWIZZLE = 4;  // band of row tiles walked together
+// one group of epilogue warps leaves room for six stages, two groups for five
+__host__ __device__ constexpr int t_stages(int groups) { return groups == 1 ? 6 : 5; }
+__host__ __device__ constexpr int t_threads(int groups) { return 64 + 128 * groups; }
+__host__ __device__ constexpr int t_smem(int groups) {
+  return t_stages(groups) * T_STAGE_BYTES + groups * T_STAGING + 1024 + 256;
+}
 constexpr int T_EPI_FIRST = 64;
 
 struct K2Params {
@@ -52,38 +58,67 @@ struct K2Params {
   int a_mn, b_mn;
   const int* group_offsets;
   int k_chunk, k_rows;  // regular groups of k_chunk rows instead of group_offsets
+  const int* tile_group;  // grouped by rows: expert of a 128-row tile, pairs of such tiles, their number
+  const int* pair_tile;
+  const int* num_pairs;
+  int b_group_rows, split_n;
+  int band;           // row tiles walked together
+  const int* group_order;  // grouped by K: the groups, longest first
+  int cols_per_tile;  // output columns of a tile (256; 128 with the SwiGLU forward: gate in one CTA's half of B, up in the other's)
+  int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
   int* status;
   unsigned long long timeout_ns;
 };
 
 struct Tile2 {
-  int m0, n0, group, a_k0, b_k0, k_blocks;
+  int m0, n0, group, a_k0, k_blocks;
+  int b_n, b_k0;  // this CTA's half of B: first N index, first K index
+  bool lone;      // only the first CTA has rows
 };
 
-__device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, int n_tiles) {
+__device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, int n_tiles, int cta) {
   Tile2 ti;
   int g = 0;
   if (p.mode == GEMM_GROUPED_K) {
     g = t / (m_tiles * n_tiles);
     t -= g * m_tiles * n_tiles;
+    if (p.group_order != nullptr) g = p.group_order[g];
   }
-  const int band = t / (T_SWIZZLE * n_tiles);
-  const int r = t - band * T_SWIZZLE * n_tiles;
-  const int band_rows = min(T_SWIZZLE, m_tiles - band * T_SWIZZLE);
-  ti.m0 = (band * T_SWIZZLE + r % band_rows) * T_BM;
-  ti.n0 = (r / band_rows) * T_BN;
-  ti.group = g;
+  const int band = t / (p.band * n_tiles);
+  const int r = t - band * p.band * n_tiles;
+  const int band_rows = min(p.band, m_tiles - band * p.band);
+  const int mt = band * p.band + r % band_rows;
+  ti.m0 = mt * T_BM;
+  ti.n0 = (r / band_rows) * p.cols_per_tile;
+  ti.b_n = ti.n0 + cta * 128;
+  ti.a_k0 = ti.b_k0 = 0;
+  ti.lone = false;
+  ti.k_blocks = (p.K + T_BK - 1) / T_BK;
   if (p.mode == GEMM_GROUPED_K) {
     const int r0 = p.k_chunk > 0 ? min(g * p.k_chunk, p.k_rows) : p.group_offsets[g];
     const int r1 = p.k_chunk > 0 ? min((g + 1) * p.k_chunk, p.k_rows) : p.group_offsets[g + 1];
     ti.a_k0 = ti.b_k0 = r0;
     ti.k_blocks = (r1 - r0 + T_BK - 1) / T_BK;
-  } else {
-    ti.a_k0 = ti.b_k0 = 0;
-    ti.k_blocks = (p.K + T_BK - 1) / T_BK;
+  } else if (p.mode == GEMM_GROUPED_M) {
+    const int v = p.pair_tile[mt];
+    ti.m0 = (v >> 1) * 128;
+    ti.lone = (v & 1) != 0;
+    g = p.tile_group[v >> 1];
+    if (p.b_mn) {
+      ti.b_k0 = g * p.b_group_rows;
+    } else {
+      ti.b_n = g * p.b_group_rows + (p.split_n ? ti.n0 + cta * p.split_n : ti.b_n);
+    }
   }
+  ti.group = g;
   return ti;
+}
+
+// The tile of cluster c in the round of tiles that starts at r0 (one per cluster).  With the groups sorted by length
+// the rounds go back and forth, so that a cluster which got the longest tile of one round gets the shortest of the next.
+__device__ __forceinline__ int tile_of_round(const K2Params& p, int r0, int c, int n_clusters) {
+  return p.group_order != nullptr && ((r0 / n_clusters) & 1) != 0 ? r0 + n_clusters - 1 - c : r0 + c;
 }
 
 // ---- cluster / two-SM PTX -------------------------------------------------------------------------------------
@@ -142,20 +177,23 @@ __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t d_tmem, uint64_t a_de
       : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T_THREADS, 1)
+template <int EPI, int GROUPS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(t_threads(GROUPS), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-             const __grid_constant__ CUtensorMap tmD, const K2Params p) {
+             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmE, const K2Params p) {
+  constexpr int T_STAGES = t_stages(GROUPS);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + T_STAGES * T_A_BYTES;
   uint8_t* stg = smem + T_STAGES * T_STAGE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T_STAGES * T_STAGE_BYTES + T_STAGING);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T_STAGES * T_STAGE_BYTES + GROUPS * T_STAGING);
   uint64_t* full_bar = bars;                    // [T_STAGES]  (used in the leader)
   uint64_t* empty_bar = bars + T_STAGES;        // [T_STAGES]
   uint64_t* tfull_bar = bars + 2 * T_STAGES;    // [2]
   uint64_t* tempty_bar = bars + 2 * T_STAGES + 2;  // [2]       (used in the leader)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T_STAGES + 4);
+  uint64_t* gfull_bar = bars + 2 * T_STAGES + 4;   // [GROUPS][2] saved gate|up pieces (SwiGLU backward)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T_STAGES + 4 + 2 * T_MAX_GROUPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -171,12 +209,14 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 256);
+      mbar_init(&tempty_bar[a], 256 * GROUPS);
     }
+    for (int a = 0; a < 2 * GROUPS; ++a) mbar_init(&gfull_bar[a], 1);
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmD);
+    if (EPI != EPI_STORE) tma_prefetch_desc(&tmE);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, T_TMEM_COLS);
@@ -193,8 +233,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   wc.status = p.status;
   wc.timeout_ns = p.timeout_ns;
 
-  const int m_tiles = (p.M + T_BM - 1) / T_BM;
-  const int n_tiles = (p.N + T_BN - 1) / T_BN;
+  const int m_tiles = p.mode == GEMM_GROUPED_M ? *p.num_pairs : (p.M + T_BM - 1) / T_BM;
+  const int n_tiles = (p.N + p.cols_per_tile - 1) / p.cols_per_tile;
   const int n_total = (p.mode == GEMM_GROUPED_K ? p.groups : 1) * m_tiles * n_tiles;
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
@@ -205,27 +245,31 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       int stage = 0;
       uint32_t phase = 0;
       const int moff = static_cast<int>(cta) * 128;  // this CTA's rows of A and its half of B
-      for (int t = cluster_id; t < n_total; t += n_clusters) {
-        const Tile2 ti = decode2(p, t, m_tiles, n_tiles);
+      for (int r0 = 0; r0 < n_total; r0 += n_clusters) {
+        const int t = tile_of_round(p, r0, cluster_id, n_clusters);
+        if (t >= n_total) break;  // in the last round only
+        const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta));
         if (ti.k_blocks == 0) continue;
+        const bool have_a = leader || !ti.lone;  // the MMA reads this CTA's stale rows; their results are not stored
         for (int kb = 0; kb < ti.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
           const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * T_STAGE_BYTES);
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * T_STAGE_BYTES - (ti.lone ? T_A_BYTES : 0));
           uint8_t* a_dst = sA + stage * T_A_BYTES;
           uint8_t* b_dst = sB + stage * T_B_BYTES;
           const int k = kb * T_BK;
-          if (p.a_mn) {
+          if (!have_a) {
+          } else if (p.a_mn) {
             tma_load_2d_pair(a_dst, &tmA, fb, ti.m0 + moff, ti.a_k0 + k);
             tma_load_2d_pair(a_dst + T_CHUNK_BYTES, &tmA, fb, ti.m0 + moff + 64, ti.a_k0 + k);
           } else {
             tma_load_2d_pair(a_dst, &tmA, fb, ti.a_k0 + k, ti.m0 + moff);
           }
           if (p.b_mn) {
-            tma_load_2d_pair(b_dst, &tmB, fb, ti.n0 + moff, ti.b_k0 + k);
-            tma_load_2d_pair(b_dst + T_CHUNK_BYTES, &tmB, fb, ti.n0 + moff + 64, ti.b_k0 + k);
+            tma_load_2d_pair(b_dst, &tmB, fb, ti.b_n, ti.b_k0 + k);
+            tma_load_2d_pair(b_dst + T_CHUNK_BYTES, &tmB, fb, ti.b_n + 64, ti.b_k0 + k);
           } else {
-            tma_load_2d_pair(b_dst, &tmB, fb, ti.b_k0 + k, ti.n0 + moff);
+            tma_load_2d_pair(b_dst, &tmB, fb, ti.b_k0 + k, ti.b_n);
           }
           if (++stage == T_STAGES) {
             stage = 0;
@@ -247,8 +291,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
-      for (int t = cluster_id; t < n_total; t += n_clusters) {
-        const Tile2 ti = decode2(p, t, m_tiles, n_tiles);
+      for (int r0 = 0; r0 < n_total; r0 += n_clusters) {
+        const int t = tile_of_round(p, r0, cluster_id, n_clusters);
+        if (t >= n_total) break;  // in the last round only
+        const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta));
         if (ti.k_blocks == 0) continue;
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, wc, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
@@ -283,19 +329,52 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
   } else {
     // ------------------------------------------------------------------ epilogue (this CTA's 128 rows)
+    // With two groups of four warps, a group takes every second piece of columns and has its own staging buffers.
+    const int grp = GROUPS == 1 ? 0 : (warp - 2) >> 2;
+    const bool issuer = threadIdx.x == T_EPI_FIRST + 128 * grp;  // of this group's TMA copies
+    uint8_t* my_stg = stg + grp * T_STAGING;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const int sw = row_in_tile & 7;
-    const int unit_cols = p.d_fp32 ? 32 : 64;
+    const int gsw = (row_in_tile >> 1) & 3;  // 64-byte swizzle: 16-byte chunk j of row r sits at j ^ ((r / 2) % 4)
+    const int unit_cols = EPI != EPI_STORE || p.d_fp32 ? 32 : 64;
+    // one named barrier per group and piece; it carries the OR of "a wait failed / abort seen", so that all 128
+    // threads leave the loop together
+    auto any_failed = [&](bool bad_here) {
+      int any;
+      asm volatile(
+          "{\n\t.reg .pred q, r;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.or.pred r, %2, 128, q;\n\t"
+          "selp.s32 %0, 1, 0, r;\n\t}"
+          : "=r"(any)
+          : "r"((bad_here || *abort_flag) ? 1 : 0), "r"(1 + grp)
+          : "memory");
+      return any != 0;
+    };
     int acc = 0;
     uint32_t acc_phase = 0;
     uint32_t stage_ctr = 0;
-    for (int t = cluster_id; t < n_total; t += n_clusters) {
-      const Tile2 ti = decode2(p, t, m_tiles, n_tiles);
+    for (int r0 = 0; r0 < n_total; r0 += n_clusters) {
+      const int t = tile_of_round(p, r0, cluster_id, n_clusters);
+      if (t >= n_total) break;  // in the last round only
+      const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta));
       const int row0 = ti.m0 + static_cast<int>(cta) * 128;
       const bool have_acc = ti.k_blocks != 0;
-      if (!have_acc && p.reduce) continue;  // adding zero: nothing to do
+      if (!have_acc && (p.reduce || EPI != EPI_STORE)) continue;  // adding zero: nothing to do (K > 0 otherwise)
+      const bool mine = p.mode == GEMM_GROUPED_M ? (leader || !ti.lone) : row0 < p.M;  // this CTA has rows
+      // SwiGLU backward: asks for the saved gate and up values of a piece (128 rows x 32 columns each)
+      auto gu_issue = [&](uint32_t ctr, int col) {
+        const uint32_t b = ctr & 1u;
+        uint8_t* dst = my_stg + b * T_STAGING_BUF;
+        uint64_t* bar = &gfull_bar[2 * grp + b];
+        mbar_arrive_expect_tx(bar, T_STAGING_BUF);
+        tma_load_2d(dst, &tmD, bar, col, row0);
+        tma_load_2d(dst + T_STAGING_BUF / 2, &tmD, bar, p.N + col, row0);
+      };
+      if (EPI == EPI_SWIGLU_BWD && issuer && mine && ti.n0 + grp * 32 < p.N) {
+        bulk_wait_group_read<1>();  // this piece's buffer was last read by the store issued two pieces ago
+        gu_issue(stage_ctr, ti.n0 + grp * 32);
+      }
       bool ok = true;
       if (have_acc) {
         ok = mbar_wait(&tfull_bar[acc], acc_phase, wc, ST_TIMEOUT_TMEM_FULL);
@@ -303,11 +382,96 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       }
       const uint32_t t_acc = tmem_base + acc * T_BN + lane_base;
       bool any_bad = false;
+      const int units = p.cols_per_tile / unit_cols;
 #pragma unroll 1
-      for (int u = 0; u < T_BN / unit_cols; ++u) {
+      for (int u = grp; u < units; u += GROUPS) {
         const int col0 = ti.n0 + u * unit_cols;
         if (col0 >= p.N) break;  // uniform
-        uint8_t* buf = stg + (stage_ctr & 1) * T_STAGING_BUF;
+        if (EPI == EPI_SWIGLU_BWD) {
+          // every thread turns its row of the piece into dGate / dUp in place
+          if (!mine) break;
+          const uint32_t b = stage_ctr & 1u;
+          if (issuer && u + GROUPS < units && col0 + 32 * GROUPS < p.N) {
+            bulk_wait_group_read<0>();  // the store of the previous piece has read the other buffer
+            gu_issue(stage_ctr + 1, col0 + 32 * GROUPS);
+          }
+          const bool got = mbar_wait(&gfull_bar[2 * grp + b], (stage_ctr >> 1) & 1u, wc, ST_TIMEOUT_SMEM_FULL);
+          uint8_t* grow = my_stg + b * T_STAGING_BUF + row_in_tile * 64;
+          if (ok && got) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(t_acc + u * 32, r);
+            uint4 cg[4], cu[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              cg[j] = *reinterpret_cast<const uint4*>(grow + ((j ^ gsw) << 4));
+              cu[j] = *reinterpret_cast<const uint4*>(grow + T_STAGING_BUF / 2 + ((j ^ gsw) << 4));
+            }
+            tmem_ld_wait();
+            swiglu_bwd_math(r, cg, cu);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              *reinterpret_cast<uint4*>(grow + ((j ^ gsw) << 4)) = cg[j];
+              *reinterpret_cast<uint4*>(grow + T_STAGING_BUF / 2 + ((j ^ gsw) << 4)) = cu[j];
+            }
+          }
+          fence_proxy_async_smem();
+          any_bad = any_failed(!ok || !got);
+          if (any_bad) break;
+          if (issuer) {
+            tma_store_3d(&tmE, my_stg + b * T_STAGING_BUF, col0, 0, row0);                      // dGate
+            tma_store_3d(&tmE, my_stg + b * T_STAGING_BUF + T_STAGING_BUF / 2, col0, 1, row0);  // dUp
+            bulk_commit_group();
+          }
+          ++stage_ctr;
+          continue;
+        }
+        if (EPI == EPI_SWIGLU_FWD) {
+          // accumulator columns [0, 128) = gate, [128, 256) = up: h, gate and up leave as three pieces of 128 rows x
+          // 64 bytes out of one staging area; two barriers per piece (area free, area filled)
+          if (!mine) break;
+          uint8_t* hrow = my_stg + row_in_tile * 64;
+          uint32_t ph[16], pg[16], pu[16];
+          if (ok) {
+            uint32_t rg[32], ru[32];
+            tmem_ld_32x32b_x32(t_acc + u * 32, rg);
+            tmem_ld_32x32b_x32(t_acc + 128 + u * 32, ru);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float g0 = __uint_as_float(rg[2 * j]), g1 = __uint_as_float(rg[2 * j + 1]);
+              const float u0 = __uint_as_float(ru[2 * j]), u1 = __uint_as_float(ru[2 * j + 1]);
+              ph[j] = pack_bf16x2(g0 * sigmoidf_fast(g0) * u0, g1 * sigmoidf_fast(g1) * u1);
+              pg[j] = pack_bf16x2(g0, g1);
+              pu[j] = pack_bf16x2(u0, u1);
+            }
+          }
+          if (issuer) bulk_wait_group_read<0>();  // the stores of the previous piece have read the area
+          any_bad = any_failed(!ok);
+          if (any_bad) break;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int o = (j ^ gsw) << 4;
+            *reinterpret_cast<uint4*>(hrow + o) = make_uint4(ph[4 * j], ph[4 * j + 1], ph[4 * j + 2], ph[4 * j + 3]);
+            if (p.has_aux) {
+              *reinterpret_cast<uint4*>(hrow + T_STAGING_BUF / 2 + o) =
+                  make_uint4(pg[4 * j], pg[4 * j + 1], pg[4 * j + 2], pg[4 * j + 3]);
+              *reinterpret_cast<uint4*>(hrow + T_STAGING_BUF + o) =
+                  make_uint4(pu[4 * j], pu[4 * j + 1], pu[4 * j + 2], pu[4 * j + 3]);
+            }
+          }
+          fence_proxy_async_smem();
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+          if (issuer) {
+            tma_store_3d(&tmD, my_stg, col0, row0, 0);
+            if (p.has_aux) {
+              tma_store_3d(&tmE, my_stg + T_STAGING_BUF / 2, col0, 0, row0);  // gate half
+              tma_store_3d(&tmE, my_stg + T_STAGING_BUF, col0, 1, row0);      // up half
+            }
+            bulk_commit_group();
+          }
+          continue;
+        }
+        uint8_t* buf = my_stg + (stage_ctr & 1) * T_STAGING_BUF;
         uint8_t* myrow = buf + row_in_tile * 128;
         if (ok) {
           if (p.d_fp32) {
@@ -354,20 +518,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           }
         }
         fence_proxy_async_smem();
-        if (threadIdx.x == T_EPI_FIRST) bulk_wait_group_read<0>();
-        {
-          const int bad = (!ok || *abort_flag) ? 1 : 0;
-          int any;
-          asm volatile(
-              "{\n\t.reg .pred q, r;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.or.pred r, 1, 128, q;\n\t"
-              "selp.s32 %0, 1, 0, r;\n\t}"
-              : "=r"(any)
-              : "r"(bad)
-              : "memory");
-          any_bad = any != 0;
-        }
+        if (issuer) bulk_wait_group_read<0>();
+        any_bad = any_failed(!ok);
         if (any_bad) break;
-        if (threadIdx.x == T_EPI_FIRST && row0 < p.M) {
+        if (issuer && mine) {
           const int zgrp = (p.mode == GEMM_GROUPED_K) ? ti.group : 0;
           if (p.reduce)
             tma_reduce_add_3d(&tmD, buf, col0, row0, zgrp);
@@ -378,7 +532,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         ++stage_ctr;
       }
       if (have_acc) {
-        // the leader's MMA warp may reuse this accumulator once all 256 epilogue threads of the pair have read it
+        // the leader's MMA warp may reuse this accumulator once all epilogue threads of the pair have read it
         tc_fence_before();
         mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
         acc ^= 1;
@@ -386,7 +540,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       }
       if (any_bad) break;
     }
-    if (threadIdx.x == T_EPI_FIRST) bulk_wait_group<0>();
+    if (issuer) bulk_wait_group<0>();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -404,92 +558,67 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 
 }  // namespace
 
-// bf16 row-major [rows, cols], box 64 columns x box_rows rows, 128-byte swizzle (same layout as gemm.cu's operand maps)
-static cudaError_t encode_operand_map(CUtensorMap* out, const void* ptr, long long rows, long long cols, long long ld,
-                                      int box_rows);
-static cudaError_t encode_output_map(CUtensorMap* out, const void* ptr, int fp32, long long groups, long long rows,
-                                     long long cols, long long ld, long long gstride);
-
-typedef CUresult (*EncodeTiledFn2)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn2 encode_fn2() {
-  static EncodeTiledFn2 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn2>(ptr);
-  });
-  return fn;
-}
-
-static cudaError_t encode_operand_map(CUtensorMap* out, const void* ptr, long long rows, long long cols, long long ld,
-                                      int box_rows) {
-  EncodeTiledFn2 enc = encode_fn2();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0 || (ld * 2) % 16 != 0 || cols <= 0 || rows <= 0)
-    return cudaErrorInvalidValue;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estride[2] = {1u, 1u};
-  return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estride,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-             ? cudaSuccess
-             : cudaErrorInvalidValue;
-}
-
-static cudaError_t encode_output_map(CUtensorMap* out, const void* ptr, int fp32, long long groups, long long rows,
-                                     long long cols, long long ld, long long gstride) {
-  EncodeTiledFn2 enc = encode_fn2();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  const long long es = fp32 ? 4 : 2;
-  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(groups)};
-  cuuint64_t gstr[2] = {static_cast<cuuint64_t>(ld * es), static_cast<cuuint64_t>(gstride * es)};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / es), 128u, 1u};
-  cuuint32_t estride[3] = {1u, 1u, 1u};
-  return enc(out, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-             const_cast<void*>(ptr), gdim, gstr, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-             ? cudaSuccess
-             : cudaErrorInvalidValue;
-}
-
 bool gemm_2cta_supported(const GemmArgs& a) {
-  if (a.epilogue != EPI_STORE || a.scatter_row_slot != nullptr || a.pull_row_slot != nullptr ||
-      a.ready_flags != nullptr)
-    return false;
+  if (a.scatter_row_slot != nullptr || a.pull_row_slot != nullptr || a.ready_flags != nullptr) return false;
+  if (a.N % 8 != 0 || a.N <= 0) return false;
+  const auto aligned = [](const void* ptr, long long ld, long long es) {
+    return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0 && (ld * es) % 16 == 0;
+  };
+  const long long es = a.d_fp32 ? 4 : 2;
+  long long gstride = static_cast<long long>(a.M) * a.ldd;
   if (a.mode == GEMM_DENSE) {
-    if (a.a_mn) return false;
+    if (a.a_mn || a.M <= 0) return false;
   } else if (a.mode == GEMM_GROUPED_K) {
-    if (!(a.a_mn && a.b_mn) || (a.group_offsets == nullptr && (a.k_chunk <= 0 || a.k_chunk % 64 != 0))) return false;
+    if (!(a.a_mn && a.b_mn) || (a.group_offsets == nullptr && (a.k_chunk <= 0 || a.k_chunk % 64 != 0)) || a.M <= 0)
+      return false;
+    gstride = a.d_group_stride;
   } else {
-    return false;
+    if (a.pair_tile == nullptr || a.a_mn || a.K <= 0 || a.accumulate) return false;
+    gstride = 0;
+  }
+  if (a.epilogue != EPI_STORE) {
+    if (a.mode != GEMM_GROUPED_M || a.d_fp32 || !aligned(a.D, a.ldd, 2)) return false;
+    if (a.epilogue == EPI_SWIGLU_FWD)
+      return !a.b_mn && a.split_n > 0 && a.ldd >= a.N &&
+             (a.aux_out == nullptr || (aligned(a.aux_out, a.ld_aux_out, 2) && a.ld_aux_out >= 2LL * a.N));
+    return a.epilogue == EPI_SWIGLU_BWD && a.aux_in != nullptr && aligned(a.aux_in, a.ld_aux_in, 2) &&
+           a.ld_aux_in >= 2LL * a.N && a.ldd >= 2LL * a.N;
   }
   if (a.accumulate && !a.d_fp32) return false;
-  if (a.N % 8 != 0 || a.N <= 0 || a.M <= 0) return false;
-  const long long es = a.d_fp32 ? 4 : 2;
-  const long long gstride = a.mode == GEMM_GROUPED_K ? a.d_group_stride : static_cast<long long>(a.M) * a.ldd;
-  return (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 && (a.ldd * es) % 16 == 0 && (gstride * es) % 16 == 0 &&
-         a.ldd >= a.N;
+  return aligned(a.D, a.ldd, es) && (gstride * es) % 16 == 0 && a.ldd >= a.N;
+}
+
+template <int EPI, int GROUPS>
+static cudaError_t launch_pairs(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
+                                const CUtensorMap& tmE, const K2Params& kp, long long clusters, cudaStream_t stream) {
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(gemm2_kernel<EPI, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(GROUPS));
+  if (configured != cudaSuccess) return configured;
+  gemm2_kernel<EPI, GROUPS>
+      <<<static_cast<unsigned>(2 * clusters), t_threads(GROUPS), t_smem(GROUPS), stream>>>(tmA, tmB, tmD, tmE, kp);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   if (!gemm_2cta_supported(a)) return cudaErrorInvalidValue;
-  CUtensorMap tmA, tmB, tmD;
-  cudaError_t e = encode_operand_map(&tmA, a.A, a.a_rows, a.a_cols, a.a_ld, a.a_mn ? 64 : 128);
+  CUtensorMap tmA, tmB, tmD, tmE;
+  cudaError_t e = make_tmap(&tmA, a.A, a.a_rows, a.a_cols, a.a_ld, a.a_mn ? 64 : 128);
   if (e != cudaSuccess) return e;
-  e = encode_operand_map(&tmB, a.B, a.b_rows, a.b_cols, a.b_ld, a.b_mn ? 64 : 128);
+  e = make_tmap(&tmB, a.B, a.b_rows, a.b_cols, a.b_ld, a.b_mn ? 64 : 128);
   if (e != cudaSuccess) return e;
   const long long groups = a.mode == GEMM_GROUPED_K ? a.groups : 1;
-  const long long gstride = a.mode == GEMM_GROUPED_K ? a.d_group_stride : static_cast<long long>(a.M) * a.ldd;
-  e = encode_output_map(&tmD, a.D, a.d_fp32, groups, a.M, a.N, a.ldd, gstride);
+  const long long d_rows = a.mode == GEMM_GROUPED_M ? a.a_rows : a.M;
+  const long long gstride = a.mode == GEMM_GROUPED_K ? a.d_group_stride : d_rows * a.ldd;
+  tmE = tmA;  // placeholder where the epilogue has no second map
+  if (a.epilogue == EPI_STORE) {
+    e = make_tmap_out(&tmD, a.D, a.d_fp32, groups, d_rows, a.N, a.ldd, gstride);
+  } else if (a.epilogue == EPI_SWIGLU_FWD) {
+    e = make_tmap_out(&tmD, a.D, 0, 1, d_rows, a.N, a.ldd, gstride, 64);
+    if (e == cudaSuccess && a.aux_out != nullptr) e = make_tmap_halves(&tmE, a.aux_out, d_rows, a.N, a.ld_aux_out);
+  } else {
+    e = make_tmap(&tmD, a.aux_in, d_rows, 2LL * a.N, a.ld_aux_in, 128, 32);
+    if (e == cudaSuccess) e = make_tmap_halves(&tmE, a.D, d_rows, a.N, a.ldd);
+  }
   if (e != cudaSuccess) return e;
 
   K2Params kp;
@@ -503,6 +632,21 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   kp.group_offsets = a.group_offsets;
   kp.k_chunk = a.k_chunk;
   kp.k_rows = static_cast<int>(a.a_rows);
+  kp.tile_group = a.tile_group;
+  kp.pair_tile = a.pair_tile;
+  kp.num_pairs = a.num_pairs;
+  kp.b_group_rows = static_cast<int>(a.b_group_rows);
+  kp.split_n = a.epilogue == EPI_SWIGLU_FWD ? a.split_n : 0;
+  kp.group_order = a.mode == GEMM_GROUPED_K ? a.group_order : nullptr;
+  // A band of row tiles is walked column by column, and B is read once per band: eight row tiles where B is the larger
+  // operand and a group has that many, four otherwise (a band across several groups reads more of B at a time).
+  // 8 experts x 2048 rows, H 4096, F 14336: first GEMM 3260 -> 3110 us, gradient of the activation 1695 -> 1630;
+  // 833 rows per expert: 755 -> 760.
+  const long long group_rows = a.mode == GEMM_GROUPED_M ? a.rows_per_group : a.M;
+  const long long b_extent = a.epilogue == EPI_SWIGLU_FWD ? 2LL * a.N : a.N;
+  kp.band = b_extent > group_rows && group_rows >= 8 * T_BM ? 8 : 4;
+  kp.cols_per_tile = a.epilogue == EPI_SWIGLU_FWD ? 128 : T_BN;
+  kp.has_aux = a.aux_out != nullptr;
   kp.d_fp32 = a.d_fp32;
   kp.reduce = a.accumulate;
   kp.status = a.status;
@@ -516,19 +660,19 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
     e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
   }
-  const long long m_tiles = (a.M + T_BM - 1) / T_BM, n_tiles = (a.N + T_BN - 1) / T_BN;
-  const long long tiles = m_tiles * n_tiles * groups;
+  // grouped by rows: an expert's last pair may have one tile only, so up to max_m_tiles pairs
+  const long long m_tiles = a.mode == GEMM_GROUPED_M ? a.max_m_tiles : (a.M + T_BM - 1) / T_BM;
+  const long long tiles = m_tiles * ((a.N + kp.cols_per_tile - 1) / kp.cols_per_tile) * groups;
   if (tiles <= 0) return cudaSuccess;
-  long long clusters = num_sms / 2;
-  if (tiles < clusters) clusters = tiles;
-  static bool configured = false;
-  if (!configured) {
-    e = cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T_SMEM);
-    if (e != cudaSuccess) return e;
-    configured = true;
+  const long long clusters = tiles < num_sms / 2 ? tiles : num_sms / 2;
+  switch (a.epilogue) {
+    case EPI_STORE:
+      return launch_pairs<EPI_STORE, 1>(tmA, tmB, tmD, tmE, kp, clusters, stream);
+    case EPI_SWIGLU_FWD:
+      return launch_pairs<EPI_SWIGLU_FWD, 1>(tmA, tmB, tmD, tmE, kp, clusters, stream);
+    default:
+      return launch_pairs<EPI_SWIGLU_BWD, 2>(tmA, tmB, tmD, tmE, kp, clusters, stream);
   }
-  gemm2_kernel<<<static_cast<unsigned>(2 * clusters), T_THREADS, T_SMEM, stream>>>(tmA, tmB, tmD, kp);
-  return cudaGetLastError();
 }
 
 }  // namespace cmoe

@@ -101,6 +101,9 @@ struct MoePlanArgs {
   int* tile_group = nullptr;
   int* num_m_tiles = nullptr;
   int* counts_kept = nullptr;
+  int* pair_tile = nullptr;  // optional, with num_pairs: the tiles in pairs of one expert (GemmArgs::pair_tile), [cap_rows/128]
+  int* num_pairs = nullptr;
+  int* group_order = nullptr;  // optional [n_local]: the experts by descending (padded) rows
   int* scratch = nullptr;
   int* overflow = nullptr;  // optional counter: slots dropped because cap_rows was too small for the routing
 };

@@ -89,9 +89,9 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(const MoePlanArgs a, in
 }
 
 // int words of working storage of one CTA of the ranking kernel: warp counts, slots before this unit, totals, first
-// row of every bin, first row of every expert
+// row of every bin, first row and first tile pair of every expert
 __host__ __device__ inline long long rank_words(int warps, int nbins, int n_local) {
-  return (static_cast<long long>(warps) + 3) * nbins + n_local + 1;
+  return (static_cast<long long>(warps) + 3) * nbins + 2 * (n_local + 1);
 }
 
 // SINGLE: one CTA does everything.  Otherwise CTA u ranks the slots of unit u; `prescanned` says that
@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
   int* s_tot = s_pre + nbins;           // all slots of the bin
   int* s_base = s_tot + nbins;          // first row of the bin
   int* s_goff = s_base + nbins;         // [n_local + 1] first row of the expert
+  int* s_pair = s_goff + a.n_local + 1; // [n_local + 1] first pair of its tiles
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int unit = blockIdx.x;
   const unsigned below = (1u << lane) - 1u;
@@ -192,6 +193,7 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
   const int cap128 = static_cast<int>(a.cap_rows / 128 * 128);
   if (warp == 0) {
     long long carry = 0;
+    int pair_carry = 0;
     for (int e0 = 0; e0 < a.n_local; e0 += 32) {
       const int e = e0 + lane;
       int cnt = 0;
@@ -206,8 +208,16 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
       }
       const long long raw = carry + incl - padded;
       const int off = raw < cap128 ? static_cast<int>(raw) : cap128;
+      const int pairs = ((raw + padded < cap128 ? static_cast<int>(raw) + padded : cap128) - off + 255) / 256;
+      int pincl = pairs;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, pincl, o);
+        if (lane >= o) pincl += v;
+      }
       if (e < a.n_local) {
         s_goff[e] = off;
+        s_pair[e] = pair_carry + pincl - pairs;
         int base = off;
         for (int k = 0; k < kb; ++k) {
           s_base[e * kb + k] = base;
@@ -221,6 +231,7 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
         }
       }
       carry += __shfl_sync(0xffffffffu, incl, 31);
+      pair_carry += __shfl_sync(0xffffffffu, pincl, 31);
     }
     if (lane == 0) {
       const int off = carry < cap128 ? static_cast<int>(carry) : cap128;
@@ -228,6 +239,7 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
       if (unit == 0) {
         a.group_offsets[a.n_local] = off;
         *a.num_m_tiles = off / 128;
+        if (a.num_pairs != nullptr) *a.num_pairs = pair_carry;
       }
     }
   }
@@ -259,6 +271,18 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
       }
     }
   }
+  // the experts by descending rows, equal ones in order
+  if (a.group_order != nullptr) {
+    for (int e = unit * T + tid; e < a.n_local; e += gridDim.x * T) {
+      const int rows = s_goff[e + 1] - s_goff[e];
+      int rank = 0;
+      for (int o = 0; o < a.n_local; ++o) {
+        const int r = s_goff[o + 1] - s_goff[o];
+        rank += r > rows || (r == rows && o < e) ? 1 : 0;
+      }
+      a.group_order[rank] = e;
+    }
+  }
   // expert of every tile, spread over the CTAs
   const int tiles = s_goff[a.n_local] / 128, all_tiles = static_cast<int>((a.cap_rows + 127) / 128);
   for (int t = unit * T + tid; t < all_tiles; t += gridDim.x * T) {
@@ -270,6 +294,10 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
         if (s_goff[mid] <= t * 128) lo = mid; else hi = mid;
       }
       e = lo;
+      if (a.pair_tile != nullptr) {
+        const int in_group = t - s_goff[e] / 128;
+        if ((in_group & 1) == 0) a.pair_tile[s_pair[e] + in_group / 2] = 2 * t + (s_goff[e + 1] <= (t + 1) * 128 ? 1 : 0);
+      }
     }
     a.tile_group[t] = e;
   }

@@ -32,6 +32,7 @@ _SOURCES = [
     "bindings_router.cpp",
     "bindings_moe.cpp",
     "host_ops.cpp",
+    "tensor_maps.cpp",
     "gemm.cu",
     "gemm2.cu",
     "router.cu",
