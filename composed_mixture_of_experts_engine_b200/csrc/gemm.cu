@@ -6,10 +6,11 @@
 // Replaces the per-expert Python loop of three cuBLAS calls in the reference
 // (pkg/distributed/moe_layer.py:197-198, 327-337) with one launch per GEMM of the layer.
 //
-// CTA layout (192 threads, one CTA per SM):
-//   warp 0      TMA producer (one elected lane)
-//   warp 1      TMEM allocation + MMA issue (one lane)
+// CTA layout (224 threads, one CTA per SM):
+//   warp 0      TMA loads of A (one elected thread)
+//   warp 1      TMEM allocation + MMA issue (one elected thread)
 //   warps 2..5  epilogue: each warp owns the TMEM lane quadrant (warp_id % 4)
+//   last warp   TMA loads of B (one elected thread)
 // Tile 128 x 256 x 64, 4 shared-memory stages (48 KiB each), two accumulators of 256 TMEM
 // columns so that the epilogue of tile i overlaps the main loop of tile i+1.
 // Plain results leave through a 32 KiB swizzled staging area and TMA: `cp.async.bulk.tensor` stores, or
@@ -38,8 +39,8 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int CHUNK_BYTES = 64 * BK * 2;  // one 64 x 64 bf16 box (MN-major operands) = 8 KiB
-constexpr int GEMM_THREADS = 192;
-constexpr int GEMM_THREADS_PULL = 320;  // + four row-pull warps (fused expert-parallel dispatch)
+constexpr int GEMM_THREADS = 224;
+constexpr int GEMM_THREADS_PULL = 352;  // + four row-pull warps (fused expert-parallel dispatch)
 constexpr int PULL_SUBS = 4;            // the pull warps fill a 128-row tile in quarters, each with its own ready flag
 constexpr int TMEM_COLS = 2 * BN;  // 512: two accumulators
 constexpr int GROUP_M_SWIZZLE = 8;
@@ -270,7 +271,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -308,67 +309,95 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int n_tiles = (p.N + p.n_cols_per_tile - 1) / p.n_cols_per_tile;
   const int n_total = total_tiles(p, m_tiles, n_tiles);
 
+  const int b_warp = (blockDim.x >> 5) - 1;  // behind the epilogue warps and, where there are any, the pull warps
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    // One elected lane issues the loads.  With the fused row pull the whole warp walks the tiles: lanes 0..3 each
+    // ------------------------------------------------------------------ TMA producer of A
+    // One elected thread issues the loads.  With the fused row pull the whole warp walks the tiles: lanes 0..3 each
     // poll one of the tile's four quarter flags at the same time (one L2 round trip per tile instead of four in a
-    // row, which the four buffered stages hide), then lane 0 goes on alone.
-    const bool pulling = p.pull_row_slot != nullptr;
-    if (lane == 0 || pulling) {
+    // row, which the four buffered stages hide), then one thread goes on alone.
+    int stage = 0;
+    uint32_t phase = 0;
+    auto load_tile = [&](const Tile& ti) {
+      for (int kb = 0; kb < ti.k_blocks; ++kb) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
+        mbar_arrive_expect_tx(&full_bar[stage], A_STAGE_BYTES);
+        uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
+        const int k = ti.a_k0 + kb * BK;
+        if (p.a_mn) {
+          tma_load_2d(a_dst, &tmA, &full_bar[stage], ti.a_mn0, k);
+          tma_load_2d(a_dst + CHUNK_BYTES, &tmA, &full_bar[stage], ti.a_mn0 + 64, k);
+        } else {
+          tma_load_2d(a_dst, &tmA, &full_bar[stage], k, ti.a_mn0);
+        }
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    };
+    if (p.pull_row_slot != nullptr) {
+      for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
+        const Tile ti = decode_tile(p, t, m_tiles, n_tiles);
+        if (ti.skip || ti.k_blocks == 0) continue;
+        // the rows of this tile are written by the pull warps of some CTAs of this launch
+        if (lane < PULL_SUBS) flag_wait_ge_gpu(p.tile_ready + (ti.m0 / BM) * PULL_SUBS + lane, p.pull_epoch, wc);
+        __syncwarp();
+        if (lane == 0) {
+          asm volatile("fence.proxy.async.global;" ::: "memory");  // generic-proxy writes -> TMA reads
+          load_tile(ti);
+        }
+        __syncwarp();
+        if (*abort_flag) break;
+      }
+    } else if (elect_one()) {
+      for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
+        const Tile ti = decode_tile(p, t, m_tiles, n_tiles);
+        if (ti.skip || ti.k_blocks == 0) continue;
+        if (p.ready_flags != nullptr) {
+          const uint32_t* f = p.ready_flags + (long long)ti.group * p.ready_stride;
+          for (int s = 0; s < p.ready_count; ++s) flag_wait_ge(f + s, p.ready_target, wc);
+        }
+        load_tile(ti);
+        if (*abort_flag) break;
+      }
+    }
+  } else if (warp == b_warp) {
+    // ------------------------------------------------------------------ TMA producer of B
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
         const Tile ti = decode_tile(p, t, m_tiles, n_tiles);
         if (ti.skip || ti.k_blocks == 0) continue;
-        if (lane == 0 && p.ready_flags != nullptr) {
-          const uint32_t* f = p.ready_flags + (long long)ti.group * p.ready_stride;
-          for (int s = 0; s < p.ready_count; ++s) flag_wait_ge(f + s, p.ready_target, wc);
-        }
-        if (pulling) {
-          // the rows of this tile are written by the pull warps of some CTAs of this launch
-          if (lane < PULL_SUBS) flag_wait_ge_gpu(p.tile_ready + (ti.m0 / BM) * PULL_SUBS + lane, p.pull_epoch, wc);
-          __syncwarp();
-          if (lane == 0) asm volatile("fence.proxy.async.global;" ::: "memory");  // generic-proxy writes -> TMA reads
-        }
-        if (lane == 0) {
-          for (int kb = 0; kb < ti.k_blocks; ++kb) {
-            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
-            mbar_arrive_expect_tx(&full_bar[stage], STAGE_BYTES);
-            uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
-            uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
-            const int k = kb * BK;
-            if (p.a_mn) {
-              tma_load_2d(a_dst, &tmA, &full_bar[stage], ti.a_mn0, ti.a_k0 + k);
-              tma_load_2d(a_dst + CHUNK_BYTES, &tmA, &full_bar[stage], ti.a_mn0 + 64, ti.a_k0 + k);
-            } else {
-              tma_load_2d(a_dst, &tmA, &full_bar[stage], ti.a_k0 + k, ti.a_mn0);
-            }
-            if (p.b_mn) {
+        for (int kb = 0; kb < ti.k_blocks; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
+          mbar_arrive_expect_tx(&full_bar[stage], B_STAGE_BYTES);
+          uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
+          const int k = ti.b_k0 + kb * BK;
+          if (p.b_mn) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                tma_load_2d(b_dst + j * CHUNK_BYTES, &tmB, &full_bar[stage], ti.b_n0 + 64 * j, ti.b_k0 + k);
-            } else {
-              tma_load_2d(b_dst, &tmB, &full_bar[stage], ti.b_k0 + k, ti.b_n0);
-              tma_load_2d(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], ti.b_k0 + k, ti.b_n1);
-            }
-            if (++stage == STAGES) {
-              stage = 0;
-              phase ^= 1u;
-            }
+            for (int j = 0; j < 4; ++j)
+              tma_load_2d(b_dst + j * CHUNK_BYTES, &tmB, &full_bar[stage], ti.b_n0 + 64 * j, k);
+          } else {
+            tma_load_2d(b_dst, &tmB, &full_bar[stage], k, ti.b_n0);
+            tma_load_2d(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], k, ti.b_n1);
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
           }
         }
-        if (pulling) __syncwarp();
         if (*abort_flag) break;
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
-      const uint32_t a_lbo = p.a_mn ? CHUNK_BYTES : 16;
-      const uint32_t b_lbo = p.b_mn ? CHUNK_BYTES : 16;
-      const uint32_t a_kstep = p.a_mn ? 2048u : 32u;  // bytes per UMMA_K = 16 step
-      const uint32_t b_kstep = p.b_mn ? 2048u : 32u;
+      const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(sA), p.a_mn ? CHUNK_BYTES : 16, 1024);
+      const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sB), p.b_mn ? CHUNK_BYTES : 16, 1024);
+      const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;  // per UMMA_K = 16 step, in descriptor units of 16 bytes
+      const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -387,14 +416,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             atomicMin(p.pull_stamps + 2, global_timer_ns());
             stamped = true;
           }
-          const uint32_t a_addr = smem_u32(sA + stage * A_STAGE_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * B_STAGE_BYTES);
+          const uint64_t ad = a_desc0 + static_cast<uint32_t>(stage * (A_STAGE_BYTES >> 4));
+          const uint64_t bd = b_desc0 + static_cast<uint32_t>(stage * (B_STAGE_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t ad = make_smem_desc_sw128(a_addr + k * a_kstep, a_lbo, 1024);
-            const uint64_t bd = make_smem_desc_sw128(b_addr + k * b_kstep, b_lbo, 1024);
-            umma_bf16_ss(d_tmem, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16_ss(d_tmem, ad + k * a_kstep, bd + k * b_kstep, idesc, (kb | k) != 0 ? 1u : 0u);
           umma_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
           if (++stage == STAGES) {
             stage = 0;

@@ -12,17 +12,22 @@
 // one-CTA kernel).
 // What bounds it: the tensor pipe at the clock that the power limit leaves (1.55 GHz of 1.96 in a capture of the expert
 // GEMMs; pipe active 78 - 84 % of the cycles), so what counts is operand traffic per FLOP and evenly filled SMs.
+// The single threads that load and issue matter as much: a k-block is 512 cycles of MMAs, and an issue loop that rebuilt
+// its descriptors under a `lane == 0` branch needed about 590 (the elected form 250 to 340); a load takes its thread 100 to
+// 200 cycles, so A and B have a warp each.  LM-head GEMMs of 4096 rows, H 2048, 50304 columns, before / after: forward
+// 549 / 509 us, token gradient 568 / 550, weight gradient 600 / 549.
 // Measured on a B200: dense 8192^3 1543 TFLOP/s against 1407 for the one-CTA kernel (cuBLAS in the same run: 1707),
-// grouped weight gradient with fp32 accumulation 1352 against 1144; expert layer of 64 experts, 2048 rows each, H 2048,
-// F 1024, one-CTA / this kernel: first GEMM 869 / 823 us, second 475 / 436, gradient of the activation 513 / 482 (481
-// with two groups of epilogue warps, 497 with one), gradient of the tokens 884 / 838.
+// grouped weight gradient with fp32 accumulation 1352 against 1144 (both with the slower issue loop); expert layer of 64
+// experts, 2048 rows each, H 2048, F 1024, one-CTA kernel / this one / with the faster issue loop: first GEMM 869 / 823 /
+// 781 us, second 475 / 436 / 413, gradient of the activation 513 / 482 / 457 (two groups of epilogue warps; 497 with
+// one, slower loop), gradient of the tokens 884 / 838 / 824.
 //
-// CTA layout (192 threads, 320 with two epilogue groups): warp 0 TMA producer, warp 1 TMEM allocation (both CTAs) + MMA issue (leader only),
-// warps 2.. epilogue of this CTA's 128 rows.  Barriers:
-//   full[s]   in the leader: one arrival with the byte count of both CTAs' loads; both CTAs' TMA loads complete on it
+// CTA layout (224 threads, 352 with two epilogue groups): warp 0 TMA loads of A, the last warp those of B, warp 1 TMEM
+// allocation (both CTAs) + MMA issue (leader only), the others epilogue of this CTA's 128 rows.  Barriers:
+//   full[s]   in the leader: two arrivals (A, B) with the byte counts of both CTAs' loads, which complete on it
 //   empty[s]  in each CTA: the leader's MMA commits to its own and to the peer's barrier
 //   tfull[a]  in each CTA: committed by the leader to both when an accumulator is complete
-//   tempty[a] in the leader: 256 arrivals, the epilogue threads of both CTAs
+//   tempty[a] in the leader: the epilogue threads of both CTAs
 // Every wait is bounded as in gemm.cu; a wait that runs out ends the kernel normally with a status code.
 #include "gemm.cuh"
 
@@ -47,7 +52,7 @@ constexpr int T_MAX_GROUPS = 2;
 constexpr int T_TMEM_COLS = 512;
 // one group of epilogue warps leaves room for six stages, two groups for five
 __host__ __device__ constexpr int t_stages(int groups) { return groups == 1 ? 6 : 5; }
-__host__ __device__ constexpr int t_threads(int groups) { return 64 + 128 * groups; }
+__host__ __device__ constexpr int t_threads(int groups) { return 96 + 128 * groups; }
 __host__ __device__ constexpr int t_smem(int groups) {
   return t_stages(groups) * T_STAGE_BYTES + groups * T_STAGING + 1024 + 256;
 }
@@ -160,10 +165,12 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// arrives once on the barrier at `cluster_addr` (own or peer CTA) when all MMAs issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
-               : "memory");
+// arrives once on the barrier at this shared-memory offset in both CTAs when all MMAs issued so far have completed
+__device__ __forceinline__ void umma_commit_both(uint32_t smem_addr) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
 }
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                   uint32_t accumulate) {
@@ -204,7 +211,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < T_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -239,37 +246,40 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+  if (warp == 0 || warp == 2 + 4 * GROUPS) {
+    // ------------------------------------------------------------------ TMA producers (both CTAs)
+    // One warp loads A, one B: a thread needs 100 - 200 cycles to issue a load, and a k-block has two to four of them.
+    if (elect_one()) {
+      const bool is_a = warp == 0;
+      const CUtensorMap* tm = is_a ? &tmA : &tmB;
+      const bool mn = is_a ? p.a_mn != 0 : p.b_mn != 0;
+      uint8_t* const dst0 = is_a ? sA : sB;
+      const uint32_t fb0 = map_to_cta(smem_u32(full_bar), 0);
+      const int moff = static_cast<int>(cta) * 128;  // this CTA's rows of A
       int stage = 0;
       uint32_t phase = 0;
-      const int moff = static_cast<int>(cta) * 128;  // this CTA's rows of A and its half of B
       for (int r0 = 0; r0 < n_total; r0 += n_clusters) {
         const int t = tile_of_round(p, r0, cluster_id, n_clusters);
         if (t >= n_total) break;  // in the last round only
         const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta));
         if (ti.k_blocks == 0) continue;
-        const bool have_a = leader || !ti.lone;  // the MMA reads this CTA's stale rows; their results are not stored
-        for (int kb = 0; kb < ti.k_blocks; ++kb) {
+        const int x = is_a ? ti.m0 + moff : ti.b_n;
+        int k = is_a ? ti.a_k0 : ti.b_k0;
+        const bool skip = is_a && ti.lone;  // one CTA's rows only; the MMA reads stale ones there, which are not stored
+        const uint32_t bytes = (skip ? 1 : 2) * T_A_BYTES;
+        const bool load = leader || !skip;
+        for (int kb = 0; kb < ti.k_blocks; ++kb, k += T_BK) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
-          const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * T_STAGE_BYTES - (ti.lone ? T_A_BYTES : 0));
-          uint8_t* a_dst = sA + stage * T_A_BYTES;
-          uint8_t* b_dst = sB + stage * T_B_BYTES;
-          const int k = kb * T_BK;
-          if (!have_a) {
-          } else if (p.a_mn) {
-            tma_load_2d_pair(a_dst, &tmA, fb, ti.m0 + moff, ti.a_k0 + k);
-            tma_load_2d_pair(a_dst + T_CHUNK_BYTES, &tmA, fb, ti.m0 + moff + 64, ti.a_k0 + k);
-          } else {
-            tma_load_2d_pair(a_dst, &tmA, fb, ti.a_k0 + k, ti.m0 + moff);
-          }
-          if (p.b_mn) {
-            tma_load_2d_pair(b_dst, &tmB, fb, ti.b_n, ti.b_k0 + k);
-            tma_load_2d_pair(b_dst + T_CHUNK_BYTES, &tmB, fb, ti.b_n + 64, ti.b_k0 + k);
-          } else {
-            tma_load_2d_pair(b_dst, &tmB, fb, ti.b_k0 + k, ti.b_n);
+          const uint32_t fb = fb0 + stage * 8;
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
+          uint8_t* dst = dst0 + stage * T_A_BYTES;
+          if (load) {
+            if (mn) {
+              tma_load_2d_pair(dst, tm, fb, x, k);
+              tma_load_2d_pair(dst + T_CHUNK_BYTES, tm, fb, x + 64, k);
+            } else {
+              tma_load_2d_pair(dst, tm, fb, k, x);
+            }
           }
           if (++stage == T_STAGES) {
             stage = 0;
@@ -281,12 +291,14 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    // The loop body is what one thread issues while the tensor pipe works on 512 cycles' worth of MMAs: the elected
+    // thread is known to be alone (no loop over the lanes around each instruction) and the descriptors only advance.
+    if (leader && elect_one()) {
       const uint32_t idesc = make_idesc_bf16(T_BM, T_BN, p.a_mn, p.b_mn);
-      const uint32_t a_lbo = p.a_mn ? T_CHUNK_BYTES : 16;
-      const uint32_t b_lbo = p.b_mn ? T_CHUNK_BYTES : 16;
-      const uint32_t a_kstep = p.a_mn ? 2048u : 32u;
-      const uint32_t b_kstep = p.b_mn ? 2048u : 32u;
+      const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(sA), p.a_mn ? T_CHUNK_BYTES : 16, 1024);
+      const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sB), p.b_mn ? T_CHUNK_BYTES : 16, 1024);
+      const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;
+      const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -302,26 +314,18 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         for (int kb = 0; kb < ti.k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, wc, ST_TIMEOUT_SMEM_FULL)) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * T_A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * T_B_BYTES);
+          const uint64_t ad = a_desc0 + static_cast<uint32_t>(stage * (T_A_BYTES >> 4));
+          const uint64_t bd = b_desc0 + static_cast<uint32_t>(stage * (T_B_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < T_BK / 16; ++k) {
-            const uint64_t ad = make_smem_desc_sw128(a_addr + k * a_kstep, a_lbo, 1024);
-            const uint64_t bd = make_smem_desc_sw128(b_addr + k * b_kstep, b_lbo, 1024);
-            umma_bf16_ss_pair(d_tmem, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          // the stage is free in both CTAs once these MMAs have read it
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          umma_commit_pair(eb);
-          umma_commit_pair(map_to_cta(eb, 1));
+          for (int k = 0; k < T_BK / 16; ++k)
+            umma_bf16_ss_pair(d_tmem, ad + k * a_kstep, bd + k * b_kstep, idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit_both(smem_u32(&empty_bar[stage]));  // the stage is free in both CTAs once these MMAs have read it
           if (++stage == T_STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        const uint32_t tb = smem_u32(&tfull_bar[acc]);
-        umma_commit_pair(tb);
-        umma_commit_pair(map_to_cta(tb, 1));
+        umma_commit_both(smem_u32(&tfull_bar[acc]));
         if (*abort_flag) break;
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;

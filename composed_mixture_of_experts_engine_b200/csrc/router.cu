@@ -15,6 +15,9 @@
 //     gate weights, which every tile reads whole; the logits meet through distributed shared memory and every CTA
 //     finishes its share of the rows.  (Splitting H instead would add the logits up in another order, and with it
 //     decide near-ties between experts differently for different token counts.);
+//   * every k-block costs its issue: on few tokens the loop over H is as long as single threads need to wait, load and
+//     issue.  The gate weights have a loading warp of their own, two k-blocks share a barrier, and the MMA loop only
+//     advances its descriptors (590 -> 310 cycles per k-block of 64);
 //   * the epilogue runs on 16 warps with four lanes per row over logits in shared memory.  A thread per row straight
 //     out of tensor memory took longer than the GEMM: 54 us of 88 at 8190 tokens, E 256, top-8.
 // Launch to end with a cold L2, first form (128-row tiles, a thread per row) and now: 8190 tokens H 4096 E 256 top-8
@@ -44,8 +47,10 @@ constexpr int RT_BM = 128;
 constexpr int RT_BK = 64;
 constexpr int RT_CHUNK_BYTES = 64 * RT_BK * 2;  // 8 KiB: 64 experts x 64 k
 constexpr int RT_EPI = 512;                     // epilogue threads (warps 2..17)
-constexpr int RT_THREADS = 64 + RT_EPI;
-constexpr int RT_MAX_STAGES = 24;
+constexpr int RT_W_WARP = 2 + RT_EPI / 32;      // the last warp: loads of the gate weights
+constexpr int RT_THREADS = 96 + RT_EPI;
+constexpr int RT_SUB = 2;  // k-blocks of a stage: one wait and one commit for eight MMAs
+constexpr int RT_MAX_STAGES = 12;
 constexpr int RT_SMEM_BUDGET = 200 * 1024;
 
 struct RouterParams {
@@ -124,11 +129,12 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int b_bytes = p.n_chunks * RT_CHUNK_BYTES;
   const int a_bytes = p.rows * RT_BK * 2;
-  const int stage_bytes = a_bytes + b_bytes;
+  const int stage_bytes = RT_SUB * (a_bytes + b_bytes);
   const int SE = rt_row_stride(p.E);
   const int front = max(p.stages * stage_bytes, p.rows * SE * 4);
   float* s_logit = reinterpret_cast<float*>(smem);  // [rows][SE], over the drained pipeline stages
-  uint8_t* sB = smem + p.stages * a_bytes;  // behind all of A: what an MMA reads past a short tile's rows is ours
+  // behind all of A: what an MMA reads past a short tile's rows is ours
+  uint8_t* sB = smem + p.stages * RT_SUB * a_bytes;
   uint8_t* tail = smem + front;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(tail);   // [RT_MAX_STAGES]
   uint64_t* empty_bar = full_bar + RT_MAX_STAGES;           // [RT_MAX_STAGES]
@@ -154,7 +160,7 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     *abort_flag = 0;
     *s_last = 0;
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(tfull_bar, 1);
@@ -179,16 +185,37 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   const int et = static_cast<int>(threadIdx.x) - 64;  // epilogue thread
   const int E = p.E;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = 0; kb < k_blocks; kb += RT_SUB) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
-        mbar_arrive_expect_tx(&full_bar[stage], stage_bytes);
-        uint8_t* b_dst = sB + stage * b_bytes;
-        tma_load_2d(smem + stage * a_bytes, &tmX, &full_bar[stage], kb * RT_BK, static_cast<int>(row0));
-        for (int j = 0; j < p.n_chunks; ++j)
-          tma_load_2d(b_dst + j * RT_CHUNK_BYTES, &tmW, &full_bar[stage], 64 * (rank * p.n_chunks + j), kb * RT_BK);
+        const int sub = min(RT_SUB, k_blocks - kb);
+        mbar_arrive_expect_tx(&full_bar[stage], sub * a_bytes);
+        for (int s = 0; s < sub; ++s)
+          tma_load_2d(smem + (stage * RT_SUB + s) * a_bytes, &tmX, &full_bar[stage], (kb + s) * RT_BK,
+                      static_cast<int>(row0));
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == RT_W_WARP) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < k_blocks; kb += RT_SUB) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
+        const int sub = min(RT_SUB, k_blocks - kb);
+        mbar_arrive_expect_tx(&full_bar[stage], sub * b_bytes);
+        for (int s = 0; s < sub; ++s) {
+          uint8_t* b_dst = sB + (stage * RT_SUB + s) * b_bytes;
+          for (int j = 0; j < p.n_chunks; ++j)
+            tma_load_2d(b_dst + j * RT_CHUNK_BYTES, &tmW, &full_bar[stage], 64 * (rank * p.n_chunks + j),
+                        (kb + s) * RT_BK);
+        }
         if (++stage == p.stages) {
           stage = 0;
           phase ^= 1u;
@@ -197,20 +224,22 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+      const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sB), RT_CHUNK_BYTES, 1024);
       const uint32_t idesc = make_idesc_bf16(RT_BM, p.umma_n, 0, 1);
       int stage = 0;
       uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = 0; kb < k_blocks; kb += RT_SUB) {
         if (!mbar_wait(&full_bar[stage], phase, wc, ST_TIMEOUT_SMEM_FULL)) break;
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(smem + stage * a_bytes);
-        const uint32_t b_addr = smem_u32(sB + stage * b_bytes);
+        const int sub = min(RT_SUB, k_blocks - kb);
+        for (int q = 0; q < sub; ++q) {
+          const uint64_t ad = a_desc0 + static_cast<uint32_t>((stage * RT_SUB + q) * (a_bytes >> 4));
+          const uint64_t bd = b_desc0 + static_cast<uint32_t>((stage * RT_SUB + q) * (b_bytes >> 4));
 #pragma unroll
-        for (int k = 0; k < RT_BK / 16; ++k) {
-          const uint64_t ad = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc_sw128(b_addr + k * 2048, RT_CHUNK_BYTES, 1024);
-          umma_bf16_ss(tmem_base, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < RT_BK / 16; ++k)
+            umma_bf16_ss(tmem_base, ad + k * (32 >> 4), bd + k * (2048 >> 4), idesc, (kb | q | k) != 0 ? 1u : 0u);
         }
         umma_commit(&empty_bar[stage]);
         if (++stage == p.stages) {
@@ -252,7 +281,7 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     rt_cluster_arrive();
     rt_cluster_wait();
   }
-  if (warp >= 2) {
+  if (warp >= 2 && warp != RT_W_WARP) {
     const int R = p.rows / split;  // this CTA finishes the rows [r_lo, r_lo + R) of the tile
     const int r_lo = rank * R;
     if (split == 1) epi_sync();
@@ -280,7 +309,7 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     }
   }
   if (split > 1) rt_cluster_arrive();  // done with the other CTAs' shared memory; waited for before the exit
-  if (warp >= 2) {
+  if (warp >= 2 && warp != RT_W_WARP) {
     const int R = p.rows / split;
     const int r_lo = rank * R;
     const int t = et >> 2, l = et & 3;  // row of this CTA's share, lane of the row
@@ -644,11 +673,11 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   const unsigned tiles = static_cast<unsigned>(tiles_of(p.rows));
   const int e_cta = a.E / p.split;
   p.n_chunks = (e_cta + 63) / 64;
-  const int stage_bytes = p.rows * RT_BK * 2 + p.n_chunks * RT_CHUNK_BYTES;
-  const int k_blocks = (a.H + RT_BK - 1) / RT_BK;
+  const int stage_bytes = RT_SUB * (p.rows * RT_BK * 2 + p.n_chunks * RT_CHUNK_BYTES);
+  const int k_steps = (a.H + RT_SUB * RT_BK - 1) / (RT_SUB * RT_BK);
   int stages = RT_SMEM_BUDGET / stage_bytes;
   if (stages > RT_MAX_STAGES) stages = RT_MAX_STAGES;
-  p.stages = stages < k_blocks ? stages : k_blocks;
+  p.stages = stages < k_steps ? stages : k_steps;
   p.umma_n = ((e_cta + 15) / 16) * 16;
   int cols = 32;
   while (cols < p.umma_n) cols <<= 1;
@@ -675,7 +704,7 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   const int ring = p.stages * stage_bytes;
   int smem = (ring > tile_bytes ? ring : tile_bytes) + 1024 + RT_TABLES;
   // an MMA reads 128 rows of A whatever the tile's rows: the last stage's must end inside this CTA's shared memory
-  const int reach = (p.stages - 1) * p.rows * RT_BK * 2 + RT_BM * RT_BK * 2 + 1024;
+  const int reach = (p.stages * RT_SUB - 1) * p.rows * RT_BK * 2 + RT_BM * RT_BK * 2 + 1024;
   if (smem < reach) smem = reach;
   if (a.E <= 32) return launch_router_variant<1>(tmX, tmW, p, tiles, smem, stream);
   if (a.E <= 64) return launch_router_variant<2>(tmX, tmW, p, tiles, smem, stream);
