@@ -407,6 +407,14 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
         se += __shfl_xor_sync(0xffffffffu, se, 1);
         se += __shfl_xor_sync(0xffffffffu, se, 2);
+        if (p.K == 1) {
+          // the gate weight is 1 whatever the logits: its gradient with respect to them is the rounding of lse and
+          // nothing else, so the sum keeps the order of the experts here, which that rounding has always had
+          __syncwarp();
+          se = 0.f;
+#pragma unroll 8
+          for (int e = 0; e < E; ++e) se += mine[e - l];
+        }
         if (l == 0) {
           const float lse = mx + logf(se);
           if (row_ok && p.lse != nullptr) p.lse[row] = lse;
