@@ -89,6 +89,7 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   g.status = status;
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.epilogue = epilogue;
+  g.b_early = 1;  // weights and row plan are older than the kernel before each of these launches
   // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs 0.85 of the time of a tile (it loads
   // a third less per FLOP) but wastes one of its SMs where an expert has an odd number of tiles, and rounds are counted
   // in whole tiles.  So the rounds of both are estimated, every expert ending in half a tile or pair on average.

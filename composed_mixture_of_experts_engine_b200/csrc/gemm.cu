@@ -24,6 +24,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "launch.h"
 #include "swiglu_epilogue.cuh"
 #include "tensor_maps.h"
 
@@ -97,6 +98,7 @@ struct KParams {
   long long scatter_slots_per_rank;
   PeerTable scatter_out;
   long long scatter_ld;
+  int b_early;     // B does not depend on the kernel before this one
   int out_mode;    // OutMode (EPI_STORE only)
   int fwd_staged;  // SwiGLU forward: h (tmD) and gate|up (tmE) leave through the staging area and TMA stores
   int bwd_staged;  // SwiGLU backward: dGate|dUp (tmE) leave through the piece's own staging buffer and TMA stores
@@ -300,6 +302,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   wc.status = p.status;
   wc.timeout_ns = p.timeout_ns;
 
+  const int b_warp = (blockDim.x >> 5) - 1;  // behind the epilogue warps and, where there are any, the pull warps
+  // what the kernel before this one wrote (or still reads) is touched behind this line only; weights that nobody writes
+  // and the row plan, which is older than that kernel, may be loaded ahead of it
+  if (!(p.b_early && warp == b_warp)) {
+    chain_wait();
+    chain_trigger();
+  }
+
   int m_tiles;
   if (p.mode == GEMM_GROUPED_M) {
     m_tiles = *p.num_m_tiles;
@@ -309,7 +319,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int n_tiles = (p.N + p.n_cols_per_tile - 1) / p.n_cols_per_tile;
   const int n_total = total_tiles(p, m_tiles, n_tiles);
 
-  const int b_warp = (blockDim.x >> 5) - 1;  // behind the epilogue warps and, where there are any, the pull warps
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer of A
     // One elected thread issues the loads.  With the fused row pull the whole warp walks the tiles: lanes 0..3 each
@@ -965,7 +974,9 @@ cudaError_t launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  const int threads = kp.pull_row_slot != nullptr ? GEMM_THREADS_PULL : GEMM_THREADS;
+  if (kp.pull_row_slot == nullptr && kp.scatter_row_slot == nullptr && kp.ready_flags == nullptr)
+    return launch_chained(gemm_kernel<EPI>, grid, GEMM_THREADS, SMEM_BYTES, stream, tmA, tmB, tmD, tmE, kp);
+  const int threads = kp.pull_row_slot != nullptr ? GEMM_THREADS_PULL : GEMM_THREADS;  // exchange with other ranks
   gemm_kernel<EPI><<<grid, threads, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmE, kp);
   return cudaGetLastError();
 }
@@ -1081,6 +1092,7 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.ready_count = a.ready_count;
   kp.ready_target = a.ready_target;
   kp.status = a.status;
+  kp.b_early = a.b_early;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
   kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? 128 : BN;
 

@@ -108,6 +108,10 @@ struct GemmArgs {
   PeerTable scatter_out = {};
   long long scatter_ld = 0;
 
+  // B is not written by the kernel that the stream runs before this launch (nor, with grouped-M, are the tables of the
+  // row plan): its loads may start before that kernel has ended
+  int b_early = 0;
+
   int* status = nullptr;  // device int, set to a StatusCode when a wait ran out
   unsigned long long timeout_ns = 0;  // 0: default
   int num_sms = 0;                    // 0: query the current device

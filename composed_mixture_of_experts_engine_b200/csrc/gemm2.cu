@@ -32,6 +32,7 @@
 #include "gemm.cuh"
 
 #include "common.cuh"
+#include "launch.h"
 #include "swiglu_epilogue.cuh"
 #include "tensor_maps.h"
 
@@ -70,6 +71,7 @@ struct K2Params {
   int band;           // row tiles walked together
   const int* group_order;  // grouped by K: the groups, longest first
   int cols_per_tile;  // output columns of a tile (256; 128 with the SwiGLU forward: gate in one CTA's half of B, up in the other's)
+  int b_early;        // B does not depend on the kernel before this one
   int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
   int* status;
@@ -239,6 +241,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   wc.abort_flag = abort_flag;
   wc.status = p.status;
   wc.timeout_ns = p.timeout_ns;
+
+  // what the kernel before this one wrote (or still reads) is touched behind this line only; weights that nobody writes
+  // and the row plan, which is older than that kernel, may be loaded ahead of it
+  if (!(p.b_early && warp == 2 + 4 * GROUPS)) {
+    chain_wait();
+    chain_trigger();
+  }
 
   const int m_tiles = p.mode == GEMM_GROUPED_M ? *p.num_pairs : (p.M + T_BM - 1) / T_BM;
   const int n_tiles = (p.N + p.cols_per_tile - 1) / p.cols_per_tile;
@@ -598,9 +607,8 @@ static cudaError_t launch_pairs(const CUtensorMap& tmA, const CUtensorMap& tmB, 
   static const cudaError_t configured =
       cudaFuncSetAttribute(gemm2_kernel<EPI, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(GROUPS));
   if (configured != cudaSuccess) return configured;
-  gemm2_kernel<EPI, GROUPS>
-      <<<static_cast<unsigned>(2 * clusters), t_threads(GROUPS), t_smem(GROUPS), stream>>>(tmA, tmB, tmD, tmE, kp);
-  return cudaGetLastError();
+  return launch_chained(gemm2_kernel<EPI, GROUPS>, static_cast<unsigned>(2 * clusters), t_threads(GROUPS),
+                        t_smem(GROUPS), stream, tmA, tmB, tmD, tmE, kp);
 }
 
 cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
@@ -650,6 +658,7 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   const long long b_extent = a.epilogue == EPI_SWIGLU_FWD ? 2LL * a.N : a.N;
   kp.band = b_extent > group_rows && group_rows >= 8 * T_BM ? 8 : 4;
   kp.cols_per_tile = a.epilogue == EPI_SWIGLU_FWD ? 128 : T_BN;
+  kp.b_early = a.b_early;
   kp.has_aux = a.aux_out != nullptr;
   kp.d_fp32 = a.d_fp32;
   kp.reduce = a.accumulate;

@@ -10,6 +10,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 
@@ -56,6 +57,8 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
                                                                  __nv_bfloat16* __restrict__ y,
                                                                  float* __restrict__ rstd, long long rows, int H,
                                                                  float eps) {
+  chain_wait();
+  chain_trigger();
   __shared__ float red[RN_THREADS / 32];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + row * H;
@@ -110,6 +113,8 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
                                                                  __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                                                                  float* __restrict__ dw_partial, long long rows,
                                                                  int H) {
+  chain_wait();
+  chain_trigger();
   __shared__ float red[RN_THREADS / 32];
   extern __shared__ uint4 rn_ring[];  // [stages][x | dy][VEC][RN_THREADS]: every thread's own 16-byte pieces
   constexpr int S = rn_bwd_stages(VEC);
@@ -212,6 +217,8 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
 // leaves the result in row y (only slice y ever touches those rows).  Stage 2, grid (ceil(H / 128)): dw[c] += the
 // `slices` stage-1 rows, again in order.
 __global__ void __launch_bounds__(128) colsum_stage1_kernel(float* __restrict__ partial, int n_rows, int H) {
+  chain_wait();
+  chain_trigger();
   const int c = blockIdx.x * 128 + threadIdx.x;
   if (c >= H) return;
   float s = 0.f;
@@ -221,6 +228,8 @@ __global__ void __launch_bounds__(128) colsum_stage1_kernel(float* __restrict__ 
 }
 __global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* __restrict__ partial, float* __restrict__ dw,
                                                             int slices, int H) {
+  chain_wait();
+  chain_trigger();
   const int c = blockIdx.x * 128 + threadIdx.x;
   if (c >= H) return;
   float s = 0.f;
@@ -233,6 +242,8 @@ __global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* __restr
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ t, const float* __restrict__ cos_tab,
                             const float* __restrict__ sin_tab, long long rows, int seq, int heads, int head_dim,
                             long long row_stride, int inverse) {
+  chain_wait();
+  chain_trigger();
   const int half = head_dim / 2;
   const int vec_per_head = half / 8;
   const long long total = rows * heads * vec_per_head;
@@ -273,6 +284,8 @@ struct QkvGradSrc {
 __global__ void qkv_grad_pack_kernel(QkvGradSrc dq, QkvGradSrc dk, QkvGradSrc dv, __nv_bfloat16* __restrict__ out,
                                      const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
                                      long long rows, int seq, int nh, int nkv, int head_dim) {
+  chain_wait();
+  chain_trigger();
   const int heads = nh + 2 * nkv;
   const int half = head_dim / 2;
   const int vec_per_head = half / 8;
@@ -315,6 +328,8 @@ __global__ void qkv_grad_pack_kernel(QkvGradSrc dq, QkvGradSrc dk, QkvGradSrc dv
 
 // ------------------------------------------------------------------------------------ AdamW
 __global__ void adamw_kernel(const AdamWArgs a) {
+  chain_wait();
+  chain_trigger();
   float gs = a.grad_scale;
   if (a.max_norm > 0.f && a.sumsq != nullptr) {
     const float norm = sqrtf(*a.sumsq);  // sumsq already refers to the scaled gradients
@@ -388,6 +403,8 @@ __global__ void adamw_kernel(const AdamWArgs a) {
 
 __global__ void __launch_bounds__(256) sumsq_kernel(const void* x, int is_bf16, long long n, float* out,
                                                     float* __restrict__ partials) {
+  chain_wait();
+  chain_trigger();
   __shared__ float red[8];
   float acc = 0.f;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -427,6 +444,8 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const void* x, int is_bf16, 
 // out += sum of `n` per-block partial sums, always in the same order (one block, fixed tree)
 __global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restrict__ partials, int n,
                                                           float* __restrict__ out) {
+  chain_wait();
+  chain_trigger();
   __shared__ float red[8];
   float acc = 0.f;
   for (int i = threadIdx.x; i < n; i += 256) acc += partials[i];
@@ -439,6 +458,8 @@ __global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restric
 template <int OUT>  // 0: fp32 store, 1: fp32 add, 2: bf16 store
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float4* __restrict__ part, int parts, long long n4,
                                                             void* __restrict__ out) {
+  chain_wait();
+  chain_trigger();
   const long long i = blockIdx.x * 256ll + threadIdx.x;
   if (i >= n4) return;
   float4 acc = __ldcs(part + i);
@@ -466,6 +487,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
                                                                    float* __restrict__ loss_sum,
                                                                    float* __restrict__ row_loss, long long rows, int V,
                                                                    long long ld, float grad_scale) {
+  chain_wait();
+  chain_trigger();
   __shared__ float red[CE_THREADS / 32];
   __shared__ float s_max, s_sum;
   const long long row = blockIdx.x;
@@ -543,6 +566,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
                                    int slot_div, const float* __restrict__ slot_scale,
                                    __nv_bfloat16* __restrict__ out, long long cap_rows,
                                    const int* __restrict__ num_m_tiles, int H, long long ld_src, long long ld_out) {
+  chain_wait();
+  chain_trigger();
   const long long n_rows = num_m_tiles ? min(static_cast<long long>(*num_m_tiles) * 128, cap_rows) : cap_rows;
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -555,7 +580,15 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
     } else {
       const __nv_bfloat16* s = src + static_cast<long long>(slot / slot_div) * ld_src;
       if (slot_scale == nullptr) {
-        for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = *reinterpret_cast<const uint4*>(s + c);
+        for (int c = lane * 8; c < H; c += 1024) {  // four loads in flight
+          uint4 v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (c + q * 256 < H) v[q] = *reinterpret_cast<const uint4*>(s + c + q * 256);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (c + q * 256 < H) *reinterpret_cast<uint4*>(o + c + q * 256) = v[q];
+        }
       } else {
         const float sc = slot_scale[slot];
         for (int c = lane * 8; c < H; c += 256) {
@@ -573,6 +606,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
 __global__ void combine_rows_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
                                     const float* __restrict__ w, __nv_bfloat16* __restrict__ y, long long n_tokens,
                                     int K, int H, long long ld_rows, long long ld_y) {
+  chain_wait();
+  chain_trigger();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long t = blockIdx.x * static_cast<long long>(warps_per_block) + (threadIdx.x >> 5); t < n_tokens;
@@ -597,15 +632,22 @@ __global__ void combine_rows_kernel(const __nv_bfloat16* __restrict__ rows, cons
 
 // Same sum for a compile-time K: the K (row, weight) pairs of a token are looked up once (lane k loads pair k, the
 // warp shares them by shuffle) and the loads of all K rows of a column block are issued before the first use, so a
-// lane keeps K x 16 bytes in flight instead of 16.  The order of the additions is that of the kernel above.
+// lane keeps K x 16 bytes in flight instead of 16.  The order of the additions is that of the kernel above.  Few
+// tokens are cut into pieces of columns (multiples of 256), one per warp, until the warps fill the GPU: a warp that
+// walks a row of 2048 columns alone waits eight times for memory (64 tokens, top-8: 10.4 us).
 template <int KK>
 __global__ void combine_rows_k_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
                                       const float* __restrict__ w, __nv_bfloat16* __restrict__ y, long long n_tokens,
-                                      int H, long long ld_rows, long long ld_y) {
+                                      int H, long long ld_rows, long long ld_y, int pieces, int piece_cols) {
+  chain_wait();
+  chain_trigger();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
-  for (long long t = blockIdx.x * static_cast<long long>(warps_per_block) + (threadIdx.x >> 5); t < n_tokens;
-       t += static_cast<long long>(gridDim.x) * warps_per_block) {
+  for (long long i = blockIdx.x * static_cast<long long>(warps_per_block) + (threadIdx.x >> 5); i < n_tokens * pieces;
+       i += static_cast<long long>(gridDim.x) * warps_per_block) {
+    const long long t = pieces == 1 ? i : i / pieces;
+    const int c0 = pieces == 1 ? 0 : static_cast<int>(i - t * pieces) * piece_cols;
+    const int c1 = min(H, c0 + piece_cols);
     int my_r = -1;
     float my_w = 0.f;
     if (lane < KK) {
@@ -620,7 +662,7 @@ __global__ void combine_rows_k_kernel(const __nv_bfloat16* __restrict__ rows, co
       wk[k] = __shfl_sync(0xffffffffu, my_w, k);
       src[k] = r >= 0 ? rows + static_cast<long long>(r) * ld_rows : nullptr;
     }
-    for (int c = lane * 8; c < H; c += 256) {
+    for (int c = c0 + lane * 8; c < c1; c += 256) {
       uint4 v[KK];
 #pragma unroll
       for (int k = 0; k < KK; ++k)
@@ -644,6 +686,8 @@ __global__ void combine_rows_k_kernel(const __nv_bfloat16* __restrict__ rows, co
 __global__ void combine_bwd_w_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
                                      const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw, long long n_tokens,
                                      int K, int H, long long ld_rows, long long ld_dy) {
+  chain_wait();
+  chain_trigger();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const long long n_slots = n_tokens * K;
@@ -690,10 +734,10 @@ cudaError_t launch_rmsnorm_fwd(const void* x, const void* w, void* y, float* rst
   auto wb = reinterpret_cast<const __nv_bfloat16*>(w);
   auto yb = reinterpret_cast<__nv_bfloat16*>(y);
   switch (rn_vec_for(H)) {
-    case 1: rmsnorm_fwd_kernel<1><<<grid, RN_THREADS, 0, stream>>>(xb, wb, yb, rstd, rows, H, eps); break;
-    case 2: rmsnorm_fwd_kernel<2><<<grid, RN_THREADS, 0, stream>>>(xb, wb, yb, rstd, rows, H, eps); break;
-    case 4: rmsnorm_fwd_kernel<4><<<grid, RN_THREADS, 0, stream>>>(xb, wb, yb, rstd, rows, H, eps); break;
-    default: rmsnorm_fwd_kernel<8><<<grid, RN_THREADS, 0, stream>>>(xb, wb, yb, rstd, rows, H, eps); break;
+    case 1: launch_chained(rmsnorm_fwd_kernel<1>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
+    case 2: launch_chained(rmsnorm_fwd_kernel<2>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
+    case 4: launch_chained(rmsnorm_fwd_kernel<4>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
+    default: launch_chained(rmsnorm_fwd_kernel<8>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
   }
   return cudaGetLastError();
 }
@@ -718,15 +762,20 @@ cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
     configured = true;
   }
   switch (rn_vec_for(H)) {
-    case 1: rmsnorm_bwd_kernel<1><<<grid, RN_THREADS, rn_bwd_smem(1), stream>>>(dyb, xb, wb, rstd, dxb, dw, dw_partial, rows, H); break;
-    case 2: rmsnorm_bwd_kernel<2><<<grid, RN_THREADS, rn_bwd_smem(2), stream>>>(dyb, xb, wb, rstd, dxb, dw, dw_partial, rows, H); break;
-    case 4: rmsnorm_bwd_kernel<4><<<grid, RN_THREADS, rn_bwd_smem(4), stream>>>(dyb, xb, wb, rstd, dxb, dw, dw_partial, rows, H); break;
-    default: rmsnorm_bwd_kernel<8><<<grid, RN_THREADS, rn_bwd_smem(8), stream>>>(dyb, xb, wb, rstd, dxb, dw, dw_partial, rows, H); break;
+    case 1: launch_chained(rmsnorm_bwd_kernel<1>, grid, RN_THREADS, rn_bwd_smem(1), stream, dyb, xb, wb, rstd, dxb,
+                           dw, dw_partial, rows, H); break;
+    case 2: launch_chained(rmsnorm_bwd_kernel<2>, grid, RN_THREADS, rn_bwd_smem(2), stream, dyb, xb, wb, rstd, dxb,
+                           dw, dw_partial, rows, H); break;
+    case 4: launch_chained(rmsnorm_bwd_kernel<4>, grid, RN_THREADS, rn_bwd_smem(4), stream, dyb, xb, wb, rstd, dxb,
+                           dw, dw_partial, rows, H); break;
+    default: launch_chained(rmsnorm_bwd_kernel<8>, grid, RN_THREADS, rn_bwd_smem(8), stream, dyb, xb, wb, rstd, dxb,
+                            dw, dw_partial, rows, H); break;
   }
   if (dw_partial != nullptr) {
     const unsigned slices = grid < 16u ? grid : 16u;
-    colsum_stage1_kernel<<<dim3((H + 127) / 128, slices), 128, 0, stream>>>(dw_partial, static_cast<int>(grid), H);
-    colsum_stage2_kernel<<<(H + 127) / 128, 128, 0, stream>>>(dw_partial, dw, static_cast<int>(slices), H);
+    launch_chained(colsum_stage1_kernel, dim3((H + 127) / 128, slices), 128, 0, stream, dw_partial,
+                   static_cast<int>(grid), H);
+    launch_chained(colsum_stage2_kernel, (H + 127) / 128, 128, 0, stream, dw_partial, dw, static_cast<int>(slices), H);
   }
   return cudaGetLastError();
 }
@@ -735,8 +784,8 @@ cudaError_t launch_rope(void* t, const float* cos_tab, const float* sin_tab, lon
                         int head_dim, long long row_stride, int inverse, cudaStream_t stream) {
   if (head_dim % 16 != 0 || rows <= 0) return cudaErrorInvalidValue;
   const long long total = rows * heads * (head_dim / 16);
-  rope_kernel<<<grid_for(total, 256, 148 * 16), 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(t), cos_tab, sin_tab,
-                                                                  rows, seq, heads, head_dim, row_stride, inverse);
+  launch_chained(rope_kernel, grid_for(total, 256, 148 * 16), 256, 0, stream, reinterpret_cast<__nv_bfloat16*>(t),
+                 cos_tab, sin_tab, rows, seq, heads, head_dim, row_stride, inverse);
   return cudaGetLastError();
 }
 
@@ -752,15 +801,15 @@ cudaError_t launch_qkv_grad_pack(const void* dq, const long long* dq_strides, co
     if (st[0] % 8 != 0 || st[1] % 8 != 0 || st[2] % 8 != 0) return cudaErrorInvalidValue;  // 16-byte vector loads
   const long long rows = batch * seq;
   const long long total = rows * (nh + 2 * nkv) * (head_dim / 16);
-  qkv_grad_pack_kernel<<<grid_for(total, 256, 148 * 16), 256, 0, stream>>>(
-      mk(dq, dq_strides), mk(dk, dk_strides), mk(dv, dv_strides), reinterpret_cast<__nv_bfloat16*>(out), cos_tab,
-      sin_tab, rows, seq, nh, nkv, head_dim);
+  launch_chained(qkv_grad_pack_kernel, grid_for(total, 256, 148 * 16), 256, 0, stream, mk(dq, dq_strides), mk(dk,
+                 dk_strides), mk(dv, dv_strides), reinterpret_cast<__nv_bfloat16*>(out), cos_tab, sin_tab, rows, seq,
+                 nh, nkv, head_dim);
   return cudaGetLastError();
 }
 
 cudaError_t launch_adamw(const AdamWArgs& a, cudaStream_t stream) {
   if (a.n <= 0) return cudaSuccess;
-  adamw_kernel<<<grid_for(a.n / 4 + 1, 256, 148 * 16), 256, 0, stream>>>(a);
+  launch_chained(adamw_kernel, grid_for(a.n / 4 + 1, 256, 148 * 16), 256, 0, stream, a);
   return cudaGetLastError();
 }
 
@@ -769,8 +818,8 @@ int sumsq_partial_count(long long n) { return n <= 0 ? 0 : static_cast<int>(grid
 cudaError_t launch_sumsq(const void* x, int is_bf16, long long n, float* out, float* partials, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   const unsigned grid = static_cast<unsigned>(sumsq_partial_count(n));
-  sumsq_kernel<<<grid, 256, 0, stream>>>(x, is_bf16, n, out, partials);
-  if (partials != nullptr) sumsq_final_kernel<<<1, 256, 0, stream>>>(partials, static_cast<int>(grid), out);
+  launch_chained(sumsq_kernel, grid, 256, 0, stream, x, is_bf16, n, out, partials);
+  if (partials != nullptr) launch_chained(sumsq_final_kernel, 1, 256, 0, stream, partials, static_cast<int>(grid), out);
   return cudaGetLastError();
 }
 
@@ -781,9 +830,9 @@ cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void
   const long long n4 = n / 4;
   const unsigned grid = static_cast<unsigned>((n4 + 255) / 256);
   const float4* p = reinterpret_cast<const float4*>(part);
-  if (out_bf16) splitk_reduce_kernel<2><<<grid, 256, 0, stream>>>(p, parts, n4, out);
-  else if (accumulate) splitk_reduce_kernel<1><<<grid, 256, 0, stream>>>(p, parts, n4, out);
-  else splitk_reduce_kernel<0><<<grid, 256, 0, stream>>>(p, parts, n4, out);
+  if (out_bf16) launch_chained(splitk_reduce_kernel<2>, grid, 256, 0, stream, p, parts, n4, out);
+  else if (accumulate) launch_chained(splitk_reduce_kernel<1>, grid, 256, 0, stream, p, parts, n4, out);
+  else launch_chained(splitk_reduce_kernel<0>, grid, 256, 0, stream, p, parts, n4, out);
   return cudaGetLastError();
 }
 
@@ -791,8 +840,8 @@ cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* 
                                  long long rows, int V, long long ld, float grad_scale, cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   if (ld % 8 != 0) return cudaErrorInvalidValue;
-  cross_entropy_kernel<<<static_cast<unsigned>(rows), CE_THREADS, 0, stream>>>(
-      reinterpret_cast<__nv_bfloat16*>(logits), targets, loss_sum, row_loss, rows, V, ld, grad_scale);
+  launch_chained(cross_entropy_kernel, static_cast<unsigned>(rows), CE_THREADS, 0, stream,
+                 reinterpret_cast<__nv_bfloat16*>(logits), targets, loss_sum, row_loss, rows, V, ld, grad_scale);
   return cudaGetLastError();
 }
 
@@ -800,9 +849,9 @@ cudaError_t launch_gather_rows(const void* src, const int* row_slot, int slot_di
                                long long cap_rows, const int* num_m_tiles, int H, long long ld_src, long long ld_out,
                                cudaStream_t stream) {
   if (H % 8 != 0 || cap_rows <= 0 || slot_div <= 0) return cudaErrorInvalidValue;
-  gather_rows_kernel<<<grid_for(cap_rows, 8, 148 * 8), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(src), row_slot, slot_div, slot_scale,
-      reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out);
+  launch_chained(gather_rows_kernel, grid_for(cap_rows, 8, 148 * 8), 256, 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(src), row_slot, slot_div, slot_scale,
+                 reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out);
   return cudaGetLastError();
 }
 
@@ -814,29 +863,36 @@ cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const flo
     return v != nullptr && v[0] != '\0' && v[0] != '0';
   }();
   if (!generic_only && (K == 8 || K == 6 || K == 4 || K == 2)) {
-    const unsigned grid = grid_for(n_tokens, 8, 148 * 8);
+    const long long want = 148 * 32 / n_tokens, blocks256 = (H + 255) / 256;
+    const int piece_cols = static_cast<int>(want <= 1 ? blocks256 : (blocks256 + want - 1) / want) * 256;
+    const int pieces = (H + piece_cols - 1) / piece_cols;
+    const unsigned grid = grid_for(n_tokens * pieces, 8, 148 * 8);
     auto rb = reinterpret_cast<const __nv_bfloat16*>(rows);
     auto yb = reinterpret_cast<__nv_bfloat16*>(y);
     switch (K) {
-      case 8: combine_rows_k_kernel<8><<<grid, 256, 0, stream>>>(rb, slot_row, w, yb, n_tokens, H, ld_rows, ld_y); break;
-      case 6: combine_rows_k_kernel<6><<<grid, 256, 0, stream>>>(rb, slot_row, w, yb, n_tokens, H, ld_rows, ld_y); break;
-      case 4: combine_rows_k_kernel<4><<<grid, 256, 0, stream>>>(rb, slot_row, w, yb, n_tokens, H, ld_rows, ld_y); break;
-      default: combine_rows_k_kernel<2><<<grid, 256, 0, stream>>>(rb, slot_row, w, yb, n_tokens, H, ld_rows, ld_y); break;
+      case 8: launch_chained(combine_rows_k_kernel<8>, grid, 256, 0, stream, rb, slot_row, w, yb, n_tokens, H,
+                             ld_rows, ld_y, pieces, piece_cols); break;
+      case 6: launch_chained(combine_rows_k_kernel<6>, grid, 256, 0, stream, rb, slot_row, w, yb, n_tokens, H,
+                             ld_rows, ld_y, pieces, piece_cols); break;
+      case 4: launch_chained(combine_rows_k_kernel<4>, grid, 256, 0, stream, rb, slot_row, w, yb, n_tokens, H,
+                             ld_rows, ld_y, pieces, piece_cols); break;
+      default: launch_chained(combine_rows_k_kernel<2>, grid, 256, 0, stream, rb, slot_row, w, yb, n_tokens, H,
+                              ld_rows, ld_y, pieces, piece_cols); break;
     }
     return cudaGetLastError();
   }
-  combine_rows_kernel<<<grid_for(n_tokens, 8, 148 * 8), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(rows), slot_row, w, reinterpret_cast<__nv_bfloat16*>(y), n_tokens, K, H,
-      ld_rows, ld_y);
+  launch_chained(combine_rows_kernel, grid_for(n_tokens, 8, 148 * 8), 256, 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(rows), slot_row, w, reinterpret_cast<__nv_bfloat16*>(y),
+                 n_tokens, K, H, ld_rows, ld_y);
   return cudaGetLastError();
 }
 
 cudaError_t launch_combine_bwd_w(const void* rows, const int* slot_row, const void* dy, float* dw, long long n_tokens,
                                  int K, int H, long long ld_rows, long long ld_dy, cudaStream_t stream) {
   if (H % 8 != 0 || n_tokens <= 0) return cudaErrorInvalidValue;
-  combine_bwd_w_kernel<<<grid_for(n_tokens * K, 8, 148 * 8), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(rows), slot_row, reinterpret_cast<const __nv_bfloat16*>(dy), dw, n_tokens,
-      K, H, ld_rows, ld_dy);
+  launch_chained(combine_bwd_w_kernel, grid_for(n_tokens * K, 8, 148 * 8), 256, 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(rows), slot_row, reinterpret_cast<const __nv_bfloat16*>(dy),
+                 dw, n_tokens, K, H, ld_rows, ld_dy);
   return cudaGetLastError();
 }
 

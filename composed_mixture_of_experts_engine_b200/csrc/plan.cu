@@ -15,6 +15,7 @@
 #include "ops.cuh"
 
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 
@@ -36,6 +37,8 @@ __device__ __forceinline__ int plan_bin(const MoePlanArgs& a, long long slot) {
 // hist[unit][bin]; also clears the row -> slot table
 __global__ void __launch_bounds__(kCountThreads) plan_count_kernel(const MoePlanArgs a, int nbins, int unit_slots,
                                                                    int in_smem) {
+  chain_wait();
+  chain_trigger();
   extern __shared__ int plan_smem[];
   int* hist = a.scratch + static_cast<long long>(blockIdx.x) * nbins;
   int* h = in_smem ? plan_smem : hist;
@@ -62,6 +65,8 @@ __global__ void __launch_bounds__(kCountThreads) plan_count_kernel(const MoePlan
 // In place: hist[unit][bin] -> sum over the units before it; total[bin] behind the histograms.  A CTA takes 32 bins,
 // its 32 warps a chunk of the units each.
 __global__ void __launch_bounds__(1024) plan_scan_kernel(const MoePlanArgs a, int nbins, int n_units) {
+  chain_wait();
+  chain_trigger();
   __shared__ int part[32][33];
   int* hist = a.scratch;
   int* total = a.scratch + static_cast<long long>(n_units) * nbins;
@@ -100,6 +105,8 @@ __host__ __device__ inline long long rank_words(int warps, int nbins, int n_loca
 template <int WARPS, bool SINGLE>
 __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs a, int nbins, int unit_slots,
                                                                int n_units, int prescanned, int* work) {
+  chain_wait();
+  chain_trigger();
   extern __shared__ int plan_smem[];
   constexpr int T = WARPS * 32;
   int* s_warp = work != nullptr ? work + blockIdx.x * rank_words(WARPS, nbins, a.n_local) : plan_smem;  // [WARPS][nbins]
@@ -339,18 +346,18 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
   if (configured != cudaSuccess) return configured;
   if (s.single) {
     const size_t smem = rank_words(kWarpsSingle, s.nbins, a.n_local) * 4;
-    plan_rank_kernel<kWarpsSingle, true>
-        <<<1, kWarpsSingle * 32, smem, stream>>>(a, s.nbins, s.unit_slots, 1, 0, nullptr);
-    return cudaGetLastError();
+    return launch_chained(plan_rank_kernel<kWarpsSingle, true>, 1, kWarpsSingle * 32, smem, stream, a, s.nbins,
+                          s.unit_slots, 1, 0, nullptr);
   }
   const bool hist_in_smem = s.nbins * 4 <= 48 * 1024;
-  plan_count_kernel<<<s.n_units, kCountThreads, hist_in_smem ? s.nbins * 4 : 0, stream>>>(a, s.nbins, s.unit_slots,
-                                                                                          hist_in_smem ? 1 : 0);
-  if (s.scan) plan_scan_kernel<<<(s.nbins + 31) / 32, 1024, 0, stream>>>(a, s.nbins, s.n_units);
+  cudaError_t e = launch_chained(plan_count_kernel, s.n_units, kCountThreads, hist_in_smem ? s.nbins * 4 : 0, stream, a,
+                                 s.nbins, s.unit_slots, hist_in_smem ? 1 : 0);
+  if (e != cudaSuccess) return e;
+  if (s.scan) e = launch_chained(plan_scan_kernel, (s.nbins + 31) / 32, 1024, 0, stream, a, s.nbins, s.n_units);
+  if (e != cudaSuccess) return e;
   const size_t smem = s.wide ? 0 : rank_words(kWarpsMulti, s.nbins, a.n_local) * 4;
-  plan_rank_kernel<kWarpsMulti, false><<<s.n_units, kWarpsMulti * 32, smem, stream>>>(
-      a, s.nbins, s.unit_slots, s.n_units, s.scan ? 1 : 0, s.wide ? a.scratch + s.hist_words() : nullptr);
-  return cudaGetLastError();
+  return launch_chained(plan_rank_kernel<kWarpsMulti, false>, s.n_units, kWarpsMulti * 32, smem, stream, a, s.nbins,
+                        s.unit_slots, s.n_units, s.scan ? 1 : 0, s.wide ? a.scratch + s.hist_words() : nullptr);
 }
 
 }  // namespace cmoe

@@ -38,6 +38,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 
@@ -176,6 +177,8 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_wait();
+  chain_trigger();
 
   WaitCtx wc;
   wc.abort_flag = abort_flag;
@@ -537,6 +540,8 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 // dense values, and the lane of a pick then overwrites that one value.  A warp per token that compared every expert
 // with every pick was bound by its instructions: 26.6 us at 16384 tokens, E 64, top-8 (6 MB).
 __global__ void __launch_bounds__(256) router_bwd_kernel(const RouterBwdArgs a) {
+  chain_wait();
+  chain_trigger();
   const long long row_raw = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) >> 3;
   const int l = threadIdx.x & 7;
   const bool live = row_raw < a.n_tokens;
@@ -651,12 +656,14 @@ static cudaError_t launch_router_variant(const CUtensorMap& tmX, const CUtensorM
   cfg.blockDim = dim3(RT_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.split;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = p.split;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.split > 1 ? 1 : 0;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, router_fwd_kernel<NG>, tmX, tmW, p);
 }
 
@@ -724,8 +731,7 @@ cudaError_t launch_router_bwd(const RouterBwdArgs& a, cudaStream_t stream) {
   if (a.E <= 0 || a.E > kRouterMaxExperts || a.E % 8 != 0 || a.K <= 0 || a.K > kRouterMaxTopK || a.n_tokens <= 0)
     return cudaErrorInvalidValue;
   const unsigned grid = static_cast<unsigned>((a.n_tokens * 8 + 255) / 256);
-  router_bwd_kernel<<<grid, 256, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(router_bwd_kernel, grid, 256, 0, stream, a);
 }
 
 }  // namespace cmoe
