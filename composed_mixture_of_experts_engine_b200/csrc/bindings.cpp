@@ -314,6 +314,38 @@ void sumsq(const Tensor& x, Tensor& out) {
                                 cur_stream()),
              "sumsq");
 }
+// out (fp32) += scale * x, or out (bf16) = scale * x; scale is a one-element fp32 tensor
+void scaled_out(const Tensor& x, const Tensor& scale, Tensor& out) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const bool add = out.scalar_type() == at::kFloat;
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.is_contiguous() && out.is_contiguous() &&
+                  out.numel() == x.numel() && (add || out.scalar_type() == at::kBFloat16) && x.numel() % 4 == 0,
+              "scaled_out: contiguous fp32 input and fp32 / bf16 output of one size, a multiple of 4");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0,
+              "scaled_out: tensors must start on 16-byte boundaries");
+  TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() == 1, "scaled_out: bad scale");
+  check_cuda(cmoe::launch_scaled_out(x.data_ptr<float>(), scale.data_ptr<float>(), x.numel(), out.data_ptr(), add,
+                                     cur_stream()),
+             "scaled_out");
+}
+
+void embedding_grad(const Tensor& dy, const Tensor& keys, const Tensor& order, Tensor& main) {
+  const c10::cuda::CUDAGuard guard(dy.device());
+  const int64_t n = dy.size(0), H = dy.size(1);
+  TORCH_CHECK(dy.is_cuda() && dy.dim() == 2 && dy.is_contiguous() && dy.scalar_type() == at::kBFloat16 && H % 8 == 0 &&
+                  main.scalar_type() == at::kFloat && main.is_contiguous() && main.dim() == 2 && main.size(1) == H,
+              "embedding_grad: dy contiguous bf16 [n, H], main contiguous fp32 [vocabulary, H], H a multiple of 8");
+  TORCH_CHECK(keys.scalar_type() == at::kLong && order.scalar_type() == at::kLong && keys.is_contiguous() &&
+                  order.is_contiguous() && keys.numel() == n && order.numel() == n,
+              "embedding_grad: keys and order must be contiguous int64 [n]");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(main.data_ptr()) % 16 == 0,
+              "embedding_grad: tensors must start on 16-byte boundaries");
+  check_cuda(cmoe::launch_embedding_grad(dy.data_ptr(), reinterpret_cast<const long long*>(keys.data_ptr<int64_t>()),
+                                         reinterpret_cast<const long long*>(order.data_ptr<int64_t>()),
+                                         main.data_ptr<float>(), n, static_cast<int>(H), cur_stream()),
+             "embedding_grad");
+}
+
 void cross_entropy(Tensor& logits, const Tensor& targets, Tensor& loss_sum, double grad_scale) {
   const c10::cuda::CUDAGuard guard(logits.device());
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.scalar_type() == at::kBFloat16);
@@ -415,6 +447,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("adamw", &adamw);
   m.def("sumsq", &sumsq);
   m.def("cross_entropy", &cross_entropy);
+  m.def("scaled_out", &scaled_out);
+  m.def("embedding_grad", &embedding_grad);
   m.def("moe_plan_scratch_words", &moe_plan_scratch_words);
   m.def("moe_plan", &moe_plan);
   m.def("gather_rows", &gather_rows);

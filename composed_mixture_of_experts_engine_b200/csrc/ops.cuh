@@ -64,6 +64,15 @@ cudaError_t launch_sumsq(const void* x, int is_bf16, long long n, float* out, fl
 cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void* out, int out_bf16, int accumulate,
                                  cudaStream_t stream);
 
+// out[i] += *scale * x[i] (fp32, add != 0) or out[i] = *scale * x[i] rounded to bf16.  n % 4 == 0, 16-byte aligned
+// pointers; scale is a device scalar.
+cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int add, cudaStream_t stream);
+
+// ---- embedding gradient: main[keys[i], :] += dy[order[i], :] for sorted keys (fp32 sums in that order); dy [n, H] bf16
+// and main [vocabulary, H] fp32 are contiguous and start on 16-byte boundaries, H % 8 == 0.
+cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main, long long n,
+                                  int H, cudaStream_t stream);
+
 // ---- cross-entropy, forward and gradient in one pass ------------------------------------------
 // logits [rows, V] bf16 are overwritten with d(loss)/d(logits) = (softmax - onehot) * grad_scale;
 // *loss_sum += sum over rows of the per-row loss (fp32), or, with `row_loss` [rows], the per-row losses are written

@@ -103,6 +103,13 @@ class DecoderBlock(nn.Module):
         return x + y
 
 
+class TokenEmbedding(nn.Embedding):
+    """``nn.Embedding`` whose weight gradient goes straight to the weight's fp32 ``main_grad`` when it has one."""
+
+    def forward(self, ids: torch.Tensor) -> torch.Tensor:
+        return OF.embedding(ids, self.weight)
+
+
 class _LMHeadLossFn(torch.autograd.Function):
     """sum-CE(h @ W^T, targets) * scale without keeping the logits: per chunk of rows one tcgen05 GEMM for the
     logits, the cross-entropy kernel (loss sum, logits overwritten by their gradient), and - only when a gradient
@@ -137,12 +144,17 @@ class _LMHeadLossFn(torch.autograd.Function):
         if dh is not None:
             dh = dh * g.to(dh.dtype)
         if dw is not None:
+            from ..ops import _ext
+
             main = getattr(weight, "main_grad", None)
-            if main is not None:
+            out = torch.empty_like(weight) if main is None else main
+            if dw.numel() % 4 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0:
+                _ext.ext().scaled_out(dw, g.to(torch.float32), out)
+            elif main is not None:
                 main.addcmul_(dw, g.to(torch.float32))
-                dw = None
             else:
-                dw = (dw * g.to(torch.float32)).to(weight.dtype)
+                out.copy_(dw * g.to(torch.float32))
+            dw = out if main is None else None
         return dh, dw, None, None, None
 
 
@@ -166,7 +178,7 @@ class MoEDecoder(nn.Module):
         self.stage_layers = list(partition_layers(m.num_layers, topology.pp_size)[topology.pp_rank])
         self.is_first_stage, self.is_last_stage = topology.is_first_pp_stage(), topology.is_last_pp_stage()
         self.sequence_parallel = bool(cfg.parallelism.sequence_parallel) and topology.tp_size > 1
-        self.embed = nn.Embedding(m.vocab_size, m.hidden_dim, dtype=dtype) if self.is_first_stage else None
+        self.embed = TokenEmbedding(m.vocab_size, m.hidden_dim, dtype=dtype) if self.is_first_stage else None
         self.blocks = nn.ModuleList([DecoderBlock(cfg, topology, dtype) for _ in self.stage_layers])
         self.norm = RMSNorm(m.hidden_dim, eps=m.norm_eps, dtype=dtype) if self.is_last_stage else None
         self.lm_head = nn.Linear(m.hidden_dim, m.vocab_size, bias=False, dtype=dtype) if self.is_last_stage else None

@@ -63,6 +63,36 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.T
     return rmsnorm_reference(x, weight, eps)
 
 
+# ------------------------------------------------------------------------------------------ token embedding
+class _EmbeddingFn(torch.autograd.Function):
+    """Embedding look-up of a weight with an fp32 ``main_grad``: the backward adds the rows of dy to it in the order of
+    the sorted ids (equal ids in token order, so equal inputs give equal bits) instead of filling a dense bf16 gradient
+    that is then added to it."""
+
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids, weight)
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        ids, weight = ctx.saved_tensors
+        main = getattr(weight, "main_grad", None)
+        if main is None or not main.is_contiguous() or main.data_ptr() % 16 != 0:
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, weight.shape[0], -1, False)
+        keys, order = torch.sort(ids.reshape(-1), stable=True)
+        _ext.ext().embedding_grad(rows_for_tma(dy.reshape(-1, dy.shape[-1])), keys, order, main.view(weight.shape))
+        return None, None
+
+
+def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    if (torch.is_grad_enabled() and weight.requires_grad and getattr(weight, "main_grad", None) is not None
+            and on_device_path(weight) and weight.dim() == 2 and weight.shape[1] % 8 == 0 and ids.dtype == torch.int64
+            and ids.numel() > 0):
+        return _EmbeddingFn.apply(ids, weight)
+    return F.embedding(ids, weight)
+
+
 # ------------------------------------------------------------------------------------------ dense linear
 def rows_for_tma(t: torch.Tensor) -> torch.Tensor:
     """``t`` [rows, cols] as a contiguous tensor whose first element sits on a 16-byte boundary (what a TMA
