@@ -27,7 +27,7 @@ int* status_ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr<int>() 
 // The tables of a row plan in one int32 buffer (see MoePlanArgs in ops.cuh for their meaning).
 struct PlanTables {
   int64_t n_slots, cap_rows, E;
-  int64_t row_slot, group_offsets, tile_group, pair_tile, num_pairs, group_order, num_m_tiles, counts_kept, words;  // offsets; slot_row is at 0
+  int64_t row_slot, group_offsets, tile_group, pair_tile, num_pairs, tile_rows, group_order, num_m_tiles, counts_kept, words;  // offsets; slot_row is at 0
   PlanTables(int64_t n_slots_, int64_t E_) : n_slots(n_slots_), E(E_) {
     // worst case of the padded layout: every slot kept, up to 127 padding rows for every expert that has a slot
     cap_rows = (n_slots + std::min(E, n_slots) * 127 + 127) / 128 * 128;
@@ -36,7 +36,8 @@ struct PlanTables {
     tile_group = group_offsets + E + 1;
     pair_tile = tile_group + cap_rows / 128;
     num_pairs = pair_tile + cap_rows / 128;
-    group_order = num_pairs + 1;
+    tile_rows = num_pairs + 1;
+    group_order = tile_rows + cap_rows / 128;
     num_m_tiles = group_order + E;
     counts_kept = num_m_tiles + 1;
     words = counts_kept + E;
@@ -64,7 +65,7 @@ Shapes check_shapes(const Tensor& x, const Tensor& idx32, const Tensor& w13, con
 // a grouped-by-rows launch over the tiles of `plan`: D[rows, N] = A[rows, K] * B (one [b_rows, b_cols] block per expert)
 cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_rows, bool b_mn, const Tensor& D, int64_t N,
                             int64_t K, const PlanTables& pt, int* plan, int* status,
-                            int epilogue = cmoe::EPI_STORE) {
+                            int epilogue = cmoe::EPI_STORE, bool short_tiles = false) {
   cmoe::GemmArgs g;
   g.A = A.data_ptr();
   g.a_rows = A.size(0);
@@ -90,6 +91,10 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.epilogue = epilogue;
   g.b_early = 1;  // weights and row plan are older than the kernel before each of these launches
+  if (short_tiles) {
+    g.tile_rows = plan + pt.tile_rows;
+    return g;
+  }
   // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs 0.85 of the time of a tile (it loads
   // a third less per FLOP) but wastes one of its SMs where an expert has an odd number of tiles, and rounds are counted
   // in whole tiles.  So the rounds of both are estimated, every expert ending in half a tile or pair on average.
@@ -138,6 +143,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
     a.tile_group = plan + pt.tile_group;
     a.pair_tile = plan + pt.pair_tile;
     a.num_pairs = plan + pt.num_pairs;
+    a.tile_rows = plan + pt.tile_rows;
     a.group_order = plan + pt.group_order;
     a.num_m_tiles = plan + pt.num_m_tiles;
     a.counts_kept = plan + pt.counts_kept;
@@ -145,14 +151,20 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
     a.overflow = status_ptr(overflow);
     check(cmoe::launch_moe_plan(a, stream), "moe_plan");
   }
+  // Without a backward pass nobody reads the padding rows, so they are not filled, and where experts have few rows the
+  // GEMMs load and store only the 32-row pieces that hold any: at 64 tokens, E 64 top-8 (8 rows per expert), H 2048,
+  // F 1024 the padding was 33 MB to fill, 400 MB to load from L2 and 50 MB to store, next to 805 MB of weights.  From 64
+  // rows per expert on, most pieces are live and whole tiles take fewer loads.
+  const bool short_tiles = !keep && pt.n_slots <= 64 * s.E;
   Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
   check(cmoe::launch_gather_rows(x.data_ptr(), plan + pt.row_slot, static_cast<int>(s.K), nullptr, xp.data_ptr(),
-                                 pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(s.H), x.stride(0), s.H, stream),
+                                 pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(s.H), x.stride(0), s.H, stream, keep),
         "gather_rows");
   Tensor hact = at::empty({pt.cap_rows, s.F}, bf);
   OptTensor gu;
   {
-    cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status), cmoe::EPI_SWIGLU_FWD);
+    cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status), cmoe::EPI_SWIGLU_FWD,
+                                     short_tiles);
     g.split_n = static_cast<int>(s.F);
     if (keep) {
       gu = at::empty({pt.cap_rows, 2 * s.F}, bf);
@@ -162,7 +174,9 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
     cmoe::launch_gemm_any(g, stream);
   }
   Tensor yp = at::empty({pt.cap_rows, s.H}, bf);
-  cmoe::launch_gemm_any(grouped_rows(hact, w2, s.H, false, yp, s.H, s.F, pt, plan, status_ptr(status)), stream);
+  cmoe::launch_gemm_any(grouped_rows(hact, w2, s.H, false, yp, s.H, s.F, pt, plan, status_ptr(status),
+                                      cmoe::EPI_STORE, short_tiles),
+                         stream);
   Tensor y = at::empty({s.N, s.H}, bf);
   check(cmoe::launch_combine_rows(yp.data_ptr(), plan, gate_w32.data_ptr<float>(), y.data_ptr(), s.N,
                                   static_cast<int>(s.K), static_cast<int>(s.H), s.H, s.H, stream),

@@ -40,6 +40,7 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int CHUNK_BYTES = 64 * BK * 2;  // one 64 x 64 bf16 box (MN-major operands) = 8 KiB
+constexpr int PIECE_ROWS = 32;
 constexpr int GEMM_THREADS = 224;
 constexpr int GEMM_THREADS_PULL = 352;  // + four row-pull warps (fused expert-parallel dispatch)
 constexpr int PULL_SUBS = 4;            // the pull warps fill a 128-row tile in quarters, each with its own ready flag
@@ -65,6 +66,7 @@ struct KParams {
   int b_group_rows, split_n;
   const int* tile_group;
   const int* num_m_tiles;
+  const int* tile_rows;
   const int* group_offsets;
   int k_chunk, k_rows;
   void* D;
@@ -113,6 +115,7 @@ struct Tile {
   int b_n1;      // B K-major: row coordinate of tile rows 128..255
   int b_k0;      // B: first K index (inner coordinate if K-major, row coordinate if N-major)
   int k_blocks;  // number of 64-wide K blocks
+  int pieces;    // 32-row pieces of the tile that are loaded and stored (4 unless the tile's live rows are known)
   bool skip;
 };
 
@@ -123,6 +126,7 @@ __device__ __forceinline__ int total_tiles(const KParams& p, int m_tiles, int n_
 __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles, int n_tiles) {
   Tile ti;
   ti.skip = false;
+  ti.pieces = 4;
   int g = 0;
   if (p.mode == GEMM_GROUPED_K) {
     g = t / (m_tiles * n_tiles);
@@ -148,6 +152,7 @@ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles
   } else if (p.mode == GEMM_GROUPED_M) {
     g = p.tile_group[mt];
     ti.group = g;
+    if (p.tile_rows != nullptr) ti.pieces = (p.tile_rows[mt] + PIECE_ROWS - 1) / PIECE_ROWS;
     if (g < 0) {
       ti.skip = true;
       g = 0;
@@ -329,12 +334,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     auto load_tile = [&](const Tile& ti) {
       for (int kb = 0; kb < ti.k_blocks; ++kb) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
-        mbar_arrive_expect_tx(&full_bar[stage], A_STAGE_BYTES);
+        mbar_arrive_expect_tx(&full_bar[stage], ti.pieces * (A_STAGE_BYTES / 4));
         uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
         const int k = ti.a_k0 + kb * BK;
         if (p.a_mn) {
           tma_load_2d(a_dst, &tmA, &full_bar[stage], ti.a_mn0, k);
           tma_load_2d(a_dst + CHUNK_BYTES, &tmA, &full_bar[stage], ti.a_mn0 + 64, k);
+        } else if (p.tile_rows != nullptr) {
+          // rows beyond stay as the stage was: they only reach rows of the result that nobody reads
+          for (int r = 0; r < ti.pieces; ++r)
+            tma_load_2d(a_dst + r * (A_STAGE_BYTES / 4), &tmA, &full_bar[stage], k, ti.a_mn0 + r * PIECE_ROWS);
         } else {
           tma_load_2d(a_dst, &tmA, &full_bar[stage], k, ti.a_mn0);
         }
@@ -676,7 +685,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
           } else if (threadIdx.x == EPI_FIRST_THREAD) {
             const int zgrp = (p.mode == GEMM_GROUPED_K) ? ti.group : 0;
-            if (p.out_mode == OUT_TMA_REDUCE)
+            if (p.tile_rows != nullptr)
+              for (int r = 0; r < ti.pieces; ++r)
+                tma_store_3d(&tmD, buf + r * (STAGING_BUF_BYTES / 4), col0, ti.m0 + r * PIECE_ROWS, zgrp);
+            else if (p.out_mode == OUT_TMA_REDUCE)
               tma_reduce_add_3d(&tmD, buf, col0, ti.m0, zgrp);  // rows and columns past the edge are clipped
             else
               tma_store_3d(&tmD, buf, col0, ti.m0, zgrp);
@@ -744,10 +756,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           fence_proxy_async_smem();
           asm volatile("bar.sync 1, 128;" ::: "memory");
           if (threadIdx.x == EPI_FIRST_THREAD) {
-            tma_store_3d(&tmD, stg, col, ti.m0, 0);
-            if (p.aux_out != nullptr) {
-              tma_store_3d(&tmE, stg + STAGING_BUF_BYTES / 2, col, 0, ti.m0);  // gate half
-              tma_store_3d(&tmE, stg + STAGING_BUF_BYTES, col, 1, ti.m0);      // up half
+            const int n = p.tile_rows != nullptr ? ti.pieces : 1;
+            for (int r = 0; r < n; ++r) {
+              const int o = r * (STAGING_BUF_BYTES / 8), row = ti.m0 + r * PIECE_ROWS;
+              tma_store_3d(&tmD, stg + o, col, row, 0);
+              if (p.aux_out != nullptr) {
+                tma_store_3d(&tmE, stg + STAGING_BUF_BYTES / 2 + o, col, 0, row);  // gate half
+                tma_store_3d(&tmE, stg + STAGING_BUF_BYTES + o, col, 1, row);      // up half
+              }
             }
             bulk_commit_group();
           }
@@ -991,7 +1007,12 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   if (a.epilogue == EPI_SWIGLU_FWD && (a.b_mn || a.split_n <= 0)) return cudaErrorInvalidValue;
 
   CUtensorMap tmA, tmB;
-  cudaError_t e = make_tmap(&tmA, a.A, a.a_rows, a.a_cols, a.a_ld, a.a_mn ? 64 : 128);
+  const bool short_tiles = a.tile_rows != nullptr;
+  if (short_tiles && (a.mode != GEMM_GROUPED_M || a.pull_row_slot != nullptr || a.scatter_row_slot != nullptr ||
+                      a.accumulate || a.epilogue == EPI_SWIGLU_BWD))
+    return cudaErrorInvalidValue;
+  const int piece_rows = short_tiles ? PIECE_ROWS : BM;
+  cudaError_t e = make_tmap(&tmA, a.A, a.a_rows, a.a_cols, a.a_ld, a.a_mn ? 64 : piece_rows);
   if (e != cudaSuccess) return e;
   e = make_tmap(&tmB, a.B, a.b_rows, a.b_cols, a.b_ld, a.b_mn ? 64 : 128);
   if (e != cudaSuccess) return e;
@@ -1008,6 +1029,7 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.split_n = a.split_n;
   kp.tile_group = a.tile_group;
   kp.num_m_tiles = a.num_m_tiles;
+  kp.tile_rows = a.tile_rows;
   kp.group_offsets = a.group_offsets;
   kp.k_chunk = a.k_chunk;
   kp.k_rows = static_cast<int>(a.a_rows);
@@ -1056,7 +1078,7 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
       const long long gstride = a.mode == GEMM_GROUPED_K ? a.d_group_stride : d_rows * a.ldd;
       const bool aligned = (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 && (a.ldd * es) % 16 == 0 &&
                            (gstride * es) % 16 == 0 && a.ldd >= a.N && d_rows > 0;
-      if (aligned && make_tmap_out(&tmD, a.D, a.d_fp32, groups, d_rows, a.N, a.ldd, gstride) == cudaSuccess)
+      if (aligned && make_tmap_out(&tmD, a.D, a.d_fp32, groups, d_rows, a.N, a.ldd, gstride, 128, piece_rows) == cudaSuccess)
         kp.out_mode = a.accumulate ? OUT_TMA_REDUCE : OUT_TMA_STORE;
     }
   }
@@ -1067,11 +1089,11 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
     // h [rows, N] and the optional gate|up copy [rows, 2N] (as [2 halves, rows, N]) leave through TMA stores
     const long long d_rows = a.mode == GEMM_GROUPED_M ? a.a_rows : a.M;
     bool okmaps = !a.d_fp32 && (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 && (a.ldd * 2) % 16 == 0 && d_rows > 0 &&
-                  make_tmap_out(&tmD, a.D, 0, 1, d_rows, a.N, a.ldd, d_rows * a.ldd, 64) == cudaSuccess;
+                  make_tmap_out(&tmD, a.D, 0, 1, d_rows, a.N, a.ldd, d_rows * a.ldd, 64, piece_rows) == cudaSuccess;
     if (okmaps && a.aux_out != nullptr) {
       okmaps = (reinterpret_cast<uintptr_t>(a.aux_out) & 15u) == 0 && (a.ld_aux_out * 2) % 16 == 0 &&
                a.ld_aux_out >= 2LL * a.N &&
-               make_tmap_halves(&tmE, a.aux_out, d_rows, a.N, a.ld_aux_out) == cudaSuccess;
+               make_tmap_halves(&tmE, a.aux_out, d_rows, a.N, a.ld_aux_out, piece_rows) == cudaSuccess;
     }
     kp.fwd_staged = okmaps ? 1 : 0;
   }

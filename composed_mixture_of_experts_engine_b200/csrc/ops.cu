@@ -625,7 +625,8 @@ __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ row_slot,
                                    int slot_div, const float* __restrict__ slot_scale,
                                    __nv_bfloat16* __restrict__ out, long long cap_rows,
-                                   const int* __restrict__ num_m_tiles, int H, long long ld_src, long long ld_out) {
+                                   const int* __restrict__ num_m_tiles, int H, long long ld_src, long long ld_out,
+                                   int zero_padding) {
   chain_wait();
   chain_trigger();
   const long long n_rows = num_m_tiles ? min(static_cast<long long>(*num_m_tiles) * 128, cap_rows) : cap_rows;
@@ -636,7 +637,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
     const int slot = row_slot[r];
     __nv_bfloat16* o = out + r * ld_out;
     if (slot < 0) {
-      for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = make_uint4(0u, 0u, 0u, 0u);
+      if (zero_padding)
+        for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = make_uint4(0u, 0u, 0u, 0u);
     } else {
       const __nv_bfloat16* s = src + static_cast<long long>(slot / slot_div) * ld_src;
       if (slot_scale == nullptr) {
@@ -927,11 +929,11 @@ cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* 
 
 cudaError_t launch_gather_rows(const void* src, const int* row_slot, int slot_div, const float* slot_scale, void* out,
                                long long cap_rows, const int* num_m_tiles, int H, long long ld_src, long long ld_out,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool zero_padding) {
   if (H % 8 != 0 || cap_rows <= 0 || slot_div <= 0) return cudaErrorInvalidValue;
   launch_chained(gather_rows_kernel, grid_for(cap_rows, 8, 148 * 8), 256, 0, stream,
                  reinterpret_cast<const __nv_bfloat16*>(src), row_slot, slot_div, slot_scale,
-                 reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out);
+                 reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out, zero_padding ? 1 : 0);
   return cudaGetLastError();
 }
 

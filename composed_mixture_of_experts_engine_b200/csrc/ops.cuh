@@ -112,6 +112,7 @@ struct MoePlanArgs {
   int* counts_kept = nullptr;
   int* pair_tile = nullptr;  // optional, with num_pairs: the tiles in pairs of one expert (GemmArgs::pair_tile), [cap_rows/128]
   int* num_pairs = nullptr;
+  int* tile_rows = nullptr;    // optional [cap_rows/128]: live rows of each tile (GemmArgs::tile_rows)
   int* group_order = nullptr;  // optional [n_local]: the experts by descending (padded) rows
   int* scratch = nullptr;
   int* overflow = nullptr;  // optional counter: slots dropped because cap_rows was too small for the routing
@@ -119,11 +120,11 @@ struct MoePlanArgs {
 size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_bins);
 cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream);
 
-// out[r, :] = scale * src[row_slot[r] / slot_div, :]  (zeros where row_slot[r] < 0), for r < *n_rows_dev * 128
+// out[r, :] = scale * src[row_slot[r] / slot_div, :]  (zeros where row_slot[r] < 0, or nothing with !zero_padding), for r < *n_rows_dev * 128
 // (n_rows_dev = num_m_tiles) or r < cap_rows when n_rows_dev is nullptr.  slot_scale (fp32 per slot) optional.
 cudaError_t launch_gather_rows(const void* src, const int* row_slot, int slot_div, const float* slot_scale, void* out,
                                long long cap_rows, const int* num_m_tiles, int H, long long ld_src, long long ld_out,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool zero_padding = true);
 // y[t, :] = sum_k w[t,k] * rows[slot_row[t*K+k], :]  (slots with row -1 skipped), fp32 accumulate, bf16 out
 cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const float* w, void* y, long long n_tokens,
                                 int K, int H, long long ld_rows, long long ld_y, cudaStream_t stream);

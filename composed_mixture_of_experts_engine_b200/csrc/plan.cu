@@ -301,6 +301,12 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
         if (s_goff[mid] <= t * 128) lo = mid; else hi = mid;
       }
       e = lo;
+      if (a.tile_rows != nullptr) {
+        // the rows of an expert are its kept slots, in front of its padding
+        int rows = 0;
+        for (int k = 0; k < kb; ++k) rows += s_tot[e * kb + k];
+        a.tile_rows[t] = max(0, min(128, s_goff[e] + rows - t * 128));
+      }
       if (a.pair_tile != nullptr) {
         const int in_group = t - s_goff[e] / 128;
         if ((in_group & 1) == 0) a.pair_tile[s_pair[e] + in_group / 2] = 2 * t + (s_goff[e + 1] <= (t + 1) * 128 ? 1 : 0);

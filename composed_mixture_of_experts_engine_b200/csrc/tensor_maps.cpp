@@ -54,22 +54,23 @@ cudaError_t make_tmap(CUtensorMap* out, const void* ptr, long long rows, long lo
 }
 
 cudaError_t make_tmap_out(CUtensorMap* out, const void* ptr, int fp32, long long groups, long long rows,
-                          long long cols, long long ld, long long gstride, int box_bytes) {
+                          long long cols, long long ld, long long gstride, int box_bytes, int box_rows) {
   if (box_bytes != 128 && box_bytes != 64) return cudaErrorInvalidValue;
   const long long es = fp32 ? 4 : 2;
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows),
                               static_cast<cuuint64_t>(groups)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld * es), static_cast<cuuint64_t>(gstride * es)};
-  const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_bytes / es), static_cast<cuuint32_t>(kMapTileRows), 1u};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_bytes / es), static_cast<cuuint32_t>(box_rows), 1u};
   return encode(out, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides,
                 box, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                 CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
-cudaError_t make_tmap_halves(CUtensorMap* out, const void* ptr, long long rows, long long n, long long ld) {
+cudaError_t make_tmap_halves(CUtensorMap* out, const void* ptr, long long rows, long long n, long long ld,
+                             int box_rows) {
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(n), 2u, static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(n * 2), static_cast<cuuint64_t>(ld * 2)};
-  const cuuint32_t box[3] = {32u, 1u, static_cast<cuuint32_t>(kMapTileRows)};
+  const cuuint32_t box[3] = {32u, 1u, static_cast<cuuint32_t>(box_rows)};
   return encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B,
                 CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
