@@ -13,14 +13,14 @@
 // What bounds it: the tensor pipe at the clock that the power limit leaves (1.55 GHz of 1.96 in a capture of the expert
 // GEMMs; pipe active 78 - 84 % of the cycles), so what counts is operand traffic per FLOP and evenly filled SMs.
 // The single threads that load and issue matter as much: a k-block is 512 cycles of MMAs, and an issue loop that rebuilt
-// its descriptors under a `lane == 0` branch needed about 590 (the elected form 250 to 340); a load takes its thread 100 to
-// 200 cycles, so A and B have a warp each.  LM-head GEMMs of 4096 rows, H 2048, 50304 columns, before / after: forward
-// 549 / 509 us, token gradient 568 / 550, weight gradient 600 / 549.
+// its descriptors under a `lane == 0` branch needed about 590 (the elected form 250 to 340); a load takes its thread
+// 100 to 200 cycles, so A and B have a warp each.  LM-head GEMMs of 4096 rows, H 2048, 50304 columns, before / after:
+// forward 549 / 509 us, token gradient 568 / 550, weight gradient 600 / 549.
 // Measured on a B200: dense 8192^3 1543 TFLOP/s against 1407 for the one-CTA kernel (cuBLAS in the same run: 1707),
-// grouped weight gradient with fp32 accumulation 1352 against 1144 (both with the slower issue loop); expert layer of 64
-// experts, 2048 rows each, H 2048, F 1024, one-CTA kernel / this one / with the faster issue loop: first GEMM 869 / 823 /
-// 781 us, second 475 / 436 / 413, gradient of the activation 513 / 482 / 457 (two groups of epilogue warps; 497 with
-// one, slower loop), gradient of the tokens 884 / 838 / 824.
+// grouped weight gradient with fp32 accumulation 1352 against 1144 (both with the slower issue loop); expert layer of
+// 64 experts, 2048 rows each, H 2048, F 1024, one-CTA kernel / this one / with the faster issue loop: first GEMM
+// 869 / 823 / 781 us, second 475 / 436 / 413, gradient of the activation 513 / 482 / 457 (two groups of epilogue warps;
+// 497 with one, slower loop), gradient of the tokens 884 / 838 / 824.
 //
 // CTA layout (224 threads, 352 with two epilogue groups): warp 0 TMA loads of A, the last warp those of B, warp 1 TMEM
 // allocation (both CTAs) + MMA issue (leader only), the others epilogue of this CTA's 128 rows.  Barriers:
@@ -70,7 +70,7 @@ struct K2Params {
   int b_group_rows, split_n;
   int band;           // row tiles walked together
   const int* group_order;  // grouped by K: the groups, longest first
-  int cols_per_tile;  // output columns of a tile (256; 128 with the SwiGLU forward: gate in one CTA's half of B, up in the other's)
+  int cols_per_tile;  // output columns of a tile (256; SwiGLU forward 128: gate in one CTA's half of B, up in the other's)
   int b_early;        // B does not depend on the kernel before this one
   int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
