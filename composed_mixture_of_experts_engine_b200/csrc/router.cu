@@ -389,41 +389,42 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
         __syncwarp();
       }
-      // gate weights: lane l takes the picks l and l + 4; the first pick is the row maximum
+      // Softmax statistics; the exponentials replace the logits, and the first pick is the row maximum.  The log-sum-exp
+      // adds them in the order of the experts and the gate weights exp(v - lse) are added in the order of the picks,
+      // whatever the tile, the cluster or the lanes: a last bit of a gate weight moves roundings in all that follows, and
+      // with top-1 routing, where the weight is 1, the rounding of lse is all that its gradient consists of.  All four
+      // lanes add the same E numbers (16-byte reads that they share).
       const float mx = s_topv[t];
-      const float w0 = l < p.K ? expf(s_topv[l * RT_BM + t] - mx) : 0.f;
-      const float w1 = l + 4 < p.K ? expf(s_topv[(l + 4) * RT_BM + t] - mx) : 0.f;
-      float psum = w0 + w1;
-      psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-      psum += __shfl_xor_sync(0xffffffffu, psum, 2);
-      const float inv_psum = 1.f / psum;  // the shuffles above also order every lane's reads before these writes
+#pragma unroll 8
+      for (int j = 0; j < n; ++j) mine[4 * j] = expf(mine[4 * j] - mx);
+      __syncwarp();
+      const float4* ex = reinterpret_cast<const float4*>(mine - l);
+      float se = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const float4 v = ex[j];
+        se += v.x;
+        se += v.y;
+        se += v.z;
+        se += v.w;
+      }
+      const float lse = mx + logf(se);
+      // gate weights: lane l takes the picks l and l + 4
+      const float w0 = l < p.K ? expf(s_topv[l * RT_BM + t] - lse) : 0.f;
+      const float w1 = l + 4 < p.K ? expf(s_topv[(l + 4) * RT_BM + t] - lse) : 0.f;
+      if (l < p.K) s_topv[l * RT_BM + t] = w0;
+      if (l + 4 < p.K) s_topv[(l + 4) * RT_BM + t] = w1;
+      __syncwarp();
+      float psum = 0.f;
+      for (int kk = 0; kk < p.K; ++kk) psum += s_topv[kk * RT_BM + t];
+      const float inv_psum = 1.f / psum;
+      __syncwarp();
       if (l < p.K) s_topv[l * RT_BM + t] = w0 * inv_psum;
       if (l + 4 < p.K) s_topv[(l + 4) * RT_BM + t] = w1 * inv_psum;
-      // softmax statistics; the exponentials replace the logits
-      if (p.stats != nullptr || p.lse != nullptr) {
-        float se = 0.f;
-#pragma unroll 8
-        for (int j = 0; j < n; ++j) {
-          const float ex = expf(mine[4 * j] - mx);
-          mine[4 * j] = ex;
-          se += ex;
-        }
-        se += __shfl_xor_sync(0xffffffffu, se, 1);
-        se += __shfl_xor_sync(0xffffffffu, se, 2);
-        if (p.K == 1) {
-          // the gate weight is 1 whatever the logits: its gradient with respect to them is the rounding of lse and
-          // nothing else, so the sum keeps the order of the experts here, which that rounding has always had
-          __syncwarp();
-          se = 0.f;
-#pragma unroll 8
-          for (int e = 0; e < E; ++e) se += mine[e - l];
-        }
-        if (l == 0) {
-          const float lse = mx + logf(se);
-          if (row_ok && p.lse != nullptr) p.lse[row] = lse;
-          s_inv[t] = row_ok ? 1.f / se : 0.f;
-          s_z[t] = row_ok ? lse * lse : 0.f;
-        }
+      if (l == 0) {
+        if (row_ok && p.lse != nullptr) p.lse[row] = lse;
+        s_inv[t] = row_ok ? 1.f / se : 0.f;
+        s_z[t] = row_ok ? lse * lse : 0.f;
       }
     }
     epi_sync();
