@@ -20,13 +20,20 @@ using OptTensor = std::optional<Tensor>;
 
 // Statistics workspace, zero between launches (the kernel leaves it so).  One per (device, stream): launches on one
 // stream run in order, launches on two streams must not share the accumulators.  At most kMaxWorkspaces are kept
-// (3 KiB each); further streams get a fresh zeroed one per call.
+// (3 KiB each); further streams get a fresh zeroed one per call.  So does a call under capture: a graph may be replayed
+// on any stream, before or beside others that were captured on the same one, and its memory and the zero fill belong to
+// that graph alone.
 constexpr size_t kMaxWorkspaces = 256;
 Tensor router_workspace(const c10::Device& dev, cudaStream_t stream) {
   static std::mutex mu;
-  static std::map<std::pair<int, cudaStream_t>, Tensor> kept;
+  // never destroyed: at exit the allocator may be gone before this table
+  static auto& kept = *new std::map<std::pair<int, cudaStream_t>, Tensor>;
   const auto opt = at::TensorOptions().device(dev).dtype(at::kInt);
   const int64_t words = static_cast<int64_t>(cmoe::router_workspace_words(cmoe::kRouterMaxExperts));
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
+  TORCH_CHECK(e == cudaSuccess, "cmoe: cudaStreamIsCapturing failed: ", cudaGetErrorString(e));
+  if (capturing != cudaStreamCaptureStatusNone) return at::zeros({words}, opt);
   const std::lock_guard<std::mutex> lk(mu);
   const auto key = std::make_pair(static_cast<int>(dev.index()), stream);
   auto it = kept.find(key);
