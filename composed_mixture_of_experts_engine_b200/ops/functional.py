@@ -526,7 +526,7 @@ def local_moe(x: torch.Tensor, gate_w: torch.Tensor, idx: torch.Tensor, w13: tor
         gate_w32, idx32 = gate_w.float().contiguous(), idx.to(torch.int32).contiguous()
         if _local_fused() or debug.enabled():
             return _LocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
-        if torch.is_grad_enabled() and any(t.requires_grad for t in (x, gate_w32, w13, w2)):
+        if kernels.needs_autograd(x, gate_w32, w13, w2):
             return _NativeLocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
         return _native_forward(x, gate_w32, idx32, w13, w2, capacity, False, holder)[0]
     keep = None

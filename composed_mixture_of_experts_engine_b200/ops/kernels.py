@@ -10,6 +10,7 @@ from __future__ import annotations
 from typing import Dict, Optional, Tuple
 
 import torch
+import torch.autograd.forward_ad as _forward_ad
 
 from . import _ext
 
@@ -30,6 +31,20 @@ STATUS_NAMES = {
 
 class KernelTimeoutError(RuntimeError):
     """A bounded wait inside a kernel ran out; the CUDA context is still usable."""
+
+
+def needs_autograd(*tensors: torch.Tensor) -> bool:
+    """Whether a call on ``tensors`` has to go through its autograd function: a gradient is wanted, the call is being
+    traced (the trace would hold a native call's results as constants), or a tensor carries a forward-mode tangent,
+    which the function refuses and a native call would drop.  (``torch.func`` transforms need no look: their wrappers
+    have no storage, so the native calls refuse them too.)"""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return True
+    if torch.jit.is_tracing():
+        return True
+    # no level is open in ordinary calls; unpacking every tensor would cost a small routing call a tenth of its time
+    return (getattr(_forward_ad, "_current_level", 0) >= 0
+            and any(_forward_ad.unpack_dual(t).tangent is not None for t in tensors))
 
 
 _status: Dict[int, torch.Tensor] = {}

@@ -27,7 +27,7 @@ from typing import Any, Dict, Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import _ext
+from . import _ext, kernels
 
 TRITON_AVAILABLE = False  # there is no Triton path in this package
 MIN_TRITON_DIM = 16       # smallest N/H/E for which the reference dispatched its device kernel
@@ -122,9 +122,7 @@ class RouterOutput:
 
 
 def fused_router_forward(tokens: torch.Tensor, gate_w_bf16: torch.Tensor, k: int, timed: bool = False) -> RouterOutput:
-    from .kernels import status_word
-
-    ext, status = _ext.ext(), status_word(tokens.device)
+    ext, status = _ext.ext(), kernels.status_word(tokens.device)
     if not timed:
         return RouterOutput(*ext.router_route(tokens, gate_w_bf16, k, True, status))
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -138,18 +136,12 @@ def _bf16_gate(gate_w: torch.Tensor) -> torch.Tensor:
     return (gate_w if gate_w.dtype == torch.bfloat16 else gate_w.to(torch.bfloat16)).contiguous()
 
 
-def _needs_grad(*tensors: torch.Tensor) -> bool:
-    return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
-
-
 def _fused_router_backward(ctx, tokens, gw16, logits, lse, idx32, counts, grad_w32, grad_w16, grad_aux, grad_z,
                            gate_dtype):
     """(grad_tokens, grad_gate): the analytic d(logits) kernel and the two contractions with it."""
-    from .kernels import status_word
-
     gt, gg = _ext.ext().router_grad(tokens, gw16, logits, lse, idx32, counts, grad_w32, grad_w16, grad_aux, grad_z,
                                     ctx.needs_input_grad[0], ctx.needs_input_grad[1], gate_dtype == torch.bfloat16,
-                                    status_word(tokens.device))
+                                    kernels.status_word(tokens.device))
     return gt, (gg if gg is None or gg.dtype == gate_dtype else gg.to(gate_dtype))
 
 
@@ -230,11 +222,9 @@ def moe_topk_route(tokens: torch.Tensor, gate_w: torch.Tensor, k: int, force_ref
         raise ValueError(f"tokens must be [B,S,H] or [N,H], got shape {list(tokens.shape)}")
     if not (1 <= k <= gate_w.shape[1]):
         raise ValueError(f"k={k} must be in [1, {gate_w.shape[1]}]")
-    if not _needs_grad(tokens, gate_w) and _should_use_fused(tokens, gate_w, force_reference, k):
+    if not kernels.needs_autograd(tokens, gate_w) and _should_use_fused(tokens, gate_w, force_reference, k):
         # no gradient wanted: one native call, one kernel, and only the decision itself is written
-        from .kernels import status_word
-
-        out = _ext.ext().router_route(tokens, _bf16_gate(gate_w), k, False, status_word(tokens.device))
+        out = _ext.ext().router_route(tokens, _bf16_gate(gate_w), k, False, kernels.status_word(tokens.device))
         return out[2], out[3]
     return MoERouterFunction.apply(tokens, gate_w, k, force_reference, None)
 
@@ -347,7 +337,7 @@ class MoERouter(nn.Module):
         E, K = self.num_experts, self.top_k
         fused = self.bias is None and _should_use_fused(tokens, self.gate_w, force_reference, K)
         if fused:
-            if _needs_grad(tokens, self.gate_w):
+            if kernels.needs_autograd(tokens, self.gate_w):
                 holder: Dict[str, Any] = {}
                 w32, w, aux, z, idx32, idx = FusedRouterFunction.apply(tokens, self.gate_w, K, holder,
                                                                        self.profile_timing)
