@@ -340,9 +340,13 @@ void embedding_grad(const Tensor& dy, const Tensor& keys, const Tensor& order, T
               "embedding_grad: keys and order must be contiguous int64 [n]");
   TORCH_CHECK(reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(main.data_ptr()) % 16 == 0,
               "embedding_grad: tensors must start on 16-byte boundaries");
+  const int64_t words = cmoe::embedding_grad_partial_floats(n, static_cast<int>(H));
+  Tensor partial;
+  if (words > 0) partial = at::empty({words}, main.options());
   check_cuda(cmoe::launch_embedding_grad(dy.data_ptr(), reinterpret_cast<const long long*>(keys.data_ptr<int64_t>()),
                                          reinterpret_cast<const long long*>(order.data_ptr<int64_t>()),
-                                         main.data_ptr<float>(), n, static_cast<int>(H), cur_stream()),
+                                         main.data_ptr<float>(), words > 0 ? partial.data_ptr<float>() : nullptr, n,
+                                         static_cast<int>(H), cur_stream()),
              "embedding_grad");
 }
 

@@ -16,10 +16,12 @@ namespace cmoe {
 
 namespace {
 
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
-  const uint4 x = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack8(const uint4& x, float (&f)[8]) {
   const float2 a = unpack_bf16x2(x.x), b = unpack_bf16x2(x.y), c = unpack_bf16x2(x.z), d = unpack_bf16x2(x.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
+  unpack8(*reinterpret_cast<const uint4*>(p), f);
 }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   uint4 o;
@@ -593,31 +595,115 @@ __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* __restric
 }
 
 // ------------------------------------------------------------------------------------ embedding gradient
-// main[keys[i]] += sum over the run of equal keys that starts at i of dy[order[j]], in the order of the run.  A CTA per
-// sorted position; those inside a run leave at once, so every row of main has one writer and a fixed order of additions.
-// What bounds it: dy once and the touched rows of main twice (16384 tokens of 2048: 67 + 268 MB, 50 us at the copy rate).
+// main[keys[i]] += sum over the run of equal keys of dy[order[j]].  Runs are cut at every kEmbSeg sorted positions, a CTA
+// per piece (the CTAs of the other positions leave at once): a piece that is a whole run is added to main directly,
+// pieces of a longer run are written to `partial` (two rows of H per kEmbSeg positions: [0] of a run that comes in from
+// the left, [1] of one that starts here and goes on) and added up, in order, by the join kernel.  So every row of main
+// has one writer and a fixed order of additions, and a token that fills the batch is no longer a chain of dependent reads
+// in one CTA.  What bounds it: dy once and the touched rows of main twice (16384 tokens of 2048, all distinct: 67 +
+// 268 MB, 50 us at the copy rate).
+constexpr int kEmbSeg = 32;  // one ballot finds a piece's end and its source rows
 __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16* __restrict__ dy,
                                                              const long long* __restrict__ keys,
                                                              const long long* __restrict__ order,
-                                                             float* __restrict__ main, long long n, int H) {
+                                                             float* __restrict__ main, float* __restrict__ partial,
+                                                             long long n, int H) {
   chain_wait();
   chain_trigger();
   const long long i = blockIdx.x;
   const long long key = keys[i];
-  if (i > 0 && keys[i - 1] == key) return;
-  for (int c = threadIdx.x * 8; c < H; c += blockDim.x * 8) {
-    float4* m = reinterpret_cast<float4*>(main + key * H + c);
-    const float4 m0 = m[0], m1 = m[1];
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (long long j = i; j < n && keys[j] == key; ++j) {
-      float f[8];
-      load8(dy + order[j] * H + c, f);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] += f[q];
+  const bool from_left = i > 0 && keys[i - 1] == key;
+  if (from_left && i % kEmbSeg != 0) return;
+  const int lane = threadIdx.x & 31;
+  const long long piece_end = min(n, (i / kEmbSeg + 1) * kEmbSeg);
+  const bool same = i + lane < piece_end && keys[i + lane] == key;
+  const unsigned different = ~__ballot_sync(0xffffffffu, same);
+  const int len = different == 0u ? 32 : __ffs(different) - 1;
+  const long long src = same ? order[i + lane] : 0;
+  const bool goes_on = i + len == piece_end && piece_end < n && keys[piece_end] == key;
+  const bool whole = !from_left && !goes_on;
+  float* out = whole ? main + key * H : partial + (i / kEmbSeg * 2 + (from_left ? 0 : 1)) * H;
+  for (int c0 = (threadIdx.x & ~31) * 8; c0 < H; c0 += blockDim.x * 8) {  // whole warps, for the shuffles
+    const int c = c0 + lane * 8;
+    const bool on = c < H;
+    float4* m = reinterpret_cast<float4*>(out + c);
+    float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
+    if (on && whole) {
+      m0 = m[0];
+      m1 = m[1];
     }
-    m[0] = make_float4(m0.x + acc[0], m0.y + acc[1], m0.z + acc[2], m0.w + acc[3]);
-    m[1] = make_float4(m1.x + acc[4], m1.y + acc[5], m1.z + acc[6], m1.w + acc[7]);
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int j = 0; j < len; j += 4) {
+      uint4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long row = __shfl_sync(0xffffffffu, src, (j + q) & 31);
+        if (on && j + q < len) v[q] = *reinterpret_cast<const uint4*>(dy + row * H + c);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (on && j + q < len) {
+          float f[8];
+          unpack8(v[q], f);
+#pragma unroll
+          for (int x = 0; x < 8; ++x) acc[x] += f[x];
+        }
+      }
+    }
+    if (on) {
+      m[0] = make_float4(m0.x + acc[0], m0.y + acc[1], m0.z + acc[2], m0.w + acc[3]);
+      m[1] = make_float4(m1.x + acc[4], m1.y + acc[5], m1.z + acc[6], m1.w + acc[7]);
+    }
+  }
+}
+
+// The runs that cross a multiple of kEmbSeg: main[key] += the sums of their pieces, in order.  A CTA looks through 32
+// pieces for runs that start there and go on and takes 128 columns of each; its eight warps add an eighth of the pieces
+// each, so that a run of 16384 equal ids is 64 additions deep.
+__global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long long* __restrict__ keys,
+                                                                  const float* __restrict__ partial,
+                                                                  float* __restrict__ main, long long n, int H) {
+  chain_wait();
+  chain_trigger();
+  __shared__ float4 sums[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.y * 128 + lane * 4;
+  const long long pieces = (n + kEmbSeg - 1) / kEmbSeg, p0 = blockIdx.x * 32ll;
+  bool mine = false;
+  if ((p0 + lane + 1) * kEmbSeg < n) {
+    const long long first = (p0 + lane) * kEmbSeg, next = first + kEmbSeg;
+    const long long key = keys[next];
+    mine = keys[next - 1] == key && !(first > 0 && keys[first - 1] == key);
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, mine); todo != 0u; todo &= todo - 1u) {  // the same in every warp
+    const long long p = p0 + __ffs(todo) - 1;
+    const long long key = keys[(p + 1) * kEmbSeg];
+    long long lo = p + 1, hi = pieces;  // the last piece whose first position still belongs to the run
+    while (hi - lo > 1) {
+      const long long mid = (lo + hi) >> 1;
+      if (keys[mid * kEmbSeg] == key) lo = mid; else hi = mid;
+    }
+    const long long count = lo - p + 1;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < H) {
+#pragma unroll 8
+      for (long long s = count * warp / 8; s < count * (warp + 1) / 8; ++s) {
+        const float4 v = *reinterpret_cast<const float4*>(partial + ((p + s) * 2 + (s == 0 ? 1 : 0)) * H + c);
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+    }
+    sums[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && c < H) {
+      for (int w = 1; w < 8; ++w) {
+        const float4 v = sums[w][lane];
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+      float4* m = reinterpret_cast<float4*>(main + key * H + c);
+      const float4 v = *m;
+      *m = make_float4(v.x + acc.x, v.y + acc.y, v.z + acc.z, v.w + acc.w);
+    }
+    __syncthreads();
   }
 }
 
@@ -909,13 +995,21 @@ cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, v
                               out);
 }
 
-cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main, long long n,
-                                  int H, cudaStream_t stream) {
+long long embedding_grad_partial_floats(long long n, int H) {
+  return n <= kEmbSeg ? 0 : (n + kEmbSeg - 1) / kEmbSeg * 2 * H;
+}
+
+cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main,
+                                  float* partial, long long n, int H, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  if (H % 8 != 0) return cudaErrorInvalidValue;
+  if (H % 8 != 0 || (n > kEmbSeg && partial == nullptr)) return cudaErrorInvalidValue;
   const int threads = H / 8 >= 256 ? 256 : (H / 8 + 31) / 32 * 32;
-  return launch_chained(embedding_grad_kernel, static_cast<unsigned>(n), threads, 0, stream,
-                        reinterpret_cast<const __nv_bfloat16*>(dy), keys, order, main, n, H);
+  const cudaError_t e = launch_chained(embedding_grad_kernel, static_cast<unsigned>(n), threads, 0, stream,
+                                       reinterpret_cast<const __nv_bfloat16*>(dy), keys, order, main, partial, n, H);
+  if (e != cudaSuccess || n <= kEmbSeg) return e;
+  const long long pieces = (n + kEmbSeg - 1) / kEmbSeg;
+  return launch_chained(embedding_grad_join_kernel, dim3(static_cast<unsigned>((pieces + 31) / 32), (H + 127) / 128), 256,
+                        0, stream, keys, partial, main, n, H);
 }
 
 cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* loss_sum, float* row_loss,

@@ -68,10 +68,12 @@ cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void
 // pointers; scale is a device scalar.
 cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int add, cudaStream_t stream);
 
-// ---- embedding gradient: main[keys[i], :] += dy[order[i], :] for sorted keys (fp32 sums in that order); dy [n, H] bf16
-// and main [vocabulary, H] fp32 are contiguous and start on 16-byte boundaries, H % 8 == 0.
-cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main, long long n,
-                                  int H, cudaStream_t stream);
+// ---- embedding gradient: main[keys[i], :] += dy[order[i], :] for sorted keys (fp32 sums in a fixed order); dy [n, H] bf16,
+// main [vocabulary, H] and the working storage `partial` (embedding_grad_partial_floats words, unless that is 0) fp32 are
+// contiguous and start on 16-byte boundaries, H % 8 == 0.
+long long embedding_grad_partial_floats(long long n, int H);
+cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main,
+                                  float* partial, long long n, int H, cudaStream_t stream);
 
 // ---- cross-entropy, forward and gradient in one pass ------------------------------------------
 // logits [rows, V] bf16 are overwritten with d(loss)/d(logits) = (softmax - onehot) * grad_scale;
