@@ -6,6 +6,12 @@
 // so by the time a kernel starts, everything before its immediate predecessor has completed.  What overlaps is the
 // launch itself and the set-up of barriers, tensor memory and descriptors: 1 to 2 us for each kernel of a chain of
 // short ones.
+//
+// What a predecessor may still be writing must not be read ahead of chain_wait(), neither by the source nor by the
+// compiler.  So kernels that start this way take plain pointers.  `const T* __restrict__` would promise memory that
+// nobody writes while the kernel runs: the compiler could fetch it along the non-coherent path, and in front of the wait,
+// whose memory clobber does not cover such an argument.  Loads through plain pointers stay behind the wait, and so do the
+// caching-hint loads (volatile assembly, like the wait itself).
 #pragma once
 #include <cuda_runtime.h>
 

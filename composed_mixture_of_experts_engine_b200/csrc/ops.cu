@@ -54,10 +54,10 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 constexpr int RN_THREADS = 128;
 
 template <int VEC>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                 const __nv_bfloat16* __restrict__ w,
-                                                                 __nv_bfloat16* __restrict__ y,
-                                                                 float* __restrict__ rstd, long long rows, int H,
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* x,
+                                                                 const __nv_bfloat16* w,
+                                                                 __nv_bfloat16* y,
+                                                                 float* rstd, long long rows, int H,
                                                                  float eps) {
   chain_wait();
   chain_trigger();
@@ -77,13 +77,19 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
     }
     ss = block_sum<RN_THREADS>(ss, red);
     const float r = rsqrtf(ss / H + eps);
+    uint4 wq[VEC];  // all loads ahead of the first store
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      const int c = (i * RN_THREADS + threadIdx.x) * 8;
+      if (c < H) wq[i] = *reinterpret_cast<const uint4*>(w + c);
+    }
     if (threadIdx.x == 0 && rstd) rstd[row] = r;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * RN_THREADS + threadIdx.x) * 8;
       if (c < H) {
         float wv[8], o[8];
-        load8(w + c, wv);
+        unpack8(wq[i], wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = v[i][j] * r * wv[j];
         store8(y + row * H + c, o);
@@ -108,12 +114,12 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 template <int VEC>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                                 const __nv_bfloat16* __restrict__ x,
-                                                                 const __nv_bfloat16* __restrict__ w,
-                                                                 const float* __restrict__ rstd,
-                                                                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
-                                                                 float* __restrict__ dw_partial, long long rows,
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* dy,
+                                                                 const __nv_bfloat16* x,
+                                                                 const __nv_bfloat16* w,
+                                                                 const float* rstd,
+                                                                 __nv_bfloat16* dx, float* dw,
+                                                                 float* dw_partial, long long rows,
                                                                  int H) {
   chain_wait();
   chain_trigger();
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
 // finishes first).  Stage 1, grid (ceil(H / 128), slices): slice y adds the rows y, y + slices, ... in that order and
 // leaves the result in row y (only slice y ever touches those rows).  Stage 2, grid (ceil(H / 128)): dw[c] += the
 // `slices` stage-1 rows, again in order.
-__global__ void __launch_bounds__(128) colsum_stage1_kernel(float* __restrict__ partial, int n_rows, int H) {
+__global__ void __launch_bounds__(128) colsum_stage1_kernel(float* partial, int n_rows, int H) {
   chain_wait();
   chain_trigger();
   const int c = blockIdx.x * 128 + threadIdx.x;
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(128) colsum_stage1_kernel(float* __restrict__ 
   for (int b = blockIdx.y; b < n_rows; b += gridDim.y) s += partial[static_cast<long long>(b) * H + c];  // loads ahead, adds in order
   partial[static_cast<long long>(blockIdx.y) * H + c] = s;
 }
-__global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* __restrict__ partial, float* __restrict__ dw,
+__global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* partial, float* dw,
                                                             int slices, int H) {
   chain_wait();
   chain_trigger();
@@ -241,8 +247,8 @@ __global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* __restr
 }
 
 // ------------------------------------------------------------------------------------ RoPE
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ t, const float* __restrict__ cos_tab,
-                            const float* __restrict__ sin_tab, long long rows, int seq, int heads, int head_dim,
+__global__ void rope_kernel(__nv_bfloat16* t, const float* cos_tab,
+                            const float* sin_tab, long long rows, int seq, int heads, int head_dim,
                             long long row_stride, int inverse) {
   chain_wait();
   chain_trigger();
@@ -283,8 +289,8 @@ struct QkvGradSrc {
   long long sb, sh, ss;  // strides (elements) of batch, head, sequence position
 };
 
-__global__ void qkv_grad_pack_kernel(QkvGradSrc dq, QkvGradSrc dk, QkvGradSrc dv, __nv_bfloat16* __restrict__ out,
-                                     const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
+__global__ void qkv_grad_pack_kernel(QkvGradSrc dq, QkvGradSrc dk, QkvGradSrc dv, __nv_bfloat16* out,
+                                     const float* cos_tab, const float* sin_tab,
                                      long long rows, int seq, int nh, int nkv, int head_dim) {
   chain_wait();
   chain_trigger();
@@ -404,7 +410,7 @@ __global__ void adamw_kernel(const AdamWArgs a) {
 }
 
 __global__ void __launch_bounds__(256) sumsq_kernel(const void* x, int is_bf16, long long n, float* out,
-                                                    float* __restrict__ partials) {
+                                                    float* partials) {
   chain_wait();
   chain_trigger();
   __shared__ float red[8];
@@ -444,8 +450,8 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const void* x, int is_bf16, 
 }
 
 // out += sum of `n` per-block partial sums, always in the same order (one block, fixed tree)
-__global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restrict__ partials, int n,
-                                                          float* __restrict__ out) {
+__global__ void __launch_bounds__(256) sumsq_final_kernel(const float* partials, int n,
+                                                          float* out) {
   chain_wait();
   chain_trigger();
   __shared__ float red[8];
@@ -458,8 +464,8 @@ __global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restric
 // Sum of the partial results of a contraction that was cut into `parts` pieces, always in the same order; the result
 // replaces or is added to fp32, or is rounded once to bf16.
 template <int OUT>  // 0: fp32 store, 1: fp32 add, 2: bf16 store
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float4* __restrict__ part, int parts, long long n4,
-                                                            void* __restrict__ out) {
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float4* part, int parts, long long n4,
+                                                            void* out) {
   chain_wait();
   chain_trigger();
   const long long i = blockIdx.x * 256ll + threadIdx.x;
@@ -484,10 +490,10 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float4* __rest
 
 // ------------------------------------------------------------------------------------ cross-entropy
 constexpr int CE_THREADS = 512;
-__global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
-                                                                   const long long* __restrict__ targets,
-                                                                   float* __restrict__ loss_sum,
-                                                                   float* __restrict__ row_loss, long long rows, int V,
+__global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* logits,
+                                                                   const long long* targets,
+                                                                   float* loss_sum,
+                                                                   float* row_loss, long long rows, int V,
                                                                    long long ld, float grad_scale) {
   chain_wait();
   chain_trigger();
@@ -566,8 +572,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
 // out (fp32) += *scale * x, or out (bf16) = *scale * x.  One pass over each; what bounds it is those passes.  Library
 // operations took a multiply, a cast and a temporary for the second, and 361 us for 103 M elements of the first.
 template <bool ADD>
-__global__ void __launch_bounds__(256) scaled_out_kernel(const float4* __restrict__ x, const float* __restrict__ scale,
-                                                         long long n4, void* __restrict__ out) {
+__global__ void __launch_bounds__(256) scaled_out_kernel(const float4* x, const float* scale,
+                                                         long long n4, void* out) {
   chain_wait();
   chain_trigger();
   const float s = *scale;
@@ -603,10 +609,10 @@ __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* __restric
 // in one CTA.  What bounds it: dy once and the touched rows of main twice (16384 tokens of 2048, all distinct: 67 +
 // 268 MB, 50 us at the copy rate).
 constexpr int kEmbSeg = 32;  // one ballot finds a piece's end and its source rows
-__global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                             const long long* __restrict__ keys,
-                                                             const long long* __restrict__ order,
-                                                             float* __restrict__ main, float* __restrict__ partial,
+__global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16* dy,
+                                                             const long long* keys,
+                                                             const long long* order,
+                                                             float* main, float* partial,
                                                              long long n, int H) {
   chain_wait();
   chain_trigger();
@@ -660,9 +666,9 @@ __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16
 // The runs that cross a multiple of kEmbSeg: main[key] += the sums of their pieces, in order.  A CTA looks through 32
 // pieces for runs that start there and go on and takes 128 columns of each; its eight warps add an eighth of the pieces
 // each, so that a run of 16384 equal ids is 64 additions deep.
-__global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long long* __restrict__ keys,
-                                                                  const float* __restrict__ partial,
-                                                                  float* __restrict__ main, long long n, int H) {
+__global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long long* keys,
+                                                                  const float* partial,
+                                                                  float* main, long long n, int H) {
   chain_wait();
   chain_trigger();
   __shared__ float4 sums[8][32];
@@ -708,10 +714,10 @@ __global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long lon
 }
 
 // ------------------------------------------------------------------------------------ gather / combine
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ row_slot,
-                                   int slot_div, const float* __restrict__ slot_scale,
-                                   __nv_bfloat16* __restrict__ out, long long cap_rows,
-                                   const int* __restrict__ num_m_tiles, int H, long long ld_src, long long ld_out,
+__global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot,
+                                   int slot_div, const float* slot_scale,
+                                   __nv_bfloat16* out, long long cap_rows,
+                                   const int* num_m_tiles, int H, long long ld_src, long long ld_out,
                                    int zero_padding) {
   chain_wait();
   chain_trigger();
@@ -751,8 +757,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
   }
 }
 
-__global__ void combine_rows_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
-                                    const float* __restrict__ w, __nv_bfloat16* __restrict__ y, long long n_tokens,
+__global__ void combine_rows_kernel(const __nv_bfloat16* rows, const int* slot_row,
+                                    const float* w, __nv_bfloat16* y, long long n_tokens,
                                     int K, int H, long long ld_rows, long long ld_y) {
   chain_wait();
   chain_trigger();
@@ -784,8 +790,8 @@ __global__ void combine_rows_kernel(const __nv_bfloat16* __restrict__ rows, cons
 // tokens are cut into pieces of columns (multiples of 256), one per warp, until the warps fill the GPU: a warp that
 // walks a row of 2048 columns alone waits eight times for memory (64 tokens, top-8: 10.4 us).
 template <int KK>
-__global__ void combine_rows_k_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
-                                      const float* __restrict__ w, __nv_bfloat16* __restrict__ y, long long n_tokens,
+__global__ void combine_rows_k_kernel(const __nv_bfloat16* rows, const int* slot_row,
+                                      const float* w, __nv_bfloat16* y, long long n_tokens,
                                       int H, long long ld_rows, long long ld_y, int pieces, int piece_cols) {
   chain_wait();
   chain_trigger();
@@ -831,8 +837,8 @@ __global__ void combine_rows_k_kernel(const __nv_bfloat16* __restrict__ rows, co
   }
 }
 
-__global__ void combine_bwd_w_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ slot_row,
-                                     const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw, long long n_tokens,
+__global__ void combine_bwd_w_kernel(const __nv_bfloat16* rows, const int* slot_row,
+                                     const __nv_bfloat16* dy, float* dw, long long n_tokens,
                                      int K, int H, long long ld_rows, long long ld_dy) {
   chain_wait();
   chain_trigger();
