@@ -8,7 +8,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <optional>
+#include <string>
 #include <tuple>
 
 #include "host_ops.h"
@@ -110,47 +112,76 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   return g;
 }
 
+// The row plan of `idx32` [N, K] over all E experts; capacity > 0: slots kept per (expert, k)
+Tensor build_plan(const Tensor& idx32, int64_t E, int64_t capacity, const OptTensor& overflow, cudaStream_t stream) {
+  const PlanTables pt(idx32.numel(), E);
+  const int K = static_cast<int>(idx32.size(1)), per_k = capacity > 0;
+  Tensor plan_t = at::empty({pt.words}, idx32.options());
+  Tensor scratch = at::empty(
+      {static_cast<int64_t>(cmoe::moe_plan_scratch_words(pt.n_slots, static_cast<int>(E), K, per_k))}, idx32.options());
+  int* plan = plan_t.data_ptr<int>();
+  cmoe::MoePlanArgs a;
+  a.topk_idx = idx32.data_ptr<int>();
+  a.n_slots = pt.n_slots;
+  a.K = K;
+  a.num_experts = a.n_local = static_cast<int>(E);
+  a.per_k_bins = per_k;
+  a.capacity = static_cast<int>(capacity);
+  a.cap_rows = pt.cap_rows;
+  a.slot_row = plan;
+  a.row_slot = plan + pt.row_slot;
+  a.group_offsets = plan + pt.group_offsets;
+  a.tile_group = plan + pt.tile_group;
+  a.pair_tile = plan + pt.pair_tile;
+  a.num_pairs = plan + pt.num_pairs;
+  a.tile_rows = plan + pt.tile_rows;
+  a.group_order = plan + pt.group_order;
+  a.num_m_tiles = plan + pt.num_m_tiles;
+  a.counts_kept = plan + pt.counts_kept;
+  a.scratch = scratch.data_ptr<int>();
+  a.overflow = status_ptr(overflow);
+  check(cmoe::launch_moe_plan(a, stream), "moe_plan");
+  return plan_t;
+}
+// ... as a call of its own, and its tables by name (views), for checks between the plan and the kernels that read it
+Tensor moe_local_plan(const Tensor& idx32, int64_t E, int64_t capacity, const OptTensor& overflow) {
+  TORCH_CHECK(idx32.is_cuda() && idx32.scalar_type() == at::kInt && idx32.dim() == 2 && idx32.is_contiguous(),
+              "idx must be contiguous int32 [N, K]");
+  const c10::cuda::CUDAGuard guard(idx32.device());
+  return build_plan(idx32, E, capacity, overflow, at::cuda::getCurrentCUDAStream().stream());
+}
+std::map<std::string, Tensor> moe_local_tables(const Tensor& plan, int64_t n_slots, int64_t E) {
+  const PlanTables pt(n_slots, E);
+  TORCH_CHECK(plan.dim() == 1 && plan.numel() == pt.words, "the row plan belongs to another layer call");
+  const int64_t tiles = pt.cap_rows / 128;
+  const auto part = [&](int64_t at, int64_t n) { return plan.narrow(0, at, n); };
+  return {{"slot_row", part(0, n_slots)},
+          {"row_slot", part(pt.row_slot, pt.cap_rows)},
+          {"group_offsets", part(pt.group_offsets, E + 1)},
+          {"tile_group", part(pt.tile_group, tiles)},
+          {"pair_tile", part(pt.pair_tile, tiles)},
+          {"num_pairs", part(pt.num_pairs, 1)},
+          {"tile_rows", part(pt.tile_rows, tiles)},
+          {"group_order", part(pt.group_order, E)},
+          {"num_m_tiles", part(pt.num_m_tiles, 1)},
+          {"counts_kept", part(pt.counts_kept, E)}};
+}
+
 // (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads)
 using Forward = std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor>;
 Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
                           const Tensor& w2, int64_t capacity, bool keep, const OptTensor& status,
-                          const OptTensor& overflow) {
+                          const OptTensor& overflow, const OptTensor& made_plan) {
   const c10::cuda::CUDAGuard guard(x.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
   const Shapes s = check_shapes(x, idx32, w13, w2);
   TORCH_CHECK(gate_w32.scalar_type() == at::kFloat && gate_w32.is_contiguous() && gate_w32.numel() == s.N * s.K,
               "gate weights must be contiguous fp32 [N, K]");
   const PlanTables pt(s.N * s.K, s.E);
-  const auto i32 = x.options().dtype(at::kInt), bf = x.options();
-  Tensor plan_t = at::empty({pt.words}, i32);
+  const auto bf = x.options();
+  const Tensor plan_t = made_plan.has_value() ? *made_plan : build_plan(idx32, s.E, capacity, overflow, stream);
+  TORCH_CHECK(plan_t.scalar_type() == at::kInt && plan_t.numel() == pt.words, "the row plan belongs to another layer call");
   int* plan = plan_t.data_ptr<int>();
-  {
-    const int per_k = capacity > 0;
-    Tensor scratch = at::empty(
-        {static_cast<int64_t>(cmoe::moe_plan_scratch_words(pt.n_slots, static_cast<int>(s.E), static_cast<int>(s.K), per_k))},
-        i32);
-    cmoe::MoePlanArgs a;
-    a.topk_idx = idx32.data_ptr<int>();
-    a.n_slots = pt.n_slots;
-    a.K = static_cast<int>(s.K);
-    a.num_experts = a.n_local = static_cast<int>(s.E);
-    a.per_k_bins = per_k;
-    a.capacity = static_cast<int>(capacity);
-    a.cap_rows = pt.cap_rows;
-    a.slot_row = plan;
-    a.row_slot = plan + pt.row_slot;
-    a.group_offsets = plan + pt.group_offsets;
-    a.tile_group = plan + pt.tile_group;
-    a.pair_tile = plan + pt.pair_tile;
-    a.num_pairs = plan + pt.num_pairs;
-    a.tile_rows = plan + pt.tile_rows;
-    a.group_order = plan + pt.group_order;
-    a.num_m_tiles = plan + pt.num_m_tiles;
-    a.counts_kept = plan + pt.counts_kept;
-    a.scratch = scratch.data_ptr<int>();
-    a.overflow = status_ptr(overflow);
-    check(cmoe::launch_moe_plan(a, stream), "moe_plan");
-  }
   // Without a backward pass nobody reads the padding rows, so they are not filled, and where experts have few rows the
   // GEMMs load and store only the 32-row pieces that hold any: at 64 tokens, E 64 top-8 (8 rows per expert), H 2048,
   // F 1024 the padding was 33 MB to fill, 400 MB to load from L2 and 50 MB to store, next to 805 MB of weights.  From 64
@@ -278,6 +309,8 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
 }  // namespace
 
 void register_moe(pybind11::module_& m) {
+  m.def("moe_local_plan", &moe_local_plan);
+  m.def("moe_local_tables", &moe_local_tables);
   m.def("moe_local_forward", &moe_local_forward);
   m.def("moe_local_backward", &moe_local_backward);
 }

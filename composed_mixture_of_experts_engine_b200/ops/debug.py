@@ -44,10 +44,16 @@ def _first_bad(mask: torch.Tensor) -> Optional[int]:
 
 
 def check_plan(slot_row: torch.Tensor, row_slot: torch.Tensor, tile_group: torch.Tensor, num_m_tiles: torch.Tensor,
-               group_offsets: torch.Tensor, n_local: int, cap_rows: int, n_slots: Optional[int] = None) -> None:
+               group_offsets: torch.Tensor, n_local: int, cap_rows: int, n_slots: Optional[int] = None,
+               pair_tile: Optional[torch.Tensor] = None, num_pairs: Optional[torch.Tensor] = None,
+               tile_rows: Optional[torch.Tensor] = None, group_order: Optional[torch.Tensor] = None,
+               counts_kept: Optional[torch.Tensor] = None) -> None:
     """Validate one row plan.  ``slot_row`` [n_slots] (row of each (token, k) slot or -1), ``row_slot`` [cap_rows]
     (slot of each row or -1), ``tile_group`` [cap_rows / 128] (expert of each 128-row tile or -1), ``num_m_tiles``
-    [1], ``group_offsets`` [n_local + 1]."""
+    [1], ``group_offsets`` [n_local + 1].  The tables of the expert layer's own plan, where given: ``pair_tile``
+    [cap_rows / 128] / ``num_pairs`` [1] (2 * first tile + 1 if the pair has only that one), ``tile_rows``
+    [cap_rows / 128] (live rows of each tile), ``group_order`` [n_local] (experts from most to fewest padded rows),
+    ``counts_kept`` [n_local] (live rows of each expert)."""
     n_slots = int(slot_row.numel()) if n_slots is None else n_slots
     tiles = int(num_m_tiles.reshape(-1)[0])
     if tiles < 0 or tiles * 128 > cap_rows or tiles > tile_group.numel():
@@ -89,6 +95,49 @@ def check_plan(slot_row: torch.Tensor, row_slot: torch.Tensor, tile_group: torch
         if i is not None:
             raise PlanBoundsError(f"tile {i} names expert {int(tg[i])} whose rows are [{int(go[tg[i]])}, "
                                   f"{int(go[tg[i] + 1])})")
+    # every expert's live rows lie in front of its padding
+    live_rows = (rs >= 0).long()
+    before = torch.cat([live_rows.new_zeros(1), live_rows.cumsum(0)])
+    per_expert = before[go[1:]] - before[go[:-1]]
+    if counts_kept is not None:
+        i = _first_bad(counts_kept.reshape(-1).long() != per_expert)
+        if i is not None:
+            raise PlanBoundsError(f"counts_kept[{i}] = {int(counts_kept.reshape(-1)[i])}, but expert {i} has "
+                                  f"{int(per_expert[i])} rows")
+    if tile_rows is not None and tiles:
+        got = tile_rows.reshape(-1)[:tiles].long()
+        per_tile = live_rows.view(tiles, 128)
+        want = per_tile.sum(1)
+        i = _first_bad(got != want)
+        if i is not None:
+            raise PlanBoundsError(f"tile_rows[{i}] = {int(got[i])}, but the tile has {int(want[i])} live rows")
+        i = _first_bad((per_tile[:, 1:] > per_tile[:, :-1]).any(1))
+        if i is not None:
+            raise PlanBoundsError(f"tile {i} has a live row behind padding")
+    if group_order is not None:
+        order, padded = group_order.reshape(-1).long(), go[1:] - go[:-1]
+        i = _first_bad((order < 0) | (order >= n_local))
+        if i is not None:
+            raise PlanBoundsError(f"group_order[{i}] = {int(order[i])} is outside [0, {n_local})")
+        i = _first_bad(torch.bincount(order, minlength=n_local) != 1)
+        if i is not None:
+            raise PlanBoundsError(f"group_order names expert {i} not exactly once")
+        i = _first_bad(padded[order][1:] > padded[order][:-1])
+        if i is not None:
+            raise PlanBoundsError(f"group_order[{i + 1}] = {int(order[i + 1])} has more rows than the expert before it")
+    if pair_tile is not None and num_pairs is not None:
+        # tiles t of an expert with an even distance from its first one start a pair, alone where no other follows
+        t = torch.arange(tiles, device=tg.device)
+        first, last = go[tg] // 128, go[tg + 1] // 128 - 1
+        starts = (t - first) % 2 == 0
+        want = (2 * t + (t == last).long())[starts]
+        n = int(num_pairs.reshape(-1)[0])
+        if n != want.numel():
+            raise PlanBoundsError(f"num_pairs = {n}, but the tiles make {want.numel()} pairs")
+        got = pair_tile.reshape(-1)[:n].long()
+        i = _first_bad(got != want)
+        if i is not None:
+            raise PlanBoundsError(f"pair_tile[{i}] = {int(got[i])}, expected {int(want[i])}")
 
 
 class Canary:

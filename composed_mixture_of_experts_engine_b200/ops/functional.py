@@ -14,7 +14,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from . import _ext, kernels
+from . import _ext, debug, kernels
 from . import attention_sm100 as _attn_sm100
 from .kernels import EPI_SWIGLU_BWD, EPI_SWIGLU_FWD, GEMM_GROUPED_K, GEMM_GROUPED_M, MoEPlan
 
@@ -404,12 +404,11 @@ def _local_fused() -> bool:
 
 
 class _LocalMoEFn(torch.autograd.Function):
-    """Route-sorted expert FFN on one GPU: plan -> gather -> grouped SwiGLU GEMMs -> weighted combine.
-
-    Fused form (``CMOE_LOCAL_FUSED=1``): the first GEMM of each direction brings its own rows in (row-pull warps reading the token
-    buffer through a one-entry "peer" table, so the gather overlaps the MMAs), and the last GEMM of each direction
-    stores its result rows at their (token, k) slot, which turns the combine into a streaming weighted sum of K
-    consecutive rows instead of an indexed gather."""
+    """Route-sorted expert FFN on one GPU with the row transfers inside the grouped GEMMs (``CMOE_LOCAL_FUSED=1``): the
+    first GEMM of each direction brings its own rows in (row-pull warps reading the token buffer through a one-entry
+    "peer" table, so the gather overlaps the MMAs), and the last GEMM of each direction stores its result rows at their
+    (token, k) slot, which turns the combine into a streaming weighted sum of K consecutive rows instead of an indexed
+    gather."""
 
     @staticmethod
     def forward(ctx, x, gate_w32, idx32, w13, w2, capacity: int, holder: Optional[dict]):
@@ -417,25 +416,17 @@ class _LocalMoEFn(torch.autograd.Function):
         N, K = idx32.shape
         H = x.shape[1]
         plan = kernels.moe_plan(idx32, E, capacity=capacity)
-        fused = _local_fused() and H % 8 == 0
-        ctx.fused = fused
-        if fused:
-            x = x.contiguous()
-            xp = torch.empty(plan.cap_rows, H, device=x.device, dtype=torch.bfloat16)
-            ar = torch.arange(N * K, device=x.device, dtype=torch.int32)
-            ident = torch.where(plan.slot_row >= 0, ar, torch.full_like(ar, -1))  # slot -> its own row, -1 if dropped
-            ys = torch.empty(N * K, H, device=x.device, dtype=torch.bfloat16)
-            hact, gu, _ = grouped_swiglu_forward(
-                xp, w13, w2, plan, pull=dict(src_ptrs=[x.data_ptr()], slots_per_src=N * K, pull_K=K, ld_src=H),
-                scatter=dict(row_slot=plan.row_slot, slots_per_rank=N * K, out_ptrs=[ys.data_ptr()], out_ld=H))
-            y = torch.empty(N, H, device=x.device, dtype=torch.bfloat16)
-            _ext.ext().combine_rows(ys, ident, gate_w32, y, K)
-            ctx.save_for_backward(xp, hact, gu, ys, gate_w32, w13, w2, ident)
-        else:  # debug checks on: the plan is validated between the launches
-            xp = kernels.gather_rows(x, plan)
-            hact, gu, yp = grouped_swiglu_forward(xp, w13, w2, plan)
-            y = kernels.combine_rows(yp, plan, gate_w32)
-            ctx.save_for_backward(xp, hact, gu, yp, gate_w32, w13, w2)
+        x = x.contiguous()
+        xp = torch.empty(plan.cap_rows, H, device=x.device, dtype=torch.bfloat16)
+        ar = torch.arange(N * K, device=x.device, dtype=torch.int32)
+        ident = torch.where(plan.slot_row >= 0, ar, torch.full_like(ar, -1))  # slot -> its own row, -1 if dropped
+        ys = torch.empty(N * K, H, device=x.device, dtype=torch.bfloat16)
+        hact, gu, _ = grouped_swiglu_forward(
+            xp, w13, w2, plan, pull=dict(src_ptrs=[x.data_ptr()], slots_per_src=N * K, pull_K=K, ld_src=H),
+            scatter=dict(row_slot=plan.row_slot, slots_per_rank=N * K, out_ptrs=[ys.data_ptr()], out_ld=H))
+        y = torch.empty(N, H, device=x.device, dtype=torch.bfloat16)
+        _ext.ext().combine_rows(ys, ident, gate_w32, y, K)
+        ctx.save_for_backward(xp, hact, gu, ys, gate_w32, w13, w2, ident)
         ctx.plan = plan
         if holder is not None:
             holder["plan"] = plan
@@ -445,34 +436,27 @@ class _LocalMoEFn(torch.autograd.Function):
     def backward(ctx, dy):
         plan = ctx.plan
         dy = dy.contiguous()
-        if ctx.fused:
-            xp, hact, gu, ys, gate_w32, w13, w2, ident = ctx.saved_tensors
-            N, K = gate_w32.shape
-            H = xp.shape[1]
-            ext = _ext.ext()
-            d_gate = None
-            if ctx.needs_input_grad[1]:
-                d_gate = torch.empty(N, K, device=dy.device, dtype=torch.float32)
-                ext.combine_bwd_w(ys, ident, dy, d_gate, K)
-            dyp = torch.empty(plan.cap_rows, H, device=dy.device, dtype=torch.bfloat16)
-            need_dx = ctx.needs_input_grad[0]
-            dxs = torch.empty(N * K, H, device=dy.device, dtype=torch.bfloat16) if need_dx else None
-            _, dw13, dw2 = grouped_swiglu_backward(
-                dyp, xp, hact, gu, w13, w2, plan, need_dx=need_dx,
-                pull=dict(src_ptrs=[dy.data_ptr()], slots_per_src=N * K, pull_K=K, ld_src=H,
-                          slot_scale=gate_w32.reshape(-1)),
-                scatter=dict(row_slot=plan.row_slot, slots_per_rank=N * K, out_ptrs=[dxs.data_ptr()], out_ld=H)
-                if need_dx else None)
-            dx = None
-            if need_dx:
-                dx = torch.empty(N, H, device=dy.device, dtype=torch.bfloat16)
-                ext.combine_rows(dxs, ident, None, dx, K)
-            return dx, d_gate, None, dw13, dw2, None, None
-        xp, hact, gu, yp, gate_w32, w13, w2 = ctx.saved_tensors
-        d_gate = kernels.combine_bwd_w(yp, plan, dy) if ctx.needs_input_grad[1] else None
-        dyp = kernels.gather_rows(dy, plan, slot_scale=gate_w32.reshape(-1))
-        dxp, dw13, dw2 = grouped_swiglu_backward(dyp, xp, hact, gu, w13, w2, plan, need_dx=ctx.needs_input_grad[0])
-        dx = kernels.combine_rows(dxp, plan, None) if dxp is not None else None
+        xp, hact, gu, ys, gate_w32, w13, w2, ident = ctx.saved_tensors
+        N, K = gate_w32.shape
+        H = xp.shape[1]
+        ext = _ext.ext()
+        d_gate = None
+        if ctx.needs_input_grad[1]:
+            d_gate = torch.empty(N, K, device=dy.device, dtype=torch.float32)
+            ext.combine_bwd_w(ys, ident, dy, d_gate, K)
+        dyp = torch.empty(plan.cap_rows, H, device=dy.device, dtype=torch.bfloat16)
+        need_dx = ctx.needs_input_grad[0]
+        dxs = torch.empty(N * K, H, device=dy.device, dtype=torch.bfloat16) if need_dx else None
+        _, dw13, dw2 = grouped_swiglu_backward(
+            dyp, xp, hact, gu, w13, w2, plan, need_dx=need_dx,
+            pull=dict(src_ptrs=[dy.data_ptr()], slots_per_src=N * K, pull_K=K, ld_src=H,
+                      slot_scale=gate_w32.reshape(-1)),
+            scatter=dict(row_slot=plan.row_slot, slots_per_rank=N * K, out_ptrs=[dxs.data_ptr()], out_ld=H)
+            if need_dx else None)
+        dx = None
+        if need_dx:
+            dx = torch.empty(N, H, device=dy.device, dtype=torch.bfloat16)
+            ext.combine_rows(dxs, ident, None, dx, K)
         return dx, d_gate, None, dw13, dw2, None, None
 
 
@@ -489,10 +473,19 @@ class _LocalPlan:
         return self.buf[-self.n_local:]
 
 
+def _checked_plan(idx32: torch.Tensor, num_experts: int, capacity: int) -> torch.Tensor:
+    """The layer's own row plan, built ahead of it and validated before any kernel reads an index from it."""
+    plan = _ext.ext().moe_local_plan(idx32, num_experts, capacity, kernels.overflow_counter(idx32.device))
+    tables = _ext.ext().moe_local_tables(plan, idx32.numel(), num_experts)
+    debug.check_plan(**tables, n_local=num_experts, cap_rows=tables["row_slot"].numel())
+    return plan
+
+
 def _native_forward(x, gate_w32, idx32, w13, w2, capacity: int, keep: bool, holder: Optional[dict]):
     dev = x.device
+    plan = _checked_plan(idx32, w13.shape[0], capacity) if debug.enabled() else None
     out = _ext.ext().moe_local_forward(x, gate_w32, idx32, w13, w2, capacity, keep, kernels.status_word(dev),
-                                       kernels.overflow_counter(dev))
+                                       kernels.overflow_counter(dev), plan)
     if holder is not None:
         holder["plan"] = _LocalPlan(out[1], w13.shape[0])
     return out
@@ -521,10 +514,8 @@ def local_moe(x: torch.Tensor, gate_w: torch.Tensor, idx: torch.Tensor, w13: tor
               capacity: int = 0, holder: Optional[dict] = None) -> torch.Tensor:
     """All experts on this rank.  ``x`` [N,H], ``gate_w`` [N,K] gate weights, ``idx`` [N,K] expert ids."""
     if on_device_path(x, w13, w2):
-        from . import debug
-
         gate_w32, idx32 = gate_w.float().contiguous(), idx.to(torch.int32).contiguous()
-        if _local_fused() or debug.enabled():
+        if _local_fused() and x.shape[1] % 8 == 0:
             return _LocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
         if kernels.needs_autograd(x, gate_w32, w13, w2):
             return _NativeLocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
