@@ -399,11 +399,17 @@ void moe_plan(const Tensor& topk_idx, int64_t K, int64_t num_experts, int64_t ex
   a.overflow = opt_ptr<int>(overflow);
   check_cuda(cmoe::launch_moe_plan(a, cur_stream()), "moe_plan");
 }
+// the row kernels read and write rows in 16-byte vectors
+void check_rows(const Tensor& t, const char* name) {
+  check_bf16_2d(t, name);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && (t.size(0) <= 1 || t.stride(0) % 8 == 0), name,
+              ": rows must start on 16-byte boundaries");
+}
 void gather_rows(const Tensor& src, const Tensor& row_slot, int64_t slot_div, const OptTensor& slot_scale, Tensor& out,
                  const OptTensor& num_m_tiles) {
   const c10::cuda::CUDAGuard guard(src.device());
-  check_bf16_2d(src, "src");
-  check_bf16_2d(out, "out");
+  check_rows(src, "src");
+  check_rows(out, "out");
   check_cuda(cmoe::launch_gather_rows(src.data_ptr(), row_slot.data_ptr<int>(), static_cast<int>(slot_div),
                                       opt_ptr<const float>(slot_scale), out.data_ptr(), out.size(0),
                                       opt_ptr<const int>(num_m_tiles), static_cast<int>(src.size(1)), src.stride(0),
@@ -412,8 +418,8 @@ void gather_rows(const Tensor& src, const Tensor& row_slot, int64_t slot_div, co
 }
 void combine_rows(const Tensor& rows, const Tensor& slot_row, const OptTensor& w, Tensor& y, int64_t K) {
   const c10::cuda::CUDAGuard guard(rows.device());
-  check_bf16_2d(rows, "rows");
-  check_bf16_2d(y, "y");
+  check_rows(rows, "rows");
+  check_rows(y, "y");
   check_cuda(cmoe::launch_combine_rows(rows.data_ptr(), slot_row.data_ptr<int>(), opt_ptr<const float>(w), y.data_ptr(),
                                        y.size(0), static_cast<int>(K), static_cast<int>(y.size(1)), rows.stride(0),
                                        y.stride(0), cur_stream()),
@@ -421,8 +427,8 @@ void combine_rows(const Tensor& rows, const Tensor& slot_row, const OptTensor& w
 }
 void combine_bwd_w(const Tensor& rows, const Tensor& slot_row, const Tensor& dy, Tensor& dw, int64_t K) {
   const c10::cuda::CUDAGuard guard(rows.device());
-  check_bf16_2d(rows, "rows");
-  check_bf16_2d(dy, "dy");
+  check_rows(rows, "rows");
+  check_rows(dy, "dy");
   check_cuda(cmoe::launch_combine_bwd_w(rows.data_ptr(), slot_row.data_ptr<int>(), dy.data_ptr(), dw.data_ptr<float>(),
                                         dy.size(0), static_cast<int>(K), static_cast<int>(dy.size(1)), rows.stride(0),
                                         dy.stride(0), cur_stream()),

@@ -46,12 +46,20 @@ struct PlanTables {
   }
 };
 
+// the row kernels read and write rows in 16-byte vectors
+void check_rows(const Tensor& t, const char* name) {
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && (t.size(0) <= 1 || t.stride(0) % 8 == 0) &&
+                  t.size(1) % 8 == 0,
+              name, ": rows must be multiples of 8 columns and start on 16-byte boundaries");
+}
+
 struct Shapes {
   int64_t N, K, H, E, F;
 };
 Shapes check_shapes(const Tensor& x, const Tensor& idx32, const Tensor& w13, const Tensor& w2) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1,
               "x must be a CUDA bf16 matrix with unit inner stride");
+  check_rows(x, "x");
   TORCH_CHECK(idx32.scalar_type() == at::kInt && idx32.dim() == 2 && idx32.is_contiguous() && idx32.size(0) == x.size(0),
               "idx must be contiguous int32 [N, K]");
   TORCH_CHECK(w13.scalar_type() == at::kBFloat16 && w13.dim() == 3 && w13.is_contiguous() && w13.size(2) == x.size(1) &&
@@ -269,6 +277,9 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
   const int64_t N = gate_w32.size(0), K = gate_w32.size(1), H = xp.size(1), E = w13.size(0), F = hact.size(1);
   TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && dy.size(0) == N && dy.size(1) == H, "bad dy");
+  check_rows(dy, "dy");
+  check_rows(xp, "saved rows");
+  check_rows(yp, "saved expert rows");
   const PlanTables pt(N * K, E);
   TORCH_CHECK(plan_t.numel() == pt.words && xp.size(0) == pt.cap_rows, "the row plan belongs to another layer call");
   int* plan = plan_t.data_ptr<int>();

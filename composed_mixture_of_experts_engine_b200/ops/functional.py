@@ -102,6 +102,14 @@ def rows_for_tma(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+def rows_for_vectors(t: torch.Tensor) -> torch.Tensor:
+    """``t`` [rows, cols] for the kernels that take any row stride but read rows in 16-byte vectors: a copy only where a
+    row would start off a 16-byte boundary.  (Other layouts are passed on, for the kernels' bindings to refuse.)"""
+    if t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0:
+        return t
+    return t if t.dim() != 2 or t.stride(1) != 1 else t.clone(memory_format=torch.contiguous_format)
+
+
 class _LinearFn(torch.autograd.Function):
     """``y = x @ W^T`` on the two-SM tcgen05 GEMM: forward K-major x K-major, input gradient with W read
     N-major (no transposed copy), weight gradient as a contraction over the rows whose fp32 result is added into
@@ -504,7 +512,7 @@ class _NativeLocalMoEFn(torch.autograd.Function):
     def backward(ctx, dy):
         plan, xp, hact, gu, yp, gate_w32, w13, w2 = ctx.saved_tensors
         dx, d_gate, dw13, dw2 = _ext.ext().moe_local_backward(
-            dy.contiguous(), plan, xp, hact, gu, yp, gate_w32, w13, w2, ctx.needs_input_grad[0],
+            rows_for_tma(dy), plan, xp, hact, gu, yp, gate_w32, w13, w2, ctx.needs_input_grad[0],
             ctx.needs_input_grad[1], getattr(w13, "main_grad", None), getattr(w2, "main_grad", None),
             kernels.status_word(dy.device))
         return dx, d_gate, None, dw13, dw2, None, None
@@ -514,6 +522,7 @@ def local_moe(x: torch.Tensor, gate_w: torch.Tensor, idx: torch.Tensor, w13: tor
               capacity: int = 0, holder: Optional[dict] = None) -> torch.Tensor:
     """All experts on this rank.  ``x`` [N,H], ``gate_w`` [N,K] gate weights, ``idx`` [N,K] expert ids."""
     if on_device_path(x, w13, w2):
+        x = rows_for_vectors(x)
         gate_w32, idx32 = gate_w.float().contiguous(), idx.to(torch.int32).contiguous()
         if _local_fused() and x.shape[1] % 8 == 0:
             return _LocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
