@@ -105,8 +105,8 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& D, int64_t mode, int64_t epi
 }
 
 // out (+)= a^T @ b over the rows, cut into pieces where the output alone would leave SMs idle
-void wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, const OptTensor& status) {
-  cmoe::dense_wgrad(a, b, out, accumulate, opt_ptr<int>(status));
+void wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, const OptTensor& status, int64_t pieces) {
+  cmoe::dense_wgrad(a, b, out, accumulate, opt_ptr<int>(status), pieces);
 }
 
 // GEMM (dense or grouped-M) whose output rows are scattered by the epilogue: row r goes to rank

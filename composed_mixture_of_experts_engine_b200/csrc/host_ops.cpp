@@ -92,16 +92,21 @@ void launch_gemm_any(const GemmArgs& g, cudaStream_t stream) {
 Tensor dense_nt(const Tensor& x, const Tensor& w, Tensor out, int* status) { return dense(x, w, false, out, status); }
 Tensor dense_nn(const Tensor& x, const Tensor& w, Tensor out, int* status) { return dense(x, w, true, out, status); }
 
-void dense_wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, int* status) {
+void dense_wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, int* status, int64_t want_pieces) {
   const c10::cuda::CUDAGuard guard(a.device());
   GemmArgs g = operands(a, true, b, true);
   const int64_t R = a.size(0), M = a.size(1), N = b.size(1);
   const bool fp32 = out.scalar_type() == at::kFloat;
-  TORCH_CHECK(b.size(0) == R && out.dim() == 2 && out.size(0) == M && out.size(1) == N && out.is_contiguous() &&
+  TORCH_CHECK(b.size(0) == R && out.dim() == 2 && out.size(0) == M && out.size(1) == N && out.stride(1) == 1 &&
                   (fp32 || (out.scalar_type() == at::kBFloat16 && !accumulate)),
               "wgrad: bad output");
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-  const int pieces = (M * N) % 4 == 0 ? wgrad_pieces(R, M, N, g.num_sms) : 1;
+  // every way of writing `out` uses 16-byte vectors, the sum of the pieces over all of it as one run
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0 && out.stride(0) * (fp32 ? 4 : 2) % 16 == 0,
+              "wgrad: the rows of the output must start on 16-byte boundaries");
+  int pieces = 1;
+  if (out.is_contiguous() && (M * N) % 4 == 0)
+    pieces = want_pieces > 0 ? static_cast<int>(want_pieces) : wgrad_pieces(R, M, N, g.num_sms);
   const int64_t chunk = ((R + pieces - 1) / pieces + 63) / 64 * 64;
   g.mode = GEMM_GROUPED_K;
   g.M = static_cast<int>(M);
@@ -109,7 +114,7 @@ void dense_wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate,
   g.groups = pieces;
   g.k_chunk = static_cast<int>(chunk);
   g.d_group_stride = M * N;
-  g.ldd = N;
+  g.ldd = pieces > 1 ? N : out.stride(0);
   g.status = status;
   Tensor part;
   if (pieces > 1) {

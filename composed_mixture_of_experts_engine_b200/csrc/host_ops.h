@@ -13,7 +13,9 @@ void launch_gemm_any(const GemmArgs& g, cudaStream_t stream);
 torch::Tensor dense_nt(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
 // y[M, K] = x[M, N] @ w[N, K]
 torch::Tensor dense_nn(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
-// out[M, N] (+)= a[R, M]^T @ b[R, N]; out fp32 (stored, or added to) or bf16 (stored)
-void dense_wgrad(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool accumulate, int* status);
+// out[M, N] (+)= a[R, M]^T @ b[R, N]; out fp32 (stored, or added to) or bf16 (stored), its rows on 16-byte
+// boundaries.  The contraction is cut into `pieces` (0: as many as are worth it) that run side by side where out is contiguous.
+void dense_wgrad(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool accumulate, int* status,
+                 int64_t pieces = 0);
 
 }  // namespace cmoe

@@ -130,21 +130,29 @@ def linear_nn(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
 
 
 def linear_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
-              out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+              splits: int = 0, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """out[M, N] = a[R, M]^T @ b[R, N]: the weight-gradient contraction over R rows (fp32 accumulation; a bf16 result
-    is rounded once).  Small outputs are cut into pieces of rows that run side by side and are added in order
-    (csrc/host_ops.cpp)."""
+    is rounded once).  Small outputs are cut into ``splits`` pieces of rows (0: as many as are worth it) that run side by
+    side and are added in order (csrc/host_ops.cpp).  An ``out`` that the kernels cannot write to (another type, no unit
+    inner stride, rows off 16-byte boundaries) or add to (bf16) takes the fp32 result by an ordinary copy or addition."""
     if out is None:
-        out = torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=out_dtype)
-    _ext.ext().wgrad(a, b, out, accumulate, status_word(a.device))
+        out, accumulate = torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=out_dtype), False
+    direct = (out.dtype == torch.float32 or (out.dtype == torch.bfloat16 and not accumulate)) and (
+        out.stride(1) == 1 and out.stride(0) * out.element_size() % 16 == 0 and out.data_ptr() % 16 == 0)
+    res = out if direct else torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=torch.float32)
+    _ext.ext().wgrad(a, b, res, accumulate and direct, status_word(a.device), splits)
+    if not direct:
+        if accumulate:
+            out.add_(res.to(out.dtype))
+        else:
+            out.copy_(res)
     return out
 
 
 def linear_tn_acc(a: torch.Tensor, b: torch.Tensor, acc: torch.Tensor, accumulate: bool = True) -> torch.Tensor:
     """acc[M, N] (fp32, in place) += a[R, M]^T @ b[R, N]; one piece adds with the kernel's TMA reduce-add epilogue (no
     read-modify-write pass over ``acc`` on the SMs, no temporary); ``accumulate=False`` stores."""
-    _ext.ext().wgrad(a, b, acc, accumulate, status_word(a.device))
-    return acc
+    return linear_tn(a, b, acc, accumulate)
 
 
 _overflow: Dict[int, torch.Tensor] = {}
