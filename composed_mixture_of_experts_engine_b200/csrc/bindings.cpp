@@ -314,18 +314,20 @@ void sumsq(const Tensor& x, Tensor& out) {
                                 cur_stream()),
              "sumsq");
 }
-// out (fp32) += scale * x, or out (bf16) = scale * x; scale is a one-element fp32 tensor
-void scaled_out(const Tensor& x, const Tensor& scale, Tensor& out) {
+// out += scale * x (fp32) or out = scale * x (fp32 or bf16); scale is a one-element fp32 tensor.  A caller that does not
+// say adds to fp32 and stores bf16.
+void scaled_out(const Tensor& x, const Tensor& scale, Tensor& out, std::optional<bool> accumulate) {
   const c10::cuda::CUDAGuard guard(x.device());
-  const bool add = out.scalar_type() == at::kFloat;
+  const bool fp32 = out.scalar_type() == at::kFloat;
+  const bool add = accumulate.value_or(fp32);
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.is_contiguous() && out.is_contiguous() &&
-                  out.numel() == x.numel() && (add || out.scalar_type() == at::kBFloat16) && x.numel() % 4 == 0,
-              "scaled_out: contiguous fp32 input and fp32 / bf16 output of one size, a multiple of 4");
+                  out.numel() == x.numel() && (fp32 || (out.scalar_type() == at::kBFloat16 && !add)) && x.numel() % 4 == 0,
+              "scaled_out: contiguous fp32 input and an fp32 output, or a bf16 one to store to, of one size, a multiple of 4");
   TORCH_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0,
               "scaled_out: tensors must start on 16-byte boundaries");
   TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() == 1, "scaled_out: bad scale");
-  check_cuda(cmoe::launch_scaled_out(x.data_ptr<float>(), scale.data_ptr<float>(), x.numel(), out.data_ptr(), add,
-                                     cur_stream()),
+  check_cuda(cmoe::launch_scaled_out(x.data_ptr<float>(), scale.data_ptr<float>(), x.numel(), out.data_ptr(), !fp32,
+                                     add, cur_stream()),
              "scaled_out");
 }
 
@@ -457,7 +459,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("adamw", &adamw);
   m.def("sumsq", &sumsq);
   m.def("cross_entropy", &cross_entropy);
-  m.def("scaled_out", &scaled_out);
+  m.def("scaled_out", &scaled_out, pybind11::arg("x"), pybind11::arg("scale"), pybind11::arg("out"),
+        pybind11::arg("accumulate") = pybind11::none());
   m.def("embedding_grad", &embedding_grad);
   m.def("moe_plan_scratch_words", &moe_plan_scratch_words);
   m.def("moe_plan", &moe_plan);

@@ -569,9 +569,9 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   }
 }
 
-// out (fp32) += *scale * x, or out (bf16) = *scale * x.  One pass over each; what bounds it is those passes.  Library
+// out (+)= *scale * x in fp32, or out = *scale * x in bf16.  One pass over each; what bounds it is those passes.  Library
 // operations took a multiply, a cast and a temporary for the second, and 361 us for 103 M elements of the first.
-template <bool ADD>
+template <int OUT>  // 0: fp32 store, 1: fp32 add, 2: bf16 store
 __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* x, const float* scale,
                                                          long long n4, void* out) {
   chain_wait();
@@ -584,16 +584,18 @@ __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* x, const 
     const long long i = i0 + q * 256;
     if (i < n4) {
       v[q] = __ldcs(x + i);
-      if (ADD) o[q] = __ldcs(reinterpret_cast<const float4*>(out) + i);
+      if (OUT == 1) o[q] = __ldcs(reinterpret_cast<const float4*>(out) + i);
     }
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const long long i = i0 + q * 256;
     if (i < n4) {
-      if (ADD)
+      if (OUT == 1)
         __stcs(reinterpret_cast<float4*>(out) + i, make_float4(o[q].x + s * v[q].x, o[q].y + s * v[q].y,
                                                                o[q].z + s * v[q].z, o[q].w + s * v[q].w));
+      else if (OUT == 0)
+        reinterpret_cast<float4*>(out)[i] = make_float4(s * v[q].x, s * v[q].y, s * v[q].z, s * v[q].w);
       else
         reinterpret_cast<uint2*>(out)[i] = make_uint2(pack_bf16x2(s * v[q].x, s * v[q].y), pack_bf16x2(s * v[q].z, s * v[q].w));
     }
@@ -990,15 +992,16 @@ cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void
   return cudaGetLastError();
 }
 
-cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int add, cudaStream_t stream) {
+cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int out_bf16, int accumulate,
+                              cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  if (n % 4 != 0) return cudaErrorInvalidValue;
+  if (n % 4 != 0 || (out_bf16 && accumulate)) return cudaErrorInvalidValue;
   const long long n4 = n / 4;
   const unsigned grid = static_cast<unsigned>((n4 + 1023) / 1024);
   const float4* x4 = reinterpret_cast<const float4*>(x);
-  return add ? launch_chained(scaled_out_kernel<true>, grid, 256, 0, stream, x4, scale, n4,
-                              out) : launch_chained(scaled_out_kernel<false>, grid, 256, 0, stream, x4, scale, n4,
-                              out);
+  if (out_bf16) return launch_chained(scaled_out_kernel<2>, grid, 256, 0, stream, x4, scale, n4, out);
+  if (accumulate) return launch_chained(scaled_out_kernel<1>, grid, 256, 0, stream, x4, scale, n4, out);
+  return launch_chained(scaled_out_kernel<0>, grid, 256, 0, stream, x4, scale, n4, out);
 }
 
 long long embedding_grad_partial_floats(long long n, int H) {

@@ -64,9 +64,10 @@ cudaError_t launch_sumsq(const void* x, int is_bf16, long long n, float* out, fl
 cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void* out, int out_bf16, int accumulate,
                                  cudaStream_t stream);
 
-// out[i] += *scale * x[i] (fp32, add != 0) or out[i] = *scale * x[i] rounded to bf16.  n % 4 == 0, 16-byte aligned
-// pointers; scale is a device scalar.
-cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int add, cudaStream_t stream);
+// out[i] (fp32: stored or added to; bf16: stored) = *scale * x[i].  n % 4 == 0, 16-byte aligned pointers; scale is a device
+// scalar.
+cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int out_bf16, int accumulate,
+                              cudaStream_t stream);
 
 // ---- embedding gradient: main[keys[i], :] += dy[order[i], :] for sorted keys (fp32 sums in a fixed order); dy [n, H] bf16,
 // main [vocabulary, H] and the working storage `partial` (embedding_grad_partial_floats words, unless that is 0) fp32 are

@@ -148,8 +148,9 @@ class _LMHeadLossFn(torch.autograd.Function):
 
             main = getattr(weight, "main_grad", None)
             out = torch.empty_like(weight) if main is None else main
-            if dw.numel() % 4 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0:
-                _ext.ext().scaled_out(dw, g.to(torch.float32), out)
+            if (dw.numel() % 4 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0
+                    and (out.dtype == torch.float32 or (out.dtype == torch.bfloat16 and main is None))):
+                _ext.ext().scaled_out(dw, g.to(torch.float32), out, main is not None)
             elif main is not None:
                 main.addcmul_(dw, g.to(torch.float32))
             else:
