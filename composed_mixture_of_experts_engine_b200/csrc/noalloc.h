@@ -13,9 +13,10 @@
 // cudaMalloc, cudaFree or any other allocating call.
 //
 // Limits and rules:
-//   * The problem must fit the fixed array: cmoe_moe_plan_noalloc_words(...) <= CMOE_NOALLOC_SCRATCH_WORDS (about
-//     ceil(n_slots / 1024) * bins words up to 512 bins, where bins = n_local * (per_k_bins ? K : 1)).  Larger problems
-//     are rejected with CMOE_NOALLOC_TOO_LARGE and nothing is launched.
+//   * The problem must fit the fixed array: cmoe_moe_plan_noalloc_words(...) <= CMOE_NOALLOC_SCRATCH_WORDS.  Everything
+//     with (ceil(n_slots / 256) + 2) * bins <= CMOE_NOALLOC_SCRATCH_WORDS does, where bins = n_local * (per_k_bins ? K :
+//     1), and with up to 3900 bins about four times as many slots.  Larger problems are rejected with
+//     CMOE_NOALLOC_TOO_LARGE and nothing is launched.
 //   * The first call on each device looks up the device address of the array (one cudaGetSymbolAddress, with
 //     that device current).  Make that first call outside any stream capture.  Two host threads may make their
 //     first calls on a device at the same time: the address is published through an atomic and both arrive at

@@ -9,7 +9,9 @@
 //   * more: a counting launch (histogram per unit of slots), then one launch whose CTAs each add up the histograms of
 //     the units before theirs (a few KiB out of L2, redundantly, which is cheaper than a launch or a last-CTA hand-over
 //     in between), derive the expert offsets and rank their slots;
-//   * only where units x bins exceed 16384 words a scan launch replaces the redundant sums.
+//   * only where units x bins exceed 16384 words a scan launch replaces the redundant sums;
+//   * few slots over thousands of bins: one CTA with two words per bin, since eight warps' counts of every bin would be
+//     more work to clear and add up than the slots are.
 // The first form took two memsets and three launches, one of them a single CTA whose first thread walked the experts
 // through global memory: 22.8 us of kernels for 64 tokens x top-8 of 64 experts, 41 us for 16384 tokens.
 #include "ops.cuh"
@@ -26,6 +28,7 @@ constexpr int kWarpsMulti = 8;
 constexpr int kWarpsSingle = 32;
 constexpr int kSingleSlots = 8192;
 constexpr int kRedundantWords = 16384;
+constexpr int kSparseSlots = 4096;
 constexpr int kSmemLimit = 200 * 1024;
 
 __device__ __forceinline__ int plan_bin(const MoePlanArgs& a, long long slot) {
@@ -316,18 +319,162 @@ __global__ void __launch_bounds__(WARPS * 32) plan_rank_kernel(const MoePlanArgs
   }
 }
 
+// Few slots, many bins: one CTA.  The slots are counted by all threads and ranked by one warp, 32 at a time; `work` holds
+// the next row and the end of every bin ([2][nbins], shared memory where it fits).
+__global__ void __launch_bounds__(1024) plan_sparse_kernel(const MoePlanArgs a, int nbins, int* work) {
+  chain_wait();
+  chain_trigger();
+  extern __shared__ int plan_smem[];
+  __shared__ long long s_sum[32];
+  int* next = work != nullptr ? work : plan_smem;
+  int* end = next + nbins;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int kb = a.per_k_bins ? a.K : 1;
+  const int cap128 = static_cast<int>(a.cap_rows / 128 * 128);
+  // exclusive prefix over the threads and the total of all of them
+  auto block_prefix = [&](long long v, long long& total) {
+    long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    long long before = 0;
+    total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += s_sum[w];
+      total += s_sum[w];
+    }
+    __syncthreads();
+    return before + incl - v;
+  };
+
+  for (int b = tid; b < nbins; b += 1024) next[b] = 0;
+  for (long long r = tid; r < a.cap_rows; r += 1024) a.row_slot[r] = -1;
+  __syncthreads();
+  for (long long s = tid; s < a.n_slots; s += 1024) {
+    const int bin = plan_bin(a, s);
+    if (bin >= 0) atomicAdd(next + bin, 1);
+  }
+  __syncthreads();
+  // every thread takes a run of neighbouring experts: their padded rows, the rows before them, then bin by bin
+  const int per = (a.n_local + 1023) / 1024;
+  const int e0 = min(a.n_local, tid * per), e1 = min(a.n_local, e0 + per);
+  auto kept_of = [&](int bin) { return a.capacity > 0 ? min(next[bin], a.capacity) : next[bin]; };
+  long long mine = 0, total = 0;
+  for (int e = e0; e < e1; ++e) {
+    int cnt = 0;
+    for (int k = 0; k < kb; ++k) cnt += kept_of(e * kb + k);
+    mine += (cnt + 127) / 128 * 128;
+  }
+  long long raw = block_prefix(mine, total);
+  for (int e = e0; e < e1; ++e) {
+    const int off = raw < cap128 ? static_cast<int>(raw) : cap128;
+    int cnt = 0;
+    for (int k = 0; k < kb; ++k) {
+      const int bin = e * kb + k, n = kept_of(bin);
+      next[bin] = off + cnt;
+      cnt += n;
+      end[bin] = off + cnt;
+    }
+    // rows that do not fit the buffer are dropped below (and counted in `overflow`)
+    const long long room = a.cap_rows - off;
+    a.counts_kept[e] = cnt > room ? static_cast<int>(room > 0 ? room : 0) : cnt;
+    a.group_offsets[e] = off;
+    raw += (cnt + 127) / 128 * 128;
+  }
+  if (tid == 0) {
+    const int off = total < cap128 ? static_cast<int>(total) : cap128;
+    a.group_offsets[a.n_local] = off;
+    *a.num_m_tiles = off / 128;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    for (long long s0 = 0; s0 < a.n_slots; s0 += 32) {
+      const long long slot = s0 + lane;
+      const int bin = slot < a.n_slots ? plan_bin(a, slot) : -1;
+      const unsigned peers = __match_any_sync(0xffffffffu, bin);
+      int row = -1;
+      if (bin >= 0) {
+        row = next[bin] + __popc(peers & below);
+        if (row >= end[bin]) {
+          row = -1;  // beyond the capacity
+        } else if (row >= a.cap_rows) {  // the row buffer is full: drop the slot and report it
+          row = -1;
+          if (a.overflow) atomicAdd(a.overflow, 1);
+        }
+      }
+      __syncwarp();
+      if (bin >= 0 && (peers & below) == 0u) next[bin] += __popc(peers);
+      __syncwarp();
+      if (slot < a.n_slots) {
+        a.slot_row[slot] = row;
+        if (row >= 0) a.row_slot[row] = static_cast<int>(slot);
+      }
+    }
+  }
+  __syncthreads();
+  if (a.pair_tile != nullptr) {  // the first pair of every expert, where the bins were
+    long long n = 0;
+    for (int e = e0; e < e1; ++e) n += (a.group_offsets[e + 1] - a.group_offsets[e] + 255) / 256;
+    long long first = block_prefix(n, total);
+    for (int e = e0; e < e1; ++e) {
+      next[e] = static_cast<int>(first);
+      first += (a.group_offsets[e + 1] - a.group_offsets[e] + 255) / 256;
+    }
+    if (tid == 0) *a.num_pairs = static_cast<int>(total);
+    __syncthreads();
+  }
+  const int* goff = a.group_offsets;
+  if (a.group_order != nullptr) {
+    for (int e = tid; e < a.n_local; e += 1024) {
+      const int rows = goff[e + 1] - goff[e];
+      int rank = 0;
+      for (int o = 0; o < a.n_local; ++o) {
+        const int r = goff[o + 1] - goff[o];
+        rank += r > rows || (r == rows && o < e) ? 1 : 0;
+      }
+      a.group_order[rank] = e;
+    }
+  }
+  const int tiles = goff[a.n_local] / 128, all_tiles = static_cast<int>((a.cap_rows + 127) / 128);
+  for (int t = tid; t < all_tiles; t += 1024) {
+    int e = -1;
+    if (t < tiles) {
+      int lo = 0, hi = a.n_local;  // largest e with goff[e] <= row
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (goff[mid] <= t * 128) lo = mid; else hi = mid;
+      }
+      e = lo;
+      if (a.tile_rows != nullptr) a.tile_rows[t] = max(0, min(128, goff[e] + a.counts_kept[e] - t * 128));
+      if (a.pair_tile != nullptr) {
+        const int in_group = t - goff[e] / 128;
+        if ((in_group & 1) == 0) a.pair_tile[next[e] + in_group / 2] = 2 * t + (goff[e + 1] <= (t + 1) * 128 ? 1 : 0);
+      }
+    }
+    a.tile_group[t] = e;
+  }
+}
+
 struct PlanShape {
   int nbins, unit_slots, n_units;
   bool single, scan, wide;  // wide: the ranking kernel's working storage lies in global memory
+  bool sparse;              // few slots over bins that do not fit the ranking kernel's shared memory
   PlanShape(long long n_slots, int n_local, int K, int per_k_bins) {
     nbins = n_local * (per_k_bins ? K : 1);
     single = n_slots <= kSingleSlots && rank_words(kWarpsSingle, nbins, n_local) * 4 <= kSmemLimit;
     wide = !single && rank_words(kWarpsMulti, nbins, n_local) * 4 > kSmemLimit;
+    sparse = wide && n_slots <= kSparseSlots;
     // a unit has at least as many slots as bins twice over, so that its histogram is not larger than its slots
     unit_slots = single ? static_cast<int>((n_slots + 1023) / 1024 * 1024) : 1024 * ((nbins + 511) / 512);
     n_units = single ? 1 : static_cast<int>((n_slots + unit_slots - 1) / unit_slots);
     scan = !single && static_cast<long long>(n_units) * nbins > kRedundantWords;
   }
+  bool sparse_in_smem() const { return 8ll * nbins <= kSmemLimit; }
   long long hist_words() const { return single ? 0 : (static_cast<long long>(n_units) + 1) * nbins; }
 };
 
@@ -335,6 +482,7 @@ struct PlanShape {
 
 size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_bins) {
   const PlanShape s(n_slots, n_local, K, per_k_bins);
+  if (s.sparse) return s.sparse_in_smem() ? 1 : 2 * static_cast<size_t>(s.nbins);
   const long long work = s.wide ? s.n_units * rank_words(kWarpsMulti, s.nbins, n_local) : 0;
   return static_cast<size_t>(s.hist_words() + work + 1);
 }
@@ -346,14 +494,21 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(plan_rank_kernel<kWarpsSingle, true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(plan_rank_kernel<kWarpsMulti, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSmemLimit);
+    e = cudaFuncSetAttribute(plan_rank_kernel<kWarpsMulti, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSmemLimit);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(plan_sparse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   }();
   if (configured != cudaSuccess) return configured;
   if (s.single) {
     const size_t smem = rank_words(kWarpsSingle, s.nbins, a.n_local) * 4;
     return launch_chained(plan_rank_kernel<kWarpsSingle, true>, 1, kWarpsSingle * 32, smem, stream, a, s.nbins,
                           s.unit_slots, 1, 0, nullptr);
+  }
+  if (s.sparse) {
+    const bool in_smem = s.sparse_in_smem();
+    return launch_chained(plan_sparse_kernel, 1, 1024, in_smem ? 8ull * s.nbins : 0, stream, a, s.nbins,
+                          in_smem ? nullptr : a.scratch);
   }
   const bool hist_in_smem = s.nbins * 4 <= 48 * 1024;
   cudaError_t e = launch_chained(plan_count_kernel, s.n_units, kCountThreads, hist_in_smem ? s.nbins * 4 : 0, stream, a,
