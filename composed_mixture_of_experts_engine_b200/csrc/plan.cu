@@ -487,27 +487,29 @@ size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_b
   return static_cast<size_t>(s.hist_words() + work + 1);
 }
 
+// Launches with more than the 48 KiB of shared memory that need no asking for.  Asked for on every such call: the answer
+// belongs to one device, and a process may plan on several.
+template <typename... P, typename... A>
+static cudaError_t launch_large(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                A&&... args) {
+  if (smem > 47 * 1024) {  // the rest is for the kernels' fixed arrays
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_chained(kernel, grid, threads, smem, stream, std::forward<A>(args)...);
+}
+
 cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
   if (a.n_slots <= 0 || a.n_local <= 0) return cudaErrorInvalidValue;
   const PlanShape s(a.n_slots, a.n_local, a.K, a.per_k_bins);
-  static const cudaError_t configured = [] {
-    cudaError_t e = cudaFuncSetAttribute(plan_rank_kernel<kWarpsSingle, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(plan_rank_kernel<kWarpsMulti, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmemLimit);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(plan_sparse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-  }();
-  if (configured != cudaSuccess) return configured;
   if (s.single) {
     const size_t smem = rank_words(kWarpsSingle, s.nbins, a.n_local) * 4;
-    return launch_chained(plan_rank_kernel<kWarpsSingle, true>, 1, kWarpsSingle * 32, smem, stream, a, s.nbins,
+    return launch_large(plan_rank_kernel<kWarpsSingle, true>, 1, kWarpsSingle * 32, smem, stream, a, s.nbins,
                           s.unit_slots, 1, 0, nullptr);
   }
   if (s.sparse) {
     const bool in_smem = s.sparse_in_smem();
-    return launch_chained(plan_sparse_kernel, 1, 1024, in_smem ? 8ull * s.nbins : 0, stream, a, s.nbins,
+    return launch_large(plan_sparse_kernel, 1, 1024, in_smem ? 8ull * s.nbins : 0, stream, a, s.nbins,
                           in_smem ? nullptr : a.scratch);
   }
   const bool hist_in_smem = s.nbins * 4 <= 48 * 1024;
@@ -517,7 +519,7 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
   if (s.scan) e = launch_chained(plan_scan_kernel, (s.nbins + 31) / 32, 1024, 0, stream, a, s.nbins, s.n_units);
   if (e != cudaSuccess) return e;
   const size_t smem = s.wide ? 0 : rank_words(kWarpsMulti, s.nbins, a.n_local) * 4;
-  return launch_chained(plan_rank_kernel<kWarpsMulti, false>, s.n_units, kWarpsMulti * 32, smem, stream, a, s.nbins,
+  return launch_large(plan_rank_kernel<kWarpsMulti, false>, s.n_units, kWarpsMulti * 32, smem, stream, a, s.nbins,
                         s.unit_slots, s.n_units, s.scan ? 1 : 0, s.wide ? a.scratch + s.hist_words() : nullptr);
 }
 

@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
     (400, 8, 1024, 5, 0, 1024),     # capacity per (expert, k)
     (512, 8, 4500, 0, 0, 4500),     # the most slots of this launch
     (513, 8, 4500, 0, 0, 4500),     # one token more: the general launches
+    (200, 4, 6144, 0, 0, 6144),     # exactly 48 KiB of shared memory
     (37, 4, 9000, 0, 1000, 5000),   # experts of one rank only
     (100, 2, 40000, 0, 0, 40000),   # bins beyond shared memory
 ])
