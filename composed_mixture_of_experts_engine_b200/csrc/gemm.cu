@@ -101,6 +101,7 @@ struct KParams {
   PeerTable scatter_out;
   long long scatter_ld;
   int b_early;     // B does not depend on the kernel before this one
+  int chained;     // launched to overlap its neighbours in the stream
   int out_mode;    // OutMode (EPI_STORE only)
   int fwd_staged;  // SwiGLU forward: h (tmD) and gate|up (tmE) leave through the staging area and TMA stores
   int bwd_staged;  // SwiGLU backward: dGate|dUp (tmE) leave through the piece's own staging buffer and TMA stores
@@ -310,9 +311,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int b_warp = (blockDim.x >> 5) - 1;  // behind the epilogue warps and, where there are any, the pull warps
   // what the kernel before this one wrote (or still reads) is touched behind this line only; weights that nobody writes
   // and the row plan, which is older than that kernel, may be loaded ahead of it
+  // (a launch that waits for other ranks lets no successor start: its CTAs would take SM resources while this one spins)
   if (!(p.b_early && warp == b_warp)) {
     chain_wait();
-    chain_trigger();
+    if (p.chained) chain_trigger();
   }
 
   int m_tiles;
@@ -990,7 +992,7 @@ cudaError_t launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (kp.pull_row_slot == nullptr && kp.scatter_row_slot == nullptr && kp.ready_flags == nullptr)
+  if (kp.chained)
     return launch_chained(gemm_kernel<EPI>, grid, GEMM_THREADS, SMEM_BYTES, stream, tmA, tmB, tmD, tmE, kp);
   const int threads = kp.pull_row_slot != nullptr ? GEMM_THREADS_PULL : GEMM_THREADS;  // exchange with other ranks
   gemm_kernel<EPI><<<grid, threads, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmE, kp);
@@ -1114,7 +1116,8 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.ready_count = a.ready_count;
   kp.ready_target = a.ready_target;
   kp.status = a.status;
-  kp.b_early = a.b_early;
+  kp.chained = gemm_overlaps_neighbours(a);
+  kp.b_early = a.b_early && kp.chained;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
   kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? 128 : BN;
 

@@ -120,6 +120,12 @@ struct GemmArgs {
   int num_sms = 0;                    // 0: query the current device
 };
 
+// Whether a launch may start before its predecessor in the stream has ended and let its successor do the same: not where
+// it exchanges rows with other ranks (and may wait for them).
+inline bool gemm_overlaps_neighbours(const GemmArgs& a) {
+  return a.pull_row_slot == nullptr && a.scatter_row_slot == nullptr && a.ready_flags == nullptr;
+}
+
 // Enqueues the GEMM on `stream`.  Returns cudaSuccess or the first CUDA error met while
 // encoding tensor maps or launching.
 cudaError_t launch_gemm(const GemmArgs& args, cudaStream_t stream);

@@ -17,3 +17,13 @@ def test_chained_kernels_take_plain_pointers(name):
     for k in chained:
         signature = k[: k.index("{")]
         assert "__restrict__" not in signature, signature
+
+
+def test_launches_that_wait_for_other_ranks_hold_their_successor_back():
+    """A successor that starts early would occupy the SMs while this kernel waits for its peers; `chained` is set by
+    `gemm_overlaps_neighbours` (csrc/gemm.cuh), which no launch with a row pull, a scatter or ready flags passes."""
+    text = (CSRC_DIR / "gemm.cu").read_text()
+    triggers = re.findall(r".*chain_trigger\(\);", text)
+    assert triggers and all("if (p.chained)" in line for line in triggers)
+    rule = re.search(r"inline bool gemm_overlaps_neighbours\(.*?\{(.*?)\}", (CSRC_DIR / "gemm.cuh").read_text(), re.S).group(1)
+    assert all(f"a.{name} == nullptr" in rule for name in ("pull_row_slot", "scatter_row_slot", "ready_flags"))
