@@ -124,7 +124,8 @@ __device__ __forceinline__ int total_tiles(const KParams& p, int m_tiles, int n_
   return (p.mode == GEMM_GROUPED_K ? p.groups : 1) * m_tiles * n_tiles;
 }
 
-__device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles, int n_tiles) {
+// `ahead`: called by the warp that does not wait for the predecessor
+__device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles, int n_tiles, bool ahead = false) {
   Tile ti;
   ti.skip = false;
   ti.pieces = 4;
@@ -151,7 +152,7 @@ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t, int m_tiles
     ti.b_k0 = 0;
     ti.k_blocks = (p.K + BK - 1) / BK;
   } else if (p.mode == GEMM_GROUPED_M) {
-    g = p.tile_group[mt];
+    g = ahead ? load_ahead_of_wait(p.tile_group + mt) : p.tile_group[mt];
     ti.group = g;
     if (p.tile_rows != nullptr) ti.pieces = (p.tile_rows[mt] + PIECE_ROWS - 1) / PIECE_ROWS;
     if (g < 0) {
@@ -312,14 +313,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // what the kernel before this one wrote (or still reads) is touched behind this line only; weights that nobody writes
   // and the row plan, which is older than that kernel, may be loaded ahead of it
   // (a launch that waits for other ranks lets no successor start: its CTAs would take SM resources while this one spins)
-  if (!(p.b_early && warp == b_warp)) {
+  const bool ahead = p.b_early && warp == b_warp;
+  if (!ahead) {
     chain_wait();
     if (p.chained) chain_trigger();
   }
 
   int m_tiles;
   if (p.mode == GEMM_GROUPED_M) {
-    m_tiles = *p.num_m_tiles;
+    m_tiles = ahead ? load_ahead_of_wait(p.num_m_tiles) : *p.num_m_tiles;
   } else {
     m_tiles = (p.M + BM - 1) / BM;
   }
@@ -387,7 +389,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int stage = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
-        const Tile ti = decode_tile(p, t, m_tiles, n_tiles);
+        const Tile ti = decode_tile(p, t, m_tiles, n_tiles, ahead);
         if (ti.skip || ti.k_blocks == 0) continue;
         for (int kb = 0; kb < ti.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;

@@ -84,7 +84,8 @@ struct Tile2 {
   bool lone;      // only the first CTA has rows
 };
 
-__device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, int n_tiles, int cta) {
+// `ahead`: called by the warp that does not wait for the predecessor
+__device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, int n_tiles, int cta, bool ahead = false) {
   Tile2 ti;
   int g = 0;
   if (p.mode == GEMM_GROUPED_K) {
@@ -108,10 +109,10 @@ __device__ __forceinline__ Tile2 decode2(const K2Params& p, int t, int m_tiles, 
     ti.a_k0 = ti.b_k0 = r0;
     ti.k_blocks = (r1 - r0 + T_BK - 1) / T_BK;
   } else if (p.mode == GEMM_GROUPED_M) {
-    const int v = p.pair_tile[mt];
+    const int v = ahead ? load_ahead_of_wait(p.pair_tile + mt) : p.pair_tile[mt];
     ti.m0 = (v >> 1) * 128;
     ti.lone = (v & 1) != 0;
-    g = p.tile_group[v >> 1];
+    g = ahead ? load_ahead_of_wait(p.tile_group + (v >> 1)) : p.tile_group[v >> 1];
     if (p.b_mn) {
       ti.b_k0 = g * p.b_group_rows;
     } else {
@@ -244,12 +245,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 
   // what the kernel before this one wrote (or still reads) is touched behind this line only; weights that nobody writes
   // and the row plan, which is older than that kernel, may be loaded ahead of it
-  if (!(p.b_early && warp == 2 + 4 * GROUPS)) {
+  const bool ahead = p.b_early && warp == 2 + 4 * GROUPS;
+  if (!ahead) {
     chain_wait();
     chain_trigger();
   }
 
-  const int m_tiles = p.mode == GEMM_GROUPED_M ? *p.num_pairs : (p.M + T_BM - 1) / T_BM;
+  const int m_tiles = p.mode == GEMM_GROUPED_M ? (ahead ? load_ahead_of_wait(p.num_pairs) : *p.num_pairs) : (p.M + T_BM - 1) / T_BM;
   const int n_tiles = (p.N + p.cols_per_tile - 1) / p.cols_per_tile;
   const int n_total = (p.mode == GEMM_GROUPED_K ? p.groups : 1) * m_tiles * n_tiles;
   const int cluster_id = blockIdx.x >> 1;
@@ -270,7 +272,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       for (int r0 = 0; r0 < n_total; r0 += n_clusters) {
         const int t = tile_of_round(p, r0, cluster_id, n_clusters);
         if (t >= n_total) break;  // in the last round only
-        const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta));
+        const Tile2 ti = decode2(p, t, m_tiles, n_tiles, static_cast<int>(cta), ahead);
         if (ti.k_blocks == 0) continue;
         const int x = is_a ? ti.m0 + moff : ti.b_n;
         int k = is_a ? ti.a_k0 : ti.b_k0;

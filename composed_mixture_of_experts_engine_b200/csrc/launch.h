@@ -37,6 +37,9 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, si
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A table that the kernel before the predecessor (or an older one) wrote, read without waiting for the predecessor: past
+// L1, which the wait would have made coherent.
+__device__ __forceinline__ int load_ahead_of_wait(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 

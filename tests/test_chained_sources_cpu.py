@@ -27,3 +27,12 @@ def test_launches_that_wait_for_other_ranks_hold_their_successor_back():
     assert triggers and all("if (p.chained)" in line for line in triggers)
     rule = re.search(r"inline bool gemm_overlaps_neighbours\(.*?\{(.*?)\}", (CSRC_DIR / "gemm.cuh").read_text(), re.S).group(1)
     assert all(f"a.{name} == nullptr" in rule for name in ("pull_row_slot", "scatter_row_slot", "ready_flags"))
+
+
+@pytest.mark.parametrize("name", ["gemm.cu", "gemm2.cu"])
+def test_tables_read_ahead_of_the_wait_bypass_l1(name):
+    """The warp that loads weights without waiting for the predecessor reads the row plan past L1."""
+    text = (CSRC_DIR / name).read_text()
+    for table in ("tile_group", "num_m_tiles") if name == "gemm.cu" else ("tile_group", "pair_tile", "num_pairs"):
+        assert re.search(rf"ahead \? load_ahead_of_wait\(p\.{table}", text), table
+    assert len(re.findall(r"= decode(?:_tile|2)\(.*, ahead\);", text)) == 1
