@@ -78,9 +78,12 @@ struct RouterParams {
   unsigned long long timeout_ns;
 };
 
-// row stride (floats) of the logits tile in shared memory: 4 more than a multiple of 32 banks, so that both the
+// groups of eight experts per lane, the kernel's template argument
+__host__ __device__ constexpr int rt_groups(int E) { return E <= 32 ? 1 : E <= 64 ? 2 : E <= 128 ? 4 : 8; }
+// row stride (floats) of the logits tile in shared memory: room for every expert that the lanes of that variant look at
+// (the columns past E are masked out, but no other row's), and 4 more than a multiple of 32 banks, so that both the
 // 16-byte stores of 32 neighbouring rows and the reads of 8 rows x 4 lanes touch every bank once
-__host__ __device__ constexpr int rt_row_stride(int E) { return (E + 31) / 32 * 32 + 4; }
+__host__ __device__ constexpr int rt_row_stride(int groups) { return 32 * groups + 4; }
 // per-CTA tables behind the pipeline stages (bytes); the barriers come first
 constexpr int RT_TABLES = 1024 /* barriers, slots */ + RT_BM * 4 /* 1/sum */ + RT_BM * 4 /* lse^2 */ + RT_EPI * 4 /* column partials */ +
                           kRouterMaxExperts * 4 /* counts */ + 2 * kRouterMaxTopK * RT_BM * 4 /* picks */;
@@ -131,7 +134,8 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   const int b_bytes = p.n_chunks * RT_CHUNK_BYTES;
   const int a_bytes = p.rows * RT_BK * 2;
   const int stage_bytes = RT_SUB * (a_bytes + b_bytes);
-  const int SE = rt_row_stride(p.E);
+  constexpr int SE = rt_row_stride(NG);
+  static_assert(SE >= 32 * NG, "a row has a cell for every expert its lanes look at");
   const int front = max(p.stages * stage_bytes, p.rows * SE * 4);
   float* s_logit = reinterpret_cast<float*>(smem);  // [rows][SE], over the drained pipeline stages
   // behind all of A: what an MMA reads past a short tile's rows is ours
@@ -330,7 +334,7 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int j = g * 8 + q;
-          const float v = mine[4 * j];  // columns past E lie inside the row stride
+          const float v = mine[4 * j];  // columns past E lie inside the row stride, and are masked out
           const int k = j < n ? logit_key(v) : INT_MIN;
           if (k > gk[g]) {
             gk[g] = k;
@@ -716,16 +720,18 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   e = encode_bf16_2d(&tmW, a.Wg, a.H, a.E, a.E, 64);
   if (e != cudaSuccess) return e;
-  const int tile_bytes = p.rows * rt_row_stride(a.E) * 4;
+  const int tile_bytes = p.rows * rt_row_stride(rt_groups(a.E)) * 4;
   const int ring = p.stages * stage_bytes;
   int smem = (ring > tile_bytes ? ring : tile_bytes) + 1024 + RT_TABLES;
   // an MMA reads 128 rows of A whatever the tile's rows: the last stage's must end inside this CTA's shared memory
   const int reach = (p.stages * RT_SUB - 1) * p.rows * RT_BK * 2 + RT_BM * RT_BK * 2 + 1024;
   if (smem < reach) smem = reach;
-  if (a.E <= 32) return launch_router_variant<1>(tmX, tmW, p, tiles, smem, stream);
-  if (a.E <= 64) return launch_router_variant<2>(tmX, tmW, p, tiles, smem, stream);
-  if (a.E <= 128) return launch_router_variant<4>(tmX, tmW, p, tiles, smem, stream);
-  return launch_router_variant<8>(tmX, tmW, p, tiles, smem, stream);
+  switch (rt_groups(a.E)) {
+    case 1: return launch_router_variant<1>(tmX, tmW, p, tiles, smem, stream);
+    case 2: return launch_router_variant<2>(tmX, tmW, p, tiles, smem, stream);
+    case 4: return launch_router_variant<4>(tmX, tmW, p, tiles, smem, stream);
+    default: return launch_router_variant<8>(tmX, tmW, p, tiles, smem, stream);
+  }
 }
 
 cudaError_t launch_router_bwd(const RouterBwdArgs& a, cudaStream_t stream) {

@@ -12,7 +12,9 @@ pytestmark = pytest.mark.gpu
     (300, 256, 64, 8),     # short tiles
     (129, 520, 256, 8),    # experts split over a cluster of four CTAs
     (300, 512, 128, 6),    # clusters of two CTAs
-    (1000, 256, 72, 3),    # expert count between two lane variants
+    (1000, 256, 72, 3),    # the smallest expert counts of the two widest lane variants,
+    (129, 256, 136, 8),    # whose lanes look past the last expert
+    (300, 256, 224, 4),
     (20000, 256, 32, 2),   # full tiles
 ])
 def test_weights_follow_the_definition_to_the_bit(N, H, E, K):
