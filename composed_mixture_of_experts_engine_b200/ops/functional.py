@@ -88,7 +88,8 @@ class _EmbeddingFn(torch.autograd.Function):
 def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     if (torch.is_grad_enabled() and weight.requires_grad and getattr(weight, "main_grad", None) is not None
             and on_device_path(weight) and weight.dim() == 2 and weight.shape[1] % 8 == 0 and ids.dtype == torch.int64
-            and ids.numel() > 0):
+            and ids.numel() > 0 and not kernels.traced_or_dual(weight)
+            and not torch._C._are_functorch_transforms_active()):  # what the library's look-up supports and this does not
         return _EmbeddingFn.apply(ids, weight)
     return F.embedding(ids, weight)
 

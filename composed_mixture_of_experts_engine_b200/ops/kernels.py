@@ -38,8 +38,11 @@ def needs_autograd(*tensors: torch.Tensor) -> bool:
     traced (the trace would hold a native call's results as constants), or a tensor carries a forward-mode tangent,
     which the function refuses and a native call would drop.  (``torch.func`` transforms need no look: their wrappers
     have no storage, so the native calls refuse them too.)"""
-    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
-        return True
+    return (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)) or traced_or_dual(*tensors)
+
+
+def traced_or_dual(*tensors: torch.Tensor) -> bool:
+    """Whether the call is being traced or one of ``tensors`` carries a forward-mode tangent."""
     if torch.jit.is_tracing():
         return True
     # no level is open in ordinary calls; unpacking every tensor would cost a small routing call a tenth of its time

@@ -66,3 +66,34 @@ def test_a_trace_keeps_the_call(stand_ins, name, op):
     with torch.no_grad():
         traced = torch.jit.trace(calls()[name], (x,), check_trace=False)
     assert f"^{op}" in str(traced.graph)
+
+
+def embedding_weight():
+    w = torch.randn(10, H).to(torch.bfloat16).requires_grad_()
+    w.main_grad = torch.zeros(10, H)
+    return w
+
+
+def test_embedding_under_forward_mode(stand_ins):
+    w, ids = embedding_weight(), torch.tensor([3, 1, 3])
+    with fwAD.dual_level():
+        t = torch.randn_like(w)
+        y = OF.embedding(ids, fwAD.make_dual(w.detach(), t).requires_grad_())
+        assert torch.equal(fwAD.unpack_dual(y).tangent, t[ids])
+    dual_w = torch.func.jvp(lambda v: OF.embedding(ids, v), (w.detach(),), (t,))[1]
+    assert torch.equal(dual_w, t[ids])
+
+
+def test_embedding_under_vmap(stand_ins):
+    w, ids = embedding_weight(), torch.tensor([[3, 1], [3, 9]])
+    assert torch.equal(torch.func.vmap(lambda i: OF.embedding(i, w))(ids), w[ids])
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_embedding_in_a_trace(stand_ins):
+    from composed_mixture_of_experts_engine_b200.models.decoder import TokenEmbedding
+
+    emb, ids = TokenEmbedding(10, H, dtype=torch.bfloat16), torch.tensor([3, 1, 3])
+    emb.weight.main_grad = torch.zeros(10, H)
+    traced = torch.jit.trace(emb, (ids,), check_trace=False)
+    assert "aten::embedding" in str(traced.inlined_graph) and torch.equal(traced(ids + 1), emb.weight[ids + 1])
