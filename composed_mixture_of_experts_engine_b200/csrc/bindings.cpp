@@ -198,10 +198,11 @@ void router_fwd(const Tensor& X, const Tensor& Wg, int64_t K, Tensor& logits, Te
   check_cuda(cmoe::launch_router_fwd(a, cur_stream()), "launch_router_fwd");
 }
 
-void router_bwd(const Tensor& logits, const Tensor& lse, const Tensor& topk_idx, const OptTensor& grad_w,
-                const Tensor& counts, const OptTensor& grad_aux, const OptTensor& grad_z, const OptTensor& gl_bf16,
+void router_bwd(const Tensor& logits_in, const Tensor& lse, const Tensor& topk_idx, const OptTensor& grad_w,
+                const Tensor& counts_in, const OptTensor& grad_aux, const OptTensor& grad_z, const OptTensor& gl_bf16,
                 const OptTensor& gl_f32) {
-  const c10::cuda::CUDAGuard guard(logits.device());
+  const c10::cuda::CUDAGuard guard(logits_in.device());
+  const Tensor logits = cmoe::contiguous_aligned(logits_in), counts = cmoe::contiguous_aligned(counts_in);
   cmoe::RouterBwdArgs a;
   a.logits = logits.data_ptr<float>();
   a.lse = lse.data_ptr<float>();

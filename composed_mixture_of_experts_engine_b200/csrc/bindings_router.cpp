@@ -99,12 +99,13 @@ RouteResult router_route(const Tensor& X, const Tensor& Wg, int64_t K, bool full
 
 // (grad_tokens, grad_gate) from the upstream gradients of the gate weights (fp32 and / or bf16 view of the same
 // values), the load-balance loss and the z-loss: the d(logits) kernel, then the two contractions with it.
-std::tuple<OptTensor, OptTensor> router_grad(const Tensor& X, const Tensor& Wg, const Tensor& logits, const Tensor& lse,
-                                             const Tensor& idx32, const Tensor& counts, const OptTensor& grad_w32,
+std::tuple<OptTensor, OptTensor> router_grad(const Tensor& X, const Tensor& Wg, const Tensor& logits_in, const Tensor& lse,
+                                             const Tensor& idx32, const Tensor& counts_in, const OptTensor& grad_w32,
                                              const OptTensor& grad_w16, const OptTensor& grad_aux,
                                              const OptTensor& grad_z, bool need_tokens, bool need_gate, bool gate_bf16,
                                              const OptTensor& status) {
   const c10::cuda::CUDAGuard guard(X.device());
+  const Tensor logits = cmoe::contiguous_aligned(logits_in), counts = cmoe::contiguous_aligned(counts_in);
   const auto as_f32 = [](const OptTensor& t) {
     return t.has_value() ? OptTensor(t->to(at::kFloat).contiguous()) : OptTensor();
   };

@@ -78,6 +78,11 @@ int wgrad_pieces(int64_t R, int64_t M, int64_t N, int sms) {
 
 }  // namespace
 
+Tensor contiguous_aligned(const Tensor& t) {
+  if (!t.is_contiguous()) return t.contiguous();
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+
 void launch_gemm_any(const GemmArgs& g, cudaStream_t stream) {
   static const bool two_cta = [] {
     const char* v = std::getenv("CMOE_GEMM_2CTA");

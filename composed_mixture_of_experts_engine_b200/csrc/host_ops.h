@@ -6,6 +6,10 @@
 
 namespace cmoe {
 
+// `t`, or a contiguous copy on a 16-byte boundary where it is not that already (saved tensors may come back from a hook in
+// any layout)
+torch::Tensor contiguous_aligned(const torch::Tensor& t);
+
 // Launches `g` on the two-SM kernel where it qualifies (CMOE_GEMM_2CTA=0: never), on the one-CTA kernel otherwise.
 void launch_gemm_any(const GemmArgs& g, cudaStream_t stream);
 

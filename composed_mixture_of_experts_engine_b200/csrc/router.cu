@@ -735,7 +735,9 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
 }
 
 cudaError_t launch_router_bwd(const RouterBwdArgs& a, cudaStream_t stream) {
-  if (a.E <= 0 || a.E > kRouterMaxExperts || a.E % 8 != 0 || a.K <= 0 || a.K > kRouterMaxTopK || a.n_tokens <= 0)
+  const auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };  // 16-byte vectors throughout
+  if (a.E <= 0 || a.E > kRouterMaxExperts || a.E % 8 != 0 || a.K <= 0 || a.K > kRouterMaxTopK || a.n_tokens <= 0 ||
+      off16(a.logits) || off16(a.counts) || off16(a.grad_logits_f32) || off16(a.grad_logits_bf16))
     return cudaErrorInvalidValue;
   const unsigned grid = static_cast<unsigned>((a.n_tokens * 8 + 255) / 256);
   return launch_chained(router_bwd_kernel, grid, 256, 0, stream, a);
