@@ -30,6 +30,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 
@@ -780,6 +781,7 @@ cudaError_t launch_fwd_t(const AttnFwdArgs& a, const CUtensorMap& tm, const FwdP
   });
   if (attr_err != cudaSuccess) return attr_err;
   dim3 grid(a.S / BLK, a.nh, a.B);
+  count_launch();
   attention_fwd_kernel<HD><<<grid, ATTN_THREADS, smem, stream>>>(tm, p, smem);
   return cudaGetLastError();
 }
@@ -795,6 +797,7 @@ cudaError_t launch_bwd_t(const AttnBwdArgs& a, const CUtensorMap& tq, const CUte
   });
   if (attr_err != cudaSuccess) return attr_err;
   dim3 grid(a.S / BLK, a.nkv, a.B);
+  count_launch();
   attention_bwd_kernel<HD><<<grid, ATTN_THREADS, smem, stream>>>(tq, td, tdq, p, smem);
   return cudaGetLastError();
 }
@@ -861,6 +864,7 @@ cudaError_t launch_attention_bwd(const AttnBwdArgs& a, cudaStream_t stream) {
     const long long warps = rows * a.nh;
     const int threads = 256;
     const long long blocks = (warps * 32 + threads - 1) / threads;
+    count_launch();
     attention_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
         reinterpret_cast<const __nv_bfloat16*>(a.out), reinterpret_cast<const __nv_bfloat16*>(a.dout), a.delta, rows,
         a.S, a.nh, a.hd);

@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include "attention.cuh"
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 namespace {
@@ -385,6 +386,7 @@ extern "C" int cmoe_attention_fwd2(const void* qkv, void* out, float* lse, int B
   constexpr int smem = Fwd2Smem<128>::END + 1024;
   e = cudaFuncSetAttribute(attention_fwd2_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
+  count_launch();
   attention_fwd2_kernel<128><<<grid, THREADS2, smem, (cudaStream_t)stream>>>(tm, p, smem);
   return (int)cudaGetLastError();
 }

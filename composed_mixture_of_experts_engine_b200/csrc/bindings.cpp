@@ -13,6 +13,7 @@
 
 #include "gemm.cuh"
 #include "host_ops.h"
+#include "launch.h"
 #include "ops.cuh"
 #include "router.cuh"
 
@@ -447,6 +448,7 @@ void register_moe(pybind11::module_& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "sm_100a kernels of the composed MoE engine";
+  m.def("kernel_launches", [] { return cmoe::g_kernel_launches.load(); });  // by this process so far
   m.def("gemm", &gemm);
   m.def("wgrad", &wgrad);
   m.def("gemm_pull", &gemm_pull);

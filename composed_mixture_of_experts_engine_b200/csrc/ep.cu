@@ -10,6 +10,7 @@
 #include "ep.cuh"
 
 #include "common.cuh"
+#include "launch.h"
 
 namespace cmoe {
 
@@ -337,6 +338,7 @@ cudaError_t set_peer_status_word(int* status) {
 cudaError_t launch_peer_barrier(const PeerTable& flags, int rank, int world, uint32_t epoch, int* status,
                                 unsigned long long timeout_ns, cudaStream_t stream) {
   if (world <= 0 || world > kMaxPeers || rank < 0 || rank >= world) return cudaErrorInvalidValue;
+  count_launch();
   peer_barrier_kernel<<<1, 32, 0, stream>>>(flags, rank, world, epoch, status,
                                             timeout_ns ? timeout_ns : kDefaultTimeoutNs);
   return cudaGetLastError();
@@ -345,6 +347,7 @@ cudaError_t launch_peer_barrier(const PeerTable& flags, int rank, int world, uin
 cudaError_t launch_peer_allgather(const PeerTable& src, int world, long long n_bytes, void* out, cudaStream_t stream) {
   if (n_bytes % 16 != 0 || world <= 0 || world > kMaxPeers) return cudaErrorInvalidValue;
   const long long n_vec = n_bytes / 16;
+  count_launch();
   peer_allgather_kernel<<<blocks_for(n_vec * world, 256, 148 * 4), 256, 0, stream>>>(src, world, n_vec,
                                                                                      reinterpret_cast<uint4*>(out));
   return cudaGetLastError();
@@ -354,6 +357,7 @@ cudaError_t launch_gather_rows_peer(const PeerTable& src, long long slots_per_sr
                                     const float* slot_scale, void* out, long long cap_rows, const int* num_m_tiles,
                                     int H, long long ld_src, long long ld_out, cudaStream_t stream) {
   if (H % 8 != 0 || cap_rows <= 0 || K <= 0 || slots_per_src <= 0) return cudaErrorInvalidValue;
+  count_launch();
   gather_rows_peer_kernel<<<blocks_for(cap_rows, 8, 148 * 8), 256, 0, stream>>>(
       src, slots_per_src, K, row_slot, slot_scale, reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H,
       ld_src, ld_out);
@@ -375,6 +379,7 @@ cudaError_t launch_combine_rows_peer(const PeerTable& rows, const PeerTable& slo
     auto lr = reinterpret_cast<const __nv_bfloat16*>(local_rows);
 #define CMOE_COMBINE_PEER_CASE(KK)                                                                                  \
   case KK:                                                                                                          \
+    count_launch();                                                                                                   \
     combine_rows_peer_k_kernel<KK><<<grid, 256, 0, stream>>>(rows, slot_row, idx, expert_rank, w, yb, n_tokens, H,  \
                                                              slot_base, ld_rows, ld_y, lr);                         \
     return cudaGetLastError();
@@ -389,6 +394,7 @@ cudaError_t launch_combine_rows_peer(const PeerTable& rows, const PeerTable& slo
     }
 #undef CMOE_COMBINE_PEER_CASE
   }
+  count_launch();
   combine_rows_peer_kernel<<<blocks_for(n_tokens, 8, 148 * 8), 256, 0, stream>>>(
       rows, slot_row, idx, expert_rank, w, reinterpret_cast<__nv_bfloat16*>(y), n_tokens, K, H, slot_base, ld_rows,
       ld_y, reinterpret_cast<const __nv_bfloat16*>(local_rows));
@@ -400,6 +406,7 @@ cudaError_t launch_combine_bwd_w_peer(const PeerTable& rows, const PeerTable& sl
                                       int H, long long slot_base, long long ld_rows, long long ld_dy,
                                       const void* local_rows, cudaStream_t stream) {
   if (H % 8 != 0 || n_tokens <= 0 || K <= 0) return cudaErrorInvalidValue;
+  count_launch();
   combine_bwd_w_peer_kernel<<<blocks_for(n_tokens * K, 8, 148 * 8), 256, 0, stream>>>(
       rows, slot_row, idx, expert_rank, reinterpret_cast<const __nv_bfloat16*>(dy), dw, n_tokens, K, H, slot_base,
       ld_rows, ld_dy, reinterpret_cast<const __nv_bfloat16*>(local_rows));
@@ -411,6 +418,7 @@ cudaError_t launch_reduce_scatter_cast(const PeerTable& grads, int world, int gr
   if (world <= 0 || world > kMaxPeers || n <= 0 || n % 8 != 0 || shard_lo % 8 != 0) return cudaErrorInvalidValue;
   const long long n_vec = n / (grad_is_bf16 ? 8 : 4);
   const unsigned grid = blocks_for(n_vec, 256, 148 * 8);
+  count_launch();
   if (grad_is_bf16)
     reduce_scatter_cast_kernel<true><<<grid, 256, 0, stream>>>(grads, world, shard_lo, n, scale, out);
   else
@@ -421,6 +429,7 @@ cudaError_t launch_reduce_scatter_cast(const PeerTable& grads, int world, int gr
 cudaError_t launch_reduce_rows_peer(const PeerTable& rows, int world, const int* row_map, void* out, long long n_out,
                                     int H, long long ld_rows, long long ld_out, cudaStream_t stream) {
   if (world <= 0 || world > kMaxPeers || n_out <= 0 || H % 8 != 0) return cudaErrorInvalidValue;
+  count_launch();
   reduce_rows_peer_kernel<<<blocks_for(n_out, 8, 148 * 8), 256, 0, stream>>>(
       rows, world, row_map, reinterpret_cast<__nv_bfloat16*>(out), n_out, H, ld_rows, ld_out);
   return cudaGetLastError();
@@ -429,6 +438,7 @@ cudaError_t launch_reduce_rows_peer(const PeerTable& rows, int world, const int*
 cudaError_t launch_push_shard(const PeerTable& params, int rank, int world, long long shard_lo, long long n,
                               cudaStream_t stream) {
   if (world <= 0 || world > kMaxPeers || n <= 0 || n % 8 != 0 || shard_lo % 8 != 0) return cudaErrorInvalidValue;
+  count_launch();
   push_shard_kernel<<<blocks_for(n / 8, 256, 148 * 8), 256, 0, stream>>>(params, rank, world, shard_lo, n / 8);
   return cudaGetLastError();
 }

@@ -997,6 +997,7 @@ cudaError_t launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const
   if (kp.chained)
     return launch_chained(gemm_kernel<EPI>, grid, GEMM_THREADS, SMEM_BYTES, stream, tmA, tmB, tmD, tmE, kp);
   const int threads = kp.pull_row_slot != nullptr ? GEMM_THREADS_PULL : GEMM_THREADS;  // exchange with other ranks
+  count_launch();
   gemm_kernel<EPI><<<grid, threads, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmE, kp);
   return cudaGetLastError();
 }

@@ -15,9 +15,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <utility>
 
 namespace cmoe {
+
+// Kernels that this process has launched through the package, for whoever reports them.
+inline std::atomic<long long> g_kernel_launches{0};
+inline void count_launch() { g_kernel_launches.fetch_add(1, std::memory_order_relaxed); }
 
 template <typename... P, typename... A>
 cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
@@ -32,6 +37,7 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, si
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  count_launch();
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 

@@ -669,6 +669,7 @@ static cudaError_t launch_router_variant(const CUtensorMap& tmX, const CUtensorM
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.split > 1 ? 2 : 1;
+  count_launch();
   return cudaLaunchKernelEx(&cfg, router_fwd_kernel<NG>, tmX, tmW, p);
 }
 

@@ -164,13 +164,12 @@ def build_io_lib(force: bool = False) -> Path:
     return IO_LIB
 
 
-# kernels launched by one call of each entry point (cudaMemsetAsync calls are not counted)
-_KERNELS_PER_CALL = {"moe_plan": 2, "moe_plan_scratch_words": 0, "router_grad": 3, "moe_local_forward": 5, "moe_local_backward": 7}
-_launch_counts: dict = {}
+_call_counts: dict = {}
+_launch_base = 0
 
 
 class _CountingExt:
-    """The extension module with a per-entry-point call counter (what ``bench.py`` reports as launches)."""
+    """The extension module with a per-entry-point call counter."""
 
     def __init__(self, mod: ModuleType):
         self._mod = mod
@@ -182,10 +181,9 @@ class _CountingExt:
             raw = getattr(self._mod, name)
             if not callable(raw):
                 return raw
-            per_call = _KERNELS_PER_CALL.get(name, 1)
 
-            def fn(*args, __raw=raw, __name=name, __n=per_call, **kwargs):
-                _launch_counts[__name] = _launch_counts.get(__name, 0) + __n
+            def fn(*args, __raw=raw, __name=name, **kwargs):
+                _call_counts[__name] = _call_counts.get(__name, 0) + 1
                 return __raw(*args, **kwargs)
 
             self._cache[name] = fn
@@ -210,15 +208,20 @@ def ext() -> _CountingExt:
 
 
 def reset_launch_counts() -> None:
-    _launch_counts.clear()
+    global _launch_base
+    _call_counts.clear()
+    _launch_base = ext()._mod.kernel_launches()
 
 
 def launch_counts() -> dict:
-    return dict(_launch_counts)
+    """Calls of each entry point since the last reset."""
+    return dict(_call_counts)
 
 
 def launch_counts_total() -> int:
-    return int(sum(_launch_counts.values()))
+    """Kernels of this package launched by this process since the last reset (counted where they are launched; a replayed
+    graph's kernels count once, when they are captured)."""
+    return int(ext()._mod.kernel_launches() - _launch_base)
 
 
 def available() -> bool:
