@@ -34,11 +34,10 @@
 #include "router.cuh"
 
 #include <climits>
-#include <cstdio>
-#include <mutex>
 
 #include "common.cuh"
 #include "launch.h"
+#include "tensor_maps.h"
 
 namespace cmoe {
 
@@ -616,38 +615,6 @@ __global__ void __launch_bounds__(256) router_bwd_kernel(const RouterBwdArgs a) 
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn router_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  });
-  return fn;
-}
-
-cudaError_t encode_bf16_2d(CUtensorMap* out, const void* ptr, long long rows, long long cols, long long ld,
-                           int box_rows) {
-  EncodeTiledFn enc = router_encode_fn();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0 || (ld * 2) % 16 != 0) return cudaErrorInvalidValue;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estride[2] = {1u, 1u};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estride,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
 }  // namespace
 
 template <int NG>
@@ -717,9 +684,9 @@ cudaError_t launch_router_fwd(const RouterFwdArgs& a, cudaStream_t stream) {
   p.status = a.status;
   p.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
 
-  cudaError_t e = encode_bf16_2d(&tmX, a.X, a.n_tokens, a.H, a.ldx, p.rows);
+  cudaError_t e = make_tmap(&tmX, a.X, a.n_tokens, a.H, a.ldx, p.rows);
   if (e != cudaSuccess) return e;
-  e = encode_bf16_2d(&tmW, a.Wg, a.H, a.E, a.E, 64);
+  e = make_tmap(&tmW, a.Wg, a.H, a.E, a.E, 64);
   if (e != cudaSuccess) return e;
   const int tile_bytes = p.rows * rt_row_stride(rt_groups(a.E)) * 4;
   const int ring = p.stages * stage_bytes;

@@ -1,4 +1,4 @@
-// TMA descriptors of the GEMM kernels' operands and results.
+// TMA descriptors of the GEMM and router kernels' operands and results.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
