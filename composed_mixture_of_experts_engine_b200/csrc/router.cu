@@ -24,9 +24,11 @@
 // 94 -> 47 us, 64 x 2048 E 64 top-8 33 -> 25, 1000 x 2048 E 64 top-8 35 -> 25, 16384 x 2048 E 64 top-8 41 -> 35,
 // 16384 x 4096 E 64 top-2 51 -> 47 (134 MB of tokens: 21 us at the copy rate).
 //
+// Gate weights are exp(v - lse) over their sum, with lse and that sum added in a fixed order (see the epilogue).
+//
 // Backward: the analytic gradient of the gate weights, load-balance loss and z-loss with respect
-// to the logits (one warp per token); the two contractions with it (grad_tokens, grad_gate_w) run
-// on the tcgen05 GEMM of gemm.cu.
+// to the logits (eight lanes per token); the two contractions with it (grad_tokens, grad_gate_w) run
+// on the tcgen05 GEMMs (host_ops.cpp: dense_nt, dense_wgrad).
 //
 // Counterpart in the reference: the Triton kernels _router_fwd_kernel / _router_bwd_kernel plus the
 // bincount, the second logits GEMM for the z-loss and the two cuBLAS GEMMs of the backward

@@ -233,8 +233,9 @@ def moe_topk_route(tokens: torch.Tensor, gate_w: torch.Tensor, k: int, force_ref
 # module
 # --------------------------------------------------------------------------------------------------
 def _fused_stage_bytes(num_experts: int) -> int:
-    """Shared memory of one pipeline stage of the fused router kernel (csrc/router.cu): a 128-token x 64-wide bf16
-    slice of the activations plus the matching slice of the gate weights, experts padded to a multiple of 64.
+    """Shared memory of one 64-wide k-block of a full 128-token tile of the fused router kernel (csrc/router.cu): the
+    bf16 slice of the activations plus the matching slice of the gate weights, experts padded to a multiple of 64.  (A
+    pipeline stage holds two k-blocks; few tokens get shorter tiles, and wide gates are split over a cluster.)
     Reported on every path as the on-chip working set per block, like the reference's theoretical figure
     (pkg/kernels/moe_router.py:703-714)."""
     e_chunks = max(1, (num_experts + 63) // 64)
@@ -348,8 +349,7 @@ class MoERouter(nn.Module):
                 aux, z = out.stats[0], out.stats[1]
             self._last_logits, self.last_aux_loss, self.last_z_loss = out.logits, aux, z
             self.last_idx32, self.last_w32 = idx32, w32
-            self._pending = dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2,
-                                 sram=16384 + ((E + 63) // 64) * 8192)
+            self._pending = dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2)
             return idx, w, out.counts64
         # PyTorch path (bias, CPU, fp32 tokens, shapes the kernel does not cover): fp64 math under autograd
         logits64 = tokens.to(torch.float64) @ self.gate_w.to(torch.float64)
@@ -365,5 +365,5 @@ class MoERouter(nn.Module):
         self._last_logits = logits64.detach().to(tokens.dtype)
         self.last_idx32, self.last_w32 = idx.to(torch.int32), w.float()
         self._pending = dict(counts=counts, N=N, fused=False, events=None, z_loss=self.last_z_loss.detach(),
-                             aux_loss=self.last_aux_loss.detach(), elem=tokens.element_size(), sram=0)
+                             aux_loss=self.last_aux_loss.detach(), elem=tokens.element_size())
         return idx, w, counts

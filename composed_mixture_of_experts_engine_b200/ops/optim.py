@@ -6,8 +6,8 @@ fp32 reduction).  Here the same mixed-precision contract (bf16 parameters in the
 moments in the optimizer) is one kernel launch per parameter group:
 
 * parameters are re-pointed into one flat bf16 buffer per group, gradients into one flat buffer
-  (fp32 ``main_grad``: the GEMM kernels add the weight gradients of experts, projections and LM head into it
-  directly; what autograd leaves in ``p.grad`` - norm weights, router gates, embedding - is added at step time);
+  (fp32 ``main_grad``: the kernels add the weight gradients of experts, projections, LM head and token embedding into
+  it directly; what autograd leaves in ``p.grad`` - norm weights, router gates - is added at step time);
 * the global gradient norm is a device scalar (sum-of-squares kernel), so clipping needs no host round trip;
 * with data parallelism the flat gradient is reduce-scattered, the update runs on this rank's shard only, and
   the updated bf16 parameters are all-gathered (ZeRO-style sharding of master weights and moments).  Expert
