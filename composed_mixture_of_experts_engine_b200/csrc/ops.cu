@@ -77,19 +77,13 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
     }
     ss = block_sum<RN_THREADS>(ss, red);
     const float r = rsqrtf(ss / H + eps);
-    uint4 wq[VEC];  // all loads ahead of the first store
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const int c = (i * RN_THREADS + threadIdx.x) * 8;
-      if (c < H) wq[i] = *reinterpret_cast<const uint4*>(w + c);
-    }
     if (threadIdx.x == 0 && rstd) rstd[row] = r;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * RN_THREADS + threadIdx.x) * 8;
       if (c < H) {
         float wv[8], o[8];
-        unpack8(wq[i], wv);
+        load8(w + c, wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = v[i][j] * r * wv[j];
         store8(y + row * H + c, o);
@@ -735,24 +729,24 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot
         for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = make_uint4(0u, 0u, 0u, 0u);
     } else {
       const __nv_bfloat16* s = src + static_cast<long long>(slot / slot_div) * ld_src;
-      if (slot_scale == nullptr) {
-        for (int c = lane * 8; c < H; c += 1024) {  // four loads in flight
-          uint4 v[4];
+      const float sc = slot_scale != nullptr ? slot_scale[slot] : 1.f;
+      for (int c = lane * 8; c < H; c += 1024) {  // four loads in flight, all ahead of the first store
+        uint4 v[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (c + q * 256 < H) v[q] = *reinterpret_cast<const uint4*>(s + c + q * 256);
+        for (int q = 0; q < 4; ++q)
+          if (c + q * 256 < H) v[q] = *reinterpret_cast<const uint4*>(s + c + q * 256);
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (c + q * 256 < H) *reinterpret_cast<uint4*>(o + c + q * 256) = v[q];
-        }
-      } else {
-        const float sc = slot_scale[slot];
-        for (int c = lane * 8; c < H; c += 256) {
-          float f[8];
-          load8(s + c, f);
+        for (int q = 0; q < 4; ++q) {
+          if (c + q * 256 >= H) continue;
+          if (slot_scale == nullptr) {
+            *reinterpret_cast<uint4*>(o + c + q * 256) = v[q];
+          } else {
+            float f[8];
+            unpack8(v[q], f);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] *= sc;
-          store8(o + c, f);
+            for (int j = 0; j < 8; ++j) f[j] *= sc;
+            store8(o + c + q * 256, f);
+          }
         }
       }
     }
