@@ -7,6 +7,7 @@
 // MoE layer (pkg/distributed/moe_layer.py:309-353).  RoPE has no counterpart there.
 #include "ops.cuh"
 
+#include <climits>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -603,28 +604,32 @@ __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* x, const 
 // the left, [1] of one that starts here and goes on) and added up, in order, by the join kernel.  So every row of main
 // has one writer and a fixed order of additions, and a token that fills the batch is no longer a chain of dependent reads
 // in one CTA.  What bounds it: dy once and the touched rows of main twice (16384 tokens of 2048, all distinct: 67 +
-// 268 MB, 50 us at the copy rate).
+// 268 MB, 51 us at the copy rate).  Both kernels, 16384 x 2048, a CTA per run before / now: all distinct 62 / 71 us, uniform
+// over 50304 ids 58 / 79, one id 5954 to 10068 / 85, Zipf 905 / 65, every second id the same 5161 / 66.
 constexpr int kEmbSeg = 32;  // one ballot finds a piece's end and its source rows
 __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16* dy,
                                                              const long long* keys,
                                                              const long long* order,
-                                                             float* main, float* partial,
-                                                             long long n, int H) {
+                                                             float* main, float* partial, int n, int H) {
   chain_wait();
   chain_trigger();
-  const long long i = blockIdx.x;
-  const long long key = keys[i];
-  const bool from_left = i > 0 && keys[i - 1] == key;
-  if (from_left && i % kEmbSeg != 0) return;
+  const int i = blockIdx.x;
   const int lane = threadIdx.x & 31;
-  const long long piece_end = min(n, (i / kEmbSeg + 1) * kEmbSeg);
-  const bool same = i + lane < piece_end && keys[i + lane] == key;
-  const unsigned different = ~__ballot_sync(0xffffffffu, same);
-  const int len = different == 0u ? 32 : __ffs(different) - 1;
-  const long long src = same ? order[i + lane] : 0;
+  const int piece_end = min(n, (i / kEmbSeg + 1) * kEmbSeg);
+  const long long key = keys[i], k_before = keys[max(i - 1, 0)], k_next = keys[min(i + 1, n - 1)];
+  int src = static_cast<int>(order[i]);
+  int len = 1;
+  const bool from_left = i > 0 && k_before == key;
+  if (from_left && i % kEmbSeg != 0) return;
+  if (i + 1 < piece_end && k_next == key) {  // most ids stand alone and need none of this
+    const int at = min(i + lane, n - 1);
+    const unsigned different = ~__ballot_sync(0xffffffffu, i + lane < piece_end && keys[at] == key);
+    len = different == 0u ? 32 : __ffs(different) - 1;
+    src = static_cast<int>(order[at]);
+  }
   const bool goes_on = i + len == piece_end && piece_end < n && keys[piece_end] == key;
   const bool whole = !from_left && !goes_on;
-  float* out = whole ? main + key * H : partial + (i / kEmbSeg * 2 + (from_left ? 0 : 1)) * H;
+  float* out = whole ? main + key * H : partial + (i / kEmbSeg * 2ll + (from_left ? 0 : 1)) * H;
   for (int c0 = (threadIdx.x & ~31) * 8; c0 < H; c0 += blockDim.x * 8) {  // whole warps, for the shuffles
     const int c = c0 + lane * 8;
     const bool on = c < H;
@@ -635,15 +640,15 @@ __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16
       m1 = m[1];
     }
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < len; j += 4) {
-      uint4 v[4];
+    for (int j = 0; j < len; j += 2) {
+      uint4 v[2];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2; ++q) {
         const long long row = __shfl_sync(0xffffffffu, src, (j + q) & 31);
         if (on && j + q < len) v[q] = *reinterpret_cast<const uint4*>(dy + row * H + c);
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2; ++q) {
         if (on && j + q < len) {
           float f[8];
           unpack8(v[q], f);
@@ -659,9 +664,10 @@ __global__ void __launch_bounds__(256) embedding_grad_kernel(const __nv_bfloat16
   }
 }
 
-// The runs that cross a multiple of kEmbSeg: main[key] += the sums of their pieces, in order.  A CTA looks through 32
-// pieces for runs that start there and go on and takes 128 columns of each; its eight warps add an eighth of the pieces
-// each, so that a run of 16384 equal ids is 64 additions deep.
+// The runs that cross a multiple of kEmbSeg: main[key] += the sums of their pieces, in order.  A CTA looks through eight
+// pieces for runs that start there and go on and takes 128 columns of each; its eight warps add an eighth of a run's
+// pieces each, so that a run of 16384 equal ids is 64 additions deep.
+constexpr int kEmbJoin = 8;
 __global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long long* keys,
                                                                   const float* partial,
                                                                   float* main, long long n, int H) {
@@ -670,9 +676,9 @@ __global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long lon
   __shared__ float4 sums[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.y * 128 + lane * 4;
-  const long long pieces = (n + kEmbSeg - 1) / kEmbSeg, p0 = blockIdx.x * 32ll;
+  const long long p0 = static_cast<long long>(blockIdx.x) * kEmbJoin;
   bool mine = false;
-  if ((p0 + lane + 1) * kEmbSeg < n) {
+  if (lane < kEmbJoin && (p0 + lane + 1) * kEmbSeg < n) {
     const long long first = (p0 + lane) * kEmbSeg, next = first + kEmbSeg;
     const long long key = keys[next];
     mine = keys[next - 1] == key && !(first > 0 && keys[first - 1] == key);
@@ -680,12 +686,12 @@ __global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long lon
   for (unsigned todo = __ballot_sync(0xffffffffu, mine); todo != 0u; todo &= todo - 1u) {  // the same in every warp
     const long long p = p0 + __ffs(todo) - 1;
     const long long key = keys[(p + 1) * kEmbSeg];
-    long long lo = p + 1, hi = pieces;  // the last piece whose first position still belongs to the run
-    while (hi - lo > 1) {
-      const long long mid = (lo + hi) >> 1;
-      if (keys[mid * kEmbSeg] == key) lo = mid; else hi = mid;
+    long long count = 1;  // pieces of the run: those behind p whose first position still belongs to it, 32 at a time
+    for (unsigned on = ~0u; on == ~0u;) {
+      const long long q = (p + count + lane) * kEmbSeg;
+      on = __ballot_sync(0xffffffffu, q < n && keys[min(q, n - 1)] == key);
+      count += on == ~0u ? 32 : __ffs(~on) - 1;
     }
-    const long long count = lo - p + 1;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < H) {
 #pragma unroll 8
@@ -1005,13 +1011,14 @@ long long embedding_grad_partial_floats(long long n, int H) {
 cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const long long* order, float* main,
                                   float* partial, long long n, int H, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  if (H % 8 != 0 || (n > kEmbSeg && partial == nullptr)) return cudaErrorInvalidValue;
+  if (H % 8 != 0 || n > INT_MAX - kEmbSeg || (n > kEmbSeg && partial == nullptr)) return cudaErrorInvalidValue;
   const int threads = H / 8 >= 256 ? 256 : (H / 8 + 31) / 32 * 32;
   const cudaError_t e = launch_chained(embedding_grad_kernel, static_cast<unsigned>(n), threads, 0, stream,
-                                       reinterpret_cast<const __nv_bfloat16*>(dy), keys, order, main, partial, n, H);
+                                       reinterpret_cast<const __nv_bfloat16*>(dy), keys, order, main, partial,
+                                       static_cast<int>(n), H);
   if (e != cudaSuccess || n <= kEmbSeg) return e;
   const long long pieces = (n + kEmbSeg - 1) / kEmbSeg;
-  return launch_chained(embedding_grad_join_kernel, dim3(static_cast<unsigned>((pieces + 31) / 32), (H + 127) / 128), 256,
+  return launch_chained(embedding_grad_join_kernel, dim3(static_cast<unsigned>((pieces + kEmbJoin - 1) / kEmbJoin), (H + 127) / 128), 256,
                         0, stream, keys, partial, main, n, H);
 }
 

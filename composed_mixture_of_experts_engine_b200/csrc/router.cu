@@ -398,7 +398,8 @@ router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       // adds them in the order of the experts and the gate weights exp(v - lse) are added in the order of the picks,
       // whatever the tile, the cluster or the lanes: a last bit of a gate weight moves roundings in all that follows, and
       // with top-1 routing, where the weight is 1, the rounding of lse is all that its gradient consists of.  All four
-      // lanes add the same E numbers (16-byte reads that they share).
+      // lanes add the same E numbers (16-byte reads that they share).  Where only the decision is wanted this costs 1.5 us
+      // of 28 (16384 x 4096, E 64, top-2); with statistics, which need the exponentials anyway, at most one.
       const float mx = s_topv[t];
 #pragma unroll 8
       for (int j = 0; j < n; ++j) mine[4 * j] = expf(mine[4 * j] - mx);
