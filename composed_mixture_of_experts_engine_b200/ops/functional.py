@@ -65,9 +65,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.T
 
 # ------------------------------------------------------------------------------------------ token embedding
 class _EmbeddingFn(torch.autograd.Function):
-    """Embedding look-up of a weight with an fp32 ``main_grad``: the backward adds the rows of dy to it in the order of
-    the sorted ids (equal ids in token order, so equal inputs give equal bits) instead of filling a dense bf16 gradient
-    that is then added to it."""
+    """Embedding look-up of a weight with an fp32 ``main_grad``: the backward adds the rows of dy to it, equal ids in a
+    fixed order (token order within pieces of a run, so equal inputs give equal bits), instead of filling a dense bf16
+    gradient that is then added to it."""
 
     @staticmethod
     def forward(ctx, ids, weight):

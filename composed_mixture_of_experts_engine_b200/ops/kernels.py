@@ -139,9 +139,14 @@ def linear_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     side and are added in order (csrc/host_ops.cpp).  An ``out`` that the kernels cannot write to (another type, no unit
     inner stride, rows off 16-byte boundaries) or add to (bf16) takes the fp32 result by an ordinary copy or addition."""
     if out is None:
-        out, accumulate = torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=out_dtype), False
-    direct = (out.dtype == torch.float32 or (out.dtype == torch.bfloat16 and not accumulate)) and (
-        out.stride(1) == 1 and out.stride(0) * out.element_size() % 16 == 0 and out.data_ptr() % 16 == 0)
+        out, accumulate, direct = torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=out_dtype), False, True
+    elif out.data_ptr() % 16 != 0:
+        direct = False
+    elif out.dtype == torch.float32 and out.is_contiguous() and out.stride(0) % 4 == 0:  # the gradient buffers
+        direct = True
+    else:
+        direct = ((out.dtype == torch.float32 or (out.dtype == torch.bfloat16 and not accumulate))
+                  and out.stride(1) == 1 and out.stride(0) * out.element_size() % 16 == 0)
     res = out if direct else torch.empty(a.shape[1], b.shape[1], device=a.device, dtype=torch.float32)
     _ext.ext().wgrad(a, b, res, accumulate and direct, status_word(a.device), splits)
     if not direct:
