@@ -420,6 +420,29 @@ void gather_rows(const Tensor& src, const Tensor& row_slot, int64_t slot_div, co
                                       out.stride(0), cur_stream()),
              "gather_rows");
 }
+void place_rows(const Tensor& src, const Tensor& slot_row, int64_t K, const Tensor& group_offsets, const Tensor& counts_kept,
+                Tensor& out, bool zero_padding) {
+  const c10::cuda::CUDAGuard guard(src.device());
+  check_rows(src, "src");
+  check_rows(out, "out");
+  TORCH_CHECK(slot_row.numel() == src.size(0) * K && out.size(1) == src.size(1) &&
+                  group_offsets.numel() == counts_kept.numel() + 1,
+              "place_rows: sizes do not match");
+  cmoe::PlaceRowsArgs a;
+  a.src = src.data_ptr();
+  a.n_tokens = src.size(0);
+  a.ld_src = src.stride(0);
+  a.slot_row = slot_row.data_ptr<int>();
+  a.K = static_cast<int>(K);
+  a.H = static_cast<int>(src.size(1));
+  a.out = out.data_ptr();
+  a.ld_out = out.stride(0);
+  a.zero_padding = zero_padding;
+  a.group_offsets = group_offsets.data_ptr<int>();
+  a.counts_kept = counts_kept.data_ptr<int>();
+  a.n_local = static_cast<int>(counts_kept.numel());
+  check_cuda(cmoe::launch_place_rows(a, cur_stream()), "place_rows");
+}
 void combine_rows(const Tensor& rows, const Tensor& slot_row, const OptTensor& w, Tensor& y, int64_t K) {
   const c10::cuda::CUDAGuard guard(rows.device());
   check_rows(rows, "rows");
@@ -468,6 +491,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_plan_scratch_words", &moe_plan_scratch_words);
   m.def("moe_plan", &moe_plan);
   m.def("gather_rows", &gather_rows);
+  m.def("place_rows", &place_rows);
   m.def("combine_rows", &combine_rows);
   m.def("combine_bwd_w", &combine_bwd_w);
   register_attention(m);

@@ -175,6 +175,25 @@ std::map<std::string, Tensor> moe_local_tables(const Tensor& plan, int64_t n_slo
           {"counts_kept", part(pt.counts_kept, E)}};
 }
 
+// the rows of `src` (tokens) at their places in expert order
+void place_rows(const Tensor& src, const Tensor& out, int64_t K, const PlanTables& pt, const int* plan, bool zero_padding,
+                cudaStream_t stream) {
+  cmoe::PlaceRowsArgs a;
+  a.src = src.data_ptr();
+  a.n_tokens = src.size(0);
+  a.ld_src = src.stride(0);
+  a.slot_row = plan;
+  a.K = static_cast<int>(K);
+  a.H = static_cast<int>(src.size(1));
+  a.out = out.data_ptr();
+  a.ld_out = out.stride(0);
+  a.zero_padding = zero_padding;
+  a.group_offsets = plan + pt.group_offsets;
+  a.counts_kept = plan + pt.counts_kept;
+  a.n_local = static_cast<int>(pt.E);
+  check(cmoe::launch_place_rows(a, stream), "place_rows");
+}
+
 // (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads)
 using Forward = std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor>;
 Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
@@ -196,9 +215,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   // rows per expert on, most pieces are live and whole tiles take fewer loads.
   const bool short_tiles = !keep && pt.n_slots <= 64 * s.E;
   Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
-  check(cmoe::launch_gather_rows(x.data_ptr(), plan + pt.row_slot, static_cast<int>(s.K), nullptr, xp.data_ptr(),
-                                 pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(s.H), x.stride(0), s.H, stream, keep),
-        "gather_rows");
+  place_rows(x, xp, s.K, pt, plan, keep, stream);
   Tensor hact = at::empty({pt.cap_rows, s.F}, bf);
   OptTensor gu;
   {

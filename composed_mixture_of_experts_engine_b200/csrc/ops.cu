@@ -719,8 +719,7 @@ __global__ void __launch_bounds__(256) embedding_grad_join_kernel(const long lon
 __global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot,
                                    int slot_div, const float* slot_scale,
                                    __nv_bfloat16* out, long long cap_rows,
-                                   const int* num_m_tiles, int H, long long ld_src, long long ld_out,
-                                   int zero_padding) {
+                                   const int* num_m_tiles, int H, long long ld_src, long long ld_out) {
   chain_wait();
   chain_trigger();
   const long long n_rows = num_m_tiles ? min(static_cast<long long>(*num_m_tiles) * 128, cap_rows) : cap_rows;
@@ -731,8 +730,7 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot
     const int slot = row_slot[r];
     __nv_bfloat16* o = out + r * ld_out;
     if (slot < 0) {
-      if (zero_padding)
-        for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = make_uint4(0u, 0u, 0u, 0u);
+      for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(o + c) = make_uint4(0u, 0u, 0u, 0u);
     } else {
       const __nv_bfloat16* s = src + static_cast<long long>(slot / slot_div) * ld_src;
       const float sc = slot_scale != nullptr ? slot_scale[slot] : 1.f;
@@ -756,6 +754,52 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot
         }
       }
     }
+  }
+}
+
+// The same rows without a scale, token by token: a warp loads 1024 columns of a token's row once and stores them at all K
+// places.  What bounds it: the stores (a plain zero fill writes at 5.8 TB/s here).  Row by row in expert order, a token is
+// read K times, and between those reads the stream of stores has driven it out of L2.  Row by row / this, behind GEMMs:
+// 16384 tokens x 2048 columns, top-8 of 64: 174 / 122 us; 3333 x 4096, top-8 of 32: 68 / 56; 8192 x 4096, top-2 of 8:
+// 48 / 40; 16384 x 512, top-1 of 16: 15.3 / 13.2; 16384 x 4096, top-1 of 8: 52 / 52.  (Bulk copies through shared memory
+// instead of registers: 130, 67, 57, 22, 67.)
+__global__ void place_rows_kernel(const PlaceRowsArgs a, int pieces) {
+  chain_wait();
+  chain_trigger();
+  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.src);
+  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
+  const int lane = threadIdx.x & 31;
+  const long long first = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
+  const long long step = (gridDim.x * static_cast<long long>(blockDim.x)) >> 5;
+  const long long items = a.n_tokens * pieces;
+  for (long long it = first; it < items; it += step) {
+    const long long t = it / pieces;
+    const int c0 = static_cast<int>(it - t * pieces) * 1024 + lane * 8;
+    const __nv_bfloat16* s = src + t * a.ld_src + c0;
+    uint4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c0 + q * 256 < a.H) v[q] = *reinterpret_cast<const uint4*>(s + q * 256);
+    for (int k0 = 0; k0 < a.K; k0 += 32) {
+      const int mine = k0 + lane < a.K ? a.slot_row[t * a.K + k0 + lane] : -1;
+      const int n = min(32, a.K - k0);
+      for (int k = 0; k < n; ++k) {
+        const int row = __shfl_sync(0xffffffffu, mine, k);
+        if (row < 0) continue;  // dropped
+        __nv_bfloat16* o = out + row * a.ld_out + c0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (c0 + q * 256 < a.H) *reinterpret_cast<uint4*>(o + q * 256) = v[q];
+      }
+    }
+  }
+  if (!a.zero_padding) return;
+  // an expert's rows are followed by up to 127 rows of padding
+  for (long long i = first; i < a.n_local * 128LL; i += step) {
+    const int e = static_cast<int>(i >> 7);
+    const long long row = static_cast<long long>(a.group_offsets[e]) + a.counts_kept[e] + (i & 127);
+    if (row < a.group_offsets[e + 1])
+      for (int c = lane * 8; c < a.H; c += 256) *reinterpret_cast<uint4*>(out + row * a.ld_out + c) = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -1033,11 +1077,20 @@ cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* 
 
 cudaError_t launch_gather_rows(const void* src, const int* row_slot, int slot_div, const float* slot_scale, void* out,
                                long long cap_rows, const int* num_m_tiles, int H, long long ld_src, long long ld_out,
-                               cudaStream_t stream, bool zero_padding) {
+                               cudaStream_t stream) {
   if (H % 8 != 0 || cap_rows <= 0 || slot_div <= 0) return cudaErrorInvalidValue;
   launch_chained(gather_rows_kernel, grid_for(cap_rows, 8, 148 * 8), 256, 0, stream,
                  reinterpret_cast<const __nv_bfloat16*>(src), row_slot, slot_div, slot_scale,
-                 reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out, zero_padding ? 1 : 0);
+                 reinterpret_cast<__nv_bfloat16*>(out), cap_rows, num_m_tiles, H, ld_src, ld_out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream) {
+  if (a.H % 8 != 0 || a.H <= 0 || a.K <= 0) return cudaErrorInvalidValue;
+  if (a.n_tokens <= 0) return cudaSuccess;
+  const int pieces = (a.H + 1023) / 1024;
+  const long long warps = a.n_tokens * pieces + (a.zero_padding ? a.n_local * 64LL : 0);
+  launch_chained(place_rows_kernel, grid_for(warps, 8, 148 * 8), 256, 0, stream, a, pieces);
   return cudaGetLastError();
 }
 

@@ -123,11 +123,26 @@ struct MoePlanArgs {
 size_t moe_plan_scratch_words(long long n_slots, int n_local, int K, int per_k_bins);
 cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream);
 
-// out[r, :] = scale * src[row_slot[r] / slot_div, :]  (zeros where row_slot[r] < 0, or nothing with !zero_padding), for r < *n_rows_dev * 128
+// out[r, :] = scale * src[row_slot[r] / slot_div, :]  (zeros where row_slot[r] < 0), for r < *n_rows_dev * 128
 // (n_rows_dev = num_m_tiles) or r < cap_rows when n_rows_dev is nullptr.  slot_scale (fp32 per slot) optional.
 cudaError_t launch_gather_rows(const void* src, const int* row_slot, int slot_div, const float* slot_scale, void* out,
                                long long cap_rows, const int* num_m_tiles, int H, long long ld_src, long long ld_out,
-                               cudaStream_t stream, bool zero_padding = true);
+                               cudaStream_t stream);
+// out[slot_row[t*K+k], :] = src[t, :] for every slot with a row, and zeros in the padding behind each expert's rows if
+// asked for.  Row starts on 16-byte boundaries, H a multiple of 8.
+struct PlaceRowsArgs {
+  const void* src = nullptr;
+  long long n_tokens = 0, ld_src = 0;
+  const int* slot_row = nullptr;
+  int K = 0, H = 0;
+  void* out = nullptr;
+  long long ld_out = 0;
+  bool zero_padding = true;
+  const int* group_offsets = nullptr;  // of the row plan (MoePlanArgs)
+  const int* counts_kept = nullptr;
+  int n_local = 0;
+};
+cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream);
 // y[t, :] = sum_k w[t,k] * rows[slot_row[t*K+k], :]  (slots with row -1 skipped), fp32 accumulate, bf16 out
 cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const float* w, void* y, long long n_tokens,
                                 int K, int H, long long ld_rows, long long ld_y, cudaStream_t stream);
