@@ -72,6 +72,15 @@ struct GemmArgs {
   void* aux_out = nullptr;  // SWIGLU_FWD: optional [rows, 2N] gate|up
   long long ld_aux_out = 0;
 
+  // SwiGLU epilogues of grouped-M, optional: row r carries the weight slot_weight[weight_row_slot[r]] (padding, with a
+  // negative slot, 0).  Forward: D = weight * silu(gate) * up, aux_out unchanged.  Backward: acc is the gradient of that
+  // D, and row_dot[part * row_dot_stride + r], part < 2 * ceil(N / 256), are the row's partial sums of the gradient of its
+  // weight (whole tiles of rows are written, padding too).
+  const int* weight_row_slot = nullptr;
+  const float* slot_weight = nullptr;
+  float* row_dot = nullptr;
+  long long row_dot_stride = 0;
+
   // Optional readiness flags (fused dispatch): before the first load of a 128-row tile the
   // producer waits until ready_flags[tile_group * ready_stride + s] >= ready_target for all
   // s < ready_count.  nullptr disables the wait.
