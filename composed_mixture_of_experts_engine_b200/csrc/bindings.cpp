@@ -333,6 +333,18 @@ void scaled_out(const Tensor& x, const Tensor& scale, Tensor& out, std::optional
              "scaled_out");
 }
 
+Tensor scaled_bf16(const Tensor& x, const Tensor& scale) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.numel() % 8 == 0 &&
+                  reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0,
+              "scaled_bf16: a contiguous bf16 tensor on a 16-byte boundary, its size a multiple of 8");
+  TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() == 1, "scaled_bf16: bad scale");
+  Tensor out = at::empty(x.sizes(), x.options());
+  check_cuda(cmoe::launch_scaled_bf16(x.data_ptr(), scale.data_ptr<float>(), x.numel(), out.data_ptr(), cur_stream()),
+             "scaled_bf16");
+  return out;
+}
+
 void embedding_grad(const Tensor& dy, const Tensor& keys, const Tensor& order, Tensor& main) {
   const c10::cuda::CUDAGuard guard(dy.device());
   const int64_t n = dy.size(0), H = dy.size(1);
@@ -354,13 +366,23 @@ void embedding_grad(const Tensor& dy, const Tensor& keys, const Tensor& order, T
              "embedding_grad");
 }
 
-void cross_entropy(Tensor& logits, const Tensor& targets, Tensor& loss_sum, double grad_scale) {
+// x @ w^T and the softmax statistics of its rows, or None for these where the kernel that runs leaves none
+std::tuple<Tensor, OptTensor> linear_stats(const Tensor& x, const Tensor& w, const OptTensor& status) {
+  auto [y, stats] = cmoe::dense_nt_stats(x, w, opt_ptr<int>(status));
+  return {y, stats.defined() ? OptTensor(stats) : OptTensor()};
+}
+void cross_entropy(Tensor& logits, const Tensor& targets, Tensor& loss_sum, double grad_scale, const OptTensor& stats) {
   const c10::cuda::CUDAGuard guard(logits.device());
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.scalar_type() == at::kBFloat16);
   TORCH_CHECK(targets.scalar_type() == at::kLong && targets.is_contiguous() && targets.numel() == logits.size(0));
   // per-row losses, summed by a library reduction whose order is fixed: the loss value is reproducible bit for bit
   Tensor row_loss = at::empty({logits.size(0)}, loss_sum.options());
-  check_cuda(cmoe::launch_cross_entropy(logits.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()),
+  TORCH_CHECK(!stats.has_value() || (stats->scalar_type() == at::kFloat && stats->is_contiguous() && stats->is_cuda() &&
+                                     stats->numel() == logits.size(0) * ((logits.size(1) + 255) / 256) * 2),
+              "cross_entropy: the row statistics do not belong to these logits");
+  check_cuda(cmoe::launch_cross_entropy(logits.data_ptr(),
+                                        stats.has_value() ? reinterpret_cast<const float2*>(stats->data_ptr<float>()) : nullptr,
+                                        reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()),
                                         loss_sum.data_ptr<float>(), row_loss.data_ptr<float>(), logits.size(0),
                                         static_cast<int>(logits.size(1)), logits.stride(0),
                                         static_cast<float>(grad_scale), cur_stream()),
@@ -484,9 +506,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qkv_grad_pack", &qkv_grad_pack);
   m.def("adamw", &adamw);
   m.def("sumsq", &sumsq);
-  m.def("cross_entropy", &cross_entropy);
+  m.def("linear_stats", &linear_stats);
+  m.def("cross_entropy", &cross_entropy, pybind11::arg("logits"), pybind11::arg("targets"), pybind11::arg("loss_sum"),
+        pybind11::arg("grad_scale"), pybind11::arg("stats") = pybind11::none());
   m.def("scaled_out", &scaled_out, pybind11::arg("x"), pybind11::arg("scale"), pybind11::arg("out"),
         pybind11::arg("accumulate") = pybind11::none());
+  m.def("scaled_bf16", &scaled_bf16);
   m.def("embedding_grad", &embedding_grad);
   m.def("moe_plan_scratch_words", &moe_plan_scratch_words);
   m.def("moe_plan", &moe_plan);

@@ -1033,6 +1033,7 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
     return cudaErrorInvalidValue;
   if (a.mode == GEMM_GROUPED_M && a.a_mn) return cudaErrorInvalidValue;
   if (a.epilogue == EPI_SWIGLU_FWD && (a.b_mn || a.split_n <= 0)) return cudaErrorInvalidValue;
+  if (a.row_stats != nullptr) return cudaErrorInvalidValue;
 
   CUtensorMap tmA, tmB;
   const bool short_tiles = a.tile_rows != nullptr;

@@ -81,6 +81,10 @@ struct GemmArgs {
   float* row_dot = nullptr;
   long long row_dot_stride = 0;
 
+  // Dense bf16 results on pairs of SMs, optional: row_stats[row * ceil(N / 256) + c] = (max, sum of exp(v - max)) over the
+  // values v of columns [256 c, 256 c + 256) of the row, as they are stored (a softmax over the row then needs one pass)
+  float2* row_stats = nullptr;
+
   // Optional readiness flags (fused dispatch): before the first load of a 128-row tile the
   // producer waits until ready_flags[tile_group * ready_stride + s] >= ready_target for all
   // s < ready_count.  nullptr disables the wait.

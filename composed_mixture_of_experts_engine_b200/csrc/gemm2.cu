@@ -74,6 +74,7 @@ struct K2Params {
   int b_early;        // B does not depend on the kernel before this one
   int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
+  float2* row_stats;           // dense: softmax statistics of the rows
   const int* weight_row_slot;  // SwiGLU: weights of the rows
   const float* slot_weight;
   float* row_dot;
@@ -189,6 +190,22 @@ __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t d_tmem, uint64_t a_de
       "}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// Adds 64 values of a row, packed in bf16 pairs of which the first `live` columns exist, to its running maximum and sum of
+// exp(v - maximum).  A row of minus infinities only has the sum 0.
+__device__ __forceinline__ void add_to_stats(const uint32_t (&v)[32], int live, float& mx, float& sum) {
+  float m = mx;
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    if (2 * j < live) m = fmaxf(m, fmaxf(__uint_as_float(v[j] << 16), __uint_as_float(v[j] & 0xffff0000u)));
+  const float base = m == -INFINITY ? 0.f : m;
+  sum *= __expf(mx - base);
+  mx = m;
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    if (2 * j < live)
+      sum += __expf(__uint_as_float(v[j] << 16) - base) + __expf(__uint_as_float(v[j] & 0xffff0000u) - base);
 }
 
 template <int EPI, int GROUPS>
@@ -396,6 +413,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       }
       const float weight = EPI != EPI_STORE && mine ? row_weight(p.weight_row_slot, p.slot_weight, row0 + row_in_tile) : 1.f;
       float dot = 0.f;
+      float stat_max = -INFINITY, stat_sum = 0.f;
       bool ok = true;
       if (have_acc) {
         ok = mbar_wait(&tfull_bar[acc], acc_phase, wc, ST_TIMEOUT_TMEM_FULL);
@@ -521,23 +539,21 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 #pragma unroll
               for (int j = 0; j < 32; ++j) r0[j] = r1[j] = 0u;
             }
+            uint32_t v[32];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(r0[8 * j]), __uint_as_float(r0[8 * j + 1]));
-              o.y = pack_bf16x2(__uint_as_float(r0[8 * j + 2]), __uint_as_float(r0[8 * j + 3]));
-              o.z = pack_bf16x2(__uint_as_float(r0[8 * j + 4]), __uint_as_float(r0[8 * j + 5]));
-              o.w = pack_bf16x2(__uint_as_float(r0[8 * j + 6]), __uint_as_float(r0[8 * j + 7]));
-              *reinterpret_cast<uint4*>(myrow + ((j ^ sw) << 4)) = o;
+            for (int j = 0; j < 16; ++j) {
+              v[j] = pack_bf16x2(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1]));
+              v[16 + j] = pack_bf16x2(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1]));
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(r1[8 * j]), __uint_as_float(r1[8 * j + 1]));
-              o.y = pack_bf16x2(__uint_as_float(r1[8 * j + 2]), __uint_as_float(r1[8 * j + 3]));
-              o.z = pack_bf16x2(__uint_as_float(r1[8 * j + 4]), __uint_as_float(r1[8 * j + 5]));
-              o.w = pack_bf16x2(__uint_as_float(r1[8 * j + 6]), __uint_as_float(r1[8 * j + 7]));
-              *reinterpret_cast<uint4*>(myrow + (((j + 4) ^ sw) << 4)) = o;
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(myrow + ((j ^ sw) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            if (p.row_stats != nullptr) {
+              const int live = p.N - col0;
+              if (live >= 64)
+                add_to_stats(v, 64, stat_max, stat_sum);
+              else
+                add_to_stats(v, live, stat_max, stat_sum);
             }
           }
         }
@@ -555,6 +571,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         }
         ++stage_ctr;
       }
+      if (EPI == EPI_STORE && p.row_stats != nullptr && row0 + row_in_tile < p.M)
+        p.row_stats[static_cast<long long>(row0 + row_in_tile) * n_tiles + ti.n0 / T_BN] = make_float2(stat_max, stat_sum);
       if (EPI == EPI_SWIGLU_BWD && p.row_dot != nullptr && mine)
         p.row_dot[(2 * (ti.n0 / T_BN) + grp) * p.row_dot_stride + row0 + row_in_tile] = dot;
       if (have_acc) {
@@ -594,7 +612,7 @@ bool gemm_2cta_supported(const GemmArgs& a) {
   const long long es = a.d_fp32 ? 4 : 2;
   long long gstride = static_cast<long long>(a.M) * a.ldd;
   if (a.mode == GEMM_DENSE) {
-    if (a.a_mn || a.M <= 0) return false;
+    if (a.a_mn || a.M <= 0 || (a.row_stats != nullptr && (a.d_fp32 || a.accumulate || a.epilogue != EPI_STORE))) return false;
   } else if (a.mode == GEMM_GROUPED_K) {
     if (!(a.a_mn && a.b_mn) || (a.group_offsets == nullptr && (a.k_chunk <= 0 || a.k_chunk % 64 != 0)) || a.M <= 0)
       return false;
@@ -676,6 +694,7 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   kp.has_aux = a.aux_out != nullptr;
   kp.d_fp32 = a.d_fp32;
   kp.reduce = a.accumulate;
+  kp.row_stats = a.row_stats;
   kp.weight_row_slot = a.weight_row_slot;
   kp.slot_weight = a.slot_weight;
   kp.row_dot = a.row_dot;

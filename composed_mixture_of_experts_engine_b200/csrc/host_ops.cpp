@@ -39,7 +39,15 @@ GemmArgs operands(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn) {
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   return g;
 }
-Tensor dense(const Tensor& x, const Tensor& w, bool b_mn, Tensor out, int* status) {
+bool two_cta() {
+  static const bool on = [] {
+    const char* v = std::getenv("CMOE_GEMM_2CTA");
+    return v == nullptr || (v[0] != '\0' && v[0] != '0');
+  }();
+  return on;
+}
+// `stats`, where given: takes the softmax statistics of the rows
+Tensor dense(const Tensor& x, const Tensor& w, bool b_mn, Tensor out, int* status, Tensor* stats = nullptr) {
   const c10::cuda::CUDAGuard guard(x.device());
   GemmArgs g = operands(x, false, w, b_mn);
   const int64_t M = x.size(0), N = w.size(b_mn ? 1 : 0), K = x.size(1);
@@ -52,6 +60,10 @@ Tensor dense(const Tensor& x, const Tensor& w, bool b_mn, Tensor out, int* statu
   g.D = out.data_ptr();
   g.ldd = out.stride(0);
   g.status = status;
+  if (stats != nullptr && two_cta() && gemm_2cta_supported(g)) {
+    *stats = at::empty({M, (N + 255) / 256, 2}, x.options().dtype(at::kFloat));
+    g.row_stats = reinterpret_cast<float2*>(stats->data_ptr<float>());
+  }
   launch_gemm_any(g, at::cuda::getCurrentCUDAStream().stream());
   return out;
 }
@@ -84,17 +96,18 @@ Tensor contiguous_aligned(const Tensor& t) {
 }
 
 void launch_gemm_any(const GemmArgs& g, cudaStream_t stream) {
-  static const bool two_cta = [] {
-    const char* v = std::getenv("CMOE_GEMM_2CTA");
-    return v == nullptr || (v[0] != '\0' && v[0] != '0');
-  }();
-  if (two_cta && gemm_2cta_supported(g))
+  if (two_cta() && gemm_2cta_supported(g))
     check(launch_gemm_2cta(g, stream), "launch_gemm_2cta");
   else
     check(launch_gemm(g, stream), "launch_gemm");
 }
 
 Tensor dense_nt(const Tensor& x, const Tensor& w, Tensor out, int* status) { return dense(x, w, false, out, status); }
+std::pair<Tensor, Tensor> dense_nt_stats(const Tensor& x, const Tensor& w, int* status) {
+  Tensor stats;
+  Tensor y = dense(x, w, false, Tensor(), status, &stats);
+  return {y, stats};
+}
 Tensor dense_nn(const Tensor& x, const Tensor& w, Tensor out, int* status) { return dense(x, w, true, out, status); }
 
 void dense_wgrad(const Tensor& a, const Tensor& b, Tensor& out, bool accumulate, int* status, int64_t want_pieces) {

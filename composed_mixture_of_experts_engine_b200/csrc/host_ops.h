@@ -15,6 +15,9 @@ void launch_gemm_any(const GemmArgs& g, cudaStream_t stream);
 
 // y[M, N] = x[M, K] @ w[N, K]^T (out: bf16, allocated when undefined)
 torch::Tensor dense_nt(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
+// the same with the softmax statistics of the rows (GemmArgs::row_stats, fp32 [M, ceil(N / 256), 2]) where the kernel that
+// runs can leave them; undefined otherwise
+std::pair<torch::Tensor, torch::Tensor> dense_nt_stats(const torch::Tensor& x, const torch::Tensor& w, int* status);
 // y[M, K] = x[M, N] @ w[N, K]
 torch::Tensor dense_nn(const torch::Tensor& x, const torch::Tensor& w, torch::Tensor out, int* status);
 // out[M, N] (+)= a[R, M]^T @ b[R, N]; out fp32 (stored, or added to) or bf16 (stored), its rows on 16-byte

@@ -564,6 +564,80 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   }
 }
 
+// The same loss and gradient where the GEMM that made the logits has left the maximum and the sum of exp(v - maximum) of
+// every 256 columns (GemmArgs::row_stats): the row is read and written once, with one exponential per logit.  What bounds
+// it: these passes, which take as long as a copy.  4096 x 50304 behind GEMMs, at the clock that these leave: 279 us with
+// the row read twice, 147 this way (a copy: 138); 4096 x 8192 77 / 36.  Small CTAs, whose first loads are in flight while
+// the statistics are merged, measured better than large ones: 256 threads 147, 512 155, 1024 177.
+constexpr int CS_THREADS = 256, CS_VECS = 2;
+__global__ void __launch_bounds__(CS_THREADS) cross_entropy_stats_kernel(__nv_bfloat16* logits, const float2* stats,
+                                                                         const long long* targets, float* loss_sum,
+                                                                         float* row_loss, int V, long long ld,
+                                                                         float grad_scale) {
+  chain_wait();
+  chain_trigger();
+  __shared__ float warp_m[CS_THREADS / 32], warp_s[CS_THREADS / 32];
+  const long long row = blockIdx.x;
+  __nv_bfloat16* lr = logits + row * ld;
+  const long long tgt = targets[row];
+  const int nvec = V / 8;  // V is a multiple of 8
+  uint4 v[CS_VECS];
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int q = 0; q < CS_VECS; ++q)
+      if (i0 + q * CS_THREADS < nvec) v[q] = reinterpret_cast<const uint4*>(lr)[i0 + q * CS_THREADS];
+  };
+  fetch(threadIdx.x);
+  const int n = (V + 255) / 256;
+  float mx = -INFINITY, se = 0.f;
+  // sums of parts without a finite or larger value are 0 and stay so
+  const auto scaled = [](float s, float m, float to) { return m == -INFINITY ? (isnan(s) ? s : 0.f) : s * __expf(m - to); };
+  for (int i = threadIdx.x; i < n; i += CS_THREADS) {
+    const float2 s = stats[row * n + i];
+    const float m = fmaxf(mx, s.x);
+    se = scaled(se, mx, m) + scaled(s.y, s.x, m);
+    mx = m;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float wm = warp_max(mx), ws = warp_sum(scaled(se, mx, wm));
+  if (lane == 0) {
+    warp_m[warp] = wm;
+    warp_s[warp] = ws;
+  }
+  __syncthreads();
+  const float m = lane < CS_THREADS / 32 ? warp_m[lane] : -INFINITY, s = lane < CS_THREADS / 32 ? warp_s[lane] : 0.f;
+  const float bm = warp_max(m), lse = bm + logf(warp_sum(scaled(s, m, bm)));
+  const bool ignore = tgt < 0 || tgt >= V;
+  if (threadIdx.x == 0) {
+    const float l = ignore ? 0.f : lse - __bfloat162float(lr[tgt]);
+    if (row_loss != nullptr)
+      row_loss[row] = l;
+    else if (!ignore)
+      atomicAdd(loss_sum, l);
+  }
+  __syncthreads();  // the target's logit has been read
+  const float gs = ignore ? 0.f : grad_scale;
+  for (int i0 = threadIdx.x; i0 < nvec; i0 += CS_VECS * CS_THREADS) {
+    if (i0 != static_cast<int>(threadIdx.x)) fetch(i0);
+#pragma unroll
+    for (int q = 0; q < CS_VECS; ++q) {
+      const int i = i0 + q * CS_THREADS;
+      if (i >= nvec) break;
+      float f[8], o[8];
+      unpack8(v[q], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = __expf(f[j] - lse) * gs;
+      const long long at = tgt - i * 8LL;
+      if (at >= 0 && at < 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j == at) o[j] = (__expf(f[j] - lse) - 1.f) * gs;
+      }
+      store8(lr + i * 8, o);
+    }
+  }
+}
+
 // out (+)= *scale * x in fp32, or out = *scale * x in bf16.  One pass over each; what bounds it is those passes.  Library
 // operations took a multiply, a cast and a temporary for the second, and 361 us for 103 M elements of the first.
 template <int OUT>  // 0: fp32 store, 1: fp32 add, 2: bf16 store
@@ -594,6 +668,28 @@ __global__ void __launch_bounds__(256) scaled_out_kernel(const float4* x, const 
       else
         reinterpret_cast<uint2*>(out)[i] = make_uint2(pack_bf16x2(s * v[q].x, s * v[q].y), pack_bf16x2(s * v[q].z, s * v[q].w));
     }
+  }
+}
+
+// out = *scale * x for bf16 rows, the scale rounded to bf16 first (the library's product with a bf16 scalar, which took 63 us
+// for 20 M elements, a broadcast scalar being outside its vectorised kernels; this takes 14).
+__global__ void __launch_bounds__(256) scaled_bf16_kernel(const uint4* x, const float* scale, long long n8, uint4* out) {
+  chain_wait();
+  chain_trigger();
+  const float s = __bfloat162float(__float2bfloat16(*scale));
+  const long long i0 = blockIdx.x * 1024ll + threadIdx.x;
+  uint4 v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (i0 + q * 256 < n8) v[q] = x[i0 + q * 256];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (i0 + q * 256 >= n8) break;
+    float f[8];
+    unpack8(v[q], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] *= s;
+    store8(reinterpret_cast<__nv_bfloat16*>(out + i0 + q * 256), f);
   }
 }
 
@@ -1065,6 +1161,13 @@ cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, v
   return launch_chained(scaled_out_kernel<0>, grid, 256, 0, stream, x4, scale, n4, out);
 }
 
+cudaError_t launch_scaled_bf16(const void* x, const float* scale, long long n, void* out, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (n % 8 != 0) return cudaErrorInvalidValue;
+  return launch_chained(scaled_bf16_kernel, static_cast<unsigned>((n / 8 + 1023) / 1024), 256, 0, stream,
+                        reinterpret_cast<const uint4*>(x), scale, n / 8, reinterpret_cast<uint4*>(out));
+}
+
 long long embedding_grad_partial_floats(long long n, int H) {
   return n <= kEmbSeg ? 0 : (n + kEmbSeg - 1) / kEmbSeg * 2 * H;
 }
@@ -1083,12 +1186,18 @@ cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const l
                         0, stream, keys, partial, main, n, H);
 }
 
-cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* loss_sum, float* row_loss,
-                                 long long rows, int V, long long ld, float grad_scale, cudaStream_t stream) {
+cudaError_t launch_cross_entropy(void* logits, const float2* stats, const long long* targets, float* loss_sum,
+                                 float* row_loss, long long rows, int V, long long ld, float grad_scale,
+                                 cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   if (ld % 8 != 0) return cudaErrorInvalidValue;
-  launch_chained(cross_entropy_kernel, static_cast<unsigned>(rows), CE_THREADS, 0, stream,
-                 reinterpret_cast<__nv_bfloat16*>(logits), targets, loss_sum, row_loss, rows, V, ld, grad_scale);
+  auto lb = reinterpret_cast<__nv_bfloat16*>(logits);
+  if (stats != nullptr && V % 8 == 0)
+    launch_chained(cross_entropy_stats_kernel, static_cast<unsigned>(rows), CS_THREADS, 0, stream, lb, stats, targets,
+                   loss_sum, row_loss, V, ld, grad_scale);
+  else
+    launch_chained(cross_entropy_kernel, static_cast<unsigned>(rows), CE_THREADS, 0, stream, lb, targets, loss_sum, row_loss,
+                   rows, V, ld, grad_scale);
   return cudaGetLastError();
 }
 

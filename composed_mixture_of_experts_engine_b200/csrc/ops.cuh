@@ -69,6 +69,9 @@ cudaError_t launch_splitk_reduce(const float* part, int parts, long long n, void
 cudaError_t launch_scaled_out(const float* x, const float* scale, long long n, void* out, int out_bf16, int accumulate,
                               cudaStream_t stream);
 
+// out[i] = bf16(*scale) * x[i], bf16 in and out.  n % 8 == 0, 16-byte aligned pointers; scale is a device scalar.
+cudaError_t launch_scaled_bf16(const void* x, const float* scale, long long n, void* out, cudaStream_t stream);
+
 // ---- embedding gradient: main[keys[i], :] += dy[order[i], :] for sorted keys (fp32 sums in a fixed order); dy [n, H] bf16,
 // main [vocabulary, H] and the working storage `partial` (embedding_grad_partial_floats words, unless that is 0) fp32 are
 // contiguous and start on 16-byte boundaries, H % 8 == 0.
@@ -80,9 +83,10 @@ cudaError_t launch_embedding_grad(const void* dy, const long long* keys, const l
 // logits [rows, V] bf16 are overwritten with d(loss)/d(logits) = (softmax - onehot) * grad_scale;
 // *loss_sum += sum over rows of the per-row loss (fp32), or, with `row_loss` [rows], the per-row losses are written
 // there for the caller to sum in a fixed order (*loss_sum is then left alone).  targets are int64; target < 0 is
-// ignored (its row loss is 0).
-cudaError_t launch_cross_entropy(void* logits, const long long* targets, float* loss_sum, float* row_loss,
-                                 long long rows, int V, long long ld, float grad_scale, cudaStream_t stream);
+// ignored (its row loss is 0).  stats: GemmArgs::row_stats of the launch that made the logits, or nullptr.
+cudaError_t launch_cross_entropy(void* logits, const float2* stats, const long long* targets, float* loss_sum,
+                                 float* row_loss, long long rows, int V, long long ld, float grad_scale,
+                                 cudaStream_t stream);
 
 // ---- MoE routing bookkeeping -------------------------------------------------------------------
 // Builds the expert-sorted, 128-row-padded row layout for `n_slots` (token, k) slots.

@@ -129,8 +129,8 @@ class _LMHeadLossFn(torch.autograd.Function):
         dw = torch.empty(weight.shape, device=h.device, dtype=torch.float32) if need_dw else None
         for a in range(0, N, chunk):
             b = min(a + chunk, N)
-            logits = kernels.linear_nt(h[a:b], weight)
-            ext.cross_entropy(logits, targets[a:b], loss, scale)  # logits now hold d(loss)/d(logits)
+            logits, stats = ext.linear_stats(h[a:b], weight, kernels.status_word(h.device))
+            ext.cross_entropy(logits, targets[a:b], loss, scale, stats)  # logits now hold d(loss)/d(logits)
             if need_dh:
                 kernels.linear_nn(logits, weight, out=dh[a:b])
             if need_dw:
@@ -141,11 +141,16 @@ class _LMHeadLossFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dh, dw, weight = ctx.saved_tensors
-        if dh is not None:
-            dh = dh * g.to(dh.dtype)
-        if dw is not None:
-            from ..ops import _ext
+        from ..ops import _ext, kernels
 
+        if dh is not None:
+            # (a saved tensor may come back from a hook in another layout)
+            if (dh.is_contiguous() and dh.data_ptr() % 16 == 0 and dh.numel() % 8 == 0 and g.dtype == torch.float32
+                    and not kernels.needs_autograd(g) and not torch._C._are_functorch_transforms_active()):
+                dh = _ext.ext().scaled_bf16(dh, g)
+            else:
+                dh = dh * g.to(dh.dtype)
+        if dw is not None:
             main = getattr(weight, "main_grad", None)
             out = torch.empty_like(weight) if main is None else main
             if (dw.numel() % 4 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0
