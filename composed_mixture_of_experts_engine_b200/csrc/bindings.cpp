@@ -242,6 +242,52 @@ void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tenso
                                       dw.data_ptr<float>(), partial.data_ptr<float>(), rows, H, sms, cur_stream()),
              "rmsnorm_bwd");
 }
+// (x + delta, norm of it, rstd); without delta the first is x itself
+std::tuple<Tensor, Tensor, Tensor> add_rmsnorm(const Tensor& x, const OptTensor& delta, const Tensor& w, double eps) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t H = x.size(-1), rows = x.numel() / H;
+  const auto fits = [&](const Tensor& t) {
+    return t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kBFloat16 &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  TORCH_CHECK(fits(x) && fits(w) && w.numel() == H && (!delta.has_value() || (fits(*delta) && delta->sizes() == x.sizes())),
+              "add_rmsnorm: contiguous bf16 tensors on 16-byte boundaries, weight [H], both rows of one shape");
+  Tensor sum = delta.has_value() ? at::empty_like(x) : x, y = at::empty_like(x);
+  Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+  check_cuda(cmoe::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), rows,
+                                      static_cast<int>(H), static_cast<float>(eps), cur_stream(),
+                                      delta.has_value() ? delta->data_ptr() : nullptr,
+                                      delta.has_value() ? sum.data_ptr() : nullptr),
+             "add_rmsnorm");
+  return {sum, y, rstd};
+}
+// (dx, dw) of the norm plus `dsum`, the gradient of the sum past the norm; dw is added to `main` (fp32) where there is one
+// and otherwise rounded once to the weight's type
+std::tuple<Tensor, OptTensor> add_rmsnorm_grad(const Tensor& dy, const OptTensor& dsum, const Tensor& x, const Tensor& w,
+                                               const Tensor& rstd, bool need_dw, const OptTensor& main) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t H = x.size(-1), rows = x.numel() / H;
+  const Tensor g = cmoe::contiguous_aligned(dy), xs = cmoe::contiguous_aligned(x), r = cmoe::contiguous_aligned(rstd);
+  OptTensor res;
+  if (dsum.has_value()) res = cmoe::contiguous_aligned(*dsum);
+  TORCH_CHECK(g.scalar_type() == at::kBFloat16 && xs.scalar_type() == at::kBFloat16 && g.numel() == xs.numel() &&
+                  r.scalar_type() == at::kFloat && r.numel() == rows &&
+                  (!res.has_value() || (res->scalar_type() == at::kBFloat16 && res->numel() == xs.numel())) &&
+                  (!main.has_value() || (main->scalar_type() == at::kFloat && main->is_contiguous() && main->numel() == H)),
+              "add_rmsnorm_grad: bf16 rows of one shape, fp32 rstd and main gradient");
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  Tensor dx = at::empty_like(xs), partial, dw;
+  if (need_dw) {
+    dw = main.has_value() ? *main : at::zeros({H}, r.options());
+    partial = at::empty({cmoe::rmsnorm_bwd_partial_rows(rows, sms), H}, r.options());
+  }
+  check_cuda(cmoe::launch_rmsnorm_bwd(g.data_ptr(), xs.data_ptr(), w.data_ptr(), r.data_ptr<float>(), dx.data_ptr(),
+                                      need_dw ? dw.data_ptr<float>() : nullptr, need_dw ? partial.data_ptr<float>() : nullptr,
+                                      rows, static_cast<int>(H), sms, cur_stream(),
+                                      res.has_value() ? res->data_ptr() : nullptr),
+             "add_rmsnorm_grad");
+  return {dx.view(x.sizes()), need_dw && !main.has_value() ? OptTensor(dw.to(w.scalar_type())) : OptTensor()};
+}
 void rope(Tensor& t, const Tensor& cos_tab, const Tensor& sin_tab, int64_t seq, bool inverse) {
   // t: [rows, heads, head_dim] view with unit stride on head_dim and stride head_dim on heads
   const c10::cuda::CUDAGuard guard(t.device());
@@ -502,6 +548,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("router_bwd", &router_bwd);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("add_rmsnorm", &add_rmsnorm);
+  m.def("add_rmsnorm_grad", &add_rmsnorm_grad);
   m.def("rope", &rope);
   m.def("qkv_grad_pack", &qkv_grad_pack);
   m.def("adamw", &adamw);

@@ -194,13 +194,15 @@ void place_rows(const Tensor& src, const Tensor& out, int64_t K, const PlanTable
   check(cmoe::launch_place_rows(a, stream), "place_rows");
 }
 
-// With several picks per token the gate weight enters with the SwiGLU product, h = weight * silu(gate) * up, so that the
-// result rows only have to be added up, the backward reads dy's rows as they are, and the gradient of the weight falls out
-// of the SwiGLU backward, next to the values that it needs.  A weight on the result rows instead (the form for one pick)
-// needs those rows again in the backward: 16384 tokens top-8, H 2048, F 1024 read 600 MB for it and scale 540 MB of dy's
-// rows on their way (layer, forward and backward, 5077 -> 4874 us, with the rows placed token by token).  One pick: a normalised weight is 1 and its gradient cancels to rounding noise in the router; that
-// noise is left as it always was.
-bool weight_in_ffn(int64_t K) { return K > 1; }
+// With several picks per token and a backward pass to come, the gate weight enters with the SwiGLU product,
+// h = weight * silu(gate) * up: the result rows only have to be added up, the backward reads dy's rows as they are, and
+// the gradient of the weight falls out of the SwiGLU backward, next to the values that it needs.  A weight on the result
+// rows instead needs those rows again in the backward: 16384 tokens top-8, H 2048, F 1024 read 600 MB for it and scale
+// 540 MB of dy's rows on their way (layer, forward and backward, 5077 -> 4874 us, with the rows placed token by token).
+// One pick: a normalised weight is 1 and its gradient cancels to rounding noise in the router, which is left as it always
+// was.  Without a backward pass nothing is read again, so the weight stays on the result rows: the picks of the layers
+// behind, which near-ties make depend on single roundings, stay what they were.
+bool weight_in_ffn(int64_t K, bool keep) { return keep && K > 1; }
 void set_weights(cmoe::GemmArgs& g, const Tensor& gate_w32, const PlanTables& pt, const int* plan) {
   g.weight_row_slot = plan + pt.row_slot;
   g.slot_weight = gate_w32.data_ptr<float>();
@@ -225,6 +227,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   // GEMMs load and store only the 32-row pieces that hold any: at 64 tokens, E 64 top-8 (8 rows per expert), H 2048,
   // F 1024 the padding was 33 MB to fill, 400 MB to load from L2 and 50 MB to store, next to 805 MB of weights.  From 64
   // rows per expert on, most pieces are live and whole tiles take fewer loads.
+  const bool weighted = weight_in_ffn(s.K, keep);
   const bool short_tiles = !keep && pt.n_slots <= 64 * s.E;
   Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
   place_rows(x, xp, s.K, pt, plan, keep, stream);
@@ -234,7 +237,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
     cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status), cmoe::EPI_SWIGLU_FWD,
                                      short_tiles);
     g.split_n = static_cast<int>(s.F);
-    if (weight_in_ffn(s.K)) set_weights(g, gate_w32, pt, plan);
+    if (weighted) set_weights(g, gate_w32, pt, plan);
     if (keep) {
       gu = at::empty({pt.cap_rows, 2 * s.F}, bf);
       g.aux_out = gu->data_ptr();
@@ -247,11 +250,11 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
                                       cmoe::EPI_STORE, short_tiles),
                          stream);
   Tensor y = at::empty({s.N, s.H}, bf);
-  check(cmoe::launch_combine_rows(yp.data_ptr(), plan, weight_in_ffn(s.K) ? nullptr : gate_w32.data_ptr<float>(),
+  check(cmoe::launch_combine_rows(yp.data_ptr(), plan, weighted ? nullptr : gate_w32.data_ptr<float>(),
                                   y.data_ptr(), s.N, static_cast<int>(s.K), static_cast<int>(s.H), s.H, s.H, stream),
         "combine_rows");
   if (!keep) return {y, plan_t, std::nullopt, std::nullopt, std::nullopt, std::nullopt};
-  return {y, plan_t, xp, hact, gu, weight_in_ffn(s.K) ? OptTensor() : OptTensor(yp)};
+  return {y, plan_t, xp, hact, gu, weighted ? OptTensor() : OptTensor(yp)};
 }
 
 // dW[e] = a[rows of e]^T b[rows of e]: added into the fp32 `main` buffer when there is one (returns nothing), else
@@ -309,7 +312,7 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
   TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && dy.size(0) == N && dy.size(1) == H, "bad dy");
   check_rows(dy, "dy");
   check_rows(xp, "saved rows");
-  const bool weighted = weight_in_ffn(K);
+  const bool weighted = weight_in_ffn(K, true);
   TORCH_CHECK(weighted || yp.has_value(), "the saved expert rows are missing");
   if (!weighted) check_rows(*yp, "saved expert rows");
   const PlanTables pt(N * K, E);

@@ -54,9 +54,11 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // (VEC = 1, 2, 4, 8 covers H <= 1024, 2048, 4096, 8192).  Small CTAs keep 16 rows in flight per SM.
 constexpr int RN_THREADS = 128;
 
-template <int VEC>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* x,
-                                                                 const __nv_bfloat16* w,
+// ADD: the row is x + delta, rounded to bf16 and written to `sum` first (a residual stream and the branch that joins it:
+// one pass instead of an addition of its own and a pass that reads its result).
+template <int VEC, bool ADD>
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta,
+                                                                 __nv_bfloat16* sum, const __nv_bfloat16* w,
                                                                  __nv_bfloat16* y,
                                                                  float* rstd, long long rows, int H,
                                                                  float eps) {
@@ -72,6 +74,13 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
       const int c = (i * RN_THREADS + threadIdx.x) * 8;
       if (c < H) {
         load8(xr + c, v[i]);
+        if (ADD) {
+          float d[8];
+          load8(delta + row * H + c, d);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[i][j] = __bfloat162float(__float2bfloat16(v[i][j] + d[j]));
+          store8(sum + row * H + c, v[i]);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
       }
@@ -95,7 +104,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
 
 // rows of x / dy that a CTA of the backward kernel keeps in flight (shared-memory ring)
 __host__ __device__ constexpr int rn_bwd_stages(int vec) { return vec <= 2 ? 4 : 2; }
-__host__ __device__ constexpr int rn_bwd_smem(int vec) { return rn_bwd_stages(vec) * 2 * vec * RN_THREADS * 16; }
+__host__ __device__ constexpr int rn_bwd_smem(int vec, int streams) { return rn_bwd_stages(vec) * streams * vec * RN_THREADS * 16; }
 
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
@@ -108,8 +117,9 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int VEC>
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* dy,
+// RES: `dres`, the gradient that reaches the row past the norm (a residual stream), is added to dx before it is rounded.
+template <int VEC, bool RES>
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* dres,
                                                                  const __nv_bfloat16* x,
                                                                  const __nv_bfloat16* w,
                                                                  const float* rstd,
@@ -119,8 +129,8 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
   chain_wait();
   chain_trigger();
   __shared__ float red[RN_THREADS / 32];
-  extern __shared__ uint4 rn_ring[];  // [stages][x | dy][VEC][RN_THREADS]: every thread's own 16-byte pieces
-  constexpr int S = rn_bwd_stages(VEC);
+  extern __shared__ uint4 rn_ring[];  // [stages][x | dy | dres][VEC][RN_THREADS]: every thread's own 16-byte pieces
+  constexpr int S = rn_bwd_stages(VEC), STREAMS = RES ? 3 : 2;
   float wv[VEC][8], dwacc[VEC][8];
 #pragma unroll
   for (int i = 0; i < VEC; ++i) {
@@ -136,7 +146,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
   // (`cp.async`, 16 bytes each, past L1): a CTA keeps S rows of loads in flight without holding them in registers,
   // and every thread reads back only the pieces it copied itself, so the ring needs no barrier.  One commit group per
   // row (an empty one past the end), so that "all but the newest S - 1 groups" is always the row about to be used.
-  auto slot = [&](int s, int which, int i) { return rn_ring + ((s * 2 + which) * VEC + i) * RN_THREADS + threadIdx.x; };
+  auto slot = [&](int s, int which, int i) { return rn_ring + ((s * STREAMS + which) * VEC + i) * RN_THREADS + threadIdx.x; };
   auto issue = [&](long long row, int s) {
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
@@ -144,6 +154,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
       if (row < rows && c < H) {
         cp_async_16(slot(s, 0, i), x + row * H + c);
         cp_async_16(slot(s, 1, i), dy + row * H + c);
+        if (RES) cp_async_16(slot(s, 2, i), dres + row * H + c);
       }
     }
     cp_async_commit();
@@ -155,12 +166,14 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
     cp_async_wait<S - 1>();
     const float r = rstd[row];
     float xh[VEC][8], g[VEC][8];
+    uint4 res[VEC];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * RN_THREADS + threadIdx.x) * 8;
       if (c < H) {
         const uint4 nx = *slot(s, 0, i), nd = *slot(s, 1, i);
+        if (RES) res[i] = *slot(s, 2, i);
         const uint32_t xw[4] = {nx.x, nx.y, nx.z, nx.w};
         const uint32_t dw4[4] = {nd.x, nd.y, nd.z, nd.w};
 #pragma unroll
@@ -187,6 +200,12 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
         float o[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = r * (g[i][j] - xh[i][j] * dot);
+        if (RES) {
+          float f[8];
+          unpack8(res[i], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += f[j];
+        }
         store8(dx + row * H + c, o);
       }
     }
@@ -215,29 +234,25 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
   }
 }
 
-// Column sums of the per-CTA partial rows in a fixed order (the same inputs give the same bits, whichever CTA
-// finishes first).  Stage 1, grid (ceil(H / 128), slices): slice y adds the rows y, y + slices, ... in that order and
-// leaves the result in row y (only slice y ever touches those rows).  Stage 2, grid (ceil(H / 128)): dw[c] += the
-// `slices` stage-1 rows, again in order.
-__global__ void __launch_bounds__(128) colsum_stage1_kernel(float* partial, int n_rows, int H) {
+// dw[c] += column sums of the per-CTA partial rows, in a fixed order (the same inputs give the same bits, whichever CTA
+// finishes first): 16 warps take every 16th row each, a lane per column, and their sums are added in order.  What bounds
+// it: latency.  In two launches (slices of rows, then the slices' sums) it took 13.4 us for 592 rows of 1024.
+constexpr int CSUM_WARPS = 16;
+__global__ void __launch_bounds__(CSUM_WARPS * 32) colsum_kernel(const float* partial, float* dw, int n_rows, int H) {
   chain_wait();
   chain_trigger();
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  if (c >= H) return;
+  __shared__ float sums[CSUM_WARPS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
+  if (c < H)
 #pragma unroll 8
-  for (int b = blockIdx.y; b < n_rows; b += gridDim.y) s += partial[static_cast<long long>(b) * H + c];  // loads ahead, adds in order
-  partial[static_cast<long long>(blockIdx.y) * H + c] = s;
-}
-__global__ void __launch_bounds__(128) colsum_stage2_kernel(const float* partial, float* dw,
-                                                            int slices, int H) {
-  chain_wait();
-  chain_trigger();
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  if (c >= H) return;
-  float s = 0.f;
-#pragma unroll 8
-  for (int y = 0; y < slices; ++y) s += partial[static_cast<long long>(y) * H + c];
+    for (int b = warp; b < n_rows; b += CSUM_WARPS) s += partial[static_cast<long long>(b) * H + c];  // loads ahead, adds in order
+  sums[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || c >= H) return;
+#pragma unroll
+  for (int w = 1; w < CSUM_WARPS; ++w) s += sums[w][lane];
   dw[c] += s;
 }
 
@@ -1040,17 +1055,19 @@ inline int rn_vec_for(int H) {
 }
 
 cudaError_t launch_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows, int H, float eps,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, const void* delta, void* sum) {
   if (H % 8 != 0 || H > RN_THREADS * 8 * 8 || rows <= 0) return cudaErrorInvalidValue;
   const unsigned grid = grid_for(rows, 1, 148 * 32);
-  auto xb = reinterpret_cast<const __nv_bfloat16*>(x);
-  auto wb = reinterpret_cast<const __nv_bfloat16*>(w);
-  auto yb = reinterpret_cast<__nv_bfloat16*>(y);
+  auto go = [&](auto add, auto plain) {
+    launch_chained(delta != nullptr ? add : plain, grid, RN_THREADS, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x),
+                   reinterpret_cast<const __nv_bfloat16*>(delta), reinterpret_cast<__nv_bfloat16*>(sum),
+                   reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<__nv_bfloat16*>(y), rstd, rows, H, eps);
+  };
   switch (rn_vec_for(H)) {
-    case 1: launch_chained(rmsnorm_fwd_kernel<1>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
-    case 2: launch_chained(rmsnorm_fwd_kernel<2>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
-    case 4: launch_chained(rmsnorm_fwd_kernel<4>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
-    default: launch_chained(rmsnorm_fwd_kernel<8>, grid, RN_THREADS, 0, stream, xb, wb, yb, rstd, rows, H, eps); break;
+    case 1: go(rmsnorm_fwd_kernel<1, true>, rmsnorm_fwd_kernel<1, false>); break;
+    case 2: go(rmsnorm_fwd_kernel<2, true>, rmsnorm_fwd_kernel<2, false>); break;
+    case 4: go(rmsnorm_fwd_kernel<4, true>, rmsnorm_fwd_kernel<4, false>); break;
+    default: go(rmsnorm_fwd_kernel<8, true>, rmsnorm_fwd_kernel<8, false>); break;
   }
   return cudaGetLastError();
 }
@@ -1059,38 +1076,41 @@ long long rmsnorm_bwd_partial_rows(long long rows, int num_sms) {
   return grid_for(rows, 1, (num_sms > 0 ? num_sms : 148) * 4);  // one wave of persistent CTAs
 }
 
+template <int VEC, bool RES>
+static cudaError_t launch_rmsnorm_bwd_variant(const void* dy, const void* dres, const void* x, const void* w,
+                                              const float* rstd, void* dx, float* dw, float* dw_partial, long long rows,
+                                              int H, unsigned grid, cudaStream_t stream) {
+  constexpr int smem = rn_bwd_smem(VEC, RES ? 3 : 2);
+  if (smem + 1024 > 48 * 1024) {  // static shared memory counts too; asked for on the device that launches
+    const cudaError_t e =
+        cudaFuncSetAttribute(rmsnorm_bwd_kernel<VEC, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_chained(rmsnorm_bwd_kernel<VEC, RES>, grid, RN_THREADS, smem, stream,
+                        reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(dres),
+                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w), rstd,
+                        reinterpret_cast<__nv_bfloat16*>(dx), dw, dw_partial, rows, H);
+}
+
 cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw,
-                               float* dw_partial, long long rows, int H, int num_sms, cudaStream_t stream) {
+                               float* dw_partial, long long rows, int H, int num_sms, cudaStream_t stream,
+                               const void* dres) {
   if (H % 8 != 0 || H > RN_THREADS * 8 * 8 || rows <= 0) return cudaErrorInvalidValue;
   const unsigned grid = static_cast<unsigned>(rmsnorm_bwd_partial_rows(rows, num_sms));
   if (dw == nullptr) dw_partial = nullptr;
-  auto dyb = reinterpret_cast<const __nv_bfloat16*>(dy);
-  auto xb = reinterpret_cast<const __nv_bfloat16*>(x);
-  auto wb = reinterpret_cast<const __nv_bfloat16*>(w);
-  auto dxb = reinterpret_cast<__nv_bfloat16*>(dx);
-  static bool configured = false;
-  if (!configured) {  // the largest ring (H up to 8192) is above the default 48 KiB of dynamic shared memory
-    cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, rn_bwd_smem(8));
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  auto go = [&](auto res, auto plain) {
+    return (dres != nullptr ? res : plain)(dy, dres, x, w, rstd, dx, dw, dw_partial, rows, H, grid, stream);
+  };
+  cudaError_t e;
   switch (rn_vec_for(H)) {
-    case 1: launch_chained(rmsnorm_bwd_kernel<1>, grid, RN_THREADS, rn_bwd_smem(1), stream, dyb, xb, wb, rstd, dxb,
-                           dw, dw_partial, rows, H); break;
-    case 2: launch_chained(rmsnorm_bwd_kernel<2>, grid, RN_THREADS, rn_bwd_smem(2), stream, dyb, xb, wb, rstd, dxb,
-                           dw, dw_partial, rows, H); break;
-    case 4: launch_chained(rmsnorm_bwd_kernel<4>, grid, RN_THREADS, rn_bwd_smem(4), stream, dyb, xb, wb, rstd, dxb,
-                           dw, dw_partial, rows, H); break;
-    default: launch_chained(rmsnorm_bwd_kernel<8>, grid, RN_THREADS, rn_bwd_smem(8), stream, dyb, xb, wb, rstd, dxb,
-                            dw, dw_partial, rows, H); break;
+    case 1: e = go(launch_rmsnorm_bwd_variant<1, true>, launch_rmsnorm_bwd_variant<1, false>); break;
+    case 2: e = go(launch_rmsnorm_bwd_variant<2, true>, launch_rmsnorm_bwd_variant<2, false>); break;
+    case 4: e = go(launch_rmsnorm_bwd_variant<4, true>, launch_rmsnorm_bwd_variant<4, false>); break;
+    default: e = go(launch_rmsnorm_bwd_variant<8, true>, launch_rmsnorm_bwd_variant<8, false>); break;
   }
-  if (dw_partial != nullptr) {
-    const unsigned slices = grid < 16u ? grid : 16u;
-    launch_chained(colsum_stage1_kernel, dim3((H + 127) / 128, slices), 128, 0, stream, dw_partial,
-                   static_cast<int>(grid), H);
-    launch_chained(colsum_stage2_kernel, (H + 127) / 128, 128, 0, stream, dw_partial, dw, static_cast<int>(slices), H);
-  }
-  return cudaGetLastError();
+  if (e == cudaSuccess && dw_partial != nullptr)
+    e = launch_chained(colsum_kernel, (H + 31) / 32, CSUM_WARPS * 32, 0, stream, dw_partial, dw, static_cast<int>(grid), H);
+  return e;
 }
 
 cudaError_t launch_rope(void* t, const float* cos_tab, const float* sin_tab, long long rows, int seq, int heads,

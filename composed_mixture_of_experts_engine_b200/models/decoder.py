@@ -19,6 +19,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from ..ops import functional as OF
 from ..parallel import collectives as C
@@ -64,6 +65,10 @@ class CausalSelfAttention(nn.Module):
         return self.wo(o.reshape(B, S, self.nh * self.hd))
 
 
+def _hooked(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
 class DecoderBlock(nn.Module):
     def __init__(self, cfg, topology: ParallelTopology, dtype: torch.dtype):
         super().__init__()
@@ -85,6 +90,20 @@ class DecoderBlock(nn.Module):
                 # the layer will take sequence shards: its router then sees a shard only (known now, so that the
                 # optimizer can group the gate with the other partially summed parameters)
                 self.moe.router.gate_w.sequence_parallel_grad = True
+
+    def joins_residuals(self) -> bool:
+        """Whether :meth:`forward_joined` does what calling the block does: nothing watches the block or its norms
+        (hooks, other modules in their place), and the layer takes whole sequences."""
+        return (type(self) is DecoderBlock and type(self.attn_norm) is RMSNorm and type(self.norm) is RMSNorm
+                and not self.sequence_parallel and "forward" not in self.__dict__ and not _has_any_global_hook()
+                and not any(_hooked(m) for m in (self, self.attn_norm, self.norm)))
+
+    def forward_joined(self, x: torch.Tensor, delta: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
+        """The block on ``x + delta``, its result left as (residual stream, expert output): every addition to the stream
+        is part of the norm that reads it, in both directions."""
+        x, h = OF.add_rmsnorm(x, delta, self.attn_norm.weight, self.attn_norm.eps)
+        x, h = OF.add_rmsnorm(x, self.attn(h), self.norm.weight, self.norm.eps)
+        return x, self.moe(h)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         x = x + self.attn(self.attn_norm(x))
@@ -211,27 +230,47 @@ class MoEDecoder(nn.Module):
             x = C.split(x, 1, tp_process_group(self.topology))
         return x
 
-    def run_blocks(self, x: torch.Tensor) -> torch.Tensor:
+    def _run_blocks(self, x: torch.Tensor) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+        """(residual stream, what is still to be added to it) behind the blocks."""
         recompute = bool(self.cfg.training.activation_recompute) and torch.is_grad_enabled()
+        delta = None
         for blk in self.blocks:
+            if not recompute and isinstance(blk, DecoderBlock) and blk.joins_residuals() and OF.rmsnorm_supported(
+                    x, blk.attn_norm.weight) and OF.rmsnorm_supported(x, blk.norm.weight):
+                x, delta = blk.forward_joined(x, delta)
+                continue
+            if delta is not None:
+                x, delta = x + delta, None
             if recompute:
                 from torch.utils.checkpoint import checkpoint
 
                 x = checkpoint(blk, x, use_reentrant=False)
             else:
                 x = blk(x)
-        return x
+        return x, delta
+
+    def run_blocks(self, x: torch.Tensor) -> torch.Tensor:
+        x, delta = self._run_blocks(x)
+        return x if delta is None else x + delta
 
     def final_hidden(self, x: torch.Tensor) -> torch.Tensor:
         return self.norm(x)
 
+    def _hidden(self, x: torch.Tensor) -> torch.Tensor:
+        """``final_hidden(run_blocks(x))``, the last addition joined with the norm where nothing watches that."""
+        if not (type(self.norm) is RMSNorm and not _hooked(self.norm) and not _has_any_global_hook()
+                and all(getattr(type(self), f) is getattr(MoEDecoder, f) and f not in self.__dict__
+                        for f in ("run_blocks", "final_hidden"))):
+            return self.final_hidden(self.run_blocks(x))
+        x, delta = self._run_blocks(x)
+        return self.final_hidden(x) if delta is None else OF.add_rmsnorm(x, delta, self.norm.weight, self.norm.eps)[1]
+
     def forward(self, ids_or_hidden: torch.Tensor) -> torch.Tensor:
         """Stage forward.  First stage takes token ids [B, S]; the last stage returns logits [B, S, V]."""
         x = self.embed_tokens(ids_or_hidden) if self.is_first_stage else ids_or_hidden
-        x = self.run_blocks(x)
         if not self.is_last_stage:
-            return x
-        x = self.final_hidden(x)
+            return self.run_blocks(x)
+        x = self._hidden(x)
         if self.sequence_parallel:
             x = C.all_gather(x, 1, tp_process_group(self.topology), reduce_scatter_grad=False)
         return OF.linear(x, self.lm_head.weight)
@@ -241,7 +280,7 @@ class MoEDecoder(nn.Module):
         """Cross-entropy of the next-token targets [B, S] (mean over tokens unless ``scale`` is given), computed
         without materialising the [B*S, V] logits on the device path.  Last stage only."""
         x = self.embed_tokens(ids_or_hidden) if self.is_first_stage else ids_or_hidden
-        x = self.final_hidden(self.run_blocks(x))
+        x = self._hidden(x)
         tgt = targets
         if self.sequence_parallel:
             tp, r = self.topology.tp_size, self.topology.tp_rank

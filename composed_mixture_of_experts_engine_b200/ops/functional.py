@@ -33,23 +33,28 @@ def on_device_path(*tensors: torch.Tensor) -> bool:
 
 
 # ------------------------------------------------------------------------------------------ RMSNorm
-class _RMSNormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, eps):
-        xc = x.contiguous()
-        y = torch.empty_like(xc)
-        rstd = torch.empty(xc.numel() // xc.shape[-1], device=x.device, dtype=torch.float32)
-        _ext.ext().rmsnorm_fwd(xc, weight, y, rstd, eps)
-        ctx.save_for_backward(xc, weight, rstd)
-        return y
+class _AddRMSNormFn(torch.autograd.Function):
+    """(x + delta, norm of it) in one kernel, or (x, norm of it) without ``delta``; the backward adds the gradients of
+    both results in one kernel too, and the weight's gradient into its fp32 ``main_grad`` when it has one."""
 
     @staticmethod
-    def backward(ctx, dy):
-        x, weight, rstd = ctx.saved_tensors
-        dx = torch.empty_like(x)
-        dw = torch.zeros(weight.shape, device=x.device, dtype=torch.float32)
-        _ext.ext().rmsnorm_bwd(dy.contiguous(), x, weight, rstd, dx, dw)
-        return dx, dw.to(weight.dtype), None
+    def forward(ctx, x, delta, weight, eps):
+        s, y, rstd = _ext.ext().add_rmsnorm(x, delta, weight, eps)
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(s, weight, rstd)
+        ctx.has_delta = delta is not None
+        return s, y
+
+    @staticmethod
+    def backward(ctx, ds, dy):
+        s, weight, rstd = ctx.saved_tensors
+        dw = None
+        if dy is None:
+            dx = ds
+        else:
+            dx, dw = _ext.ext().add_rmsnorm_grad(dy, ds, s, weight, rstd, ctx.needs_input_grad[2],
+                                                 getattr(weight, "main_grad", None))
+        return dx, dx if ctx.has_delta else None, dw, None
 
 
 def rmsnorm_reference(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
@@ -57,10 +62,36 @@ def rmsnorm_reference(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torc
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * weight.float()).to(x.dtype)
 
 
+def rmsnorm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    return on_device_path(x, weight) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192
+
+
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
-    if on_device_path(x, weight) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
-        return _RMSNormFn.apply(x, weight, eps)
+    if rmsnorm_supported(x, weight):
+        return add_rmsnorm(x, None, weight, eps)[1]
     return rmsnorm_reference(x, weight, eps)
+
+
+def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, eps: float = 1e-5
+                ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``s = x + delta`` (``x`` without ``delta``) and the RMSNorm of ``s``: a residual stream, the branch that joins it
+    and the norm in front of the next branch."""
+    if rmsnorm_supported(x, weight) and (delta is None or (on_device_path(delta) and delta.shape == x.shape)):
+        x = _vectors(x)
+        if delta is not None:
+            delta = _vectors(delta)
+        if kernels.needs_autograd(x, weight, *(() if delta is None else (delta,))):
+            return _AddRMSNormFn.apply(x, delta, _vectors(weight), eps)
+        s, y, _ = _ext.ext().add_rmsnorm(x, delta, _vectors(weight), eps)
+        return s, y
+    s = x if delta is None else x + delta
+    return s, rmsnorm(s, weight, eps)
+
+
+def _vectors(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte boundary (autograd sees the copy where one is needed)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 # ------------------------------------------------------------------------------------------ token embedding
