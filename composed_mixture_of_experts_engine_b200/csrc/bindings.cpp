@@ -14,13 +14,14 @@
 #include "gemm.cuh"
 #include "host_ops.h"
 #include "launch.h"
+#include "native_ops.h"
 #include "ops.cuh"
 #include "router.cuh"
 
 namespace {
 
+using cmoe::OptTensor;
 using torch::Tensor;
-using OptTensor = std::optional<Tensor>;
 
 void check_cuda(cudaError_t e, const char* what) {
   TORCH_CHECK(e == cudaSuccess, "cmoe: ", what, " failed: ", cudaGetErrorString(e));
@@ -532,7 +533,25 @@ void combine_bwd_w(const Tensor& rows, const Tensor& slot_row, const Tensor& dy,
 
 }  // namespace
 
+namespace cmoe {
+std::tuple<Tensor, Tensor, Tensor> add_rmsnorm(const Tensor& x, const OptTensor& delta, const Tensor& w, double eps) {
+  return ::add_rmsnorm(x, delta, w, eps);
+}
+std::tuple<Tensor, OptTensor> add_rmsnorm_grad(const Tensor& dy, const OptTensor& dsum, const Tensor& x, const Tensor& w,
+                                               const Tensor& rstd, bool need_dw, const OptTensor& main) {
+  return ::add_rmsnorm_grad(dy, dsum, x, w, rstd, need_dw, main);
+}
+void rope(Tensor& t, const Tensor& cos_tab, const Tensor& sin_tab, int64_t seq, bool inverse) {
+  ::rope(t, cos_tab, sin_tab, seq, inverse);
+}
+void qkv_grad_pack(const Tensor& dq, const Tensor& dk, const Tensor& dv, Tensor& out, const Tensor& cos_tab,
+                   const Tensor& sin_tab) {
+  ::qkv_grad_pack(dq, dk, dv, out, cos_tab, sin_tab);
+}
+}  // namespace cmoe
+
 void register_attention(pybind11::module_& m);
+void register_autograd(pybind11::module_& m);
 void register_ep(pybind11::module_& m);
 void register_router(pybind11::module_& m);
 void register_moe(pybind11::module_& m);
@@ -571,4 +590,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   register_ep(m);
   register_router(m);
   register_moe(m);
+  register_autograd(m);
 }

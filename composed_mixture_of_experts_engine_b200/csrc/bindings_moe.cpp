@@ -14,12 +14,15 @@
 #include <tuple>
 
 #include "host_ops.h"
+#include "native_ops.h"
 #include "ops.cuh"
 
 namespace {
 
+using cmoe::OptTensor;
+using Forward = cmoe::MoeForward;
+using Backward = cmoe::MoeBackward;
 using torch::Tensor;
-using OptTensor = std::optional<Tensor>;
 
 void check(cudaError_t e, const char* what) {
   TORCH_CHECK(e == cudaSuccess, "cmoe: ", what, " failed: ", cudaGetErrorString(e));
@@ -209,7 +212,6 @@ void set_weights(cmoe::GemmArgs& g, const Tensor& gate_w32, const PlanTables& pt
 }
 
 // (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads), yp only with one pick per token
-using Forward = std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor>;
 Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
                           const Tensor& w2, int64_t capacity, bool keep, const OptTensor& status,
                           const OptTensor& overflow, const OptTensor& made_plan) {
@@ -302,7 +304,6 @@ OptTensor expert_wgrad(const Tensor& a, const Tensor& b, const Tensor& weight, c
 }
 
 // (dx, d_gate, dw13, dw2)
-using Backward = std::tuple<OptTensor, OptTensor, OptTensor, OptTensor>;
 Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor& xp, const Tensor& hact, const Tensor& gu,
                             const OptTensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2, bool need_dx,
                             bool need_gate, const OptTensor& main13, const OptTensor& main2, const OptTensor& status) {
@@ -371,6 +372,20 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
 }
 
 }  // namespace
+
+namespace cmoe {
+MoeForward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
+                             const Tensor& w2, int64_t capacity, bool keep, const OptTensor& status,
+                             const OptTensor& overflow, const OptTensor& made_plan) {
+  return ::moe_local_forward(x, gate_w32, idx32, w13, w2, capacity, keep, status, overflow, made_plan);
+}
+MoeBackward moe_local_backward(const Tensor& dy, const Tensor& plan, const Tensor& xp, const Tensor& hact, const Tensor& gu,
+                               const OptTensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2,
+                               bool need_dx, bool need_gate, const OptTensor& main13, const OptTensor& main2,
+                               const OptTensor& status) {
+  return ::moe_local_backward(dy, plan, xp, hact, gu, yp, gate_w32, w13, w2, need_dx, need_gate, main13, main2, status);
+}
+}  // namespace cmoe
 
 void register_moe(pybind11::module_& m) {
   m.def("moe_local_plan", &moe_local_plan);

@@ -11,12 +11,14 @@
 #include <utility>
 
 #include "host_ops.h"
+#include "native_ops.h"
 #include "router.cuh"
 
 namespace {
 
+using cmoe::OptTensor;
+using cmoe::RouteResult;
 using torch::Tensor;
-using OptTensor = std::optional<Tensor>;
 
 // Statistics workspace, zero between launches (the kernel leaves it so).  One per (device, stream): launches on one
 // stream run in order, launches on two streams must not share the accumulators.  At most kMaxWorkspaces are kept
@@ -45,8 +47,6 @@ Tensor router_workspace(const c10::Device& dev, cudaStream_t stream) {
 
 // (idx32, w32, idx64, w16, logits, lse, counts, counts64, mean_prob, stats).  `full` false: only the routing decision
 // in its public types (idx64, w16) is produced, for callers that want no gradient and no statistics.
-using RouteResult = std::tuple<OptTensor, OptTensor, Tensor, Tensor, OptTensor, OptTensor, OptTensor, OptTensor,
-                               OptTensor, OptTensor>;
 RouteResult router_route(const Tensor& X, const Tensor& Wg, int64_t K, bool full, const OptTensor& status) {
   TORCH_CHECK(X.is_cuda() && X.scalar_type() == at::kBFloat16 && X.dim() == 2 && X.stride(1) == 1,
               "X must be a CUDA bf16 matrix with unit inner stride");
@@ -139,6 +139,19 @@ std::tuple<OptTensor, OptTensor> router_grad(const Tensor& X, const Tensor& Wg, 
 }
 
 }  // namespace
+
+namespace cmoe {
+RouteResult router_route(const Tensor& X, const Tensor& Wg, int64_t K, bool full, const OptTensor& status) {
+  return ::router_route(X, Wg, K, full, status);
+}
+std::tuple<OptTensor, OptTensor> router_grad(const Tensor& X, const Tensor& Wg, const Tensor& logits, const Tensor& lse,
+                                             const Tensor& idx32, const Tensor& counts, const OptTensor& grad_w32,
+                                             const OptTensor& grad_w16, const OptTensor& grad_aux, const OptTensor& grad_z,
+                                             bool need_tokens, bool need_gate, bool gate_bf16, const OptTensor& status) {
+  return ::router_grad(X, Wg, logits, lse, idx32, counts, grad_w32, grad_w16, grad_aux, grad_z, need_tokens, need_gate,
+                       gate_bf16, status);
+}
+}  // namespace cmoe
 
 void register_router(pybind11::module_& m) {
   m.def("router_route", &router_route);

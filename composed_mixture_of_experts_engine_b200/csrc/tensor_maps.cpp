@@ -32,10 +32,16 @@ cudaError_t encode(CUtensorMap* out, CUtensorMapDataType type, int rank, const v
   const EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return cudaErrorNotSupported;
   const cuuint32_t estride[3] = {1u, 1u, 1u};
-  return enc(out, type, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr), dims, strides, box, estride,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-             ? cudaSuccess
-             : cudaErrorInvalidValue;
+  const auto pack = [&] {
+    return enc(out, type, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr), dims, strides, box, estride,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  if (pack()) return cudaSuccess;
+  // A thread that has made no runtime call yet (a backward thread whose first node this is) has no current context, which
+  // the driver's encoder needs and cudaSetDevice brings.
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && pack()) return cudaSuccess;
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace

@@ -297,8 +297,9 @@ class MoEDecoder(nn.Module):
         return [blk.moe for blk in self.blocks]
 
     def aux_losses(self) -> Tuple[torch.Tensor, torch.Tensor]:
-        aux = [l.router.last_aux_loss * l.aux_scale for l in self.moe_layers() if l.router.last_aux_loss is not None]
-        z = [l.router.last_z_loss * l.aux_scale for l in self.moe_layers() if l.router.last_z_loss is not None]
+        scaled = lambda t, l: t if l.aux_scale == 1.0 else t * l.aux_scale
+        aux = [scaled(l.router.last_aux_loss, l) for l in self.moe_layers() if l.router.last_aux_loss is not None]
+        z = [scaled(l.router.last_z_loss, l) for l in self.moe_layers() if l.router.last_z_loss is not None]
         dev = next(self.parameters()).device
         zero = torch.zeros((), device=dev, dtype=torch.float32)
         n = max(self.num_layers_total, 1)

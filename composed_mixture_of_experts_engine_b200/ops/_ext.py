@@ -31,6 +31,7 @@ _SOURCES = [
     "bindings_ep.cpp",
     "bindings_router.cpp",
     "bindings_moe.cpp",
+    "bindings_autograd.cpp",
     "host_ops.cpp",
     "tensor_maps.cpp",
     "gemm.cu",

@@ -9,6 +9,7 @@ RoPE and attention are additions (the reference model has neither).
 
 from __future__ import annotations
 
+import os
 from typing import Optional, Tuple
 
 import torch
@@ -22,14 +23,21 @@ from .kernels import EPI_SWIGLU_BWD, EPI_SWIGLU_FWD, GEMM_GROUPED_K, GEMM_GROUPE
 def force_library() -> bool:
     """``CMOE_FORCE_LIBRARY=1``: every differentiable op takes its PyTorch path even on a B200 (the library arm of
     the benchmarks: cuBLAS / cuDNN / eager kernels through PyTorch, nothing of this package's device code)."""
-    import os
-
     return os.environ.get("CMOE_FORCE_LIBRARY", "0") == "1"
 
 
 def on_device_path(*tensors: torch.Tensor) -> bool:
     """True when the sm_100a kernels handle these tensors (CUDA + bf16)."""
-    return all(t.is_cuda and t.dtype == torch.bfloat16 for t in tensors) and not force_library()
+    for t in tensors:
+        if not t.is_cuda or t.dtype != torch.bfloat16:
+            return False
+    return not force_library()
+
+
+def native_nodes(*tensors: torch.Tensor) -> bool:
+    """Whether a call goes through the native autograd node of its operation (csrc/bindings_autograd.cpp): not while it
+    is traced and not with a forward-mode tangent, which the Python functions record and refuse."""
+    return tensors[0].is_cuda and not kernels.traced_or_dual(*tensors)
 
 
 # ------------------------------------------------------------------------------------------ RMSNorm
@@ -80,10 +88,13 @@ def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
         x = _vectors(x)
         if delta is not None:
             delta = _vectors(delta)
-        if kernels.needs_autograd(x, weight, *(() if delta is None else (delta,))):
-            return _AddRMSNormFn.apply(x, delta, _vectors(weight), eps)
-        s, y, _ = _ext.ext().add_rmsnorm(x, delta, _vectors(weight), eps)
-        return s, y
+        weight = _vectors(weight)
+        given = (x, weight) if delta is None else (x, weight, delta)
+        if not kernels.needs_autograd(*given):
+            return _ext.ext().add_rmsnorm(x, delta, weight, eps)[:2]
+        if native_nodes(*given):
+            return _ext.ext().add_rmsnorm_node(x, delta, weight, eps)
+        return _AddRMSNormFn.apply(x, delta, weight, eps)
     s = x if delta is None else x + delta
     return s, rmsnorm(s, weight, eps)
 
@@ -184,7 +195,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     """``x @ weight^T (+ bias)`` with ``weight`` [out, in] (the ``nn.Linear`` contraction).  Reference counterpart:
     the ``F.linear`` calls of pkg/distributed/tensor_parallel.py:121,197 and pkg/models/moe.py:186 (cuBLAS there)."""
     if linear_supported(x, weight):
-        y = _LinearFn.apply(x, weight)
+        if native_nodes(x, weight):
+            y = _ext.ext().linear(x, weight, kernels.status_word(x.device))
+        else:
+            y = _LinearFn.apply(x, weight)
         return y if bias is None else y + bias
     return F.linear(x, weight, bias)
 
@@ -309,6 +323,8 @@ def rope_causal_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
     rotary embedding on q and k.  On the device path ``qkv`` is consumed (rotated in place)."""
     B, S, heads, hd = qkv.shape
     if on_device_path(qkv) and hd % 16 == 0 and qkv.is_contiguous():
+        if nh == nkv and native_nodes(qkv) and not _attn_sm100.enabled():
+            return _ext.ext().rope_attention(qkv, cos, sin, nh)
         return _RopeAttentionFn.apply(qkv, cos, sin, nh, nkv)
     t = rope(qkv.reshape(B * S, heads, hd), cos, sin, S, nh + nkv).view(B, S, heads, hd)
     return causal_attention(t[:, :, :nh], t[:, :, nh: nh + nkv], t[:, :, nh + nkv:])
@@ -438,8 +454,6 @@ def _local_fused() -> bool:
     """Gather and combine transfers run as kernels of their own (default) or inside the grouped GEMMs
     (``CMOE_LOCAL_FUSED=1``; measured slightly slower on one B200: the row-pull warps cost the GEMM about what the
     separate gather kernel costs)."""
-    import os
-
     return os.environ.get("CMOE_LOCAL_FUSED", "0") != "0"
 
 
@@ -559,6 +573,14 @@ def local_moe(x: torch.Tensor, gate_w: torch.Tensor, idx: torch.Tensor, w13: tor
         if _local_fused() and x.shape[1] % 8 == 0:
             return _LocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
         if kernels.needs_autograd(x, gate_w32, w13, w2):
+            if native_nodes(x, gate_w32, w13, w2):
+                dev = x.device
+                y, plan = _ext.ext().moe_local_node(
+                    x, gate_w32, idx32, w13, w2, capacity, kernels.status_word(dev), kernels.overflow_counter(dev),
+                    _checked_plan(idx32, w13.shape[0], capacity) if debug.enabled() else None)
+                if holder is not None:
+                    holder["plan"] = _LocalPlan(plan, w13.shape[0])
+                return y
             return _NativeLocalMoEFn.apply(x, gate_w32, idx32, w13, w2, capacity, holder)
         return _native_forward(x, gate_w32, idx32, w13, w2, capacity, False, holder)[0]
     keep = None

@@ -21,6 +21,7 @@ The load-balance loss ``E * sum_i f_i * P_i`` and the z-loss are returned as dif
 from __future__ import annotations
 
 import math
+import os
 from dataclasses import dataclass
 from typing import Any, Dict, Optional, Tuple
 
@@ -83,8 +84,6 @@ def _should_use_fused(tokens: torch.Tensor, gate_w: torch.Tensor, force_referenc
     """Single source of truth for "will the sm_100a kernel run" (used for dispatch and for telemetry)."""
     if force_reference or not (tokens.is_cuda and gate_w.is_cuda):
         return False
-    import os
-
     if os.environ.get("CMOE_FORCE_LIBRARY", "0") == "1":  # the benchmarks' library arm: no device code of this package
         return False
     if tokens.dtype != torch.bfloat16 or tokens.dim() != 2:
@@ -338,18 +337,24 @@ class MoERouter(nn.Module):
         E, K = self.num_experts, self.top_k
         fused = self.bias is None and _should_use_fused(tokens, self.gate_w, force_reference, K)
         if fused:
-            if kernels.needs_autograd(tokens, self.gate_w):
+            if not kernels.needs_autograd(tokens, self.gate_w):
+                out = fused_router_forward(tokens, _bf16_gate(self.gate_w), K, self.profile_timing)
+                w32, w, idx32, idx = out.w32, out.w16, out.idx32, out.idx64
+                aux, z = out.stats[0], out.stats[1]
+            elif (tokens.is_cuda and self.gate_w.dtype == torch.bfloat16 and self.gate_w.is_contiguous()
+                  and not self.profile_timing and not kernels.traced_or_dual(tokens, self.gate_w)):
+                fields, aux, z = _ext.ext().router_node(tokens, self.gate_w, K, kernels.status_word(tokens.device))
+                out = RouterOutput(*fields)
+                w32, w, idx32, idx = out.w32, out.w16, out.idx32, out.idx64
+            else:
                 holder: Dict[str, Any] = {}
                 w32, w, aux, z, idx32, idx = FusedRouterFunction.apply(tokens, self.gate_w, K, holder,
                                                                        self.profile_timing)
                 out: RouterOutput = holder["out"]
-            else:
-                out = fused_router_forward(tokens, _bf16_gate(self.gate_w), K, self.profile_timing)
-                w32, w, idx32, idx = out.w32, out.w16, out.idx32, out.idx64
-                aux, z = out.stats[0], out.stats[1]
-            self._last_logits, self.last_aux_loss, self.last_z_loss = out.logits, aux, z
-            self.last_idx32, self.last_w32 = idx32, w32
-            self._pending = dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2)
+            # plain attributes, set past the module's look at each for parameters and buffers
+            self.__dict__.update(
+                _last_logits=out.logits, last_aux_loss=aux, last_z_loss=z, last_idx32=idx32, last_w32=w32,
+                _pending=dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2))
             return idx, w, out.counts64
         # PyTorch path (bias, CPU, fp32 tokens, shapes the kernel does not cover): fp64 math under autograd
         logits64 = tokens.to(torch.float64) @ self.gate_w.to(torch.float64)
