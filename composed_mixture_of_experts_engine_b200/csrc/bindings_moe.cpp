@@ -104,6 +104,7 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.epilogue = epilogue;
   g.b_early = 1;  // weights and row plan are older than the kernel before each of these launches
+  g.b_once = g.rows_per_group <= 128;  // one tile of most experts
   if (short_tiles) {
     g.tile_rows = plan + pt.tile_rows;
     return g;

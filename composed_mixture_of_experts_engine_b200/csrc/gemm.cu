@@ -104,6 +104,7 @@ struct KParams {
   long long scatter_slots_per_rank;
   PeerTable scatter_out;
   long long scatter_ld;
+  int b_once;      // B is read once
   int b_early;     // B does not depend on the kernel before this one
   int chained;     // launched to overlap its neighbours in the stream
   int out_mode;    // OutMode (EPI_STORE only)
@@ -398,6 +399,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else if (warp == b_warp) {
     // ------------------------------------------------------------------ TMA producer of B
     if (elect_one()) {
+      const uint64_t once = l2_evict_first();
       int stage = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
@@ -412,6 +414,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               tma_load_2d(b_dst + j * CHUNK_BYTES, &tmB, &full_bar[stage], ti.b_n0 + 64 * j, k);
+          } else if (p.b_once) {
+            tma_load_2d_policy(b_dst, &tmB, &full_bar[stage], k, ti.b_n0, once);
+            tma_load_2d_policy(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], k, ti.b_n1, once);
           } else {
             tma_load_2d(b_dst, &tmB, &full_bar[stage], k, ti.b_n0);
             tma_load_2d(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], k, ti.b_n1);
@@ -1148,6 +1153,7 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.row_dot_stride = a.row_dot_stride;
   kp.status = a.status;
   kp.chained = gemm_overlaps_neighbours(a);
+  kp.b_once = a.b_once;
   kp.b_early = a.b_early && kp.chained;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
   kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? 128 : BN;

@@ -71,6 +71,7 @@ struct K2Params {
   int band;           // row tiles walked together
   const int* group_order;  // grouped by K: the groups, longest first
   int cols_per_tile;  // output columns of a tile (256; SwiGLU forward 128: gate in one CTA's half of B, up in the other's)
+  int b_once;         // B is read once
   int b_early;        // B does not depend on the kernel before this one
   int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
@@ -160,6 +161,14 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_policy(void* smem_dst, const CUtensorMap* tmap, uint32_t bar_cluster_addr,
+                                                        int x, int y, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y), "l"(policy)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
@@ -287,6 +296,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       const bool mn = is_a ? p.a_mn != 0 : p.b_mn != 0;
       uint8_t* const dst0 = is_a ? sA : sB;
       const uint32_t fb0 = map_to_cta(smem_u32(full_bar), 0);
+      const uint64_t once = l2_evict_first();
+      const bool stream = !is_a && p.b_once;
       const int moff = static_cast<int>(cta) * 128;  // this CTA's rows of A
       int stage = 0;
       uint32_t phase = 0;
@@ -309,6 +320,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if (mn) {
               tma_load_2d_pair(dst, tm, fb, x, k);
               tma_load_2d_pair(dst + T_CHUNK_BYTES, tm, fb, x + 64, k);
+            } else if (stream) {
+              tma_load_2d_pair_policy(dst, tm, fb, k, x, once);
             } else {
               tma_load_2d_pair(dst, tm, fb, k, x);
             }
@@ -690,6 +703,7 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   const long long b_extent = a.epilogue == EPI_SWIGLU_FWD ? 2LL * a.N : a.N;
   kp.band = b_extent > group_rows && group_rows >= 8 * T_BM ? 8 : 4;
   kp.cols_per_tile = a.epilogue == EPI_SWIGLU_FWD ? 128 : T_BN;
+  kp.b_once = a.b_once;
   kp.b_early = a.b_early;
   kp.has_aux = a.aux_out != nullptr;
   kp.d_fp32 = a.d_fp32;
