@@ -75,6 +75,26 @@ Shapes check_shapes(const Tensor& x, const Tensor& idx32, const Tensor& w13, con
   return s;
 }
 
+// Rows of B in a tile where a layer of few rows streams its weights: the width with which nearly whole rounds of tiles
+// fill the SMs, for what counts is that all of them load all the time.  64 rows only where wider tiles leave the chip
+// half empty: a k-block of 8 KiB takes its threads as long to issue as one of 16.  64 tokens top-8, E 64 H 2048 F 1024
+// (3.46 rounds of 256, 6.92 of 128): 171.7 -> 158.9 us; 64 rows against 256 where both fill the chip: 5 tokens of the same
+// layer 111.6 / 102.9, 8 tokens top-2, E 8 H 4096 F 4096 175.9 / 157.6.
+int streamed_tile(int64_t m_tiles, int64_t N, int epilogue, int sms) {
+  int best = 256;
+  double best_fill = 0.0;
+  for (int bn : {256, 128, 64}) {
+    const int64_t cols = epilogue == cmoe::EPI_SWIGLU_FWD ? bn / 2 : bn;
+    const double rounds = static_cast<double>(m_tiles * ((N + cols - 1) / cols)) / sms;
+    const double fill = rounds / std::ceil(rounds) * (bn == 64 ? 0.75 : 1.0);
+    if (fill > 1.05 * best_fill) {
+      best = bn;
+      best_fill = fill;
+    }
+  }
+  return best;
+}
+
 // a grouped-by-rows launch over the tiles of `plan`: D[rows, N] = A[rows, K] * B (one [b_rows, b_cols] block per expert)
 cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_rows, bool b_mn, const Tensor& D, int64_t N,
                             int64_t K, const PlanTables& pt, int* plan, int* status,
@@ -107,9 +127,10 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   g.b_once = g.rows_per_group <= 128;  // one tile of most experts
   if (short_tiles) {
     g.tile_rows = plan + pt.tile_rows;
+    g.tile_n = streamed_tile(std::min(pt.E, pt.n_slots), N, epilogue, g.num_sms);
     return g;
   }
-  // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs 0.85 of the time of a tile (it loads
+  // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs about 0.85 of the time of a tile (it loads
   // a third less per FLOP) but wastes one of its SMs where an expert has an odd number of tiles, and rounds are counted
   // in whole tiles.  So the rounds of both are estimated, every expert ending in half a tile or pair on average.
   // Forward and backward of a layer, E 64 H 2048 F 1024, GEMM times on single SMs / pairs: 2048 rows per expert 2741 /
@@ -117,7 +138,9 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   // rounds of tiles face 31 of pairs, 428 / 471 where 4 face 5.
   const double tiles = pt.n_slots / 128.0 + 0.5 * pt.E, pairs = pt.n_slots / 256.0 + 0.5 * pt.E;
   const int64_t cols = (N + (epilogue == cmoe::EPI_SWIGLU_FWD ? 127 : 255)) / (epilogue == cmoe::EPI_SWIGLU_FWD ? 128 : 256);
-  if (0.85 * std::ceil(pairs * cols / (g.num_sms / 2)) < std::ceil(tiles * cols / g.num_sms)) {
+  // (0.9: near a tie single SMs, which compute fewer rows of padding; 1000 tokens top-8 of 64 experts, 125 rows each, the
+  // GEMMs of two forward layers 354 / 343 us.)
+  if (0.9 * std::ceil(pairs * cols / (g.num_sms / 2)) < std::ceil(tiles * cols / g.num_sms)) {
     g.pair_tile = plan + pt.pair_tile;
     g.num_pairs = plan + pt.num_pairs;
   }

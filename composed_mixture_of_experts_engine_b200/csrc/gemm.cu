@@ -35,9 +35,10 @@ namespace {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;
-constexpr int STAGES = 4;
+constexpr int STAGES = 4;      // of full tiles; tiles with fewer columns have more in the same space
+constexpr int MAX_STAGES = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB
+constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB (full tile)
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int CHUNK_BYTES = 64 * BK * 2;  // one 64 x 64 bf16 box (MN-major operands) = 8 KiB
 constexpr int PIECE_ROWS = 32;
@@ -85,7 +86,9 @@ struct KParams {
   long long row_dot_stride;
   int* status;
   unsigned long long timeout_ns;
-  int n_cols_per_tile;  // output columns covered by one tile (256, or 128 with the SwiGLU forward)
+  int bn;               // accumulator columns of a tile (rows of B): 256, or 128 / 64 where that fills the SMs better
+  int stages, b_boxes;  // pipeline stages, TMA boxes of B in each (K-major)
+  int n_cols_per_tile;  // output columns covered by one tile (bn, or half of it with the SwiGLU forward)
   // fused dispatch: rows of A are pulled from peers by the extra warps
   const int* pull_row_slot;
   PeerTable pull_src;
@@ -275,16 +278,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + STAGES * A_STAGE_BYTES;
+  const int b_bytes = p.bn * BK * 2;  // of a stage
+  uint8_t* sB = smem + p.stages * A_STAGE_BYTES;
   uint8_t* stg = smem + STAGES * STAGE_BYTES;  // 1024-byte aligned, as the swizzle pattern needs
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + STAGING_BYTES);
-  uint64_t* full_bar = bars;                 // [STAGES]
-  uint64_t* empty_bar = bars + STAGES;       // [STAGES]
-  uint64_t* tfull_bar = bars + 2 * STAGES;   // [2]
-  uint64_t* tempty_bar = bars + 2 * STAGES + 2;  // [2]
-  uint64_t* gfull_bar = bars + 2 * STAGES + 4;   // [2] saved gate/up pieces landed (SwiGLU backward)
-  uint64_t* gempty_bar = bars + 2 * STAGES + 6;  // [2] ... and were consumed by all epilogue threads
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8);
+  uint64_t* full_bar = bars;                     // [MAX_STAGES]
+  uint64_t* empty_bar = bars + MAX_STAGES;       // [MAX_STAGES]
+  uint64_t* tfull_bar = bars + 2 * MAX_STAGES;   // [2]
+  uint64_t* tempty_bar = bars + 2 * MAX_STAGES + 2;  // [2]
+  uint64_t* gfull_bar = bars + 2 * MAX_STAGES + 4;   // [2] saved gate/up pieces landed (SwiGLU backward)
+  uint64_t* gempty_bar = bars + 2 * MAX_STAGES + 6;  // [2] ... and were consumed by all epilogue threads
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -292,7 +296,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
@@ -364,7 +368,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else {
           tma_load_2d(a_dst, &tmA, &full_bar[stage], k, ti.a_mn0);
         }
-        if (++stage == STAGES) {
+        if (++stage == p.stages) {
           stage = 0;
           phase ^= 1u;
         }
@@ -407,8 +411,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (ti.skip || ti.k_blocks == 0) continue;
         for (int kb = 0; kb < ti.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, wc, ST_TIMEOUT_SMEM_EMPTY)) break;
-          mbar_arrive_expect_tx(&full_bar[stage], B_STAGE_BYTES);
-          uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
+          mbar_arrive_expect_tx(&full_bar[stage], b_bytes);
+          uint8_t* b_dst = sB + stage * b_bytes;
           const int k = ti.b_k0 + kb * BK;
           if (p.b_mn) {
 #pragma unroll
@@ -416,12 +420,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               tma_load_2d(b_dst + j * CHUNK_BYTES, &tmB, &full_bar[stage], ti.b_n0 + 64 * j, k);
           } else if (p.b_once) {
             tma_load_2d_policy(b_dst, &tmB, &full_bar[stage], k, ti.b_n0, once);
-            tma_load_2d_policy(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], k, ti.b_n1, once);
+            if (p.b_boxes == 2) tma_load_2d_policy(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1, once);
           } else {
             tma_load_2d(b_dst, &tmB, &full_bar[stage], k, ti.b_n0);
-            tma_load_2d(b_dst + 128 * BK * 2, &tmB, &full_bar[stage], k, ti.b_n1);
+            if (p.b_boxes == 2) tma_load_2d(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1);
           }
-          if (++stage == STAGES) {
+          if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -432,7 +436,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
+      const uint32_t idesc = make_idesc_bf16(BM, p.bn, p.a_mn, p.b_mn);
       const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(sA), p.a_mn ? CHUNK_BYTES : 16, 1024);
       const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sB), p.b_mn ? CHUNK_BYTES : 16, 1024);
       const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;  // per UMMA_K = 16 step, in descriptor units of 16 bytes
@@ -456,12 +460,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             stamped = true;
           }
           const uint64_t ad = a_desc0 + static_cast<uint32_t>(stage * (A_STAGE_BYTES >> 4));
-          const uint64_t bd = b_desc0 + static_cast<uint32_t>(stage * (B_STAGE_BYTES >> 4));
+          const uint64_t bd = b_desc0 + static_cast<uint32_t>(stage * (b_bytes >> 4));
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
             umma_bf16_ss(d_tmem, ad + k * a_kstep, bd + k * b_kstep, idesc, (kb | k) != 0 ? 1u : 0u);
           umma_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
-          if (++stage == STAGES) {
+          if (++stage == p.stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -580,7 +584,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           float z[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) z[j] = 0.f;
-          for (int c = 0; c < BN / 32; ++c) store_row_chunk(Dg, p.ldd, p.d_fp32, 0, row, ti.n0 + c * 32, p.N, z);
+          for (int c = 0; c < p.bn / 32; ++c) store_row_chunk(Dg, p.ldd, p.d_fp32, 0, row, ti.n0 + c * 32, p.N, z);
         }
         continue;
       }
@@ -642,7 +646,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
 #pragma unroll 1
-        for (int u = 0; u < BN / unit_cols; ++u) {
+        for (int u = 0; u < p.bn / unit_cols; ++u) {
           const int col0 = ti.n0 + u * unit_cols;
           if (col0 >= p.N) break;  // uniform
           uint8_t* buf = stg + (stage_ctr & 1) * STAGING_BUF_BYTES;
@@ -740,14 +744,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         uint8_t* hrow = stg + row_in_tile * 64;
         bool any_bad = false;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < p.bn / 64; ++c) {
           const int col = ti.n0 + c * 32;
           if (col >= p.N) break;  // uniform
           uint32_t ph[16], pg[16], pu[16];
           if (ok) {
             uint32_t rg[32], ru[32];
             tmem_ld_32x32b_x32(t_acc + c * 32, rg);
-            tmem_ld_32x32b_x32(t_acc + 128 + c * 32, ru);
+            tmem_ld_32x32b_x32(t_acc + p.bn / 2 + c * 32, ru);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -814,7 +818,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             float4 cur[8], nxt[8];
             prefetch_f32_chunk(drow, ti.n0, p.N, row_ok, cur);
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+            for (int c = 0; c < p.bn / 32; ++c) {
               const int col = ti.n0 + c * 32;
               if (col >= p.N) break;
               uint32_t r[32];
@@ -840,7 +844,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           } else {
             // direct bf16 / fp32 stores (and bf16 accumulate) from registers, one row per thread
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+            for (int c = 0; c < p.bn / 32; ++c) {
               if (ti.n0 + c * 32 >= p.N) break;  // uniform across the warp
               uint32_t r[32];
               tmem_ld_32x32b_x32(t_acc + c * 32, r);
@@ -856,11 +860,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else if (EPI == EPI_SWIGLU_FWD) {
           // accumulator columns [0,128) = gate, [128,256) = up for output columns n0 .. n0+127
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < p.bn / 64; ++c) {
             if (ti.n0 + c * 32 >= p.N) break;
             uint32_t rg[32], ru[32];
             tmem_ld_32x32b_x32(t_acc + c * 32, rg);
-            tmem_ld_32x32b_x32(t_acc + 128 + c * 32, ru);
+            tmem_ld_32x32b_x32(t_acc + p.bn / 2 + c * 32, ru);
             tmem_ld_wait();
             if (row_ok) {
               float g[32], u[32], h[32];
@@ -1048,7 +1052,12 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   const int piece_rows = short_tiles ? PIECE_ROWS : BM;
   cudaError_t e = make_tmap(&tmA, a.A, a.a_rows, a.a_cols, a.a_ld, a.a_mn ? 64 : piece_rows);
   if (e != cudaSuccess) return e;
-  e = make_tmap(&tmB, a.B, a.b_rows, a.b_cols, a.b_ld, a.b_mn ? 64 : 128);
+  const int bn = a.tile_n > 0 ? a.tile_n : BN;
+  if ((bn != 256 && bn != 128 && bn != 64) ||
+      (bn != BN && (a.mode != GEMM_GROUPED_M || a.b_mn || a.epilogue == EPI_SWIGLU_BWD)))
+    return cudaErrorInvalidValue;
+  const int b_boxes = a.epilogue == EPI_SWIGLU_FWD || bn == BN ? 2 : 1;
+  e = make_tmap(&tmB, a.B, a.b_rows, a.b_cols, a.b_ld, a.b_mn ? 64 : bn / b_boxes);
   if (e != cudaSuccess) return e;
 
   KParams kp;
@@ -1156,7 +1165,10 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.b_once = a.b_once;
   kp.b_early = a.b_early && kp.chained;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
-  kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? 128 : BN;
+  kp.bn = bn;
+  kp.b_boxes = b_boxes;
+  kp.stages = STAGES * STAGE_BYTES / (A_STAGE_BYTES + bn * BK * 2);  // 4, 6 or 8
+  kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? bn / 2 : bn;
 
   int num_sms = a.num_sms;
   if (num_sms <= 0) {

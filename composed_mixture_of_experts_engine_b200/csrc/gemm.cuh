@@ -54,6 +54,8 @@ struct GemmArgs {
   // grouped-M, optional: live rows of each 128-row tile (device memory).  Where it is given, only the 32-row pieces of a
   // tile that hold live rows are loaded from A and stored to D (and aux_out); plain and SwiGLU forward results only.
   const int* tile_rows = nullptr;
+  int tile_n = 0;                      // grouped-M, K-major B, plain and SwiGLU forward results, one SM per tile: rows of B
+                                       // in a tile, 256 (0), 128 or 64
   long long rows_per_group = 0;        // grouped-M: expected rows of a group (chooses the order of the tiles only)
   const int* group_order = nullptr;    // grouped-K, optional: the groups from most to fewest rows, device memory
   int max_m_tiles = 0;                 // grouped-M: upper bound on *num_m_tiles (sizes the grid)

@@ -616,7 +616,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 }  // namespace
 
 bool gemm_2cta_supported(const GemmArgs& a) {
-  if (a.scatter_row_slot != nullptr || a.pull_row_slot != nullptr || a.ready_flags != nullptr || a.tile_rows != nullptr)
+  if (a.scatter_row_slot != nullptr || a.pull_row_slot != nullptr || a.ready_flags != nullptr || a.tile_rows != nullptr ||
+      a.tile_n != 0)
     return false;
   if (a.N % 8 != 0 || a.N <= 0) return false;
   const auto aligned = [](const void* ptr, long long ld, long long es) {
