@@ -191,7 +191,7 @@ struct MoEFn : Function<MoEFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto s = ctx->get_saved_variables();
     auto [dx, d_gate, dw13, dw2] = cmoe::moe_local_backward(
-        cmoe::contiguous_aligned(g[0]), s[0], s[1], s[2], s[3], opt(s[4]), s[5], s[6], s[7], ctx->needs_input_grad(0),
+        cmoe::contiguous_aligned(g[0]), s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], ctx->needs_input_grad(0),
         ctx->needs_input_grad(1), main_grad(s[6]), main_grad(s[7]), ctx->saved_data["status"].toTensor());
     return {or_none(dx), or_none(d_gate), or_none(dw13), or_none(dw2), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }

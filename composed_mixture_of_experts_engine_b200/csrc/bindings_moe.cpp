@@ -221,21 +221,7 @@ void place_rows(const Tensor& src, const Tensor& out, int64_t K, const PlanTable
   check(cmoe::launch_place_rows(a, stream), "place_rows");
 }
 
-// With several picks per token and a backward pass to come, the gate weight enters with the SwiGLU product,
-// h = weight * silu(gate) * up: the result rows only have to be added up, the backward reads dy's rows as they are, and
-// the gradient of the weight falls out of the SwiGLU backward, next to the values that it needs.  A weight on the result
-// rows instead needs those rows again in the backward: 16384 tokens top-8, H 2048, F 1024 read 600 MB for it and scale
-// 540 MB of dy's rows on their way (layer, forward and backward, 5077 -> 4874 us, with the rows placed token by token).
-// One pick: a normalised weight is 1 and its gradient cancels to rounding noise in the router, which is left as it always
-// was.  Without a backward pass nothing is read again, so the weight stays on the result rows: the picks of the layers
-// behind, which near-ties make depend on single roundings, stay what they were.
-bool weight_in_ffn(int64_t K, bool keep) { return keep && K > 1; }
-void set_weights(cmoe::GemmArgs& g, const Tensor& gate_w32, const PlanTables& pt, const int* plan) {
-  g.weight_row_slot = plan + pt.row_slot;
-  g.slot_weight = gate_w32.data_ptr<float>();
-}
-
-// (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads), yp only with one pick per token
+// (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads)
 Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor& idx32, const Tensor& w13,
                           const Tensor& w2, int64_t capacity, bool keep, const OptTensor& status,
                           const OptTensor& overflow, const OptTensor& made_plan) {
@@ -253,7 +239,6 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   // GEMMs load and store only the 32-row pieces that hold any: at 64 tokens, E 64 top-8 (8 rows per expert), H 2048,
   // F 1024 the padding was 33 MB to fill, 400 MB to load from L2 and 50 MB to store, next to 805 MB of weights.  From 64
   // rows per expert on, most pieces are live and whole tiles take fewer loads.
-  const bool weighted = weight_in_ffn(s.K, keep);
   const bool short_tiles = !keep && pt.n_slots <= 64 * s.E;
   Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
   place_rows(x, xp, s.K, pt, plan, keep, stream);
@@ -263,7 +248,6 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
     cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status), cmoe::EPI_SWIGLU_FWD,
                                      short_tiles);
     g.split_n = static_cast<int>(s.F);
-    if (weighted) set_weights(g, gate_w32, pt, plan);
     if (keep) {
       gu = at::empty({pt.cap_rows, 2 * s.F}, bf);
       g.aux_out = gu->data_ptr();
@@ -276,11 +260,11 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
                                       cmoe::EPI_STORE, short_tiles),
                          stream);
   Tensor y = at::empty({s.N, s.H}, bf);
-  check(cmoe::launch_combine_rows(yp.data_ptr(), plan, weighted ? nullptr : gate_w32.data_ptr<float>(),
-                                  y.data_ptr(), s.N, static_cast<int>(s.K), static_cast<int>(s.H), s.H, s.H, stream),
+  check(cmoe::launch_combine_rows(yp.data_ptr(), plan, gate_w32.data_ptr<float>(), y.data_ptr(), s.N,
+                                  static_cast<int>(s.K), static_cast<int>(s.H), s.H, s.H, stream),
         "combine_rows");
   if (!keep) return {y, plan_t, std::nullopt, std::nullopt, std::nullopt, std::nullopt};
-  return {y, plan_t, xp, hact, gu, weighted ? OptTensor() : OptTensor(yp)};
+  return {y, plan_t, xp, hact, gu, yp};
 }
 
 // dW[e] = a[rows of e]^T b[rows of e]: added into the fp32 `main` buffer when there is one (returns nothing), else
@@ -329,7 +313,7 @@ OptTensor expert_wgrad(const Tensor& a, const Tensor& b, const Tensor& weight, c
 
 // (dx, d_gate, dw13, dw2)
 Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor& xp, const Tensor& hact, const Tensor& gu,
-                            const OptTensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2, bool need_dx,
+                            const Tensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2, bool need_dx,
                             bool need_gate, const OptTensor& main13, const OptTensor& main2, const OptTensor& status) {
   const c10::cuda::CUDAGuard guard(dy.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
@@ -337,49 +321,29 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
   TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && dy.size(0) == N && dy.size(1) == H, "bad dy");
   check_rows(dy, "dy");
   check_rows(xp, "saved rows");
-  const bool weighted = weight_in_ffn(K, true);
-  TORCH_CHECK(weighted || yp.has_value(), "the saved expert rows are missing");
-  if (!weighted) check_rows(*yp, "saved expert rows");
+  check_rows(yp, "saved expert rows");
   const PlanTables pt(N * K, E);
   TORCH_CHECK(plan_t.numel() == pt.words && xp.size(0) == pt.cap_rows, "the row plan belongs to another layer call");
   int* plan = plan_t.data_ptr<int>();
   int* st = status_ptr(status);
   Backward out;
-  if (need_gate && !weighted) {
+  if (need_gate) {
     Tensor d_gate = at::empty({N, K}, gate_w32.options());
-    check(cmoe::launch_combine_bwd_w(yp->data_ptr(), plan, dy.data_ptr(), d_gate.data_ptr<float>(), N,
+    check(cmoe::launch_combine_bwd_w(yp.data_ptr(), plan, dy.data_ptr(), d_gate.data_ptr<float>(), N,
                                      static_cast<int>(K), static_cast<int>(H), H, H, stream),
           "combine_bwd_w");
     std::get<1>(out) = d_gate;
   }
   Tensor dyp = at::empty({pt.cap_rows, H}, dy.options());
-  if (weighted)
-    place_rows(dy, dyp, K, pt, plan, true, stream);
-  else
-    check(cmoe::launch_gather_rows(dy.data_ptr(), plan + pt.row_slot, static_cast<int>(K), gate_w32.data_ptr<float>(),
-                                   dyp.data_ptr(), pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(H), H, H, stream),
-          "gather_rows");
+  check(cmoe::launch_gather_rows(dy.data_ptr(), plan + pt.row_slot, static_cast<int>(K), gate_w32.data_ptr<float>(),
+                                 dyp.data_ptr(), pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(H), H, H, stream),
+        "gather_rows");
   Tensor dgu = at::empty({pt.cap_rows, 2 * F}, dy.options());
   {
     cmoe::GemmArgs g = grouped_rows(dyp, w2, H, true, dgu, F, H, pt, plan, st, cmoe::EPI_SWIGLU_BWD);
     g.aux_in = gu.data_ptr();
     g.ld_aux_in = gu.stride(0);
-    const int64_t parts = 2 * ((F + 255) / 256);
-    Tensor row_dot;
-    if (weighted) {
-      set_weights(g, gate_w32, pt, plan);
-      row_dot = at::empty({parts, pt.cap_rows}, gate_w32.options());
-      g.row_dot = row_dot.data_ptr<float>();
-      g.row_dot_stride = pt.cap_rows;
-    }
     cmoe::launch_gemm_any(g, stream);
-    if (need_gate && weighted) {
-      Tensor d_gate = at::empty({N, K}, gate_w32.options());
-      check(cmoe::launch_gate_grad(g.row_dot, pt.cap_rows, static_cast<int>(parts), plan, d_gate.data_ptr<float>(), N * K,
-                                   stream),
-            "gate_grad");
-      std::get<1>(out) = d_gate;
-    }
   }
   if (need_dx) {
     Tensor dxp = at::empty({pt.cap_rows, H}, dy.options());
@@ -404,7 +368,7 @@ MoeForward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tens
   return ::moe_local_forward(x, gate_w32, idx32, w13, w2, capacity, keep, status, overflow, made_plan);
 }
 MoeBackward moe_local_backward(const Tensor& dy, const Tensor& plan, const Tensor& xp, const Tensor& hact, const Tensor& gu,
-                               const OptTensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2,
+                               const Tensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2,
                                bool need_dx, bool need_gate, const OptTensor& main13, const OptTensor& main2,
                                const OptTensor& status) {
   return ::moe_local_backward(dy, plan, xp, hact, gu, yp, gate_w32, w13, w2, need_dx, need_gate, main13, main2, status);

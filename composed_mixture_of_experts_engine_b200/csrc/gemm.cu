@@ -80,10 +80,6 @@ struct KParams {
   const uint32_t* ready_flags;
   int ready_stride, ready_count;
   uint32_t ready_target;
-  const int* weight_row_slot;  // SwiGLU: weights of the rows
-  const float* slot_weight;
-  float* row_dot;
-  long long row_dot_stride;
   int* status;
   unsigned long long timeout_ns;
   int bn;               // accumulator columns of a tile (rows of B): 256, or 128 / 64 where that fills the SMs better
@@ -249,17 +245,9 @@ __device__ __forceinline__ void prefetch_f32_chunk(const float* row_ptr, int col
 
 // ... and its results stored from registers: dGate at D[row, col..], dUp at D[row, N + col..]; columns past N hold
 // garbage and are not stored.
-__device__ __forceinline__ void swiglu_bwd_any(const KParams& p, const uint32_t (&r)[32], uint4 (&cg)[4], uint4 (&cu)[4],
-                                               int col, float weight, float& dot) {
-  if (p.row_dot != nullptr)
-    swiglu_bwd_math<true>(r, cg, cu, weight, (p.N - col) / 8, dot);
-  else
-    swiglu_bwd_math<false>(r, cg, cu, weight, 0, dot);
-}
-__device__ __forceinline__ void swiglu_bwd_chunk(const KParams& p, const uint32_t (&r)[32], uint4 (&cg)[4], uint4 (&cu)[4],
-                                                 int col, int N, void* Dg, long long ldd, long long row, float weight,
-                                                 float& dot) {
-  swiglu_bwd_any(p, r, cg, cu, col, weight, dot);
+__device__ __forceinline__ void swiglu_bwd_chunk(const uint32_t (&r)[32], uint4 (&cg)[4], uint4 (&cu)[4], int col,
+                                                 int N, void* Dg, long long ldd, long long row) {
+  swiglu_bwd_math(r, cg, cu);
   __nv_bfloat16* dgp = reinterpret_cast<__nv_bfloat16*>(Dg) + row * ldd + col;
   __nv_bfloat16* dup = dgp + N;
 #pragma unroll
@@ -606,15 +594,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (p.bwd_staged) bulk_wait_group_read<1>();
         gu_issue(stage_ctr, ti.n0);
       }
-      const float weight = EPI != EPI_STORE && row_ok ? row_weight(p.weight_row_slot, p.slot_weight, row) : 1.f;
-      float dot = 0.f;
-      // one group of epilogue warps: the second part of a tile is empty
-      auto dot_done = [&]() {
-        if (EPI != EPI_SWIGLU_BWD || p.row_dot == nullptr || !row_ok) return;
-        float* part = p.row_dot + 2 * (ti.n0 / BN) * p.row_dot_stride + row;
-        part[0] = dot;
-        part[p.row_dot_stride] = 0.f;
-      };
       const bool ok = mbar_wait(&tfull_bar[acc], acc_phase, wc, ST_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       const uint32_t t_acc = tmem_base + acc * BN + lane_base;
@@ -757,7 +736,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             for (int j = 0; j < 16; ++j) {
               const float g0 = __uint_as_float(rg[2 * j]), g1 = __uint_as_float(rg[2 * j + 1]);
               const float u0 = __uint_as_float(ru[2 * j]), u1 = __uint_as_float(ru[2 * j + 1]);
-              ph[j] = pack_bf16x2(weight * (g0 * sigmoidf_fast(g0) * u0), weight * (g1 * sigmoidf_fast(g1) * u1));
+              ph[j] = pack_bf16x2(g0 * sigmoidf_fast(g0) * u0, g1 * sigmoidf_fast(g1) * u1);
               pg[j] = pack_bf16x2(g0, g1);
               pu[j] = pack_bf16x2(u0, u1);
             }
@@ -872,7 +851,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               for (int j = 0; j < 32; ++j) {
                 g[j] = __uint_as_float(rg[j]);
                 u[j] = __uint_as_float(ru[j]);
-                h[j] = weight * (g[j] * sigmoidf_fast(g[j]) * u[j]);
+                h[j] = g[j] * sigmoidf_fast(g[j]) * u[j];
               }
               const int col = ti.n0 + c * 32;
               store_row_chunk(Dg, p.ldd, 0, 0, row, col, p.N, h);
@@ -914,7 +893,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             cu[j] = *reinterpret_cast<const uint4*>(grow + STAGING_BUF_BYTES / 2 + ((j ^ gsw) << 4));
           }
           if (ok && got) {
-            swiglu_bwd_any(p, r, cg, cu, col, weight, dot);
+            swiglu_bwd_math(r, cg, cu);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               *reinterpret_cast<uint4*>(grow + ((j ^ gsw) << 4)) = cg[j];
@@ -941,7 +920,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           ++stage_ctr;
         }
-        dot_done();
         tc_fence_before();
         mbar_arrive(&tempty_bar[acc]);
         acc ^= 1;
@@ -973,10 +951,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             cu[j] = *reinterpret_cast<const uint4*>(grow + STAGING_BUF_BYTES / 2 + ((j ^ gsw) << 4));
           }
           mbar_arrive(&gempty_bar[b]);
-          if (ok && got && row_ok) swiglu_bwd_chunk(p, r, cg, cu, col, p.N, Dg, p.ldd, row, weight, dot);
+          if (ok && got && row_ok) swiglu_bwd_chunk(r, cg, cu, col, p.N, Dg, p.ldd, row);
           ++stage_ctr;
         }
-        dot_done();
       }
       tc_fence_before();
       mbar_arrive(&tempty_bar[acc]);
@@ -1156,10 +1133,6 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.ready_stride = a.ready_stride;
   kp.ready_count = a.ready_count;
   kp.ready_target = a.ready_target;
-  kp.weight_row_slot = a.weight_row_slot;
-  kp.slot_weight = a.slot_weight;
-  kp.row_dot = a.row_dot;
-  kp.row_dot_stride = a.row_dot_stride;
   kp.status = a.status;
   kp.chained = gemm_overlaps_neighbours(a);
   kp.b_once = a.b_once;

@@ -74,15 +74,6 @@ struct GemmArgs {
   void* aux_out = nullptr;  // SWIGLU_FWD: optional [rows, 2N] gate|up
   long long ld_aux_out = 0;
 
-  // SwiGLU epilogues of grouped-M, optional: row r carries the weight slot_weight[weight_row_slot[r]] (padding, with a
-  // negative slot, 0).  Forward: D = weight * silu(gate) * up, aux_out unchanged.  Backward: acc is the gradient of that
-  // D, and row_dot[part * row_dot_stride + r], part < 2 * ceil(N / 256), are the row's partial sums of the gradient of its
-  // weight (whole tiles of rows are written, padding too).
-  const int* weight_row_slot = nullptr;
-  const float* slot_weight = nullptr;
-  float* row_dot = nullptr;
-  long long row_dot_stride = 0;
-
   // Dense bf16 results on pairs of SMs, optional: row_stats[row * ceil(N / 256) + c] = (max, sum of exp(v - max)) over the
   // values v of columns [256 c, 256 c + 256) of the row, as they are stored (a softmax over the row then needs one pass)
   float2* row_stats = nullptr;

@@ -76,10 +76,6 @@ struct K2Params {
   int has_aux;        // SwiGLU forward: gate|up is stored too
   int d_fp32, reduce;  // reduce: TMA reduce-add (fp32 accumulate) instead of store
   float2* row_stats;           // dense: softmax statistics of the rows
-  const int* weight_row_slot;  // SwiGLU: weights of the rows
-  const float* slot_weight;
-  float* row_dot;
-  long long row_dot_stride;
   int* status;
   unsigned long long timeout_ns;
 };
@@ -424,8 +420,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         bulk_wait_group_read<1>();  // this piece's buffer was last read by the store issued two pieces ago
         gu_issue(stage_ctr, ti.n0 + grp * 32);
       }
-      const float weight = EPI != EPI_STORE && mine ? row_weight(p.weight_row_slot, p.slot_weight, row0 + row_in_tile) : 1.f;
-      float dot = 0.f;
       float stat_max = -INFINITY, stat_sum = 0.f;
       bool ok = true;
       if (have_acc) {
@@ -459,10 +453,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
               cu[j] = *reinterpret_cast<const uint4*>(grow + T_STAGING_BUF / 2 + ((j ^ gsw) << 4));
             }
             tmem_ld_wait();
-            if (p.row_dot != nullptr)
-              swiglu_bwd_math<true>(r, cg, cu, weight, (p.N - col0) / 8, dot);
-            else
-              swiglu_bwd_math<false>(r, cg, cu, weight, 0, dot);
+            swiglu_bwd_math(r, cg, cu);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               *reinterpret_cast<uint4*>(grow + ((j ^ gsw) << 4)) = cg[j];
@@ -495,7 +486,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             for (int j = 0; j < 16; ++j) {
               const float g0 = __uint_as_float(rg[2 * j]), g1 = __uint_as_float(rg[2 * j + 1]);
               const float u0 = __uint_as_float(ru[2 * j]), u1 = __uint_as_float(ru[2 * j + 1]);
-              ph[j] = pack_bf16x2(weight * (g0 * sigmoidf_fast(g0) * u0), weight * (g1 * sigmoidf_fast(g1) * u1));
+              ph[j] = pack_bf16x2(g0 * sigmoidf_fast(g0) * u0, g1 * sigmoidf_fast(g1) * u1);
               pg[j] = pack_bf16x2(g0, g1);
               pu[j] = pack_bf16x2(u0, u1);
             }
@@ -586,8 +577,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       }
       if (EPI == EPI_STORE && p.row_stats != nullptr && row0 + row_in_tile < p.M)
         p.row_stats[static_cast<long long>(row0 + row_in_tile) * n_tiles + ti.n0 / T_BN] = make_float2(stat_max, stat_sum);
-      if (EPI == EPI_SWIGLU_BWD && p.row_dot != nullptr && mine)
-        p.row_dot[(2 * (ti.n0 / T_BN) + grp) * p.row_dot_stride + row0 + row_in_tile] = dot;
       if (have_acc) {
         // the leader's MMA warp may reuse this accumulator once all epilogue threads of the pair have read it
         tc_fence_before();
@@ -710,10 +699,6 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   kp.d_fp32 = a.d_fp32;
   kp.reduce = a.accumulate;
   kp.row_stats = a.row_stats;
-  kp.weight_row_slot = a.weight_row_slot;
-  kp.slot_weight = a.slot_weight;
-  kp.row_dot = a.row_dot;
-  kp.row_dot_stride = a.row_dot_stride;
   kp.status = a.status;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
 

@@ -27,7 +27,7 @@ MoeForward moe_local_forward(const torch::Tensor& x, const torch::Tensor& gate_w
                              const OptTensor& status, const OptTensor& overflow, const OptTensor& made_plan);
 using MoeBackward = std::tuple<OptTensor, OptTensor, OptTensor, OptTensor>;
 MoeBackward moe_local_backward(const torch::Tensor& dy, const torch::Tensor& plan, const torch::Tensor& xp,
-                               const torch::Tensor& hact, const torch::Tensor& gu, const OptTensor& yp,
+                               const torch::Tensor& hact, const torch::Tensor& gu, const torch::Tensor& yp,
                                const torch::Tensor& gate_w32, const torch::Tensor& w13, const torch::Tensor& w2,
                                bool need_dx, bool need_gate, const OptTensor& main13, const OptTensor& main2,
                                const OptTensor& status);

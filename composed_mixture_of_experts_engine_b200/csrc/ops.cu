@@ -1076,23 +1076,6 @@ __global__ void combine_bwd_w_kernel(const __nv_bfloat16* rows, const int* slot_
   }
 }
 
-// d(gate weight) of every slot: its row's partial sums (GemmArgs::row_dot), added in their order; 0 for dropped slots.
-// That is 4 bytes to read per slot and 128 columns of the FFN width, against 2 bytes per column of the result row for a dot
-// product with it: 6 us at 16384 tokens top-8, H 2048, F 1024, where the dot products read 600 MB (92 us at the copy rate).
-__global__ void __launch_bounds__(256) gate_grad_kernel(const float* row_dot, long long stride, int parts,
-                                                        const int* slot_row, float* dw, long long n_slots) {
-  chain_wait();
-  chain_trigger();
-  for (long long s = blockIdx.x * 256LL + threadIdx.x; s < n_slots; s += gridDim.x * 256LL) {
-    const int row = slot_row[s];
-    float acc = 0.f;
-    if (row >= 0)
-#pragma unroll 8
-      for (int i = 0; i < parts; ++i) acc += row_dot[i * stride + row];
-    dw[s] = acc;
-  }
-}
-
 inline unsigned grid_for(long long work_items, int per_block, int max_blocks) {
   long long b = (work_items + per_block - 1) / per_block;
   if (b < 1) b = 1;
@@ -1339,14 +1322,6 @@ cudaError_t launch_combine_bwd_w(const void* rows, const int* slot_row, const vo
   launch_chained(combine_bwd_w_kernel, grid_for(n_tokens * K, 8, 148 * 8), 256, 0, stream,
                  reinterpret_cast<const __nv_bfloat16*>(rows), slot_row, reinterpret_cast<const __nv_bfloat16*>(dy),
                  dw, n_tokens, K, H, ld_rows, ld_dy);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gate_grad(const float* row_dot, long long stride, int parts, const int* slot_row, float* dw,
-                             long long n_slots, cudaStream_t stream) {
-  if (n_slots <= 0) return cudaErrorInvalidValue;
-  launch_chained(gate_grad_kernel, grid_for(n_slots, 256, 148 * 8), 256, 0, stream, row_dot, stride, parts, slot_row, dw,
-                 n_slots);
   return cudaGetLastError();
 }
 

@@ -152,9 +152,6 @@ cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream);
 // y[t, :] = sum_k w[t,k] * rows[slot_row[t*K+k], :]  (slots with row -1 skipped), fp32 accumulate, bf16 out
 cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const float* w, void* y, long long n_tokens,
                                 int K, int H, long long ld_rows, long long ld_y, cudaStream_t stream);
-// dw[s] = sum over parts of row_dot[part * stride + slot_row[s]], 0 where slot_row[s] is negative
-cudaError_t launch_gate_grad(const float* row_dot, long long stride, int parts, const int* slot_row, float* dw,
-                             long long n_slots, cudaStream_t stream);
 // dw[t,k] = <dy[t,:], rows[slot_row[t*K+k], :]>
 cudaError_t launch_combine_bwd_w(const void* rows, const int* slot_row, const void* dy, float* dw, long long n_tokens,
                                  int K, int H, long long ld_rows, long long ld_dy, cudaStream_t stream);
