@@ -512,6 +512,33 @@ void place_rows(const Tensor& src, const Tensor& slot_row, int64_t K, const Tens
   a.n_local = static_cast<int>(counts_kept.numel());
   check_cuda(cmoe::launch_place_rows(a, cur_stream()), "place_rows");
 }
+void combine_grad(const Tensor& dy, const Tensor& slot_row, int64_t K, const Tensor& group_offsets, const Tensor& counts_kept,
+                  const Tensor& weight, const Tensor& rows, Tensor& out, const std::optional<Tensor>& dw) {
+  const c10::cuda::CUDAGuard guard(dy.device());
+  check_rows(dy, "dy");
+  check_rows(rows, "rows");
+  check_rows(out, "out");
+  TORCH_CHECK(slot_row.numel() == dy.size(0) * K && weight.numel() == slot_row.numel() && out.size(1) == dy.size(1) &&
+                  rows.size(1) == dy.size(1) && group_offsets.numel() == counts_kept.numel() + 1 &&
+                  weight.scalar_type() == at::kFloat && weight.is_contiguous() &&
+                  (!dw.has_value() || (dw->numel() == weight.numel() && dw->scalar_type() == at::kFloat && dw->is_contiguous())),
+              "combine_grad: sizes do not match");
+  cmoe::PlaceRowsArgs a;
+  a.src = dy.data_ptr();
+  a.n_tokens = dy.size(0);
+  a.ld_src = dy.stride(0);
+  a.slot_row = slot_row.data_ptr<int>();
+  a.K = static_cast<int>(K);
+  a.H = static_cast<int>(dy.size(1));
+  a.out = out.data_ptr();
+  a.ld_out = out.stride(0);
+  a.group_offsets = group_offsets.data_ptr<int>();
+  a.counts_kept = counts_kept.data_ptr<int>();
+  a.n_local = static_cast<int>(counts_kept.numel());
+  check_cuda(cmoe::launch_combine_grad(a, weight.data_ptr<float>(), rows.data_ptr(), rows.stride(0),
+                                       dw.has_value() ? dw->data_ptr<float>() : nullptr, cur_stream()),
+             "combine_grad");
+}
 void combine_rows(const Tensor& rows, const Tensor& slot_row, const OptTensor& w, Tensor& y, int64_t K) {
   const c10::cuda::CUDAGuard guard(rows.device());
   check_rows(rows, "rows");
@@ -584,6 +611,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_plan", &moe_plan);
   m.def("gather_rows", &gather_rows);
   m.def("place_rows", &place_rows);
+  m.def("combine_grad", &combine_grad);
   m.def("combine_rows", &combine_rows);
   m.def("combine_bwd_w", &combine_bwd_w);
   register_attention(m);

@@ -202,9 +202,9 @@ std::map<std::string, Tensor> moe_local_tables(const Tensor& plan, int64_t n_slo
           {"counts_kept", part(pt.counts_kept, E)}};
 }
 
-// the rows of `src` (tokens) at their places in expert order
-void place_rows(const Tensor& src, const Tensor& out, int64_t K, const PlanTables& pt, const int* plan, bool zero_padding,
-                cudaStream_t stream) {
+// the rows of `src` (tokens) and their places in expert order
+cmoe::PlaceRowsArgs places(const Tensor& src, const Tensor& out, int64_t K, const PlanTables& pt, const int* plan,
+                           bool zero_padding) {
   cmoe::PlaceRowsArgs a;
   a.src = src.data_ptr();
   a.n_tokens = src.size(0);
@@ -218,7 +218,7 @@ void place_rows(const Tensor& src, const Tensor& out, int64_t K, const PlanTable
   a.group_offsets = plan + pt.group_offsets;
   a.counts_kept = plan + pt.counts_kept;
   a.n_local = static_cast<int>(pt.E);
-  check(cmoe::launch_place_rows(a, stream), "place_rows");
+  return a;
 }
 
 // (y, plan, xp, hact, gu, yp); the last four only with `keep` (what the backward reads)
@@ -241,7 +241,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   // rows per expert on, most pieces are live and whole tiles take fewer loads.
   const bool short_tiles = !keep && pt.n_slots <= 64 * s.E;
   Tensor xp = at::empty({pt.cap_rows, s.H}, bf);
-  place_rows(x, xp, s.K, pt, plan, keep, stream);
+  check(cmoe::launch_place_rows(places(x, xp, s.K, pt, plan, keep), stream), "place_rows");
   Tensor hact = at::empty({pt.cap_rows, s.F}, bf);
   OptTensor gu;
   {
@@ -327,17 +327,22 @@ Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor
   int* plan = plan_t.data_ptr<int>();
   int* st = status_ptr(status);
   Backward out;
-  if (need_gate) {
-    Tensor d_gate = at::empty({N, K}, gate_w32.options());
-    check(cmoe::launch_combine_bwd_w(yp.data_ptr(), plan, dy.data_ptr(), d_gate.data_ptr<float>(), N,
-                                     static_cast<int>(K), static_cast<int>(H), H, H, stream),
-          "combine_bwd_w");
-    std::get<1>(out) = d_gate;
+  Tensor dyp = at::empty({pt.cap_rows, H}, dy.options()), d_gate;
+  if (need_gate) d_gate = at::empty({N, K}, gate_w32.options());
+  float* dw = need_gate ? d_gate.data_ptr<float>() : nullptr;
+  if (cmoe::combine_grad_supported(static_cast<int>(H))) {
+    check(cmoe::launch_combine_grad(places(dy, dyp, K, pt, plan, true), gate_w32.data_ptr<float>(), yp.data_ptr(), H, dw, stream),
+          "combine_grad");
+  } else {  // rows that do not fit a warp's registers
+    if (need_gate)
+      check(cmoe::launch_combine_bwd_w(yp.data_ptr(), plan, dy.data_ptr(), dw, N, static_cast<int>(K), static_cast<int>(H), H,
+                                       H, stream),
+            "combine_bwd_w");
+    check(cmoe::launch_gather_rows(dy.data_ptr(), plan + pt.row_slot, static_cast<int>(K), gate_w32.data_ptr<float>(),
+                                   dyp.data_ptr(), pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(H), H, H, stream),
+          "gather_rows");
   }
-  Tensor dyp = at::empty({pt.cap_rows, H}, dy.options());
-  check(cmoe::launch_gather_rows(dy.data_ptr(), plan + pt.row_slot, static_cast<int>(K), gate_w32.data_ptr<float>(),
-                                 dyp.data_ptr(), pt.cap_rows, plan + pt.num_m_tiles, static_cast<int>(H), H, H, stream),
-        "gather_rows");
+  if (need_gate) std::get<1>(out) = d_gate;
   Tensor dgu = at::empty({pt.cap_rows, 2 * F}, dy.options());
   {
     cmoe::GemmArgs g = grouped_rows(dyp, w2, H, true, dgu, F, H, pt, plan, st, cmoe::EPI_SWIGLU_BWD);

@@ -1076,6 +1076,72 @@ __global__ void combine_bwd_w_kernel(const __nv_bfloat16* rows, const int* slot_
   }
 }
 
+// Backward of the weighted combine, token by token: a warp holds the token's row of dy, multiplies it by each pick's weight
+// into the expert's row, and takes its product with that pick's result row, which is the gradient of the weight.  What
+// bounds it: reading the result rows and writing as many.  In two launches (combine_bwd_w, then gather_rows with a scale) dy
+// was read K times for each, in between the stores that drive it out of L2.  The values and the order of every sum are
+// theirs.  Both / this, behind GEMMs: 16384 tokens x 2048, top-8 of 64 286 / 192 us (1.2 GB: 175 at the copy rate);
+// 3333 x 4096, top-8 of 32 120 / 93; 8192 x 4096, top-2 of 8 85 / 75; 4096 x 1024, top-2 of 16 21.5 / 17.4; 16384 x 512,
+// top-1 of 16 23.6 / 17.4.  Q: 16-byte pieces of dy per lane, H <= 256 Q; wider rows keep the two launches.
+template <int Q>
+__global__ void __launch_bounds__(256) combine_grad_kernel(const PlaceRowsArgs a, const float* weight,
+                                                           const __nv_bfloat16* rows, long long ld_rows, float* dw) {
+  chain_wait();
+  chain_trigger();
+  const __nv_bfloat16* dy = static_cast<const __nv_bfloat16*>(a.src);
+  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
+  const int lane = threadIdx.x & 31;
+  const long long warp = (blockIdx.x * 256LL + threadIdx.x) >> 5;
+  if (warp < a.n_tokens) {
+    uint4 d[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (lane * 8 + q * 256 < a.H) d[q] = *reinterpret_cast<const uint4*>(dy + warp * a.ld_src + lane * 8 + q * 256);
+    for (int k = 0; k < a.K; ++k) {
+      const long long slot = warp * a.K + k;
+      const int row = a.slot_row[slot];
+      float acc = 0.f;
+      if (row >= 0) {
+        uint4 y[Q];
+        if (dw != nullptr) {
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if (lane * 8 + q * 256 < a.H)
+              y[q] = *reinterpret_cast<const uint4*>(rows + row * ld_rows + lane * 8 + q * 256);
+        }
+        const float w = weight[slot];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          if (lane * 8 + q * 256 >= a.H) continue;
+          float f[8], s[8];
+          unpack8(d[q], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s[j] = f[j] * w;
+          store8(out + row * a.ld_out + lane * 8 + q * 256, s);
+          if (dw != nullptr) {
+            float g[8];
+            unpack8(y[q], g);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc += g[j] * f[j];
+          }
+        }
+      }
+      if (dw != nullptr) {
+        acc = warp_sum(acc);
+        if (lane == 0) dw[slot] = acc;  // 0 for a dropped slot
+      }
+    }
+    return;
+  }
+  // the warps behind the tokens': an expert's rows are followed by up to 127 rows of padding
+  const long long i = warp - a.n_tokens;
+  if (i >= a.n_local * 128LL) return;
+  const int e = static_cast<int>(i >> 7);
+  const long long row = static_cast<long long>(a.group_offsets[e]) + a.counts_kept[e] + (i & 127);
+  if (row < a.group_offsets[e + 1])
+    for (int c = lane * 8; c < a.H; c += 256) *reinterpret_cast<uint4*>(out + row * a.ld_out + c) = make_uint4(0u, 0u, 0u, 0u);
+}
+
 inline unsigned grid_for(long long work_items, int per_block, int max_blocks) {
   long long b = (work_items + per_block - 1) / per_block;
   if (b < 1) b = 1;
@@ -1282,6 +1348,19 @@ cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream) {
   // a warp per piece: CTAs that stride over the tokens drift apart (16384 x 2048, top-8: 130 / 120 us)
   launch_chained(place_rows_kernel, grid_for(warps, 8, 1 << 24), 256, 0, stream, a, pieces);
   return cudaGetLastError();
+}
+
+bool combine_grad_supported(int H) { return H <= 4096; }
+cudaError_t launch_combine_grad(const PlaceRowsArgs& a, const float* weight, const void* rows, long long ld_rows, float* dw,
+                                cudaStream_t stream) {
+  if (a.H % 8 != 0 || a.H <= 0 || !combine_grad_supported(a.H) || a.K <= 0 || a.n_tokens <= 0) return cudaErrorInvalidValue;
+  const unsigned grid = grid_for(a.n_tokens + a.n_local * 128LL, 8, INT_MAX);
+  const int q = (a.H + 255) / 256;
+  auto go = [&](auto kernel) {
+    return launch_chained(kernel, grid, 256, 0, stream, a, weight, reinterpret_cast<const __nv_bfloat16*>(rows), ld_rows, dw);
+  };
+  return q <= 2 ? go(combine_grad_kernel<2>) : q <= 4 ? go(combine_grad_kernel<4>)
+       : q <= 8 ? go(combine_grad_kernel<8>) : go(combine_grad_kernel<16>);
 }
 
 cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const float* w, void* y, long long n_tokens,

@@ -149,6 +149,11 @@ struct PlaceRowsArgs {
   int n_local = 0;
 };
 cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream);
+// The backward of the weighted combine in one pass, H <= 4096: out[slot_row[t*K+k], :] = weight[t,k] * src[t, :] with zeros
+// in the padding, and dw[t,k] = <src[t, :], rows[slot_row[t*K+k], :]> (0 for dropped slots; nullptr: not wanted).
+bool combine_grad_supported(int H);
+cudaError_t launch_combine_grad(const PlaceRowsArgs& a, const float* weight, const void* rows, long long ld_rows, float* dw,
+                                cudaStream_t stream);
 // y[t, :] = sum_k w[t,k] * rows[slot_row[t*K+k], :]  (slots with row -1 skipped), fp32 accumulate, bf16 out
 cudaError_t launch_combine_rows(const void* rows, const int* slot_row, const float* w, void* y, long long n_tokens,
                                 int K, int H, long long ld_rows, long long ld_y, cudaStream_t stream);
