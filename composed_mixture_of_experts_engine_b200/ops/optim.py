@@ -6,8 +6,8 @@ fp32 reduction).  Here the same mixed-precision contract (bf16 parameters in the
 moments in the optimizer) is one kernel launch per parameter group:
 
 * parameters are re-pointed into one flat bf16 buffer per group, gradients into one flat buffer
-  (fp32 ``main_grad``: the kernels add the weight gradients of experts, projections, LM head and token embedding into
-  it directly; what autograd leaves in ``p.grad`` - norm weights, router gates - is added at step time);
+  (fp32 ``main_grad``: the kernels add the weight gradients of experts, projections, norms, LM head and token embedding
+  into it directly; what autograd leaves in ``p.grad`` - router gates - is added at step time);
 * the global gradient norm is a device scalar (sum-of-squares kernel), so clipping needs no host round trip;
 * with data parallelism the flat gradient is reduce-scattered, the update runs on this rank's shard only, and
   the updated bf16 parameters are all-gathered (ZeRO-style sharding of master weights and moments).  Expert
@@ -307,7 +307,7 @@ def build_optimizer(model: nn.Module, lr: float, weight_decay: float = 0.1, beta
     dense.sort(key=lambda np_: 0 if getattr(np_[1], "sequence_parallel_grad", False) else 1)
     if dense:
         # fp32 gradient buffer: the weight-gradient GEMMs of the projections and of the LM head add into it with
-        # TMA reduce-add across microbatches; vector parameters' autograd gradients are added at step time
+        # TMA reduce-add across microbatches, the norms' kernels too; what autograd holds is added at step time
         groups.append(_FlatGroup("dense", [p for _, p in dense], torch.float32,
                                  [not _no_decay(n, p) for n, p in dense], shard_group=dp_group, topology=topology,
                                  axis="ddp", param_names=[n for n, _ in dense]))
