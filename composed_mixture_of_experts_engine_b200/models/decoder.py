@@ -65,8 +65,15 @@ class CausalSelfAttention(nn.Module):
         return self.wo(o.reshape(B, S, self.nh * self.hd))
 
 
-def _hooked(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+_NORM_FORWARD = RMSNorm.forward
+
+
+def _unwatched(m: nn.Module, cls: type, forward) -> bool:
+    """Whether calling ``m`` runs ``forward`` of ``cls`` and nothing else: no hooks, no other module, method, compiled call
+    or patched ``Module.__call__`` in its place."""
+    return (type(m) is cls and cls.forward is forward and "forward" not in m.__dict__ and m._compiled_call_impl is None
+            and cls.__call__ is nn.Module._wrapped_call_impl and not _has_any_global_hook()
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
 
 
 class DecoderBlock(nn.Module):
@@ -92,11 +99,10 @@ class DecoderBlock(nn.Module):
                 self.moe.router.gate_w.sequence_parallel_grad = True
 
     def joins_residuals(self) -> bool:
-        """Whether :meth:`forward_joined` does what calling the block does: nothing watches the block or its norms
-        (hooks, other modules in their place), and the layer takes whole sequences."""
-        return (type(self) is DecoderBlock and type(self.attn_norm) is RMSNorm and type(self.norm) is RMSNorm
-                and not self.sequence_parallel and "forward" not in self.__dict__ and not _has_any_global_hook()
-                and not any(_hooked(m) for m in (self, self.attn_norm, self.norm)))
+        """Whether :meth:`forward_joined` does what calling the block does: nothing watches the block or its norms or stands
+        in their place, and the layer takes whole sequences."""
+        return (not self.sequence_parallel and _unwatched(self, DecoderBlock, _BLOCK_FORWARD)
+                and _unwatched(self.attn_norm, RMSNorm, _NORM_FORWARD) and _unwatched(self.norm, RMSNorm, _NORM_FORWARD))
 
     def forward_joined(self, x: torch.Tensor, delta: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
         """The block on ``x + delta``, its result left as (residual stream, expert output): every addition to the stream
@@ -120,6 +126,9 @@ class DecoderBlock(nn.Module):
         else:
             y = self.moe(h)
         return x + y
+
+
+_BLOCK_FORWARD = DecoderBlock.forward
 
 
 class TokenEmbedding(nn.Embedding):
@@ -258,9 +267,8 @@ class MoEDecoder(nn.Module):
 
     def _hidden(self, x: torch.Tensor) -> torch.Tensor:
         """``final_hidden(run_blocks(x))``, the last addition joined with the norm where nothing watches that."""
-        if not (type(self.norm) is RMSNorm and not _hooked(self.norm) and not _has_any_global_hook()
-                and all(getattr(type(self), f) is getattr(MoEDecoder, f) and f not in self.__dict__
-                        for f in ("run_blocks", "final_hidden"))):
+        if not (_unwatched(self.norm, RMSNorm, _NORM_FORWARD)
+                and all(getattr(type(self), f) is fn and f not in self.__dict__ for f, fn in _HIDDEN_STEPS)):
             return self.final_hidden(self.run_blocks(x))
         x, delta = self._run_blocks(x)
         return self.final_hidden(x) if delta is None else OF.add_rmsnorm(x, delta, self.norm.weight, self.norm.eps)[1]
@@ -321,6 +329,9 @@ class MoEDecoder(nn.Module):
         attn = sum(p.numel() for blk in self.blocks for p in blk.attn.parameters())
         return {"total": total, "embed": embed, "moe_router": router, "moe_experts": experts, "attention": attn,
                 "other": total - embed - router - experts - attn}
+
+
+_HIDDEN_STEPS = [(f, getattr(MoEDecoder, f)) for f in ("run_blocks", "final_hidden")]
 
 
 def finalize_sequence_parallel_grads(model: nn.Module, topology: ParallelTopology, optimizer=None) -> None:
