@@ -271,7 +271,9 @@ class MoEDecoder(nn.Module):
                 and all(getattr(type(self), f) is fn and f not in self.__dict__ for f, fn in _HIDDEN_STEPS)):
             return self.final_hidden(self.run_blocks(x))
         x, delta = self._run_blocks(x)
-        return self.final_hidden(x) if delta is None else OF.add_rmsnorm(x, delta, self.norm.weight, self.norm.eps)[1]
+        if delta is not None and OF.rmsnorm_supported(x, self.norm.weight):  # (the module rounds an fp32 weight first)
+            return OF.add_rmsnorm(x, delta, self.norm.weight, self.norm.eps)[1]
+        return self.final_hidden(x if delta is None else x + delta)
 
     def forward(self, ids_or_hidden: torch.Tensor) -> torch.Tensor:
         """Stage forward.  First stage takes token ids [B, S]; the last stage returns logits [B, S, V]."""

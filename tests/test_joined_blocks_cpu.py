@@ -73,3 +73,12 @@ def test_replaced_steps_are_taken(step, on_class, monkeypatch):
                         else lambda x: (seen.append(1), inner(model, x))[1])
     model(torch.randint(0, 64, (1, 8)))
     assert seen == [1]
+
+
+def test_a_final_norm_in_fp32_is_the_modules_own(monkeypatch):
+    """The module rounds its weight to the type of the rows; joined or not, the result has the same bits."""
+    model = _model()
+    model.norm.weight = torch.nn.Parameter(1 + 0.1 * torch.randn(32))
+    x, d = torch.randn(2, 8, 32).to(torch.bfloat16), torch.randn(2, 8, 32).to(torch.bfloat16)
+    monkeypatch.setattr(model, "_run_blocks", lambda _: (x, d))
+    assert torch.equal(model._hidden(x), model.norm(x + d))
