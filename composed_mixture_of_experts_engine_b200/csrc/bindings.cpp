@@ -245,6 +245,7 @@ void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tenso
 }
 // (x + delta, norm of it, rstd); without delta the first is x itself
 std::tuple<Tensor, Tensor, Tensor> add_rmsnorm(const Tensor& x, const OptTensor& delta, const Tensor& w, double eps) {
+  TORCH_CHECK(x.dim() > 0 && x.size(-1) > 0, "add_rmsnorm: rows must have columns");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t H = x.size(-1), rows = x.numel() / H;
   const auto fits = [&](const Tensor& t) {
