@@ -40,6 +40,7 @@ constexpr int MAX_STAGES = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB (full tile)
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int stages_of(int nb) { return STAGES * STAGE_BYTES / (A_STAGE_BYTES + nb * BK * 2); }  // 256: 4, 128: 6, 64: 8
 constexpr int CHUNK_BYTES = 64 * BK * 2;  // one 64 x 64 bf16 box (MN-major operands) = 8 KiB
 constexpr int PIECE_ROWS = 32;
 constexpr int GEMM_THREADS = 224;
@@ -82,9 +83,7 @@ struct KParams {
   uint32_t ready_target;
   int* status;
   unsigned long long timeout_ns;
-  int bn;               // accumulator columns of a tile (rows of B): 256, or 128 / 64 where that fills the SMs better
-  int stages, b_boxes;  // pipeline stages, TMA boxes of B in each (K-major)
-  int n_cols_per_tile;  // output columns covered by one tile (bn, or half of it with the SwiGLU forward)
+  int n_cols_per_tile;  // output columns covered by one tile (NB, or half of it with the SwiGLU forward)
   // fused dispatch: rows of A are pulled from peers by the extra warps
   const int* pull_row_slot;
   PeerTable pull_src;
@@ -259,15 +258,18 @@ __device__ __forceinline__ void swiglu_bwd_chunk(const uint32_t (&r)[32], uint4 
   }
 }
 
-template <int EPI>
+// NB: accumulator columns of a tile (rows of B), 256, or 128 / 64 where that fills the SMs better.  A constant: as a value
+// of the launch it costs full tiles 0.5 to 4 % (weight gradients of 300 tokens top-8, E 32 H 4096 F 2048, 470 / 487 us).
+template <int EPI, int NB>
 __global__ void __launch_bounds__(GEMM_THREADS_PULL, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmE, const KParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
-  const int b_bytes = p.bn * BK * 2;  // of a stage
-  uint8_t* sB = smem + p.stages * A_STAGE_BYTES;
+  constexpr int NSTAGES = stages_of(NB), B_BOXES = EPI == EPI_SWIGLU_FWD || NB == BN ? 2 : 1;  // boxes: K-major B
+  constexpr int b_bytes = NB * BK * 2;  // of a stage
+  uint8_t* sB = smem + NSTAGES * A_STAGE_BYTES;
   uint8_t* stg = smem + STAGES * STAGE_BYTES;  // 1024-byte aligned, as the swizzle pattern needs
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + STAGING_BYTES);
   uint64_t* full_bar = bars;                     // [MAX_STAGES]
@@ -284,7 +286,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int s = 0; s < p.stages; ++s) {
+    for (int s = 0; s < NSTAGES; ++s) {
       mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
@@ -356,7 +358,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else {
           tma_load_2d(a_dst, &tmA, &full_bar[stage], k, ti.a_mn0);
         }
-        if (++stage == p.stages) {
+        if (++stage == NSTAGES) {
           stage = 0;
           phase ^= 1u;
         }
@@ -408,12 +410,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               tma_load_2d(b_dst + j * CHUNK_BYTES, &tmB, &full_bar[stage], ti.b_n0 + 64 * j, k);
           } else if (p.b_once) {
             tma_load_2d_policy(b_dst, &tmB, &full_bar[stage], k, ti.b_n0, once);
-            if (p.b_boxes == 2) tma_load_2d_policy(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1, once);
+            if (B_BOXES == 2) tma_load_2d_policy(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1, once);
           } else {
             tma_load_2d(b_dst, &tmB, &full_bar[stage], k, ti.b_n0);
-            if (p.b_boxes == 2) tma_load_2d(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1);
+            if (B_BOXES == 2) tma_load_2d(b_dst + b_bytes / 2, &tmB, &full_bar[stage], k, ti.b_n1);
           }
-          if (++stage == p.stages) {
+          if (++stage == NSTAGES) {
             stage = 0;
             phase ^= 1u;
           }
@@ -424,7 +426,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(BM, p.bn, p.a_mn, p.b_mn);
+      const uint32_t idesc = make_idesc_bf16(BM, NB, p.a_mn, p.b_mn);
       const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(sA), p.a_mn ? CHUNK_BYTES : 16, 1024);
       const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sB), p.b_mn ? CHUNK_BYTES : 16, 1024);
       const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;  // per UMMA_K = 16 step, in descriptor units of 16 bytes
@@ -453,7 +455,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           for (int k = 0; k < BK / 16; ++k)
             umma_bf16_ss(d_tmem, ad + k * a_kstep, bd + k * b_kstep, idesc, (kb | k) != 0 ? 1u : 0u);
           umma_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
-          if (++stage == p.stages) {
+          if (++stage == NSTAGES) {
             stage = 0;
             phase ^= 1u;
           }
@@ -572,7 +574,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           float z[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) z[j] = 0.f;
-          for (int c = 0; c < p.bn / 32; ++c) store_row_chunk(Dg, p.ldd, p.d_fp32, 0, row, ti.n0 + c * 32, p.N, z);
+          for (int c = 0; c < NB / 32; ++c) store_row_chunk(Dg, p.ldd, p.d_fp32, 0, row, ti.n0 + c * 32, p.N, z);
         }
         continue;
       }
@@ -625,7 +627,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
 #pragma unroll 1
-        for (int u = 0; u < p.bn / unit_cols; ++u) {
+        for (int u = 0; u < NB / unit_cols; ++u) {
           const int col0 = ti.n0 + u * unit_cols;
           if (col0 >= p.N) break;  // uniform
           uint8_t* buf = stg + (stage_ctr & 1) * STAGING_BUF_BYTES;
@@ -723,14 +725,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         uint8_t* hrow = stg + row_in_tile * 64;
         bool any_bad = false;
 #pragma unroll 1
-        for (int c = 0; c < p.bn / 64; ++c) {
+        for (int c = 0; c < NB / 64; ++c) {
           const int col = ti.n0 + c * 32;
           if (col >= p.N) break;  // uniform
           uint32_t ph[16], pg[16], pu[16];
           if (ok) {
             uint32_t rg[32], ru[32];
             tmem_ld_32x32b_x32(t_acc + c * 32, rg);
-            tmem_ld_32x32b_x32(t_acc + p.bn / 2 + c * 32, ru);
+            tmem_ld_32x32b_x32(t_acc + NB / 2 + c * 32, ru);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -797,7 +799,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             float4 cur[8], nxt[8];
             prefetch_f32_chunk(drow, ti.n0, p.N, row_ok, cur);
 #pragma unroll 1
-            for (int c = 0; c < p.bn / 32; ++c) {
+            for (int c = 0; c < NB / 32; ++c) {
               const int col = ti.n0 + c * 32;
               if (col >= p.N) break;
               uint32_t r[32];
@@ -823,7 +825,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           } else {
             // direct bf16 / fp32 stores (and bf16 accumulate) from registers, one row per thread
 #pragma unroll 1
-            for (int c = 0; c < p.bn / 32; ++c) {
+            for (int c = 0; c < NB / 32; ++c) {
               if (ti.n0 + c * 32 >= p.N) break;  // uniform across the warp
               uint32_t r[32];
               tmem_ld_32x32b_x32(t_acc + c * 32, r);
@@ -839,11 +841,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else if (EPI == EPI_SWIGLU_FWD) {
           // accumulator columns [0,128) = gate, [128,256) = up for output columns n0 .. n0+127
 #pragma unroll 1
-          for (int c = 0; c < p.bn / 64; ++c) {
+          for (int c = 0; c < NB / 64; ++c) {
             if (ti.n0 + c * 32 >= p.N) break;
             uint32_t rg[32], ru[32];
             tmem_ld_32x32b_x32(t_acc + c * 32, rg);
-            tmem_ld_32x32b_x32(t_acc + p.bn / 2 + c * 32, ru);
+            tmem_ld_32x32b_x32(t_acc + NB / 2 + c * 32, ru);
             tmem_ld_wait();
             if (row_ok) {
               float g[32], u[32], h[32];
@@ -994,20 +996,20 @@ bool direct_epilogue_forced() {
   return forced;
 }
 
-template <int EPI>
+template <int EPI, int NB>
 cudaError_t launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                            const CUtensorMap& tmE, const KParams& kp, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<EPI, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
     configured = true;
   }
   if (kp.chained)
-    return launch_chained(gemm_kernel<EPI>, grid, GEMM_THREADS, SMEM_BYTES, stream, tmA, tmB, tmD, tmE, kp);
+    return launch_chained(gemm_kernel<EPI, NB>, grid, GEMM_THREADS, SMEM_BYTES, stream, tmA, tmB, tmD, tmE, kp);
   const int threads = kp.pull_row_slot != nullptr ? GEMM_THREADS_PULL : GEMM_THREADS;  // exchange with other ranks
   count_launch();
-  gemm_kernel<EPI><<<grid, threads, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmE, kp);
+  gemm_kernel<EPI, NB><<<grid, threads, SMEM_BYTES, stream>>>(tmA, tmB, tmD, tmE, kp);
   return cudaGetLastError();
 }
 
@@ -1138,9 +1140,6 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.b_once = a.b_once;
   kp.b_early = a.b_early && kp.chained;
   kp.timeout_ns = a.timeout_ns ? a.timeout_ns : kDefaultTimeoutNs;
-  kp.bn = bn;
-  kp.b_boxes = b_boxes;
-  kp.stages = STAGES * STAGE_BYTES / (A_STAGE_BYTES + bn * BK * 2);  // 4, 6 or 8
   kp.n_cols_per_tile = (a.epilogue == EPI_SWIGLU_FWD) ? bn / 2 : bn;
 
   int num_sms = a.num_sms;
@@ -1164,11 +1163,15 @@ cudaError_t launch_gemm(const GemmArgs& a, cudaStream_t stream) {
 
   switch (a.epilogue) {
     case EPI_STORE:
-      return launch_variant<EPI_STORE>(tmA, tmB, tmD, tmE, kp, grid, stream);
+      return bn == 256   ? launch_variant<EPI_STORE, 256>(tmA, tmB, tmD, tmE, kp, grid, stream)
+             : bn == 128 ? launch_variant<EPI_STORE, 128>(tmA, tmB, tmD, tmE, kp, grid, stream)
+                         : launch_variant<EPI_STORE, 64>(tmA, tmB, tmD, tmE, kp, grid, stream);
     case EPI_SWIGLU_FWD:
-      return launch_variant<EPI_SWIGLU_FWD>(tmA, tmB, tmD, tmE, kp, grid, stream);
+      return bn == 256   ? launch_variant<EPI_SWIGLU_FWD, 256>(tmA, tmB, tmD, tmE, kp, grid, stream)
+             : bn == 128 ? launch_variant<EPI_SWIGLU_FWD, 128>(tmA, tmB, tmD, tmE, kp, grid, stream)
+                         : launch_variant<EPI_SWIGLU_FWD, 64>(tmA, tmB, tmD, tmE, kp, grid, stream);
     case EPI_SWIGLU_BWD:
-      return launch_variant<EPI_SWIGLU_BWD>(tmA, tmB, tmD, tmE, kp, grid, stream);
+      return launch_variant<EPI_SWIGLU_BWD, 256>(tmA, tmB, tmD, tmE, kp, grid, stream);
     default:
       return cudaErrorInvalidValue;
   }

@@ -213,7 +213,9 @@ __device__ __forceinline__ void add_to_stats(const uint32_t (&v)[32], int live, 
       sum += __expf(__uint_as_float(v[j] << 16) - base) + __expf(__uint_as_float(v[j] & 0xffff0000u) - base);
 }
 
-template <int EPI, int GROUPS>
+// STATS: the softmax statistics of the rows are left too.  A kernel of its own: the registers and branches that they take
+// in the epilogue cost every other bf16 result 0.3 to 2 % (4096 x 4096 result rows of 256 terms 30.4 / 31.0 us).
+template <int EPI, int GROUPS, bool STATS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(t_threads(GROUPS), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
              const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmE, const K2Params p) {
@@ -552,7 +554,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               *reinterpret_cast<uint4*>(myrow + ((j ^ sw) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            if (p.row_stats != nullptr) {
+            if (STATS) {
               const int live = p.N - col0;
               if (live >= 64)
                 add_to_stats(v, 64, stat_max, stat_sum);
@@ -575,7 +577,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         }
         ++stage_ctr;
       }
-      if (EPI == EPI_STORE && p.row_stats != nullptr && row0 + row_in_tile < p.M)
+      if (STATS && row0 + row_in_tile < p.M)
         p.row_stats[static_cast<long long>(row0 + row_in_tile) * n_tiles + ti.n0 / T_BN] = make_float2(stat_max, stat_sum);
       if (have_acc) {
         // the leader's MMA warp may reuse this accumulator once all epilogue threads of the pair have read it
@@ -636,13 +638,13 @@ bool gemm_2cta_supported(const GemmArgs& a) {
   return aligned(a.D, a.ldd, es) && (gstride * es) % 16 == 0 && a.ldd >= a.N;
 }
 
-template <int EPI, int GROUPS>
+template <int EPI, int GROUPS, bool STATS = false>
 static cudaError_t launch_pairs(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                                 const CUtensorMap& tmE, const K2Params& kp, long long clusters, cudaStream_t stream) {
   static const cudaError_t configured =
-      cudaFuncSetAttribute(gemm2_kernel<EPI, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(GROUPS));
+      cudaFuncSetAttribute(gemm2_kernel<EPI, GROUPS, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(GROUPS));
   if (configured != cudaSuccess) return configured;
-  return launch_chained(gemm2_kernel<EPI, GROUPS>, static_cast<unsigned>(2 * clusters), t_threads(GROUPS),
+  return launch_chained(gemm2_kernel<EPI, GROUPS, STATS>, static_cast<unsigned>(2 * clusters), t_threads(GROUPS),
                         t_smem(GROUPS), stream, tmA, tmB, tmD, tmE, kp);
 }
 
@@ -717,7 +719,8 @@ cudaError_t launch_gemm_2cta(const GemmArgs& a, cudaStream_t stream) {
   const long long clusters = tiles < num_sms / 2 ? tiles : num_sms / 2;
   switch (a.epilogue) {
     case EPI_STORE:
-      return launch_pairs<EPI_STORE, 1>(tmA, tmB, tmD, tmE, kp, clusters, stream);
+      return a.row_stats != nullptr ? launch_pairs<EPI_STORE, 1, true>(tmA, tmB, tmD, tmE, kp, clusters, stream)
+                                    : launch_pairs<EPI_STORE, 1>(tmA, tmB, tmD, tmE, kp, clusters, stream);
     case EPI_SWIGLU_FWD:
       return launch_pairs<EPI_SWIGLU_FWD, 1>(tmA, tmB, tmD, tmE, kp, clusters, stream);
     default:
