@@ -269,21 +269,26 @@ std::tuple<Tensor, OptTensor> add_rmsnorm_grad(const Tensor& dy, const OptTensor
                                                const Tensor& rstd, bool need_dw, const OptTensor& main) {
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t H = x.size(-1), rows = x.numel() / H;
-  const Tensor g = cmoe::contiguous_aligned(dy), xs = cmoe::contiguous_aligned(x), r = cmoe::contiguous_aligned(rstd);
+  // (saved tensors may come back from hooks in another layout)
+  const Tensor g = cmoe::contiguous_aligned(dy), xs = cmoe::contiguous_aligned(x), r = cmoe::contiguous_aligned(rstd),
+               wt = cmoe::contiguous_aligned(w);
   OptTensor res;
   if (dsum.has_value()) res = cmoe::contiguous_aligned(*dsum);
-  TORCH_CHECK(g.scalar_type() == at::kBFloat16 && xs.scalar_type() == at::kBFloat16 && g.numel() == xs.numel() &&
-                  r.scalar_type() == at::kFloat && r.numel() == rows &&
-                  (!res.has_value() || (res->scalar_type() == at::kBFloat16 && res->numel() == xs.numel())) &&
-                  (!main.has_value() || (main->scalar_type() == at::kFloat && main->is_contiguous() && main->numel() == H)),
-              "add_rmsnorm_grad: bf16 rows of one shape, fp32 rstd and main gradient");
+  const auto bf16 = [&](const Tensor& t, int64_t n) {
+    return t.device() == x.device() && t.scalar_type() == at::kBFloat16 && t.numel() == n;
+  };
+  TORCH_CHECK(bf16(g, rows * H) && bf16(xs, rows * H) && bf16(wt, H) && r.device() == x.device() &&
+                  r.scalar_type() == at::kFloat && r.numel() == rows && (!res.has_value() || bf16(*res, rows * H)) &&
+                  (!main.has_value() || (main->device() == x.device() && main->scalar_type() == at::kFloat &&
+                                         main->is_contiguous() && main->numel() == H)),
+              "add_rmsnorm_grad: bf16 rows of one shape, weight [H], fp32 rstd and main gradient, all on one device");
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   Tensor dx = at::empty_like(xs), partial, dw;
   if (need_dw) {
     dw = main.has_value() ? *main : at::zeros({H}, r.options());
     partial = at::empty({cmoe::rmsnorm_bwd_partial_rows(rows, sms), H}, r.options());
   }
-  check_cuda(cmoe::launch_rmsnorm_bwd(g.data_ptr(), xs.data_ptr(), w.data_ptr(), r.data_ptr<float>(), dx.data_ptr(),
+  check_cuda(cmoe::launch_rmsnorm_bwd(g.data_ptr(), xs.data_ptr(), wt.data_ptr(), r.data_ptr<float>(), dx.data_ptr(),
                                       need_dw ? dw.data_ptr<float>() : nullptr, need_dw ? partial.data_ptr<float>() : nullptr,
                                       rows, static_cast<int>(H), sms, cur_stream(),
                                       res.has_value() ? res->data_ptr() : nullptr),
