@@ -285,7 +285,7 @@ std::tuple<Tensor, OptTensor> add_rmsnorm_grad(const Tensor& dy, const OptTensor
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   Tensor dx = at::empty_like(xs), partial, dw;
   if (need_dw) {
-    dw = main.has_value() ? *main : at::zeros({H}, r.options());
+    dw = main.has_value() ? *main : at::zeros(w.sizes(), r.options());
     partial = at::empty({cmoe::rmsnorm_bwd_partial_rows(rows, sms), H}, r.options());
   }
   check_cuda(cmoe::launch_rmsnorm_bwd(g.data_ptr(), xs.data_ptr(), wt.data_ptr(), r.data_ptr<float>(), dx.data_ptr(),

@@ -46,3 +46,19 @@ def test_a_moved_weight_gives_the_same_gradients(python, unpack, monkeypatch):
 def test_a_weight_that_the_kernel_cannot_read_is_refused(python, unpack, monkeypatch):
     with pytest.raises(RuntimeError, match="add_rmsnorm_grad"):
         _grads(monkeypatch, python, unpack)
+
+
+@pytest.mark.parametrize("python", [False, True])
+@pytest.mark.parametrize("shape", [(1, H), (H, 1)])
+def test_a_weight_of_more_dimensions_gets_a_gradient_of_its_shape(python, shape, monkeypatch):
+    from composed_mixture_of_experts_engine_b200.ops import functional as OF
+    from composed_mixture_of_experts_engine_b200.ops import kernels
+
+    if python:
+        monkeypatch.setattr(kernels, "traced_or_dual", lambda *t: True)
+    x = torch.randn(5, H, device="cuda").to(torch.bfloat16)
+    flat = torch.randn(H, device="cuda").to(torch.bfloat16).requires_grad_()
+    w = flat.detach().clone().view(shape).requires_grad_()
+    for weight in (flat, w):
+        OF.rmsnorm(x, weight).float().pow(2).sum().backward()
+    assert torch.equal(w.grad, flat.grad.view(shape))
