@@ -6,6 +6,7 @@
 // what only they serve: traces, which record them by name, and forward-mode tangents, which they refuse.
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
@@ -35,6 +36,23 @@ OptTensor main_grad(const Tensor& weight) {
   if (!pybind11::hasattr(o, "main_grad")) return std::nullopt;
   const pybind11::object m = o.attr("main_grad");
   return m.is_none() ? OptTensor() : OptTensor(m.cast<Tensor>());
+}
+
+// The same for a norm's weight, where its gradient may go straight into that buffer: one that the kernel can add to, while
+// nobody waits for the gradient itself - no hook on the weight or on the node that accumulates its gradient, no call that
+// asks for the gradients of given tensors.  Elsewhere autograd gets it, and the optimizer adds what is in `.grad` later.
+OptTensor norm_main_grad(const Tensor& weight) {
+  const OptTensor main = main_grad(weight);
+  if (!main.has_value() || !weight.is_leaf() || main->scalar_type() != at::kFloat || !main->is_contiguous() ||
+      main->numel() != weight.numel() || main->device() != weight.device())
+    return std::nullopt;
+  const auto* asked_for = torch::autograd::get_current_graph_task_exec_info();
+  if (asked_for != nullptr && !asked_for->empty()) return std::nullopt;
+  if (!torch::autograd::impl::hooks(weight).empty() || torch::autograd::impl::post_acc_grad_hooks(weight) != nullptr)
+    return std::nullopt;
+  const auto node = torch::autograd::impl::try_get_grad_accumulator(weight);
+  if (node != nullptr && !(node->pre_hooks().empty() && node->post_hooks().empty())) return std::nullopt;
+  return main;
 }
 
 // ---- y = x @ weight^T -------------------------------------------------------------------------------------------
@@ -99,7 +117,7 @@ struct AddRMSNormFn : Function<AddRMSNormFn> {
       // (counted over the tensors that the call was given)
       const bool need_dw = ctx->needs_input_grad(ctx->saved_data["delta"].toBool() ? 2 : 1);
       auto [d, w] = cmoe::add_rmsnorm_grad(grads[1], opt(grads[0]), saved[0], saved[1], saved[2], need_dw,
-                                           need_dw ? main_grad(saved[1]) : OptTensor());
+                                           need_dw ? norm_main_grad(saved[1]) : OptTensor());
       dx = d;
       dw = or_none(w);
     }
@@ -208,6 +226,7 @@ void register_autograd(pybind11::module_& m) {
     auto out = AddRMSNormFn::apply(x, delta, weight, eps);
     return std::make_tuple(out[0], out[1]);
   });
+  m.def("norm_main_grad", &norm_main_grad);
   m.def("rope_attention", [](const Tensor& qkv, const Tensor& cos_tab, const Tensor& sin_tab, int64_t nh) {
     const c10::cuda::CUDAGuard guard(qkv.device());
     TORCH_CHECK(qkv.dim() == 4 && qkv.is_contiguous() && qkv.size(2) == 3 * nh, "qkv must be contiguous [B, S, 3 nh, hd]");

@@ -43,7 +43,8 @@ def native_nodes(*tensors: torch.Tensor) -> bool:
 # ------------------------------------------------------------------------------------------ RMSNorm
 class _AddRMSNormFn(torch.autograd.Function):
     """(x + delta, norm of it) in one kernel, or (x, norm of it) without ``delta``; the backward adds the gradients of
-    both results in one kernel too, and the weight's gradient into its fp32 ``main_grad`` when it has one."""
+    both results in one kernel too, and the weight's gradient into its fp32 ``main_grad`` when it has one and nothing
+    (a hook, ``torch.autograd.grad``) waits for that gradient."""
 
     @staticmethod
     def forward(ctx, x, delta, weight, eps):
@@ -60,8 +61,9 @@ class _AddRMSNormFn(torch.autograd.Function):
         if dy is None:
             dx = ds
         else:
-            dx, dw = _ext.ext().add_rmsnorm_grad(dy, ds, s, weight, rstd, ctx.needs_input_grad[2],
-                                                 getattr(weight, "main_grad", None))
+            need_dw = ctx.needs_input_grad[2]
+            dx, dw = _ext.ext().add_rmsnorm_grad(dy, ds, s, weight, rstd, need_dw,
+                                                 _ext.ext().norm_main_grad(weight) if need_dw else None)
         return dx, dx if ctx.has_delta else None, dw, None
 
 
