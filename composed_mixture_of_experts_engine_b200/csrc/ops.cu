@@ -166,14 +166,12 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
     cp_async_wait<S - 1>();
     const float r = rstd[row];
     float xh[VEC][8], g[VEC][8];
-    uint4 res[VEC];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * RN_THREADS + threadIdx.x) * 8;
       if (c < H) {
         const uint4 nx = *slot(s, 0, i), nd = *slot(s, 1, i);
-        if (RES) res[i] = *slot(s, 2, i);
         const uint32_t xw[4] = {nx.x, nx.y, nx.z, nx.w};
         const uint32_t dw4[4] = {nd.x, nd.y, nd.z, nd.w};
 #pragma unroll
@@ -187,9 +185,17 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
           dwacc[i][2 * q] += dv.x * xh[i][2 * q];
           dwacc[i][2 * q + 1] += dv.y * xh[i][2 * q + 1];
         }
+        if (RES) {  // g becomes what of dx does not wait for the row's sum
+          float f[8];
+          unpack8(*slot(s, 2, i), f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) g[i][j] = fmaf(r, g[i][j], f[j]);
+        }
       }
     }
-    // the slot's values are in registers (the arithmetic above used them): refill it with the row S steps ahead
+    // Refill the slot with the row S steps ahead.  Its three pieces were read by this thread, which alone writes them, before
+    // this line: the copy's asm statement lets no read of memory past it, and a thread's own reads are ahead of a copy that
+    // it starts later.  (The sums above have used all of them, so no raw piece is held across the copy.)
     issue(row + static_cast<long long>(S) * gridDim.x, s);
     s = (s + 1 == S) ? 0 : s + 1;
     dot = block_sum<RN_THREADS>(dot, red) / H;
@@ -199,13 +205,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const __nv_bflo
       if (c < H) {
         float o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = r * (g[i][j] - xh[i][j] * dot);
-        if (RES) {
-          float f[8];
-          unpack8(res[i], f);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += f[j];
-        }
+        for (int j = 0; j < 8; ++j) o[j] = RES ? g[i][j] - xh[i][j] * (r * dot) : r * (g[i][j] - xh[i][j] * dot);
         store8(dx + row * H + c, o);
       }
     }
