@@ -928,6 +928,13 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* row_slot
 // 16384 tokens x 2048 columns, top-8 of 64: 174 / 122 us; 3333 x 4096, top-8 of 32: 68 / 56; 8192 x 4096, top-2 of 8:
 // 48 / 40; 16384 x 512, top-1 of 16: 15.3 / 13.2; 16384 x 4096, top-1 of 8: 52 / 52.  (Bulk copies through shared memory
 // instead of registers: 130, 67, 57, 22, 67.)
+// Few tokens leave mostly padding to write, up to 127 rows per expert, so it has warps of its own, kPadRows rows each, that
+// run beside the tokens'.  By the tokens' warps behind their rows it took longer than row by row: 64 x 2048, top-8 of 64
+// 11.8 us in a loop against 6.4, 1000 tokens 18.5 / 9.3; this way 9.8 and 13.3 there, and with a buffer that is not in L2,
+// as a new one, as long as row by row (12 and 15 us).  In a layer's forward and backward, whose first GEMM loads weights
+// meanwhile, 0.4 to 1 us less than behind the rows; 1, 4 and 16 rows per warp 700, 699 and 698 us for 64 tokens of E 64 H
+// 2048 F 1024, 805, 804 and 806 for 1000.
+constexpr int kPadRows = 4;
 __global__ void place_rows_kernel(const PlaceRowsArgs a, int pieces) {
   chain_wait();
   chain_trigger();
@@ -936,10 +943,22 @@ __global__ void place_rows_kernel(const PlaceRowsArgs a, int pieces) {
   const int lane = threadIdx.x & 31;
   const long long first = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const long long step = (gridDim.x * static_cast<long long>(blockDim.x)) >> 5;
-  const long long items = a.n_tokens * pieces;
+  const long long items = (a.n_tokens + (a.zero_padding ? a.n_local * (128LL / kPadRows) : 0)) * pieces;
   for (long long it = first; it < items; it += step) {
     const long long t = it / pieces;
     const int c0 = static_cast<int>(it - t * pieces) * 1024 + lane * 8;
+    if (t >= a.n_tokens) {  // rows of padding behind an expert's rows
+      const int i = static_cast<int>(t - a.n_tokens), e = i / (128 / kPadRows);
+      const long long row = static_cast<long long>(a.group_offsets[e]) + a.counts_kept[e] + i % (128 / kPadRows) * kPadRows;
+      const int end = a.group_offsets[e + 1];
+#pragma unroll
+      for (int r = 0; r < kPadRows; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (row + r < end && c0 + q * 256 < a.H)
+            *reinterpret_cast<uint4*>(out + (row + r) * a.ld_out + c0 + q * 256) = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
     const __nv_bfloat16* s = src + t * a.ld_src + c0;
     uint4 v[4];
 #pragma unroll
@@ -957,14 +976,6 @@ __global__ void place_rows_kernel(const PlaceRowsArgs a, int pieces) {
           if (c0 + q * 256 < a.H) *reinterpret_cast<uint4*>(o + q * 256) = v[q];
       }
     }
-  }
-  if (!a.zero_padding) return;
-  // an expert's rows are followed by up to 127 rows of padding
-  for (long long i = first; i < a.n_local * 128LL; i += step) {
-    const int e = static_cast<int>(i >> 7);
-    const long long row = static_cast<long long>(a.group_offsets[e]) + a.counts_kept[e] + (i & 127);
-    if (row < a.group_offsets[e + 1])
-      for (int c = lane * 8; c < a.H; c += 256) *reinterpret_cast<uint4*>(out + row * a.ld_out + c) = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -1344,7 +1355,7 @@ cudaError_t launch_place_rows(const PlaceRowsArgs& a, cudaStream_t stream) {
   if (a.H % 8 != 0 || a.H <= 0 || a.K <= 0) return cudaErrorInvalidValue;
   if (a.n_tokens <= 0) return cudaSuccess;
   const int pieces = (a.H + 1023) / 1024;
-  const long long warps = a.n_tokens * pieces + (a.zero_padding ? a.n_local * 64LL : 0);
+  const long long warps = (a.n_tokens + (a.zero_padding ? a.n_local * (128LL / kPadRows) : 0)) * pieces;
   // a warp per piece: CTAs that stride over the tokens drift apart (16384 x 2048, top-8: 130 / 120 us)
   launch_chained(place_rows_kernel, grid_for(warps, 8, 1 << 24), 256, 0, stream, a, pieces);
   return cudaGetLastError();
