@@ -1094,22 +1094,29 @@ __global__ void combine_bwd_w_kernel(const __nv_bfloat16* rows, const int* slot_
 // theirs.  Both / this, behind GEMMs: 16384 tokens x 2048, top-8 of 64 286 / 192 us (1.2 GB: 175 at the copy rate);
 // 3333 x 4096, top-8 of 32 120 / 93; 8192 x 4096, top-2 of 8 85 / 75; 4096 x 1024, top-2 of 16 21.5 / 17.4; 16384 x 512,
 // top-1 of 16 23.6 / 17.4.  Q: 16-byte pieces of dy per lane, H <= 256 Q; wider rows keep the two launches.
+// Few tokens are 2^split_log2 warps each, which share the token's picks: one warp's picks follow one another, each behind
+// its reads.  Rows in L2, two launches / one warp per token / this: 64 x 2048, top-8 of 64 9.4 / 11.6 / 6.7 us, 500 tokens
+// 11.6 / 13.4 / 8.3, 1000 18.3 / 15.2 / 11.1; 64 x 4096, top-8 of 32 11.4 / 14.6 / 7.6; 1000 x 1024, top-2 of 16 5.2 / 4.0
+// / 3.0.
 template <int Q>
 __global__ void __launch_bounds__(256) combine_grad_kernel(const PlaceRowsArgs a, const float* weight,
-                                                           const __nv_bfloat16* rows, long long ld_rows, float* dw) {
+                                                           const __nv_bfloat16* rows, long long ld_rows, float* dw,
+                                                           int split_log2) {
   chain_wait();
   chain_trigger();
   const __nv_bfloat16* dy = static_cast<const __nv_bfloat16*>(a.src);
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
   const int lane = threadIdx.x & 31;
   const long long warp = (blockIdx.x * 256LL + threadIdx.x) >> 5;
-  if (warp < a.n_tokens) {
+  const long long workers = a.n_tokens << split_log2;
+  if (warp < workers) {
+    const long long t = warp >> split_log2;
     uint4 d[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-      if (lane * 8 + q * 256 < a.H) d[q] = *reinterpret_cast<const uint4*>(dy + warp * a.ld_src + lane * 8 + q * 256);
-    for (int k = 0; k < a.K; ++k) {
-      const long long slot = warp * a.K + k;
+      if (lane * 8 + q * 256 < a.H) d[q] = *reinterpret_cast<const uint4*>(dy + t * a.ld_src + lane * 8 + q * 256);
+    for (int k = static_cast<int>(warp - (t << split_log2)); k < a.K; k += 1 << split_log2) {
+      const long long slot = t * a.K + k;
       const int row = a.slot_row[slot];
       float acc = 0.f;
       if (row >= 0) {
@@ -1145,7 +1152,7 @@ __global__ void __launch_bounds__(256) combine_grad_kernel(const PlaceRowsArgs a
     return;
   }
   // the warps behind the tokens': an expert's rows are followed by up to 127 rows of padding
-  const long long i = warp - a.n_tokens;
+  const long long i = warp - workers;
   if (i >= a.n_local * 128LL) return;
   const int e = static_cast<int>(i >> 7);
   const long long row = static_cast<long long>(a.group_offsets[e]) + a.counts_kept[e] + (i & 127);
@@ -1365,10 +1372,16 @@ bool combine_grad_supported(int H) { return H <= 4096; }
 cudaError_t launch_combine_grad(const PlaceRowsArgs& a, const float* weight, const void* rows, long long ld_rows, float* dw,
                                 cudaStream_t stream) {
   if (a.H % 8 != 0 || a.H <= 0 || !combine_grad_supported(a.H) || a.K <= 0 || a.n_tokens <= 0) return cudaErrorInvalidValue;
-  const unsigned grid = grid_for(a.n_tokens + a.n_local * 128LL, 8, INT_MAX);
+  // Shared as long as the chip is not full of warps with a row of dy each, which several would read for nothing: 6 MB of
+  // them, 40 KB per SM.  2000 x 2048, top-8 of 64: 25.6 us with one warp per token, 26.8 with two, 28.1 with four; 800 x
+  // 4096, top-8 of 32: 24.6, 25.7, 26.4; 2000 x 512, top-4 of 16: 5.4, 4.2, 4.1.
+  int split_log2 = 0;
+  while ((2 << split_log2) <= a.K && (a.n_tokens << split_log2) * a.H < (3LL << 20)) ++split_log2;
+  const unsigned grid = grid_for((a.n_tokens << split_log2) + a.n_local * 128LL, 8, INT_MAX);
   const int q = (a.H + 255) / 256;
   auto go = [&](auto kernel) {
-    return launch_chained(kernel, grid, 256, 0, stream, a, weight, reinterpret_cast<const __nv_bfloat16*>(rows), ld_rows, dw);
+    return launch_chained(kernel, grid, 256, 0, stream, a, weight, reinterpret_cast<const __nv_bfloat16*>(rows), ld_rows, dw,
+                          split_log2);
   };
   return q <= 2 ? go(combine_grad_kernel<2>) : q <= 4 ? go(combine_grad_kernel<4>)
        : q <= 8 ? go(combine_grad_kernel<8>) : go(combine_grad_kernel<16>);

@@ -13,6 +13,8 @@ pytestmark = pytest.mark.gpu
     (64, 40, 264, 48, 0),     # more picks than a warp has lanes
     (1000, 2, 2048, 8, 40),   # most slots dropped
     (33, 4, 4096, 8, 0),      # the widest row
+    (1535, 3, 2048, 8, 0),    # the last count of tokens whose picks two warps share, an odd number of picks
+    (1536, 3, 2048, 8, 0),    # the first that one warp takes
 ])
 @pytest.mark.parametrize("need_weight", [True, False])
 def test_combine_grad(N, K, H, E, capacity, need_weight):
