@@ -172,9 +172,10 @@ class _LMHeadLossFn(torch.autograd.Function):
         from ..ops import _ext, kernels
 
         if dh is not None:
-            # (a saved tensor may come back from a hook in another layout)
-            if (dh.is_contiguous() and dh.data_ptr() % 16 == 0 and dh.numel() % 8 == 0 and g.dtype == torch.float32
-                    and not kernels.needs_autograd(g) and not torch._C._are_functorch_transforms_active()):
+            # (a saved tensor may come back from a hook in another layout or type)
+            if (dh.dtype == torch.bfloat16 and dh.is_contiguous() and dh.data_ptr() % 16 == 0 and dh.numel() % 8 == 0
+                    and g.dtype == torch.float32 and not kernels.needs_autograd(g)
+                    and not torch._C._are_functorch_transforms_active()):
                 dh = _ext.ext().scaled_bf16(dh, g)
             else:
                 dh = dh * g.to(dh.dtype)
