@@ -68,12 +68,18 @@ class CausalSelfAttention(nn.Module):
 _NORM_FORWARD = RMSNorm.forward
 
 
-def _unwatched(m: nn.Module, cls: type, forward) -> bool:
-    """Whether calling ``m`` runs ``forward`` of ``cls`` and nothing else: no hooks, no other module, method, compiled call
-    or patched ``Module.__call__`` in its place."""
-    return (type(m) is cls and cls.forward is forward and "forward" not in m.__dict__ and m._compiled_call_impl is None
-            and cls.__call__ is nn.Module._wrapped_call_impl and not _has_any_global_hook()
-            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
+def _unwatched(*modules: Tuple[nn.Module, type, object]) -> bool:
+    """Whether calling each module runs the given ``forward`` of the given class and nothing else: no hooks, no other module,
+    method, compiled call or patched ``Module.__call__`` in its place."""
+    if _has_any_global_hook():
+        return False
+    for m, cls, forward in modules:
+        own = m.__dict__
+        if (type(m) is not cls or cls.forward is not forward or cls.__call__ is not nn.Module._wrapped_call_impl
+                or "forward" in own or own.get("_compiled_call_impl") is not None or own["_forward_hooks"]
+                or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"]):
+            return False
+    return True
 
 
 class DecoderBlock(nn.Module):
@@ -101,8 +107,8 @@ class DecoderBlock(nn.Module):
     def joins_residuals(self) -> bool:
         """Whether :meth:`forward_joined` does what calling the block does: nothing watches the block or its norms or stands
         in their place, and the layer takes whole sequences."""
-        return (not self.sequence_parallel and _unwatched(self, DecoderBlock, _BLOCK_FORWARD)
-                and _unwatched(self.attn_norm, RMSNorm, _NORM_FORWARD) and _unwatched(self.norm, RMSNorm, _NORM_FORWARD))
+        return not self.sequence_parallel and _unwatched(
+            (self, DecoderBlock, _BLOCK_FORWARD), (self.attn_norm, RMSNorm, _NORM_FORWARD), (self.norm, RMSNorm, _NORM_FORWARD))
 
     def forward_joined(self, x: torch.Tensor, delta: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
         """The block on ``x + delta``, its result left as (residual stream, expert output): every addition to the stream
@@ -268,7 +274,7 @@ class MoEDecoder(nn.Module):
 
     def _hidden(self, x: torch.Tensor) -> torch.Tensor:
         """``final_hidden(run_blocks(x))``, the last addition joined with the norm where nothing watches that."""
-        if not (_unwatched(self.norm, RMSNorm, _NORM_FORWARD)
+        if not (_unwatched((self.norm, RMSNorm, _NORM_FORWARD))
                 and all(getattr(type(self), f) is fn and f not in self.__dict__ for f, fn in _HIDDEN_STEPS)):
             return self.final_hidden(self.run_blocks(x))
         x, delta = self._run_blocks(x)
