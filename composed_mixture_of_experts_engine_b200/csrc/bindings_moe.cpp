@@ -121,16 +121,15 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   g.D = D.data_ptr();
   g.ldd = D.stride(0);
   g.status = status;
-  const cudaDeviceProp* prop = at::cuda::getCurrentDeviceProperties();
-  g.num_sms = prop->multiProcessorCount;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.epilogue = epilogue;
   g.b_early = 1;  // weights and row plan are older than the kernel before each of these launches
-  // Weights (here 3 N K values per expert, both matrices) that a tile of most experts reads, and that L2 would not hold for
-  // the backward pass or the next call: kept / first to leave, 20 and 50 rows per expert of E 16 to 32 H 1024, forward:
-  // 75 MB 43.6 and 46.1 / 45.1 and 46.5 us, 101 MB 47.6 and 50.7 / 48.4 and 50.2, 126 MB 56.6 and 59.1 / 52.5 and 54.1,
-  // 403 MB 99.6 and 103.5 / 93.4 and 98.8; forward and backward: 50 MB 130.2 / 132.1, 75 MB 153.0 / 154.9, 101 MB 169.8 /
-  // 170.2, 126 MB the same, 805 MB (E 64 H 2048 F 1024) 723 / 719.
-  g.b_once = !b_mn && g.rows_per_group <= 128 && 6 * pt.E * N * K >= prop->l2CacheSize / 4 * 3LL;
+  // One tile of most experts.  Whatever the size of the weights: in a model other layers' weights come before they are read
+  // again.  Decoders of layers with 50 MB of weights (E 16 H 1024 F 512), kept / first to leave: one layer 300 tokens 101.2 /
+  // 99.4 us, two 189.1 / 182.7, four 355.7 / 351.6, four at 16 tokens 309.5 / 296.2, training steps 0.1 % less.  Only a
+  // single layer of 50 to 75 MB, called again and again, would find them in L2 (forward 46.1 / 46.5, 43.6 / 45.1; forward and
+  // backward 134.7 / 136.5, 157.9 / 159.5); from 126 MB on it does not either (59.1 / 54.1 forward, 403 MB 103.5 / 98.8).
+  g.b_once = g.rows_per_group <= 128;
   if (short_tiles) {
     g.tile_rows = plan + pt.tile_rows;
     g.tile_n = streamed_tile(std::min(pt.E, pt.n_slots), N, epilogue, g.num_sms);

@@ -121,9 +121,8 @@ struct GemmArgs {
   // row plan): its loads may start before that kernel has ended
   int b_early = 0;
 
-  // grouped-M, K-major B: every part of B is read about once (few rows per expert) and B is more than L2 would hold for its
-  // next reader, so it is not kept there: what the small kernels around this launch need (tokens, tables, their own
-  // instructions) would be driven out for nothing
+  // grouped-M, K-major B: every part of B is read about once (few rows per expert), so it is not kept in L2: what the small
+  // kernels around this launch need (tokens, tables, their own instructions) would be driven out for nothing
   int b_once = 0;
 
   int* status = nullptr;  // device int, set to a StatusCode when a wait ran out
