@@ -351,10 +351,14 @@ class MoERouter(nn.Module):
                 w32, w, aux, z, idx32, idx = FusedRouterFunction.apply(tokens, self.gate_w, K, holder,
                                                                        self.profile_timing)
                 out: RouterOutput = holder["out"]
-            # plain attributes, set past the module's look at each for parameters and buffers
-            self.__dict__.update(
-                _last_logits=out.logits, last_aux_loss=aux, last_z_loss=z, last_idx32=idx32, last_w32=w32,
-                _pending=dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2))
+            left = dict(_last_logits=out.logits, last_aux_loss=aux, last_z_loss=z, last_idx32=idx32, last_w32=w32,
+                        _pending=dict(counts=out.counts, N=N, fused=True, events=out.events, stats=out.stats, elem=2))
+            if type(self) is MoERouter:
+                # plain attributes of this class, set past the module's look at each for parameters and buffers
+                self.__dict__.update(left)
+            else:
+                for name, value in left.items():
+                    setattr(self, name, value)
             return idx, w, out.counts64
         # PyTorch path (bias, CPU, fp32 tokens, shapes the kernel does not cover): fp64 math under autograd
         logits64 = tokens.to(torch.float64) @ self.gate_w.to(torch.float64)
