@@ -9,7 +9,7 @@ line under ``ncu -k regex:<kernel> -c 1`` captures one launch of the case.
 
 Cases: adamw, rmsnorm, router / router_bwd (config-2 shape: T16384 d4096 E64 top2), gemm_dense, dense_shapes,
 grouped_fwd1, grouped_fwd1_pull (fused dispatch through a local one-entry peer table), grouped_fwd2,
-grouped_dgrad, grouped_wgrad, gather, combine.
+grouped_dgrad, grouped_wgrad, gather, place, combine, combine_bwd, add_rmsnorm, cross_entropy.
 """
 
 from __future__ import annotations
@@ -113,6 +113,26 @@ def main():
         nb = rows * H * 2
         out.update(fwd_ms=f, fwd_gbs=2 * nb / f / 1e6, fwd_frac=2 * nb / f / 1e6 / hbm, bwd_ms=b,
                    bwd_gbs=3 * nb / b / 1e6, bwd_frac=3 * nb / b / 1e6 / hbm)
+    elif args.case == "add_rmsnorm":
+        # a residual addition and the norm behind it; the backward adds the stream's gradient and sums the weight's
+        rows, H = 32768 // shrink, 2048
+        x, d, ds, dy = (torch.randn(rows, H, device=dev, dtype=bf) for _ in range(4))
+        w, dw = torch.ones(H, device=dev, dtype=bf), torch.zeros(H, device=dev)
+        s, _, rstd = ext.add_rmsnorm(x, d, w, 1e-5)
+        f = time_launches(lambda: ext.add_rmsnorm(x, d, w, 1e-5), args.iters)
+        b = time_launches(lambda: ext.add_rmsnorm_grad(dy, ds, s, w, rstd, True, dw), args.iters)
+        nb = rows * H * 2
+        out.update(fwd_ms=f, fwd_gbs=4 * nb / f / 1e6, fwd_frac=4 * nb / f / 1e6 / hbm, bwd_ms=b,
+                   bwd_gbs=4 * nb / b / 1e6, bwd_frac=4 * nb / b / 1e6 / hbm)
+    elif args.case == "cross_entropy":
+        # the LM head's loss and gradient from the statistics that the logits' GEMM leaves, one chunk of rows
+        rows, V = 4096 // shrink, 50304
+        x, w = torch.randn(rows, 256, device=dev, dtype=bf), (torch.randn(V, 256, device=dev) * 0.02).to(bf)
+        targets, loss = torch.randint(0, V, (rows,), device=dev), torch.zeros(1, device=dev)
+        logits, stats = ext.linear_stats(x, w, kernels.status_word(torch.device(dev, 0)))
+        ms = time_launches(lambda: ext.cross_entropy(logits, targets, loss, 1.0, stats), args.iters)
+        nbytes = rows * (V * 4 + stats.shape[1] * 8)
+        out.update(ms=ms, gbs=nbytes / ms / 1e6, frac_of_hbm=nbytes / ms / 1e6 / hbm)
     elif args.case == "router":
         N, H, E, K = 16384 // (2 if args.small else 1), args.router_hidden, 64, args.topk
         x = torch.randn(N, H, device=dev, dtype=bf)
@@ -178,7 +198,7 @@ def main():
                                  "of_cublas": round(b / a, 3), "frac_of_peak": round(fl / a / 1e9 / tflops_peak, 3)})
             del x, w, dy, y, dx, dw, dw16
         out.update(cases=rows_out)
-    elif args.case.startswith("grouped_") or args.case in ("gather", "combine"):
+    elif args.case.startswith("grouped_") or args.case in ("gather", "place", "combine", "combine_bwd"):
         E, H, F = args.experts, args.hidden, args.ffn
         R = args.rows // shrink
         tg, nt, go, tiles = uniform_plan(R, E)
@@ -243,13 +263,20 @@ def main():
             src = torch.randn(N, H, device=dev, dtype=bf)
             rows = torch.randn(plan.cap_rows, H, device=dev, dtype=bf)
             wts = torch.rand(N, K, device=dev)
+            nbytes = (N * K + N) * H * 2
             if args.case == "gather":
                 fn = lambda: kernels.gather_rows(src, plan, out=rows)
+            elif args.case == "place":
+                fn = lambda: ext.place_rows(src, plan.slot_row, K, plan.group_offsets, plan.counts_kept, rows, True)
+            elif args.case == "combine_bwd":
+                out_rows, dw = torch.empty_like(rows), torch.empty_like(wts)
+                fn = lambda: ext.combine_grad(src, plan.slot_row, K, plan.group_offsets, plan.counts_kept, wts, rows,
+                                              out_rows, dw)
+                nbytes += N * K * H * 2
             else:
                 yv = torch.empty(N, H, device=dev, dtype=bf)
                 fn = lambda: kernels.combine_rows(rows, plan, wts, out=yv)
             ms = time_launches(fn, args.iters)
-            nbytes = (N * K + N) * H * 2
             out.update(ms=ms, gbs=nbytes / ms / 1e6, frac_of_hbm=nbytes / ms / 1e6 / hbm)
             print(json.dumps(out))
             return

@@ -77,9 +77,10 @@ Shapes check_shapes(const Tensor& x, const Tensor& idx32, const Tensor& w13, con
 
 // Rows of B in a tile where a layer of few rows streams its weights: the width with which nearly whole rounds of tiles
 // fill the SMs, for what counts is that all of them load all the time.  64 rows only where wider tiles leave the chip
-// half empty: a k-block of 8 KiB takes its threads as long to issue as one of 16.  64 tokens top-8, E 64 H 2048 F 1024
-// (3.46 rounds of 256, 6.92 of 128): 171.7 -> 158.9 us; 64 rows against 256 where both fill the chip: 5 tokens of the same
-// layer 111.6 / 102.9, 8 tokens top-2, E 8 H 4096 F 4096 175.9 / 157.6.
+// half empty: a k-block of 8 KiB takes its threads as long to issue as one of 16.  GPU time of the layer with tiles of 256 /
+// 128 / 64 rows in both GEMMs: 64 tokens top-8, E 64 H 2048 F 1024 (3.46 rounds of 256, 6.92 of 128) 170.2 / 162.3 / 196.5
+// us, 5 tokens 99.4 / 91.2 / 107.3; 8 tokens top-2, E 8 H 4096 F 4096 154.7 / 160.9 / 188.7; 250 tokens top-2, E 16 H 1024 F
+// 512 44.3 / 40.3 / 44.2.
 int streamed_tile(int64_t m_tiles, int64_t N, int epilogue, int sms) {
   int best = 256;
   double best_fill = 0.0;

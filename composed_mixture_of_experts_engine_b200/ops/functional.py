@@ -325,6 +325,8 @@ def rope_causal_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tenso
     rotary embedding on q and k.  On the device path ``qkv`` is consumed (rotated in place)."""
     B, S, heads, hd = qkv.shape
     if on_device_path(qkv) and hd % 16 == 0 and qkv.is_contiguous():
+        # (grouped heads keep the Python function: which library kernel takes them, and whether k and v are repeated for it,
+        # is found out by trying, ops/attention.py)
         if nh == nkv and native_nodes(qkv) and not _attn_sm100.enabled():
             return _ext.ext().rope_attention(qkv, cos, sin, nh)
         return _RopeAttentionFn.apply(qkv, cos, sin, nh, nkv)

@@ -7,7 +7,8 @@ moments in the optimizer) is one kernel launch per parameter group:
 
 * parameters are re-pointed into one flat bf16 buffer per group, gradients into one flat buffer
   (fp32 ``main_grad``: the kernels add the weight gradients of experts, projections, norms, LM head and token embedding
-  into it directly; what autograd leaves in ``p.grad`` - router gates - is added at step time);
+  into it directly and leave ``p.grad`` empty; what autograd leaves in ``p.grad`` - router gates, all weights under
+  activation recomputation, norms whose gradient a hook watches - is added at step time);
 * the global gradient norm is a device scalar (sum-of-squares kernel), so clipping needs no host round trip;
 * with data parallelism the flat gradient is reduce-scattered, the update runs on this rank's shard only, and
   the updated bf16 parameters are all-gathered (ZeRO-style sharding of master weights and moments).  Expert
