@@ -99,7 +99,7 @@ int streamed_tile(int64_t m_tiles, int64_t N, int epilogue, int sms) {
 // a grouped-by-rows launch over the tiles of `plan`: D[rows, N] = A[rows, K] * B (one [b_rows, b_cols] block per expert)
 cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_rows, bool b_mn, const Tensor& D, int64_t N,
                             int64_t K, const PlanTables& pt, int* plan, int* status,
-                            int epilogue = cmoe::EPI_STORE, bool short_tiles = false) {
+                            int epilogue = cmoe::EPI_STORE, bool training = true, bool short_tiles = false) {
   cmoe::GemmArgs g;
   g.A = A.data_ptr();
   g.a_rows = A.size(0);
@@ -136,7 +136,7 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
     g.tile_n = streamed_tile(std::min(pt.E, pt.n_slots), N, epilogue, g.num_sms);
     return g;
   }
-  // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs 0.85 of the time of a tile (it loads
+  // Pairs of SMs on pairs of tiles, or single SMs on single tiles?  A pair needs about 0.85 of the time of a tile (it loads
   // a third less per FLOP) but wastes one of its SMs where an expert has an odd number of tiles, and rounds are counted
   // in whole tiles.  So the rounds of both are estimated, every expert ending in half a tile or pair on average.
   // Forward and backward of a layer, E 64 H 2048 F 1024, GEMM times on single SMs / pairs: 2048 rows per expert 2741 /
@@ -144,10 +144,14 @@ cmoe::GemmArgs grouped_rows(const Tensor& A, const Tensor& B, int64_t b_group_ro
   // rounds of tiles face 31 of pairs, 428 / 471 where 4 face 5.
   const double tiles = pt.n_slots / 128.0 + 0.5 * pt.E, pairs = pt.n_slots / 256.0 + 0.5 * pt.E;
   const int64_t cols = (N + (epilogue == cmoe::EPI_SWIGLU_FWD ? 127 : 255)) / (epilogue == cmoe::EPI_SWIGLU_FWD ? 128 : 256);
-  // Near a tie too: with 0.9 in the place of 0.85, which takes single SMs there, 1000 tokens top-8 of 64 such experts take
-  // 237 us instead of 226 forward and 830 instead of 813 in training, 800 tokens top-8 of E 32 H 4096 F 2048 with equal
-  // loads 435 instead of 388 and 1564 instead of 1494.
-  if (0.85 * std::ceil(pairs * cols / (g.num_sms / 2)) < std::ceil(tiles * cols / g.num_sms)) {
+  // Near a tie it depends on the experts' loads, which the host does not know: with equal ones pairs win, where a few experts
+  // have most rows single SMs, which compute fewer rows of padding, and more so in long runs at the power limit (these, seconds
+  // of calls).  Pairs / single SMs in training, whose losses even the loads out: 800 tokens top-8, E 32 H 4096 F 2048 1781 /
+  // 1810 us with unequal loads and 1656 / 1744 with equal ones, 1500 tokens 2435 / 2484 and 2407 / 2480, 512 tokens 1550 /
+  // 1522 and 1500 / 1560, 1300 tokens E 64 H 2048 F 1024 935 / 938 and 915 / 955.  In inference: 7 rounds of pairs against 6
+  // of tiles, 512 tokens 475 / 437 and 441 / 453, 1000 tokens 263 / 260 and 249 / 245, two decoder layers of that kind 868 /
+  // 847; 8 against 7, 1300 tokens 288 / 282 and 267 / 297; 9 against 8, 800 tokens 554 / 545 and 473 / 527.
+  if ((training ? 0.85 : 0.87) * std::ceil(pairs * cols / (g.num_sms / 2)) < std::ceil(tiles * cols / g.num_sms)) {
     g.pair_tile = plan + pt.pair_tile;
     g.num_pairs = plan + pt.num_pairs;
   }
@@ -253,7 +257,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   OptTensor gu;
   {
     cmoe::GemmArgs g = grouped_rows(xp, w13, 2 * s.F, false, hact, s.F, s.H, pt, plan, status_ptr(status), cmoe::EPI_SWIGLU_FWD,
-                                     short_tiles);
+                                     keep, short_tiles);
     g.split_n = static_cast<int>(s.F);
     if (keep) {
       gu = at::empty({pt.cap_rows, 2 * s.F}, bf);
@@ -264,7 +268,7 @@ Forward moe_local_forward(const Tensor& x, const Tensor& gate_w32, const Tensor&
   }
   Tensor yp = at::empty({pt.cap_rows, s.H}, bf);
   cmoe::launch_gemm_any(grouped_rows(hact, w2, s.H, false, yp, s.H, s.F, pt, plan, status_ptr(status),
-                                      cmoe::EPI_STORE, short_tiles),
+                                      cmoe::EPI_STORE, keep, short_tiles),
                          stream);
   Tensor y = at::empty({s.N, s.H}, bf);
   check(cmoe::launch_combine_rows(yp.data_ptr(), plan, gate_w32.data_ptr<float>(), y.data_ptr(), s.N,
