@@ -322,19 +322,34 @@ OptTensor expert_wgrad(const Tensor& a, const Tensor& b, const Tensor& weight, c
   return out;
 }
 
-// (dx, d_gate, dw13, dw2)
-Backward moe_local_backward(const Tensor& dy, const Tensor& plan_t, const Tensor& xp, const Tensor& hact, const Tensor& gu,
-                            const Tensor& yp, const Tensor& gate_w32, const Tensor& w13, const Tensor& w2, bool need_dx,
-                            bool need_gate, const OptTensor& main13, const OptTensor& main2, const OptTensor& status) {
+// (dx, d_gate, dw13, dw2).  Everything but dy is a saved tensor, which a hook may hand back in another layout: brought into
+// the kernels' one, or refused.
+Backward moe_local_backward(const Tensor& dy, const Tensor& saved_plan, const Tensor& saved_xp, const Tensor& saved_hact,
+                            const Tensor& saved_gu, const Tensor& saved_yp, const Tensor& saved_gate, const Tensor& saved_w13,
+                            const Tensor& saved_w2, bool need_dx, bool need_gate, const OptTensor& main13,
+                            const OptTensor& main2, const OptTensor& status) {
   const c10::cuda::CUDAGuard guard(dy.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+  const Tensor plan_t = cmoe::contiguous_aligned(saved_plan), xp = cmoe::contiguous_aligned(saved_xp),
+               hact = cmoe::contiguous_aligned(saved_hact), gu = cmoe::contiguous_aligned(saved_gu),
+               yp = cmoe::contiguous_aligned(saved_yp), gate_w32 = cmoe::contiguous_aligned(saved_gate),
+               w13 = cmoe::contiguous_aligned(saved_w13), w2 = cmoe::contiguous_aligned(saved_w2);
+  TORCH_CHECK(gate_w32.dim() == 2 && xp.dim() == 2 && hact.dim() == 2 && w13.dim() == 3, "bad saved tensors");
   const int64_t N = gate_w32.size(0), K = gate_w32.size(1), H = xp.size(1), E = w13.size(0), F = hact.size(1);
   TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && dy.size(0) == N && dy.size(1) == H, "bad dy");
   check_rows(dy, "dy");
   check_rows(xp, "saved rows");
   check_rows(yp, "saved expert rows");
   const PlanTables pt(N * K, E);
-  TORCH_CHECK(plan_t.numel() == pt.words && xp.size(0) == pt.cap_rows, "the row plan belongs to another layer call");
+  const auto is = [&](const Tensor& t, at::ScalarType type, at::IntArrayRef sizes) {
+    return t.device() == dy.device() && t.scalar_type() == type && t.sizes() == sizes;
+  };
+  TORCH_CHECK(is(plan_t, at::kInt, {pt.words}) && is(xp, at::kBFloat16, {pt.cap_rows, H}),
+              "the row plan belongs to another layer call");
+  TORCH_CHECK(is(hact, at::kBFloat16, {pt.cap_rows, F}) && is(gu, at::kBFloat16, {pt.cap_rows, 2 * F}) &&
+                  is(yp, at::kBFloat16, {pt.cap_rows, H}) && is(gate_w32, at::kFloat, {N, K}) &&
+                  is(w13, at::kBFloat16, {E, 2 * F, H}) && is(w2, at::kBFloat16, {E, H, F}),
+              "the saved tensors of the expert layer are not what its forward left");
   int* plan = plan_t.data_ptr<int>();
   int* st = status_ptr(status);
   Backward out;
